@@ -11,9 +11,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
-
 #include <mutex>
+#include <type_traits>
 
 #include "../../include/mongoose_kernels.h"
 #include "mg_common.cuh"
@@ -32,64 +33,165 @@ static_assert(sizeof(ActBlock) == 40, "activation block is 40 bytes");
 // ---------------- fp32-activation matvecs on raw blocks ----------------
 // Raw GGUF blocks (34 / 18 bytes) are only 2-byte aligned, so a lane cannot fetch its block with a
 // vector load.  Instead a warp takes a CHUNK of 32 consecutive blocks of a row - a contiguous byte
-// range - and copies the aligned 4-byte words that cover it from global to shared memory, lane by
-// lane (coalesced, every weight byte read once); each lane then pulls the words of ITS block out of
-// shared memory, re-aligns them with a funnel shift by 16 or 32 bits, and multiplies them with the
-// activation slice staged once per CTA.  One warp walks rows warp, warp + nwarps, ...; the 32 block
-// sums meet in a shuffle reduction.
-constexpr int kRawWarps = 8;
-template <int FMT>
-__global__ void __launch_bounds__(kRawWarps * 32) raw_block_matvec_kernel(const float* __restrict__ act,
-                                                                         const uint8_t* __restrict__ w, float* out, int N,
-                                                                         int K) {
-    constexpr int BB = FMT == FMT_Q8_0 ? 34 : 18;           // bytes per block
-    constexpr int QW = FMT == FMT_Q8_0 ? 8 : 4;             // 4-byte words of quants per block
-    constexpr int CW = (32 * BB + 3) / 4 + 1;               // words that cover a chunk, whatever its alignment
-    extern __shared__ __align__(16) float raw_xs[];         // K floats, then kRawWarps * CW words
-    uint32_t* stage = reinterpret_cast<uint32_t*>(raw_xs + K) + (threadIdx.x >> 5) * CW;
-    const int lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < K; i += blockDim.x) raw_xs[i] = act[i];
-    __syncthreads();
-    const int nb = K / 32;
-    const int nwarps = gridDim.x * kRawWarps;
-    for (int row = blockIdx.x * kRawWarps + (threadIdx.x >> 5); row < N; row += nwarps) {
-        const size_t row0 = (size_t)row * nb * BB;           // byte offset of the row (always even)
-        float acc = 0.f;
-        for (int b0 = 0; b0 < nb; b0 += 32) {
-            const int nblk = min(32, nb - b0);
-            const size_t c0 = row0 + (size_t)b0 * BB, c1 = c0 + (size_t)nblk * BB;
-            const size_t a0 = ((size_t)(w + c0)) & ~(size_t)3;                       // first aligned word (address)
-            const int nw = (int)((((size_t)(w + c1)) + 3 - a0) >> 2);
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(a0);
-            for (int i = lane; i < nw; i += 32) stage[i] = __ldcs(src + i);
-            __syncwarp();
-            if (lane < nblk) {
-                const int off = (int)((size_t)(w + c0) - a0) + lane * BB;               // this block inside the staged words
-                const uint32_t* q = stage + (off >> 2);
-                const int sh = (off & 2) ? 32 : 16;                                     // quants start 2 bytes after the scale
-                const uint32_t w0 = q[0];
-                const float d = half_bits_to_float((unsigned short)((off & 2) ? (w0 >> 16) : (w0 & 0xffffu)));
-                uint32_t qw[QW];
-#pragma unroll
-                for (int i = 0; i < QW; i++) qw[i] = __funnelshift_rc(q[i], q[i + 1], sh);
-                const float4* x = reinterpret_cast<const float4*>(raw_xs + (size_t)(b0 + lane) * 32);
-                float s;
-                if (FMT == FMT_Q8_0)
-                    s = Chunk<FMT_Q8_0>::dot(make_uint4(qw[0], qw[1], qw[2], qw[3]), x) +
-                        Chunk<FMT_Q8_0>::dot(make_uint4(qw[4], qw[5], qw[6], qw[7]), x + 4);
-                else
-                    s = Chunk<FMT_Q4_0>::dot(make_uint4(qw[0], qw[1], qw[2], qw[3]), x);
-                acc = fmaf(d, s, acc);
-            }
-            __syncwarp();
-        }
-        acc = warp_sum(acc);
-        if (lane == 0) out[row] = acc;
+// range - and copies the aligned 16-byte pieces that cover it into a ring of its own in shared memory
+// (cp.async, kRawStages deep, running on over chunks and rows, so that a row's end does not drain it);
+// each lane then pulls the words of ITS block out of shared memory, re-aligns them with a funnel shift
+// by 16 or 32 bits, and multiplies them with the activation slice staged once per CTA.  A warp takes R
+// rows at a time, which share the activation reads; where rows are fewer than warps, `ks` warps share
+// a row and their sums meet in shared memory, in order.
+//
+// The bound is the instruction rate and, for wide inputs, HBM.  The activation slices of a warp's lanes
+// are 36 floats apart: 32 floats apart, all lanes of an access fell on the same four banks and the reads
+// alone took 60 of 104 us of a 3584 x 18944 Q4_0 product.
+constexpr int kRawStages = 3;
+constexpr int kXStride = 36;                                // floats between the activation slices of two blocks
+__host__ __device__ constexpr int block_bytes(int fmt) { return fmt == FMT_Q8_0 ? 34 : 18; }
+__host__ __device__ constexpr int chunk_ring(int fmt) { return 32 * block_bytes(fmt) + 16; }        // bytes: whole pieces cover a chunk, whatever its alignment
+
+// Copies bytes [src, src + n) so that they start at dst + (address of src mod V); nothing behind them is read.
+template <int V>
+__device__ __forceinline__ void copy_chunk(uint8_t* dst, const uint8_t* src, int n, int lane) {
+    const int lead = (int)(reinterpret_cast<uintptr_t>(src) & (V - 1));
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+    for (int i = lane * V; i < lead + n; i += 32 * V) {
+        const int left = min(V, lead + n - i);
+        if (V == 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + i), "l"(src - lead + i), "r"(left) : "memory");
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(to + i), "l"(src - lead + i), "r"(left) : "memory");
     }
 }
-template <int FMT>
-inline size_t raw_matvec_smem(int K) {
-    return (size_t)K * 4 + (size_t)kRawWarps * ((32 * (FMT == FMT_Q8_0 ? 34 : 18) + 3) / 4 + 1) * 4;
+
+// V: bytes per copy; 16 where the matrix starts on a 16-byte boundary (so no piece starts before it), else 4.
+// XS: the activations fit shared memory.  ks: warps per row.
+template <int FMT, int R, int V, bool XS>
+__global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __restrict__ act, const uint8_t* __restrict__ w, float* out, int N,
+                                                               int K, int ks) {
+    constexpr int BB = block_bytes(FMT), QW = FMT == FMT_Q8_0 ? 8 : 4;       // bytes, 4-byte words of quants per block
+    constexpr int ring = chunk_ring(FMT);
+    extern __shared__ __align__(16) float raw_xs[];         // kXStride floats per block, 512 R partial sums, then the rings
+    const int nb = K / 32, chunks = (nb + 31) / 32;
+    float* sums = raw_xs + (XS ? (size_t)nb * kXStride : 0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    uint8_t* stage = reinterpret_cast<uint8_t*>(sums + 16 * R) + (size_t)warp * kRawStages * R * ring;
+    const int slots = warps / ks, slot = warp / ks, part = warp - slot * ks;
+    const int tiles = (N + R - 1) / R;
+    const int mine = blockIdx.x < tiles ? (tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;        // tiles of this CTA
+    const int rounds = (mine + slots - 1) / slots;
+    pdl_launch_dependents();
+    pdl_wait();
+
+    int iround = 0, ichunk = part;                          // the next chunk to be copied
+    auto issue = [&](int s) {
+        const int k = iround * slots + slot;
+        if (k < mine) {
+            const int row0 = (blockIdx.x + k * gridDim.x) * R, n = min(32, nb - ichunk * 32) * BB;
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                if (row0 + r < N) copy_chunk<V>(stage + (s * R + r) * ring, w + ((size_t)(row0 + r) * nb + ichunk * 32) * BB, n, lane);
+            ichunk += ks;
+            if (ichunk >= chunks) { ichunk = part; iround++; }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int s = 0; s < kRawStages - 1; s++) issue(s);
+
+    if (XS) {
+        if ((reinterpret_cast<uintptr_t>(act) & 15) == 0) {
+#pragma unroll 4
+            for (int i = threadIdx.x; i < nb * 8; i += blockDim.x)
+                *reinterpret_cast<float4*>(raw_xs + (i >> 3) * kXStride + (i & 7) * 4) = reinterpret_cast<const float4*>(act)[i];
+        } else {
+            for (int i = threadIdx.x; i < K; i += blockDim.x) raw_xs[(i >> 5) * kXStride + (i & 31)] = act[i];
+        }
+        __syncthreads();
+    }
+
+    int s = 0;
+    for (int round = 0; round < rounds; round++) {
+        const int k = round * slots + slot;
+        const bool has = k < mine;
+        const int row0 = (blockIdx.x + k * gridDim.x) * R;
+        float acc[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[r] = 0.f;
+        for (int c = part; has && c < chunks; c += ks) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kRawStages - 2) : "memory");
+            __syncwarp();
+            const int b = c * 32 + lane;
+            if (b < nb) {
+                uint32_t q[R][QW];
+                float d[R], sum[R];
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const int row = min(row0 + r, N - 1);
+                    const int off = (int)(reinterpret_cast<uintptr_t>(w + ((size_t)row * nb + c * 32) * BB) & (V - 1)) + lane * BB;
+                    const uint32_t* p = reinterpret_cast<const uint32_t*>(stage + (s * R + r) * ring) + (off >> 2);
+                    const int sh = (off & 2) ? 32 : 16;                 // quants start 2 bytes after the scale
+                    uint32_t lo = p[0];
+                    d[r] = half_bits_to_float((unsigned short)((off & 2) ? (lo >> 16) : (lo & 0xffffu)));
+#pragma unroll
+                    for (int i = 0; i < QW; i++) {
+                        // the word behind a block that ends on a word's end is another's, or was never written: it is shifted out
+                        const uint32_t hi = p[i + 1];
+                        q[r][i] = __funnelshift_rc(lo, hi, sh);
+                        lo = hi;
+                    }
+                    sum[r] = 0.f;
+                }
+                const float* xb = XS ? raw_xs + (size_t)b * kXStride : act + (size_t)b * 32;
+                auto x4 = [&](int i) {
+                    return XS ? *reinterpret_cast<const float4*>(xb + 4 * i) : make_float4(xb[4 * i], xb[4 * i + 1], xb[4 * i + 2], xb[4 * i + 3]);
+                };
+                if (FMT == FMT_Q8_0) {
+#pragma unroll
+                    for (int i = 0; i < QW; i++) {
+                        const float4 x = x4(i);
+#pragma unroll
+                        for (int r = 0; r < R; r++) sum[r] = dot4_s8(q[r][i], x, sum[r]);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < QW; i++) {                      // low nibbles: elements 4i .., high ones: 16 + 4i ..
+                        const float4 x = x4(i), y = x4(4 + i);
+#pragma unroll
+                        for (int r = 0; r < R; r++) sum[r] = dot4_u4(q[r][i] >> 4 & 0x0f0f0f0fu, y, dot4_u4(q[r][i] & 0x0f0f0f0fu, x, sum[r]));
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < R; r++) acc[r] = fmaf(d[r], sum[r], acc[r]);
+            }
+            __syncwarp();
+            issue(s == 0 ? kRawStages - 1 : s - 1);
+            s = s == kRawStages - 1 ? 0 : s + 1;
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[r] = warp_sum(acc[r]);
+        if (ks == 1) {
+            if (lane == 0 && has) {
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    if (row0 + r < N) out[row0 + r] = acc[r];
+            }
+            continue;
+        }
+        if (round > 0) __syncthreads();                     // the last round's sums have been read
+        if (lane == 0) {
+#pragma unroll
+            for (int r = 0; r < R; r++) sums[warp * R + r] = acc[r];
+        }
+        __syncthreads();
+        if (lane == 0 && part == 0 && has) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                float v = 0.f;
+                for (int p = 0; p < ks; p++) v += sums[(warp + p) * R + r];
+                if (row0 + r < N) out[row0 + r] = v;
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // ---------------- activation quantizer: one warp per block of 32 ----------------
@@ -162,27 +264,79 @@ int static_fail(int code, const char* fmt, int a, int b) {
     return code;
 }
 
-// Grid: every SM gets the same number of CTAs (rows are walked with a stride), enough warps to hide
-// the loads.  Wide inputs need more than the default 48 KB of dynamic shared memory: raised once.
+// Two rows per warp where that still leaves every warp a pair; fewer rows than warps are shared by several
+// warps each.  CTAs of 8 warps, up to three per SM, while the activations are small; wide inputs, whose copy a
+// CTA's warps share, take one CTA of 16.  Measured on B200, back to back: 4864 x 896 Q8_0 10.3 -> 4.3 us
+// (the launch), 3584 x 18944 Q4_0 104 -> 26.8 us, 18944 x 3584 Q8_0 26.4 us = 2.7 TB/s.
+struct RawShape {
+    int grid, threads, ks;
+    bool pairs, xs;
+    size_t smem;
+};
+
 template <int FMT>
-static void launch_raw_matvec(const float* act, const void* w_blocks, float* out, int N, int K, cudaStream_t stream) {
+RawShape raw_shape(int N, int K, int sms) {
+    RawShape p{};
+    const int nb = K / 32, chunks = cdiv(nb, 32);
+    size_t x = (size_t)nb * kXStride * 4;
+    auto rest = [&](int warps, int R) { return (size_t)16 * R * 4 + (size_t)warps * kRawStages * R * chunk_ring(FMT); };
+    p.xs = x + rest(16, 2) <= 226 * 1024;
+    if (!p.xs) x = 0;
+    const bool wide = x > 24 * 1024;
+    const int warps = wide ? 16 : 8, most = sms * (wide ? 1 : 3);
+    p.pairs = N >= most * warps;
+    const int R = p.pairs ? 2 : 1, tiles = cdiv(N, R);
+    p.ks = 1;
+    while (2 * p.ks <= warps && 2 * p.ks <= chunks && (long long)tiles * 2 * p.ks <= (long long)most * warps) p.ks *= 2;
+    p.grid = std::min(cdiv(tiles, warps / p.ks), most);
+    p.threads = warps * 32;
+    p.smem = x + rest(warps, R);
+    return p;
+}
+
+template <int FMT, int R, int V, bool XS>
+void run_raw_matvec(const RawShape& p, int dev, const float* act, const uint8_t* w, float* out, int N, int K, cudaStream_t stream) {
+    auto kern = raw_block_matvec_kernel<FMT, R, V, XS>;
+    static std::atomic<bool> raised[kMaxDevices];
+    if (p.smem > 48 * 1024 && !(dev < kMaxDevices && raised[dev].load(std::memory_order_relaxed))) {
+        cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        if (dev < kMaxDevices) raised[dev].store(true, std::memory_order_relaxed);
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)p.grid);
+    cfg.blockDim = dim3((unsigned)p.threads);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];        // a launch may begin while the one before it ends; the kernel waits before it reads
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, act, w, out, N, K, p.ks);
+}
+
+template <int FMT>
+void launch_raw_matvec(const float* act, const void* w_blocks, float* out, int N, int K, cudaStream_t stream) {
     if (N <= 0 || K < 32 || K % 32) return;
-    static int sms = 0;
-    static bool raised = false;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
+    static std::atomic<int> sm_count[kMaxDevices];
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (dev < kMaxDevices) sms = sm_count[dev].load(std::memory_order_relaxed);
+    if (sms <= 0) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (sms <= 0) sms = 148;
+        if (dev < kMaxDevices) sm_count[dev].store(sms, std::memory_order_relaxed);
     }
-    const size_t smem = raw_matvec_smem<FMT>(K);
-    if (smem > 48 * 1024 && !raised) {
-        cudaFuncSetAttribute((const void*)raw_block_matvec_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        raised = true;
-    }
-    const int per_sm = smem > 100 * 1024 ? 1 : smem > 48 * 1024 ? 2 : 4;
-    const int grid = std::min(cdiv(N, kRawWarps), sms * per_sm);
-    raw_block_matvec_kernel<FMT><<<grid, kRawWarps * 32, smem, stream>>>(act, (const uint8_t*)w_blocks, out, N, K);
+    const RawShape p = raw_shape<FMT>(N, K, sms);
+    const uint8_t* w = static_cast<const uint8_t*>(w_blocks);
+    auto go = [&](auto r, auto v) {
+        if (p.xs) run_raw_matvec<FMT, decltype(r)::value, decltype(v)::value, true>(p, dev, act, w, out, N, K, stream);
+        else run_raw_matvec<FMT, decltype(r)::value, decltype(v)::value, false>(p, dev, act, w, out, N, K, stream);
+    };
+    using std::integral_constant;
+    const bool v16 = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+    if (p.pairs) v16 ? go(integral_constant<int, 2>{}, integral_constant<int, 16>{}) : go(integral_constant<int, 2>{}, integral_constant<int, 4>{});
+    else v16 ? go(integral_constant<int, 1>{}, integral_constant<int, 16>{}) : go(integral_constant<int, 1>{}, integral_constant<int, 4>{});
 }
 
 }  // namespace

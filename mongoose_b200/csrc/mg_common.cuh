@@ -98,6 +98,15 @@ __device__ __forceinline__ float u4_to_f32_magic(uint32_t nibbles_as_bytes, int 
     return __uint_as_float(r) - 8388616.0f;
 }
 
+// Dot of 4 nibbles, one per byte, minus 8 each, with 4 floats.
+__device__ __forceinline__ float dot4_u4(uint32_t w, float4 x, float acc) {
+    acc = fmaf(u4_to_f32_magic(w, 0), x.x, acc);
+    acc = fmaf(u4_to_f32_magic(w, 1), x.y, acc);
+    acc = fmaf(u4_to_f32_magic(w, 2), x.z, acc);
+    acc = fmaf(u4_to_f32_magic(w, 3), x.w, acc);
+    return acc;
+}
+
 // ---------------------------------------------------------------------
 // Per-format chunk traits.  A chunk is 16 bytes of the weight plane:
 //   Q8_0: 16 int8  = half a block      (x slice: 16 floats)
