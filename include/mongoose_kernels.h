@@ -421,7 +421,8 @@ MG_API int mg_create_layered(const mg_model_config* cfg, const mg_layer_config* 
  * earlier calls left: pos is 0 (a new sequence; nothing of the old one is read) or the number of tokens
  * seen so far.  logits_out (HOST, [n_want][vocab]) receives the logits after the tokens want[0..n_want)
  * (ascending places among the n).  One token takes the decode path, more the prompt path; an engine
- * made by mg_create feeds them one by one, as its mg_generate does. */
+ * made by mg_create takes the tokens between wanted places in batches, those at wanted places, and the last, one
+ * by one, as its mg_generate does. */
 MG_API int mg_forward(mg_engine* e, const int* tokens, int n, int pos, const int* want, int n_want, float* logits_out);
 
 /* ---- tensor-parallel decode over 2/4/8 GPUs of one node, one process per GPU ----------------------

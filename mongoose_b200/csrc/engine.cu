@@ -28,6 +28,7 @@
 
 #include "../../include/mongoose_kernels.h"
 #include "decode_kernels.cuh"
+#include "dense_prompt.h"
 #include "gemm_tc.h"
 #include "kernel_table.h"
 #include "layered.h"
@@ -153,6 +154,17 @@ struct Arena {
     }
 };
 
+// Workspace of prompts that go through the layers in batches (dense_host.cuh); kept with the engine, one
+// stream's worth, like its other activations.
+struct DensePrompt {
+    int cap = 0;                        // tokens per batch; 0: prompts are fed token by token
+    int* tokens = nullptr;              // [out_cap]
+    float *x = nullptr, *q = nullptr, *sums = nullptr;      // [cap][dim], [cap][dim], pieces of products
+    __nv_bfloat16 *act = nullptr, *mid = nullptr;           // [3][cap][dim], [3][cap][ffn]
+    int* status = nullptr;
+    CUtensorMap act_map[2], mid_map[2];                     // boxes of 64 and of 32 tokens
+};
+
 }  // namespace
 
 struct Layered;
@@ -197,6 +209,7 @@ struct mg_engine {
     int mk_buf = 0;
     int mk_acc_n = 0;                   // additions that complete an accumulator word
     int mk_qkv_cta0 = 0;                // first CTA that owns QKV rows
+    DensePrompt prompt;
     PhaseGeom mk_geom[5] = {};
     size_t mk_smem = 0;
     size_t tape_bytes = 0;
@@ -493,6 +506,7 @@ int set_kernel_attrs(mg_engine* e) {
     for (int hd = 32; hd <= 128; hd *= 2)
         MG_CUDA(e, cudaFuncSetAttribute((const void*)dense_kernels()->attn(hd),
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
+    MG_CUDA(e, dense_kernels()->prompt_attrs());
     return MG_OK;
 }
 
@@ -719,6 +733,7 @@ void drop_graphs(mg_engine* e) {
 }  // namespace
 
 #include "layered_host.cuh"
+#include "dense_host.cuh"
 
 namespace {
 
@@ -1162,10 +1177,13 @@ int launch_mega(mg_engine* e, int ls, int le, int mode, int head, int n_steps) {
 int check_mega_status(mg_engine* e) {
     MegaStatus* hs = reinterpret_cast<MegaStatus*>(e->pin_i + e->pin_i_cap);
     XchgStatus* hx = reinterpret_cast<XchgStatus*>(e->pin_i + e->pin_i_cap + 8);
-    static_assert(sizeof(MegaStatus) <= 32 && sizeof(XchgStatus) <= 32, "status words must fit their pinned slots");
+    static_assert(sizeof(MegaStatus) <= 28 && sizeof(XchgStatus) <= 32, "status words must fit their pinned slots");
     if (e->tp_fused) MG_CUDA(e, cudaMemcpyAsync(hx, e->xchg_status, sizeof(XchgStatus), cudaMemcpyDeviceToHost, e->stream));
     if (e->lm) MG_CUDA(e, cudaMemcpyAsync(hs, e->lm->status, 4, cudaMemcpyDeviceToHost, e->stream));
     if (e->mega_ok) MG_CUDA(e, cudaMemcpyAsync(hs, e->mk_status, sizeof(MegaStatus), cudaMemcpyDeviceToHost, e->stream));
+    int* hp = e->pin_i + e->pin_i_cap + 7;
+    *hp = 0;
+    if (e->prompt.cap) MG_CUDA(e, cudaMemcpyAsync(hp, e->prompt.status, 4, cudaMemcpyDeviceToHost, e->stream));
     MG_CUDA(e, cudaStreamSynchronize(e->stream));
     if (e->tp_fused) {
         const XchgStatus x = *hx;
@@ -1178,6 +1196,10 @@ int check_mega_status(mg_engine* e) {
     if (e->lm && *reinterpret_cast<int*>(hs)) {
         cudaMemset(e->lm->status, 0, 4);
         return fail(e, MG_ERR_TIMEOUT, "tensor-core kernel: a wait for its own copies or products ran out");
+    }
+    if (*hp) {
+        cudaMemset(e->prompt.status, 0, 4);
+        return fail(e, MG_ERR_TIMEOUT, "prompt: a tensor-core kernel's wait for its own copies or products ran out");
     }
     if (!e->mega_ok) return MG_OK;
     const MegaStatus s = *hs;
@@ -1368,6 +1390,7 @@ int mg_create(const mg_config* cfg, mg_engine** out) {
         }
         size_t want = 2 * planes + planes / 16 + kv_elems * 4 + (size_t)c.max_seq * half * 8 + (size_t)c.vocab * 8 +
                       (size_t)(c.dim * 64 + c.ffn_dim * 16) + (size_t)e->out_cap * 4 + (64u << 20);
+        dense_prompt_buffers(e, [&](void**, size_t bytes) { want += (bytes + 511) & ~(size_t)255; return MG_OK; });
         if (const char* mb = getenv("MG_ARENA_MB")) want = (size_t)atoll(mb) << 20;
         if (!e->arena.init(want)) fprintf(stderr, "[mongoose-b200] arena of %zu MB not available: falling back to one allocation per buffer\n", want >> 20);
     }
@@ -1382,6 +1405,7 @@ int mg_create(const mg_config* cfg, mg_engine** out) {
     if ((rc = dev_alloc(e, &e->mid, (size_t)c.ffn_dim))) return bail(rc);
     if ((rc = dev_alloc(e, &e->logits, (size_t)c.vocab))) return bail(rc);
     if ((rc = create_cursor(e))) return bail(rc);
+    if ((rc = dense_prompt_create(e))) return bail(rc);
 
     // RoPE tables in float64 on the host, narrowed to fp32 (cuda_fused_infer.go:181-190).
     {
@@ -1988,6 +2012,12 @@ int mg_forward(mg_engine* e, const int* tokens, int n, int pos, const int* want,
         return check_mega_status(e);
     }
     for (int i = 0, w = 0; i < n; i++) {
+        // up to the next place whose logits are wanted (or the last token, which leaves the cursor and the hidden state) in batches
+        const int stop = w < n_want ? want[w] : n - 1;
+        if (dense_prompt_takes(e, stop - i)) {
+            if ((rc = check_range(e, 0, c.n_layers, true, true)) || (rc = dense_prompt(e, tokens + i, stop - i, pos + i))) return rc;
+            i = stop;
+        }
         const bool out = w < n_want && want[w] == i;
         int next;
         if ((rc = mg_step_token(e, tokens[i], pos + i, &next, out ? logits_out + (size_t)w * c.vocab : nullptr))) return rc;
@@ -2026,10 +2056,16 @@ int mg_generate(mg_engine* e, const int* prompt, int n_prompt, int n_new, int st
     MG_CUDA(e, cudaStreamSynchronize(e->stream));
     e->pin_i[0] = start_pos; e->pin_i[1] = prompt[0]; e->pin_i[2] = 0;
     for (int i = 0; i < n_prompt; i++) e->pin_i[8 + i] = prompt[i];
-    MG_CUDA(e, cudaMemcpyAsync(e->st, e->pin_i, 12, cudaMemcpyHostToDevice, e->stream));
     const int total = n_prompt + n_new - 1;
-    for (int i = 0; i < n_prompt; i++) {
-        if (i > 0)   // prompt tokens override the fed-back argmax
+    int first = 0;
+    if (dense_prompt_takes(e, n_prompt - 1)) {      // all but the last token, which the decode path takes with the new ones
+        if ((rc = dense_prompt(e, prompt, n_prompt - 1, start_pos))) return rc;
+        first = n_prompt - 1;
+        e->pin_i[0] = start_pos + first; e->pin_i[1] = prompt[first]; e->pin_i[2] = first;
+    }
+    MG_CUDA(e, cudaMemcpyAsync(e->st, e->pin_i, 12, cudaMemcpyHostToDevice, e->stream));
+    for (int i = first; i < n_prompt; i++) {
+        if (i > first)   // prompt tokens override the fed-back argmax
             MG_CUDA(e, cudaMemcpyAsync(&e->st->token, e->pin_i + 8 + i, 4, cudaMemcpyHostToDevice, e->stream));
         if ((rc = run_step(e, 0, c.n_layers, MODE_EMBED, HEAD_ARGMAX))) return rc;
     }

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "decode_kernels.cuh"
+#include "dense_prompt.h"
 
 namespace mg {
 
@@ -14,6 +15,13 @@ struct DenseKernels {
     attn_fn_t (*attn)(int head_dim);
     const void* (*mega)();      // persistent decode kernel, one GPU
     const void* (*mega_tp)();   // the same as one rank of a tensor-parallel group
+    // prompts in batches of tokens
+    cudaError_t (*prompt_attrs)();
+    cudaError_t (*prompt_gemm)(const PromptGemm&, cudaStream_t);
+    cudaError_t (*prompt_norm)(const PromptNorm&, int tokens, cudaStream_t);
+    cudaError_t (*prompt_rope)(const PromptRope&, int tokens, cudaStream_t);
+    cudaError_t (*prompt_attn)(const PromptAttn&, int head_dim, cudaStream_t);
+    cudaError_t (*prompt_swiglu)(const PieceSums&, const SplitRows&, int tokens, cudaStream_t);
 };
 
 const void* mega_kernel_single();

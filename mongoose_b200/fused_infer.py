@@ -329,7 +329,8 @@ class CUDAFusedInference:
     def Forward(self, tokens, pos: int, want=()) -> np.ndarray:
         """Tokens at positions pos.. of the sequence, continuing the cache and state; returns the
         logits [len(want), vocab] after the tokens at the ascending places `want`.  Layer-described
-        models take several tokens as one prompt portion, the dense block one by one."""
+        models take several tokens as one prompt portion; the dense block takes the tokens between
+        wanted places in batches and those at wanted places, and the last, one by one."""
         t = np.ascontiguousarray(tokens, dtype=np.int32)
         w = np.ascontiguousarray(want, dtype=np.int32)
         out = np.empty((w.size, self.cfg.vocab), np.float32)
