@@ -86,6 +86,7 @@ int dense_prompt(mg_engine* e, const int* tokens, int n, int pos) {
     const int L = c.n_layers;
     cudaStream_t s = e->stream;
     MG_CUDA(e, cudaStreamSynchronize(s));
+    p.ran = true;
     for (int i = 0; i < n; i++) e->pin_i[8 + i] = tokens[i];
     MG_CUDA(e, cudaMemcpyAsync(p.tokens, e->pin_i + 8, (size_t)n * 4, cudaMemcpyHostToDevice, s));
     const SplitRows act{p.act, (long long)p.cap * c.dim, c.dim}, mid{p.mid, (long long)p.cap * c.ffn_dim, c.ffn_dim};

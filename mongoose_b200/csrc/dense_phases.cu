@@ -28,7 +28,7 @@ attn_fn_t attn_fn(int head_dim) {
     return head_dim == 64 ? attn_decode_kernel<64> : head_dim == 128 ? attn_decode_kernel<128> : attn_decode_kernel<32>;
 }
 
-const DenseKernels kTable = {phase_fn, attn_fn, mega_kernel_single, mega_kernel_tp, prompt_kernel_attrs, launch_prompt_gemm,
+const DenseKernels kTable = {phase_fn, attn_fn, mega_kernel_single, mega_kernel_shared, mega_kernel_tp, prompt_kernel_attrs, launch_prompt_gemm,
                              launch_prompt_norm, launch_prompt_rope, launch_prompt_attn, launch_prompt_swiglu};
 
 }  // namespace

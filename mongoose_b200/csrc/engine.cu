@@ -162,6 +162,7 @@ struct DensePrompt {
     float *x = nullptr, *q = nullptr, *sums = nullptr;      // [cap][dim], [cap][dim], pieces of products
     __nv_bfloat16 *act = nullptr, *mid = nullptr;           // [3][cap][dim], [3][cap][ffn]
     int* status = nullptr;
+    bool ran = false;                   // since the status was last read
     CUtensorMap act_map[2], mid_map[2];                     // boxes of 64 and of 32 tokens
 };
 
@@ -209,6 +210,7 @@ struct mg_engine {
     int mk_buf = 0;
     int mk_acc_n = 0;                   // additions that complete an accumulator word
     int mk_qkv_cta0 = 0;                // first CTA that owns QKV rows
+    int mk_splits = 1;                  // most CTAs that share a query head in the persistent kernel
     DensePrompt prompt;
     PhaseGeom mk_geom[5] = {};
     size_t mk_smem = 0;
@@ -491,8 +493,8 @@ int upload_planes(mg_engine* e, int idx, int fmt, int rows, int K, const std::ve
 // ------------------------------------------------------------------
 phase_fn_t phase_fn(int fmt, int epi, int R) { return dense_kernels()->phase(fmt, epi, R); }
 
-const void* mega_fn(const mg_engine* e) {
-    return e->sh.size > 1 ? dense_kernels()->mega_tp() : dense_kernels()->mega();
+const void* mega_fn(const mg_engine* e, bool shared = false) {
+    return e->sh.size > 1 ? dense_kernels()->mega_tp() : shared ? dense_kernels()->mega_shared() : dense_kernels()->mega();
 }
 
 const int kMaxDynSmem = 120 * 1024;
@@ -901,6 +903,7 @@ int build_mega(mg_engine* e) {
         int per_sm = 0;
         const void* kern = mega_fn(e);
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->mk_smem) != cudaSuccess ||
+            cudaFuncSetAttribute(mega_fn(e, true), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->mk_smem) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MK_THREADS, e->mk_smem) != cudaSuccess ||
             per_sm < 1) {
             cudaGetLastError();
@@ -1100,7 +1103,15 @@ int build_mega(mg_engine* e) {
                     MG_CUDA(e, cudaMemcpy(e->mk_bias + l * bw + offs[k], e->vecs[l * 12 + 4 + k], lens[k] * 4, cudaMemcpyDeviceToDevice));
         }
     }
-    const size_t nx = (size_t)2 * c.dim + 2 * q_dim + 2 * c.kv_dim + c.ffn_dim + 2;   // xh xhm | xq | xkv | xattn | xmid | xtok
+    {
+        // A CTA that shares a head polls words which the next layer overwrites: every CTA must own gate/up rows, whose
+        // results the next layer waits for.
+        const PhaseGeom& gu = e->mk_geom[PH_GU];
+        const int units = (c.ffn_dim + (1 << gu.ipg_shift) - 1) >> gu.ipg_shift;
+        e->mk_splits = units >= e->num_sms && e->sh.size == 1 ? std::max(1, std::min(e->num_sms / c.n_heads, MK_MAX_SPLITS)) : 1;
+    }
+    const size_t nx = (size_t)2 * c.dim + 2 * q_dim + 2 * c.kv_dim + c.ffn_dim + 2     // xh xhm | xq | xkv | xattn | xmid | xtok
+                      + (size_t)c.n_heads * (e->mk_splits - 1) * (c.head_dim + 2);     // xpart
     MG_CUDA(e, ARENA_MALLOC(e, &e->xbuf, nx * sizeof(Tagged)));
     MG_CUDA(e, cudaMemset(e->xbuf, 0, nx * sizeof(Tagged)));
     MG_CUDA(e, ARENA_MALLOC(e, &e->mk_status, sizeof(MegaStatus)));
@@ -1115,7 +1126,7 @@ int build_mega(mg_engine* e) {
 }
 
 // One launch of the persistent kernel: n_steps tokens through layers [ls, le).
-int launch_mega(mg_engine* e, int ls, int le, int mode, int head, int n_steps) {
+int launch_mega_steps(mg_engine* e, int ls, int le, int mode, int head, int n_steps, bool shared) {
     int q_dim, vocab_base;
     const mg_config c = mega_cfg(e, &q_dim, &vocab_base);
     const int L = c.n_layers;
@@ -1137,7 +1148,8 @@ int launch_mega(mg_engine* e, int ls, int le, int mode, int head, int n_steps) {
     a.cos_tab = e->cos_tab; a.sin_tab = e->sin_tab; a.kc = e->kc; a.vc = e->vc;
     Tagged* x = e->xbuf;
     a.xh = x; x += c.dim; a.xhm = x; x += c.dim; a.xq = x; x += q_dim; a.xkv = x; x += 2 * c.kv_dim;
-    a.xattn = x; x += q_dim; a.xmid = x; x += c.ffn_dim; a.xtok = x;
+    a.xattn = x; x += q_dim; a.xmid = x; x += c.ffn_dim; a.xtok = x; x += 2;
+    a.xpart = x; a.att_splits = e->mk_splits;
     a.q_dim = q_dim; a.tp_n = e->sh.size; a.tp_rank = e->sh.rank; a.vocab_base = vocab_base; a.vocab_total = e->cfg.vocab;
     if (e->sh.size > 1) {
         // the hidden-state exchanges go through the receive buffers every rank has mapped
@@ -1164,10 +1176,22 @@ int launch_mega(mg_engine* e, int ls, int le, int mode, int head, int n_steps) {
     a.trace = e->trace_next ? e->mk_trace : nullptr;
     e->trace_next = false;
     void* params[] = {&a};
-    const void* kern = mega_fn(e);
+    const void* kern = mega_fn(e, shared);
     MG_CUDA(e, cudaLaunchCooperativeKernel(kern, dim3(e->num_sms), dim3(MK_THREADS), params,
                                            e->mk_smem, e->stream));
     e->launches += 1;
+    return MG_OK;
+}
+
+// Positions from MK_SPLIT_FROM on go to the instance whose CTAs share query heads.  The host's mirror of the position only
+// chooses: both instances are right at any position.
+int launch_mega(mg_engine* e, int ls, int le, int mode, int head, int n_steps) {
+    const int plain = e->mk_splits > 1 ? std::max(0, std::min(MK_SPLIT_FROM - e->cursor, n_steps)) : n_steps;
+    if (plain > 0)
+        if (int rc = launch_mega_steps(e, ls, le, mode, head, plain, false)) return rc;
+    if (plain < n_steps)
+        if (int rc = launch_mega_steps(e, ls, le, mode, head, n_steps - plain, true)) return rc;
+    if (head != 0 && le >= e->cfg.n_layers) e->cursor += n_steps;       // lm_head moves the device's
     return MG_OK;
 }
 
@@ -1183,7 +1207,7 @@ int check_mega_status(mg_engine* e) {
     if (e->mega_ok) MG_CUDA(e, cudaMemcpyAsync(hs, e->mk_status, sizeof(MegaStatus), cudaMemcpyDeviceToHost, e->stream));
     int* hp = e->pin_i + e->pin_i_cap + 7;
     *hp = 0;
-    if (e->prompt.cap) MG_CUDA(e, cudaMemcpyAsync(hp, e->prompt.status, 4, cudaMemcpyDeviceToHost, e->stream));
+    if (e->prompt.ran) MG_CUDA(e, cudaMemcpyAsync(hp, e->prompt.status, 4, cudaMemcpyDeviceToHost, e->stream));
     MG_CUDA(e, cudaStreamSynchronize(e->stream));
     if (e->tp_fused) {
         const XchgStatus x = *hx;
@@ -1197,6 +1221,7 @@ int check_mega_status(mg_engine* e) {
         cudaMemset(e->lm->status, 0, 4);
         return fail(e, MG_ERR_TIMEOUT, "tensor-core kernel: a wait for its own copies or products ran out");
     }
+    e->prompt.ran = false;
     if (*hp) {
         cudaMemset(e->prompt.status, 0, 4);
         return fail(e, MG_ERR_TIMEOUT, "prompt: a tensor-core kernel's wait for its own copies or products ran out");
@@ -2054,14 +2079,14 @@ int mg_generate(mg_engine* e, const int* prompt, int n_prompt, int n_new, int st
         return check_mega_status(e);
     }
     MG_CUDA(e, cudaStreamSynchronize(e->stream));
-    e->pin_i[0] = start_pos; e->pin_i[1] = prompt[0]; e->pin_i[2] = 0;
+    e->pin_i[0] = e->cursor = start_pos; e->pin_i[1] = prompt[0]; e->pin_i[2] = 0;
     for (int i = 0; i < n_prompt; i++) e->pin_i[8 + i] = prompt[i];
     const int total = n_prompt + n_new - 1;
     int first = 0;
     if (dense_prompt_takes(e, n_prompt - 1)) {      // all but the last token, which the decode path takes with the new ones
         if ((rc = dense_prompt(e, prompt, n_prompt - 1, start_pos))) return rc;
         first = n_prompt - 1;
-        e->pin_i[0] = start_pos + first; e->pin_i[1] = prompt[first]; e->pin_i[2] = first;
+        e->pin_i[0] = e->cursor = start_pos + first; e->pin_i[1] = prompt[first]; e->pin_i[2] = first;
     }
     MG_CUDA(e, cudaMemcpyAsync(e->st, e->pin_i, 12, cudaMemcpyHostToDevice, e->stream));
     for (int i = first; i < n_prompt; i++) {

@@ -14,6 +14,7 @@ struct DenseKernels {
     phase_fn_t (*phase)(int fmt, int epi, int R);
     attn_fn_t (*attn)(int head_dim);
     const void* (*mega)();      // persistent decode kernel, one GPU
+    const void* (*mega_shared)();   // the same for long contexts
     const void* (*mega_tp)();   // the same as one rank of a tensor-parallel group
     // prompts in batches of tokens
     cudaError_t (*prompt_attrs)();
@@ -25,6 +26,7 @@ struct DenseKernels {
 };
 
 const void* mega_kernel_single();
+const void* mega_kernel_shared();
 const void* mega_kernel_tp();
 
 // NULL in a library built without the dense family.

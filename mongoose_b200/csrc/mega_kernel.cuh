@@ -137,6 +137,8 @@ struct MegaArgs {
     __half* vc;
     // exchange buffers
     Tagged *xh, *xhm, *xq, *xkv, *xattn, *xmid, *xtok;
+    Tagged* xpart;          // [head][att_splits - 1][head_dim + 2] partial attention outputs (see mk_attention)
+    int att_splits;         // most CTAs that share a query head
     // Tensor parallelism (tp_n > 1): dim is the model width, every other size above is this rank's
     // share.  xh / xhm are then receive buffers [tp_n][dim] that every rank writes its partial sums
     // into (peer stores), xbest [tp_n][2] receives the ranks' argmax keys.
@@ -1501,6 +1503,20 @@ __device__ __forceinline__ void mk_clear_next(const MegaArgs& a, long long* acc_
 }
 
 // ---------------------------------------------------------------------
+// CTAs that share a query head at `pos`: CTA s * n_heads + h takes the s-th run of the positions of head h.  One CTA
+// keeps up with the other phases as long as its rows sit in registers when q arrives (240 positions); beyond
+// that it fetches them behind q, 256 bytes of K and V per position through one SM.  A split costs one more
+// exchange, the partial outputs.  B200, six layers of 1.1B widths, us per token with one CTA a head / with 240 positions
+// per CTA: at 300 positions 176.8 / 177.3, 360: 182.4 / 178.3, 600: 209.3 / 185.8, 960: 246.7 / 195.4; two layers of
+// 7B widths, at 300: 251.0 / 248.2, 900: 282.7 / 250.5.  Runs of 120, 160 and 300 positions were no better.
+constexpr int MK_SPLIT_FROM = 320;
+constexpr int MK_SPLIT_POSITIONS = 240;
+constexpr int MK_MAX_SPLITS = 5;
+__device__ __forceinline__ int mk_attn_splits(const MegaArgs& a, int pos) {
+    return pos < MK_SPLIT_FROM ? 1 : min((pos + MK_SPLIT_POSITIONS) / MK_SPLIT_POSITIONS, a.att_splits);
+}
+
+// ---------------------------------------------------------------------
 // Attention for one query head on this CTA (fp16 KV cache), three barriers.
 // Cached K/V rows do not depend on this token, so they are loaded into registers BEFORE q is
 // waited for.
@@ -1509,6 +1525,8 @@ __device__ __forceinline__ void mk_clear_next(const MegaArgs& a, long long* acc_
 //   softmax: one maximum over the CTA; exp(s - max) is formed where it is used;
 //   P . V  : warp w takes positions w, w + 15, ... (the first NV from registers), a lane HD / 32
 //            adjacent dims; the warps' partial outputs and partial sums of exp meet in shared memory.
+// Where several CTAs share the head, each does this for its run of positions and the first of them
+// collects the others' outputs, maxima and sums.  Positions below are relative to the run.
 // ---------------------------------------------------------------------
 template <int VPL>
 __device__ __forceinline__ uint2 ldcg_v(const __half* p) {
@@ -1542,9 +1560,60 @@ __device__ __forceinline__ float dot8_kq(uint4 kk, uint32_t q_s) {
     return d0 + d1;
 }
 
-template <int HD>
-__device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int layer, int pos, unsigned int tag_in,
-                                             unsigned int tag_out) {
+// Element tid of a head's output and the sum of its weights over all the head's splits, from those of the first split
+// (s, l, relative to the maximum m) and the words of the n others.  All words are requested before any is
+// waited for.  Out of line: attention is expanded for every format and head size.
+static __device__ __noinline__ float2 mk_merge_splits(volatile int* abort_flag, MegaStatus* status, long long limit, const Tagged* part,
+                                                      int n, int stride, int tid, unsigned int tag, float s, float l, float m) {
+    uint2 o[MK_MAX_SPLITS - 1];
+    uint4 ml[MK_MAX_SPLITS - 1];
+#pragma unroll
+    for (int q = 0; q < MK_MAX_SPLITS - 1; q++)
+        if (q < n) {
+            o[q] = ld_poll8(part + q * stride + tid);
+            ml[q] = ld_poll16(part + q * stride + stride - 2);
+        }
+    float top = m;
+#pragma unroll
+    for (int q = 0; q < MK_MAX_SPLITS - 1; q++)
+        if (q < n) {
+            if (o[q].y != tag) {
+                const uint4 pair = mk_poll16_slow(abort_flag, status, limit, part + q * stride + (tid & ~1), tag, 0);
+                o[q].x = tid & 1 ? pair.z : pair.x;
+            }
+            if (ml[q].y != tag || ml[q].w != tag) ml[q] = mk_poll16_slow(abort_flag, status, limit, part + q * stride + stride - 2, tag, 0);
+            top = fmaxf(top, __uint_as_float(ml[q].x));
+        }
+    const float f0 = __expf(m - top);
+    s *= f0;
+    l *= f0;
+#pragma unroll
+    for (int q = 0; q < MK_MAX_SPLITS - 1; q++)
+        if (q < n) {
+            const float f = __expf(__uint_as_float(ml[q].x) - top);
+            s = fmaf(f, __uint_as_float(o[q].x), s);
+            l = fmaf(f, __uint_as_float(ml[q].z), l);
+        }
+    return make_float2(s, l);
+}
+
+// The new K and V rows of this token on a CTA that will share the head later in this launch: a CTA reads
+// back only cache rows that it has written itself, or that an earlier launch has written.
+static __device__ __noinline__ void mk_append_row(volatile int* abort_flag, MegaStatus* status, long long limit, const Tagged* k_new, int kv_dim,
+                                                  int hd, __half* k_row, __half* v_row, unsigned int tag) {
+    const int i = 2 * (int)threadIdx.x;
+    if (i >= 2 * hd) return;
+    const bool is_k = i < hd;
+    const int at = is_k ? i : i - hd;
+    const Tagged* p = k_new + (is_k ? 0 : kv_dim) + at;
+    uint4 r = ld_poll16(p);
+    if (r.y != tag || r.w != tag) r = mk_poll16_slow(abort_flag, status, limit, p, tag, 0);
+    *reinterpret_cast<__half2*>((is_k ? k_row : v_row) + at) = __floats2half2_rn(__uint_as_float(r.x), __uint_as_float(r.z));
+}
+
+template <int HD, bool SHARED>
+__device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int layer, int pos, int split, int splits,
+                                             unsigned int tag_in, unsigned int tag_out) {
     constexpr int DPL = HD / 4;                // dims per lane in the score phase
     constexpr int KV4 = DPL / 8;               // 16-byte pieces of K per lane and position
     constexpr int NPRE = HD == 128 ? 2 : 4;    // score passes whose K rows are held in registers
@@ -1552,30 +1621,34 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
     constexpr int VPL = HD / 32;               // dims per lane in P . V
     constexpr int NV = 16;                     // positions per warp whose V rows are held in registers
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int head = blockIdx.x;
+    const int head = (int)blockIdx.x - (SHARED ? split * a.n_heads : 0);
     const int kvh = head / (a.n_heads / a.n_kv_heads);
-    const size_t lbase = (size_t)layer * a.max_seq * a.kv_dim;
-    __half* kc = a.kc + lbase + kvh * HD;
-    __half* vc = a.vc + lbase + kvh * HD;
+    // this CTA's run of positions: rows 0 .. now - 1 of kc / vc are cached, row `now` is the new one where the run ends with it
+    const int run = SHARED && splits > 1 ? (pos + splits) / splits : pos + 1, first = SHARED ? split * run : 0;
+    const bool ends = !SHARED || first + run > pos;
+    const int now = ends ? pos - first : run, end = ends ? now : now - 1;
+    const size_t lbase = (size_t)layer * a.max_seq * a.kv_dim + kvh * HD;
+    const __half* kc = a.kc + lbase + (size_t)first * a.kv_dim;
+    const __half* vc = a.vc + lbase + (size_t)first * a.kv_dim;
     const uint32_t xs_s = smem_u32(mk_smem) + c.xs_off;        // q | new k | new v, HD floats each
     const int uq = lane >> 2, qp = lane & 3;
     // Warp w owns positions w, w + 15, w + 30, ...: it computes their scores AND their share of
     // P . V, so the scores never leave the warp; pass i covers its positions number 8 i .. 8 i + 7.
     const int t_first = w + MK_NW * uq;
 
-    // ---- cached rows (positions < pos) into registers ----
+    // ---- cached rows (positions < now) into registers ----
     // Everything below is guarded per warp (a warp's positions of a pass / of a group of four are
-    // known from w and pos alone), so a short context skips the passes it does not have instead of
+    // known from w and the run alone), so a short context skips the passes it does not have instead of
     // walking through their predicated-off loads.
-    const int npass = (pos - w + MK_NW * PPP) / (MK_NW * PPP);      // score passes in which this warp has a position <= pos (w <= pos)
-    const int nv = w < pos ? (pos - w + MK_NW - 1) / MK_NW : 0;     // cached positions of this warp for P . V
+    const int npass = (end - w + MK_NW * PPP) / (MK_NW * PPP);      // score passes in which this warp has a position <= end (w <= end)
+    const int nv = w < now ? (now - w + MK_NW - 1) / MK_NW : 0;     // cached positions of this warp for P . V
     uint4 kreg[NPRE][KV4];
 #pragma unroll
     for (int i = 0; i < NPRE; i++) {
         const int t = t_first + i * (MK_NW * PPP);
 #pragma unroll
         for (int j = 0; j < KV4; j++) kreg[i][j] = make_uint4(0u, 0u, 0u, 0u);
-        if (w <= pos && i < npass && t < pos) {
+        if (w <= end && i < npass && t < now) {
             const uint4* kp = reinterpret_cast<const uint4*>(kc + (size_t)t * a.kv_dim + qp * DPL);
 #pragma unroll
             for (int j = 0; j < KV4; j++) kreg[i][j] = __ldcg(kp + j);
@@ -1590,7 +1663,7 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
 #pragma unroll
             for (int j = j0; j < j0 + 4; j++) {
                 const int t = w + j * MK_NW;
-                if (t < pos) vreg[j] = ldcg_v<VPL>(vc + (size_t)t * a.kv_dim + lane * VPL);
+                if (t < now) vreg[j] = ldcg_v<VPL>(vc + (size_t)t * a.kv_dim + lane * VPL);
             }
         }
     }
@@ -1607,8 +1680,8 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
         *reinterpret_cast<float2*>(c.xs() + i) = make_float2(v0, v1);
         // every CTA of the KV group appends the (identical) new row; each CTA later reads back
         // only addresses it has written itself
-        if (which == 1) *reinterpret_cast<__half2*>(kc + (size_t)pos * a.kv_dim + d) = __floats2half2_rn(v0, v1);
-        if (which == 2) *reinterpret_cast<__half2*>(vc + (size_t)pos * a.kv_dim + d) = __floats2half2_rn(v0, v1);
+        if (which == 1) *reinterpret_cast<__half2*>(a.kc + lbase + (size_t)pos * a.kv_dim + d) = __floats2half2_rn(v0, v1);
+        if (which == 2) *reinterpret_cast<__half2*>(a.vc + lbase + (size_t)pos * a.kv_dim + d) = __floats2half2_rn(v0, v1);
     }
     consumer_sync();
     MK_ESTAMP(41);
@@ -1619,9 +1692,9 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
     float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < NPRE; i++) {
-        if (i == 0 || (w <= pos && i < npass)) {                   // uniform over the warp
+        if (i == 0 || (w <= end && i < npass)) {                   // uniform over the warp
             const int t = t_first + i * (MK_NW * PPP);
-            if (t == pos) {
+            if (t == now) {
                 // the new position's K row sits in shared memory (fp16-rounded values: the conversion is exact)
                 const float* kn = c.xs() + HD + qp * DPL;
 #pragma unroll
@@ -1638,19 +1711,19 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
             dot += __shfl_xor_sync(MG_FULL_MASK, dot, 1);
             dot += __shfl_xor_sync(MG_FULL_MASK, dot, 2);
             dot *= scale;
-            if (t <= pos) { if (qp == 0) c.sc()[t] = dot; mx = fmaxf(mx, dot); }
+            if (t <= end) { if (qp == 0) c.sc()[t] = dot; mx = fmaxf(mx, dot); }
         }
     }
-    for (int i = NPRE; w <= pos && i < npass; i++) {              // contexts beyond the registers: rows from L2
+    for (int i = NPRE; w <= end && i < npass; i++) {              // contexts beyond the registers: rows from L2
         const int t = t_first + i * (MK_NW * PPP);
         uint4 kk[KV4];
 #pragma unroll
         for (int j = 0; j < KV4; j++) kk[j] = make_uint4(0u, 0u, 0u, 0u);
-        if (t < pos) {
+        if (t < now) {
             const uint4* kp = reinterpret_cast<const uint4*>(kc + (size_t)t * a.kv_dim + qp * DPL);
 #pragma unroll
             for (int j = 0; j < KV4; j++) kk[j] = __ldcg(kp + j);
-        } else if (t == pos) {
+        } else if (t == now) {
             const float* kn = c.xs() + HD + qp * DPL;
 #pragma unroll
             for (int j = 0; j < KV4; j++) {
@@ -1666,7 +1739,7 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
         dot += __shfl_xor_sync(MG_FULL_MASK, dot, 1);
         dot += __shfl_xor_sync(MG_FULL_MASK, dot, 2);
         dot *= scale;
-        if (t <= pos) { if (qp == 0) c.sc()[t] = dot; mx = fmaxf(mx, dot); }
+        if (t <= end) { if (qp == 0) c.sc()[t] = dot; mx = fmaxf(mx, dot); }
     }
     mx = warp_max(mx);                       // -inf: the warp has no position
     __syncwarp();                            // the scores in sc[] were written by lanes of this warp
@@ -1678,7 +1751,7 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
 #pragma unroll
     for (int e = 0; e < VPL; e++) acc[e] = 0.f;
     float lsum = 0.f;
-    const int last = max(pos - 1, 0);
+    const int last = max(now - 1, 0);
 #pragma unroll
     for (int j0 = 0; j0 < NV; j0 += 4) {
         if (j0 < nv) {
@@ -1687,31 +1760,31 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
             for (int j = j0; j < j0 + 4; j++) {
                 const int t = w + j * MK_NW;
                 float p = __expf(c.sc()[min(t, last)] - mx);
-                p = t < pos ? p : 0.f;
+                p = t < now ? p : 0.f;
                 lsum += p;
                 fma_v<VPL>(acc, p, vreg[j]);
             }
         }
     }
-    for (int t0 = w + NV * MK_NW; t0 < pos; t0 += 4 * MK_NW) {   // remainder, four loads in flight
+    for (int t0 = w + NV * MK_NW; t0 < now; t0 += 4 * MK_NW) {   // remainder, four loads in flight
         uint2 vv[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int t = t0 + j * MK_NW;
             vv[j] = make_uint2(0u, 0u);
-            if (t < pos) vv[j] = ldcg_v<VPL>(vc + (size_t)t * a.kv_dim + lane * VPL);
+            if (t < now) vv[j] = ldcg_v<VPL>(vc + (size_t)t * a.kv_dim + lane * VPL);
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int t = t0 + j * MK_NW;
             float p = __expf(c.sc()[min(t, last)] - mx);
-            p = t < pos ? p : 0.f;
+            p = t < now ? p : 0.f;
             lsum += p;
             fma_v<VPL>(acc, p, vv[j]);
         }
     }
-    if (w == pos % MK_NW) {                                       // the new position belongs to one warp
-        const float p = __expf(c.sc()[pos] - mx);
+    if (ends && w == now % MK_NW) {                                       // the new position belongs to one warp
+        const float p = __expf(c.sc()[now] - mx);
         lsum += p;
         const float* vn = c.xs() + 2 * HD + lane * VPL;
 #pragma unroll
@@ -1743,6 +1816,18 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
             s = fmaf(f, c.part()[g * HD + tid], s);
             lt = fmaf(f, l[g], lt);
         }
+        if (SHARED && splits > 1) {
+            Tagged* part = a.xpart + (size_t)head * (a.att_splits - 1) * (HD + 2);
+            if (split > 0) {
+                part += (split - 1) * (HD + 2);
+                st_tagged(part + tid, s, tag_out);
+                if (tid == 0) { st_tagged(part + HD, M, tag_out); st_tagged(part + HD + 1, lt, tag_out); }
+                return;
+            }
+            const float2 all = mk_merge_splits(c.abort_flag(), c.status(), a.wait_cycles, part, splits - 1, HD + 2, tid, tag_out, s, lt, M);
+            s = all.x;
+            lt = all.y;
+        }
         st_tagged(a.xattn + head * HD + tid, __fdividef(s, lt), tag_out);
     }
 }
@@ -1753,7 +1838,7 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
 // Trace events per layer (mg_trace_step): 2p = input of phase p ready, 2p+1 = phase p done,
 // 8 = layer start, 9 = attention done (attention CTAs).
 // ---------------------------------------------------------------------
-template <bool TP>
+template <bool TP, bool SHARED>
 __device__ __forceinline__ void mk_consumer(MkCtx& c, const MegaArgs& a) {
     const int tid = threadIdx.x;
     const int L = a.n_layers;
@@ -1763,10 +1848,13 @@ __device__ __forceinline__ void mk_consumer(MkCtx& c, const MegaArgs& a) {
     const bool do_head = a.le >= L && a.head;
     const bool fused = !TP && a.ffn_fused;
     int qn = 0;                              // layers finished in this launch
+    const int my_split = SHARED ? (int)blockIdx.x / a.n_heads : (int)blockIdx.x < a.n_heads ? 0 : 1;
+    const int late_splits = SHARED ? mk_attn_splits(a, min(pos0 + a.n_steps, a.max_seq) - 1) : 1;   // of the launch's last token
 
     for (int step = 0; step < a.n_steps; step++) {
         const unsigned int ep = a.epoch + (unsigned)step * (unsigned)(L * MK_EPOCHS_PER_LAYER + 8);
         const int pos = min(pos0 + step, a.max_seq - 1);
+        const int splits = SHARED ? mk_attn_splits(a, pos) : 1;
         // ---- token of this step (greedy feedback from the previous step) ----
         if (a.embed) {
             if (step > 0) token = (int)__float_as_uint(mk_poll1(c, a.xtok, ep - 8u + 1u));
@@ -1790,12 +1878,16 @@ __device__ __forceinline__ void mk_consumer(MkCtx& c, const MegaArgs& a) {
             }                                                                                                      \
             if (l == a.ls) s0.kind = a.embed ? SRC_EMBED : SRC_PLAIN;                                              \
             mk_run_phase<PH_QKV, FMT, TP>(a, c, s0, l, base + 1, l * MK_EV, best);                                 \
-            if ((int)blockIdx.x < a.n_heads) {                                                                     \
+            if (my_split < splits) {                                                                               \
                 MK_SET_PROBE(l * MK_EV);                                                                           \
-                if (a.head_dim == 64) mk_attention<64>(a, c, l, pos, base + 1, base + 2);                          \
-                else if (a.head_dim == 128) mk_attention<128>(a, c, l, pos, base + 1, base + 2);                   \
-                else mk_attention<32>(a, c, l, pos, base + 1, base + 2);                                           \
+                if (a.head_dim == 64) mk_attention<64, SHARED>(a, c, l, pos, my_split, splits, base + 1, base + 2); \
+                else if (a.head_dim == 128) mk_attention<128, SHARED>(a, c, l, pos, my_split, splits, base + 1, base + 2); \
+                else mk_attention<32, SHARED>(a, c, l, pos, my_split, splits, base + 1, base + 2);                 \
                 mk_trace(a, step, l * MK_EV + 9);                                                                  \
+            } else if (SHARED && my_split < late_splits) {                                                         \
+                const int at = ((int)blockIdx.x - my_split * a.n_heads) / (a.n_heads / a.n_kv_heads) * a.head_dim;  \
+                const size_t row = ((size_t)l * a.max_seq + pos) * a.kv_dim + at;                                  \
+                mk_append_row(c.abort_flag(), c.status(), a.wait_cycles, a.xkv + at, a.kv_dim, a.head_dim, a.kc + row, a.vc + row, base + 1); \
             }                                                                                                      \
             if (fused) mk_clear_next(a, a.acc + (size_t)((a.acc_buf0 + qn + 1) % 3) * a.dim);                      \
             const StageSrc s1{SRC_POLL, a.xattn, base + 2, a.q_dim, nullptr, token};                               \
@@ -1917,8 +2009,10 @@ __host__ __device__ inline size_t mk_smem_bytes(int nslot, int slot_bytes, int x
            2 * MK_MAX_SLOTS * 8 + 16 + 64 + 5 * 16 * 2 + 16;
 }
 
-// TP = false: one GPU (no peer pointers are touched); TP = true: one rank of a tensor-parallel group.
-template <bool TP>
+// TP = false: one GPU (no peer pointers are touched); TP = true: one rank of a tensor-parallel group.  SHARED: query heads
+// may be shared by CTAs (mk_attention); an instance of its own, since the longer code of a layer costs the
+// launches that do not need it 2 to 5 % (instruction fetch is part of what bounds a phase).
+template <bool TP, bool SHARED>
 __global__ void __launch_bounds__(MK_THREADS, 1) mega_decode_kernel(const __grid_constant__ MegaArgs a) {
     MkCtx c(a);
     if (threadIdx.x == 0) {
@@ -1956,7 +2050,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) mega_decode_kernel(const __grid
     }
     __syncthreads();
     if (threadIdx.x >= MK_CONSUMERS) mk_producer(c, a);
-    else mk_consumer<TP>(c, a);
+    else mk_consumer<TP, SHARED>(c, a);
 }
 
 }  // namespace mg

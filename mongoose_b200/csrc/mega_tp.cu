@@ -2,4 +2,4 @@
 #include "kernel_table.h"
 #include "mega_kernel.cuh"
 
-const void* mg::mega_kernel_tp() { return (const void*)mg::mega_decode_kernel<true>; }
+const void* mg::mega_kernel_tp() { return (const void*)mg::mega_decode_kernel<true, false>; }
