@@ -283,6 +283,263 @@ __global__ void __launch_bounds__(kThreads, Geo<HP>::per_sm) gate_scores_kernel(
     if (warp == 1) tmem_free(acc, G::cols);
 }
 
+// ---- heads one at a time, mixed behind the product with the keys ---------------------------------------
+// sum over keys of (sum over g of T[h][g] w_g) v = sum over g of T[h][g] (sum over keys of w_g v): the weights are
+// multiplied by the keys first and the heads are mixed in the outputs.  A head then multiplies the keys of
+// EVERY key head, kv_heads times the products, which the tensor cores do not notice, and mixing falls from
+// every (query, key) pair to every query.  A CTA owns 128 queries of one head and up to 256 output columns
+// and walks the keys in tiles of 64: scores into one of two TMEM buffers, sigmoids in fp32 on eight warps,
+// weights as two bf16 parts, high and low, into one of two shared-memory buffers, O += (P_high + P_low) V
+// in TMEM.  The weights carry 16 bits of mantissa into an fp32 sum and are never rounded to 8.
+constexpr int kFlashKeys = 64;
+constexpr int kFlashCols = 256;
+
+struct FlashArgs {
+    CUtensorMap q, k, v;            // [rows][heads][dim_s] in boxes of 128 rows; [max_seq][kv][dim_s], 64 rows; [kv * dim][ldv], `cols` rows
+    GateAttn at;
+    int row0, rows, pos0;           // queries [row0, row0 + rows) of the portion, at positions pos0 + row
+    int kb;                         // 64-column steps of a query
+    int per, cols;                  // key heads per CTA; their columns, padded to 16
+    int tmem_cols;
+    float* o;                       // [rows][heads][kv_heads * dim]
+    int* status;
+};
+
+constexpr int flash_smem(int kb, int cols) { return kb * 128 * 128 + 4 * 128 * 128 + 2 * kb * kFlashKeys * 128 + 2 * ((cols * 128 + 1023) & ~1023) + 1024 + 256 + 8 * 2 * 32 * 4; }
+
+__global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_constant__ FlashArgs a) {
+    extern __shared__ uint8_t raw[];
+    uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
+    const GateAttn& A = a.at;
+    const int kbytes = a.kb * kFlashKeys * 128, vbytes = pad_to(a.cols * 128, 1024);
+    uint8_t* Q = base;
+    uint8_t* P = Q + a.kb * 128 * 128;                      // [2][high, low][128 x 64]
+    uint8_t* Ks = P + 4 * 128 * 128;
+    uint8_t* Vs = Ks + 2 * kbytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(Vs + 2 * vbytes);
+    uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 3, *v_full = bars + 5, *v_empty = bars + 7, *s_full = bars + 9, *p_empty = bars + 11,
+             *s_empty = bars + 13, *p_full = bars + 15;
+    uint32_t* tmem_base = reinterpret_cast<uint32_t*>(bars + 17);
+    float* rms = reinterpret_cast<float*>(Vs + 2 * vbytes + 256);               // [warp][2][32]: -log2 e / rms of the warp's keys
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = blockIdx.y, c = h / (A.heads / A.kv_heads), c0 = blockIdx.z * a.per;
+    const int tile_row = (gridDim.x - 1 - blockIdx.x) * 128;                    // the longest rows first
+    const int first = a.pos0 + a.row0 + tile_row;                               // position of the first query
+    const int last = a.pos0 + a.row0 + min(tile_row + 128, a.rows) - 1;
+    const int tiles = last / kFlashKeys + 1;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 17; i++) bar_init(bars + i, i >= 13 ? 8 : 1);
+        bar_init_fence();
+        tma_prefetch_map(&a.q); tma_prefetch_map(&a.k); tma_prefetch_map(&a.v);
+    }
+    if (warp == 1) tmem_alloc(tmem_base, a.tmem_cols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t S0 = *tmem_base, O = S0 + 2 * kFlashKeys;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            bar_expect(q_full, a.kb * 128 * 128);
+            for (int x = 0; x < a.kb; x++) tma_load_3d(Q + x * 128 * 128, &a.q, x * 64, h, a.row0 + tile_row, q_full);
+            int ki = 0, vi = 0;
+            for (int j = 0; j < tiles; j++) {
+                const int s = j & 1, use = j >> 1;
+                if (use > 0 && !bar_wait(k_empty + s, (use - 1) & 1, a.status)) break;
+                bar_expect(k_full + s, kbytes);
+                for (int x = 0; x < a.kb; x++) tma_load_3d(Ks + s * kbytes + x * kFlashKeys * 128, &a.k, x * 64, c, j * kFlashKeys, k_full + s);
+                ki = j + 1;
+                if (use > 0 && !bar_wait(v_empty + s, (use - 1) & 1, a.status)) break;
+                bar_expect(v_full + s, a.cols * 128);
+                tma_load_3d(Vs + s * vbytes, &a.v, j * kFlashKeys, c0 * A.dim, 0, v_full + s);
+                vi = j + 1;
+            }
+            // no copy may be in flight when the CTA leaves
+            bar_wait(q_full, 0, a.status);
+            for (int i = max(0, ki - 2); i < ki; i++) bar_wait(k_full + (i & 1), (i >> 1) & 1, a.status);
+            for (int i = max(0, vi - 2); i < vi; i++) bar_wait(v_full + (i & 1), (i >> 1) & 1, a.status);
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            auto scores = [&](int j) {
+                const int b = j & 1;
+                if (!bar_wait(k_full + b, (j >> 1) & 1, a.status)) return false;
+                if (j >= 2 && !bar_wait(s_empty + b, ((j >> 1) - 1) & 1, a.status)) return false;
+                tc_fence_after();
+                for (int x = 0; x < a.kb; x++) {
+                    const uint64_t da = tile_desc(Q + x * 128 * 128), db = tile_desc(Ks + b * kbytes + x * kFlashKeys * 128);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) mma_bf16(S0 + b * kFlashKeys, da + 2 * k, db + 2 * k, mma_desc(kFlashKeys), x > 0 || k > 0);
+                }
+                mma_commit(k_empty + b);
+                mma_commit(s_full + b);
+                return true;
+            };
+            bool ok = bar_wait(q_full, 0, a.status) && scores(0);
+            for (int j = 0; j < tiles && ok; j++) {
+                if (j + 1 < tiles && !(ok = scores(j + 1))) break;
+                const int b = j & 1;
+                ok = bar_wait(v_full + b, (j >> 1) & 1, a.status) && bar_wait(p_full + b, (j >> 1) & 1, a.status);
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t dh = tile_desc(P + b * 2 * 128 * 128), dl = tile_desc(P + (b * 2 + 1) * 128 * 128), db = tile_desc(Vs + b * vbytes);
+                const uint32_t desc = mma_desc(a.cols);
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    mma_bf16(O, dl + 2 * k, db + 2 * k, desc, j > 0 || k > 0);
+                    mma_bf16(O, dh + 2 * k, db + 2 * k, desc, true);
+                }
+                mma_commit(v_empty + b);
+                mma_commit(p_empty + b);
+            }
+        }
+        __syncwarp();
+    } else {
+        constexpr float kLog2e = 1.4426950408889634f;
+        const int quarter = warp & 3, half = (warp - 2) >> 2, r = quarter * 32 + lane;
+        const uint32_t mine = (uint32_t)(quarter * 32) << 16;
+        const float slope = A.slopes[h] * kLog2e, bias = -A.head_bias[h] * kLog2e;
+        float* kr = rms + (warp - 2) * 64;
+        auto key_rms = [&](int j) {
+            const int key = j * kFlashKeys + half * 32 + lane;
+            return key <= last ? -kLog2e * A.cache_r[(size_t)key * A.kv_heads + c] : 0.f;
+        };
+        const int pos = first + r;
+        float next = key_rms(0);
+        bool ok = true;
+        for (int j = 0; j < tiles; j++) {
+            const int b = j & 1, k0 = j * kFlashKeys + half * 32;
+            kr[b * 32 + lane] = next;
+            __syncwarp();
+            if (j + 1 < tiles) next = key_rms(j + 1);
+            ok = __all_sync(MG_FULL_MASK, bar_wait(s_full + b, (j >> 1) & 1, a.status));
+            if (!ok) break;
+            tc_fence_after();
+            float s[32];
+            tmem_load32(S0 + mine + b * kFlashKeys + half * 32, s);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) bar_arrive(s_empty + b);
+            const int seen = pos - k0 + 1;                  // keys of this half that the row sees
+            const bool cut = __any_sync(MG_FULL_MASK, seen < 32);
+            if (cut) {                                      // rows of the cache behind the query hold anything
+#pragma unroll
+                for (int i = 0; i < 32; i++)
+                    if (i >= seen) s[i] = 0.f;
+            }
+            // 1 / (1 + 2^t), two at a time: 1 / x = y / (x y).  Exponents are cut off at 60, where a weight is 2^-60.
+            const float line = fmaf(slope, (float)(pos - k0), bias);
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 k4 = *reinterpret_cast<const float4*>(kr + b * 32 + i);
+                const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
+                float e[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    float t = fmaf(s[i + u], kk[u], fmaf(-slope, (float)(i + u), line));
+                    asm("min.NaN.f32 %0, %1, 0f42700000;" : "=f"(t) : "f"(t));
+                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e[u]) : "f"(t));
+                    e[u] += 1.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u += 2) {
+                    float inv;
+                    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(e[u] * e[u + 1]));
+                    s[i + u] = inv * e[u + 1];
+                    s[i + u + 1] = inv * e[u];
+                }
+            }
+            if (cut) {
+#pragma unroll
+                for (int i = 0; i < 32; i++)
+                    if (i >= seen) s[i] = 0.f;
+            }
+            if (j >= 2) {
+                ok = __all_sync(MG_FULL_MASK, bar_wait(p_empty + b, ((j >> 1) - 1) & 1, a.status));
+                if (!ok) break;
+            }
+            uint8_t* high = P + b * 2 * 128 * 128 + r * 128;
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                uint32_t w[4], u[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float p = s[x * 8 + i * 2], q = s[x * 8 + i * 2 + 1];
+                    w[i] = bf16_pair(p, q);
+                    u[i] = bf16_pair(p - __uint_as_float(w[i] << 16), q - __uint_as_float(w[i] & 0xffff0000u));
+                }
+                const int at = ((half * 4 + x) ^ (r & 7)) << 4;
+                *reinterpret_cast<uint4*>(high + at) = make_uint4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<uint4*>(high + 128 * 128 + at) = make_uint4(u[0], u[1], u[2], u[3]);
+            }
+            async_proxy_fence();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) bar_arrive(p_full + b);
+        }
+        if (ok) ok = __all_sync(MG_FULL_MASK, bar_wait(p_empty + ((tiles - 1) & 1), ((tiles - 1) >> 1) & 1, a.status));
+        if (ok) {
+            tc_fence_after();
+            const int wide = A.kv_heads * A.dim, cols = min(a.per, A.kv_heads - c0) * A.dim, row = tile_row + r;
+            float* out = a.o + ((size_t)row * A.heads + h) * wide + c0 * A.dim;
+            const bool vec = (A.dim & 3) == 0;
+            for (int x = half * 32; x < cols; x += 64) {
+                float o[32];
+                tmem_load32(O + mine + x, o);
+                if (row < a.rows) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) {
+                        if (vec) {
+                            if (x + i < cols) *reinterpret_cast<float4*>(out + x + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
+                        } else {
+#pragma unroll
+                            for (int u = 0; u < 4; u++)
+                                if (x + i + u < cols) out[x + i + u] = o[i + u];
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1) tmem_free(S0, a.tmem_cols);
+}
+
+// out[row][h][d] = sum over g of T[h][g] o[row][g][key head of h][d]: a CTA per row, every element of o read once, eight heads
+// of a group at a time.
+__global__ void __launch_bounds__(256) gate_mix_kernel(GateAttn A, const float* o, __nv_bfloat16* out, int ld_out) {
+    __shared__ __align__(16) float talk[32][32];            // [g][h], heads of a group side by side
+    const int H = A.heads, group = H / A.kv_heads, wide = A.kv_heads * A.dim;
+    for (int i = threadIdx.x; i < 32 * 32; i += 256) {
+        const int h = i & 31, g = i >> 5;
+        talk[g][h] = h < H && g < H ? A.talk[h * H + g] : 0.f;
+    }
+    __syncthreads();
+    const size_t row = blockIdx.x;
+    for (int e = threadIdx.x; e < wide; e += 256) {
+        const int c = e / A.dim, d = e - c * A.dim;
+        const float* p = o + row * H * wide + e;
+        for (int h0 = 0; h0 < group; h0 += 8) {
+            float acc[8] = {};
+#pragma unroll 8
+            for (int g = 0; g < H; g++) {
+                const float v = p[(size_t)g * wide];
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[i] = fmaf(talk[g][min(c * group + h0 + i, 31)], v, acc[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (h0 + i < group) out[row * ld_out + (size_t)(c * group + h0 + i) * A.dim + d] = __float2bfloat16_rn(acc[i]);
+        }
+    }
+}
+
 // cache [len][kv][dim_s] -> vt [kv][dim][ldv], zero from len to ldv
 __global__ void __launch_bounds__(256) key_transpose_kernel(const __nv_bfloat16* cache, int kv_heads, int dim, int dim_s, int len, int ldv,
                                                             __nv_bfloat16* vt) {
@@ -306,10 +563,47 @@ cudaError_t scores(const ScoreArgs& a, cudaStream_t s) {
 
 }  // namespace
 
+namespace {
+
+// Heads one at a time where a query, two buffers of weights and two stages of keys fit shared memory; wider heads take the
+// kernel that mixes pairs.
+bool gate_flash_fits(const GateAttn& at) { return at.dim_s <= 128; }
+
+size_t bytes_per_row(const GateAttn& at, int max_seq) {
+    return gate_flash_fits(at) ? (size_t)at.heads * at.kv_heads * at.dim * 4 : (size_t)at.heads * pad_to(max_seq, 64) * 2;
+}
+
+cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* work, int block_rows, const void* vt, int ldv,
+                         void* out, int ld_out, int* status, int* launches, cudaStream_t s) {
+    FlashArgs a{};
+    a.at = at; a.pos0 = pos0; a.o = (float*)work; a.status = status;
+    a.kb = (at.dim_s + 63) / 64;
+    a.per = std::min(at.kv_heads, kFlashCols / at.dim);
+    a.cols = pad_to(a.per * at.dim, 16);
+    a.tmem_cols = 2 * kFlashKeys + pad_to(a.cols, 32) <= 256 ? 256 : 512;
+    if (!make_head_map(&a.q, qh, at.dim_s, at.heads, max_rows, at.dim_s, (long long)at.heads * at.dim_s, 128) ||
+        !make_head_map(&a.k, at.cache, at.dim_s, at.kv_heads, at.max_seq, at.dim_s, (long long)at.kv_heads * at.dim_s, kFlashKeys) ||
+        !make_tile_map(&a.v, vt, ldv, at.kv_heads * at.dim, 1, ldv, (long long)at.kv_heads * at.dim * ldv, a.cols))
+        return cudaErrorInvalidValue;
+    static const cudaError_t attr = cudaFuncSetAttribute((const void*)gate_flash_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, flash_smem(2, kFlashCols));
+    if (attr != cudaSuccess) return attr;
+    for (int q0 = 0; q0 < n; q0 += block_rows) {
+        a.row0 = q0; a.rows = std::min(block_rows, n - q0);
+        gate_flash_kernel<<<dim3((a.rows + 127) / 128, at.heads, (at.kv_heads + a.per - 1) / a.per), kThreads, flash_smem(a.kb, a.cols), s>>>(a);
+        gate_mix_kernel<<<a.rows, 256, 0, s>>>(at, a.o, (__nv_bfloat16*)out + (size_t)q0 * ld_out, ld_out);
+        *launches += 2;
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace
+
 bool gate_attn_tc_fits(const GateAttn& at) { return at.heads <= 32; }
 
+size_t gate_attn_tc_bytes(const GateAttn& at, int max_seq, int block_rows) { return bytes_per_row(at, max_seq) * block_rows; }
+
 int gate_attn_tc_rows(const GateAttn& at, int max_seq, int max_rows, size_t budget) {
-    const size_t per = (size_t)at.heads * pad_to(max_seq, 64) * 2;
+    const size_t per = bytes_per_row(at, max_seq);
     int rows = (int)std::min<size_t>(budget / per, (size_t)pad_to(max_rows, 128)) / 128 * 128;
     return rows < 128 ? 128 : rows;
 }
@@ -320,6 +614,7 @@ cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, in
     key_transpose_kernel<<<dim3(ldv / 32, (at.dim + 31) / 32, at.kv_heads), 256, 0, s>>>((const __nv_bfloat16*)at.cache, at.kv_heads, at.dim,
                                                                                        at.dim_s, len, ldv, (__nv_bfloat16*)vt);
     *launches += 1;
+    if (gate_flash_fits(at)) return launch_flash(at, qh, pos0, n, max_rows, weights, block_rows, vt, ldv, out, ld_out, status, launches, s);
     const int hp = at.heads <= 4 ? 4 : at.heads <= 8 ? 8 : at.heads <= 16 ? 16 : 32;
     ScoreArgs a{};
     a.at = at; a.pos0 = pos0; a.w = (__nv_bfloat16*)weights; a.status = status;

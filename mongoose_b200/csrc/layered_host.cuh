@@ -140,7 +140,7 @@ int layered_buffers(Layered& m, F take) {
             const size_t chunks = (T + kMemChunk - 1) / kMemChunk;
             u = std::max(u, chunks * r.heads * r.dim * r.vdim); nu = std::max(nu, chunks * r.heads * r.dim);
             if (l.block_rows) {
-                aw = std::max(aw, (size_t)a.heads * l.block_rows * ldv);
+                aw = std::max(aw, gate_attn_tc_bytes(l.at, c.max_seq, l.block_rows));
                 vt = std::max(vt, (size_t)a.kv_heads * a.dim * ldv);
             }
             part = std::max(part, (size_t)l.splits * a.heads * l.at.dim_s);
@@ -225,7 +225,7 @@ int layered_buffers(Layered& m, F take) {
     get(&m.logits, (size_t)m.logit_rows * c.vocab, 4);
     get(&m.act, (size_t)T * kw, as); get(&m.qh, (size_t)T * hd, as); get(&m.ao, (size_t)T * kat, as);
     get(&m.my, (size_t)T * kmem, as); get(&m.midr, (size_t)T * ff, as); get(&m.fin, (size_t)m.logit_rows * kw, as);
-    get(&m.aw, aw, 2); get(&m.vt, vt, 2); get(&m.keys, keys, 2);
+    get(&m.aw, aw, 1); get(&m.vt, vt, 2); get(&m.keys, keys, 2);
     get(&m.q32, q32, 4); get(&m.cq, (size_t)T * cq, as);
     if (wkv) { get(&m.hr, (size_t)T * W, 4); get(&m.mix, (size_t)5 * T * kw, as); get(&m.decay, (size_t)T * wkv, 4); get(&m.wo, (size_t)T * wkv, 4); get(&m.inner, m.f32 ? 0 : (size_t)T * ld2, 2); get(&m.inner32, (size_t)kThinSlices * T * (ld2 / 2), 4); }
     get(&m.rtr, (size_t)kThinSlices * T * rtr, 4); get(&m.moe.shared_gate, rtr ? T : 0, 4); get(&m.xmid, xmid, as); get(&m.glu, m.f32 ? xmid : 0, 4);
