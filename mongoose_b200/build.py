@@ -26,7 +26,7 @@ LIB_PATH = os.path.join(HERE, LIB_NAME)
 UNITS = {
     "engine.cu": "core",
     "legacy_ops.cu": "abi", "block_ops.cu": "abi",
-    "layered_decode.cu": "layered", "layered_prefill.cu": "layered", "gemm_tc.cu": "layered", "gate_attn_tc.cu": "layered",
+    "layered_decode.cu": "layered", "layered_prefill.cu": "layered", "gemm_tc.cu": "layered", "gemm_f32.cu": "layered", "gate_attn_tc.cu": "layered",
     "latent_attn.cu": "layered", "latent_attn_tc.cu": "layered", "wkv.cu": "layered", "moe.cu": "layered",
     "dense_phases.cu": "dense", "dense_prompt.cu": "dense", "mega_single.cu": "dense", "mega_shared.cu": "dense", "mega_tp.cu": "dense",
 }

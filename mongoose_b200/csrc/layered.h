@@ -211,7 +211,8 @@ cudaError_t launch_moe_combine(const Moe& m, int n, const MoeRows& w, float* z, 
 // `act` buffers hold bf16 or fp32 (f32 = true) rows padded to a multiple of 64 with zeros.
 cudaError_t launch_embed_rows(const WeightView& embed, int ld_embed, const float* pos_tab, const int* tokens, int pos0, int n,
                               int width, float* x, void* act, int ld_act, bool f32, cudaStream_t s);
-// out[n][ldc] = A[n][K] W[rows][K]^T, fp32 on the CUDA cores (32-bit mode, and what is 32-bit in every mode)
+// out[n][ldc] = A[n][K] W[rows][K]^T with fp32 accuracy (32-bit mode; gemm_f32.cu).  lda a multiple of 4, ldw of 8; W is zero
+// from K to ldw.
 enum : int { F32_STORE = 0, F32_GELU = 1,
              F32_SILU_MUL = 2,      // silu(aux) * the product
              F32_DECAY = 3 };       // exp(-exp(tanh(A) W^T + bias))
@@ -225,7 +226,9 @@ struct GemmF32 {
     const float* aux;               // [n][ldc]
     const float* bias;              // [rows]
     const int* group;               // per 128 rows of A: which of the stacked matrices (-1: none); NULL: one matrix
-    long long group_stride;         // elements between the stacked matrices
+    int groups;                     // stacked matrices
+    long long group_stride;         // elements between them
+    int* status;                    // set by a wait that ran out
 };
 cudaError_t launch_gemm_f32(const GemmF32& g, cudaStream_t s);
 // queries: normed, times temperature, score scale and key-norm weight; keys: raw rows into the cache

@@ -752,7 +752,7 @@ int layered_matmul(mg_engine* e, const void* act, int act_rows, int ld, const ui
     if (m.f32) {
         GemmF32 g{};
         g.A = (const float*)act; g.lda = ld; g.W = w; g.ldw = ld; g.out = (float*)out; g.ldc = ldc; g.n = n; g.rows = rows; g.K = ld;
-        g.epi = gelu ? F32_GELU : F32_STORE;
+        g.epi = gelu ? F32_GELU : F32_STORE; g.status = m.status;
         MG_CUDA(e, launch_gemm_f32(g, e->stream));
         return MG_OK;
     }
@@ -818,13 +818,13 @@ int layered_glu(mg_engine* e, const void* act, int act_rows, int ld, const uint8
     if (m.f32) {
         GemmF32 g{};
         g.A = (const float*)act; g.lda = ld; g.W = gate; g.ldw = ld; g.out = m.glu; g.ldc = ffs; g.n = n; g.rows = ff; g.K = ld;
-        g.group = group; g.group_stride = (long long)ff * ld;
+        g.group = group; g.groups = count; g.group_stride = (long long)ff * ld; g.status = m.status;
         MG_CUDA(e, launch_gemm_f32(g, e->stream));
         g.W = up; g.out = (float*)m.xmid; g.epi = F32_SILU_MUL; g.aux = m.glu;
         MG_CUDA(e, launch_gemm_f32(g, e->stream));
         g = GemmF32{};
         g.A = (const float*)m.xmid; g.lda = ffs; g.W = down; g.ldw = ffs; g.out = (float*)z; g.ldc = W; g.n = n; g.rows = W; g.K = ffs;
-        g.group = group; g.group_stride = (long long)W * ffs;
+        g.group = group; g.groups = count; g.group_stride = (long long)W * ffs; g.status = m.status;
         MG_CUDA(e, launch_gemm_f32(g, e->stream));
         return MG_OK;
     }
@@ -910,7 +910,7 @@ int wkv_rows(mg_engine* e, const LayerRun& run, LayerWeights& l, int pos, int n)
     if (m.f32) {
         GemmF32 g{};
         g.A = m.inner32; g.lda = ldi; g.W = l.w2; g.ldw = wk.ld2; g.out = m.decay; g.ldc = d; g.n = n; g.rows = d; g.K = wk.rank;
-        g.epi = F32_DECAY; g.bias = l.w0;
+        g.epi = F32_DECAY; g.bias = l.w0; g.status = m.status;
         MG_CUDA(e, launch_gemm_f32(g, s));
     } else {
         const int ld = 2 * wk.ld2;

@@ -1,4 +1,4 @@
-// Portions of a prompt of a layer-described model: row-wise kernels, the 32-bit matrix product, attention on
+// Portions of a prompt of a layer-described model: row-wise kernels, attention on
 // the CUDA cores (32-bit mode and head counts the tensor-core kernel does not take), and the matrix
 // memory in chunked form: every chunk's contribution in parallel, one pass over the chunks, then every
 // chunk's outputs in parallel.
@@ -17,68 +17,6 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(WeightView embed, int l
         x[(size_t)r * width + i] = v;
         from_f32(v, act + (size_t)r * ld_act + i);
     }
-}
-
-// 64 x 64 tile, 16 columns of K per step, 4 x 4 outputs per thread.  W's rows are padded with zeros to a multiple
-// of 16 at least; A's columns from K on are not read.
-__global__ void __launch_bounds__(256) gemm_f32_kernel(const GemmF32 g) {
-    __shared__ __align__(16) float As[16][68], Ws[16][68];
-    const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
-    const __nv_bfloat16* W = reinterpret_cast<const __nv_bfloat16*>(g.W);
-    if (g.group) {
-        const int e = g.group[r0 / 128];
-        if (e < 0) return;
-        W += e * g.group_stride;
-    }
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 4;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < g.K; k0 += 16) {
-        float a4[4] = {0.f, 0.f, 0.f, 0.f};
-        float2 w0 = make_float2(0.f, 0.f), w1 = w0;
-        if (r0 + lr < g.n) {
-            const float* ap = g.A + (size_t)(r0 + lr) * g.lda + k0 + lk;
-            if (k0 + lk + 4 <= g.K) {
-                const float4 av = *reinterpret_cast<const float4*>(ap);
-                a4[0] = av.x; a4[1] = av.y; a4[2] = av.z; a4[3] = av.w;
-            } else {
-                for (int i = 0; i < 4; i++)
-                    if (k0 + lk + i < g.K) a4[i] = ap[i];
-            }
-            if (g.epi == F32_DECAY)
-                for (int i = 0; i < 4; i++) a4[i] = tanhf(a4[i]);
-        }
-        if (c0 + lr < g.rows) {
-            const __nv_bfloat16* wp = W + (size_t)(c0 + lr) * g.ldw + k0 + lk;
-            w0 = pair_f32(wp);
-            w1 = pair_f32(wp + 2);
-        }
-        As[lk][lr] = a4[0]; As[lk + 1][lr] = a4[1]; As[lk + 2][lr] = a4[2]; As[lk + 3][lr] = a4[3];
-        Ws[lk][lr] = w0.x; Ws[lk + 1][lr] = w0.y; Ws[lk + 2][lr] = w1.x; Ws[lk + 3][lr] = w1.y;
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const float4 a = *reinterpret_cast<const float4*>(&As[k][ty * 4]), w = *reinterpret_cast<const float4*>(&Ws[k][tx * 4]);
-            const float aa[4] = {a.x, a.y, a.z, a.w}, ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(aa[i], ww[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int r = r0 + ty * 4 + i, c = c0 + tx * 4 + j;
-            if (r >= g.n || c >= g.rows) continue;
-            float v = acc[i][j];
-            if (g.epi == F32_GELU) v = gelu_tanh(v);
-            else if (g.epi == F32_SILU_MUL) v *= silu(g.aux[(size_t)r * g.ldc + c]);
-            else if (g.epi == F32_DECAY) v = expf(-expf(v + g.bias[c]));
-            g.out[(size_t)r * g.ldc + c] = v;
-        }
 }
 
 // One warp per (token, query head or key head).
@@ -551,11 +489,6 @@ cudaError_t launch_embed_rows(const WeightView& embed, int ld_embed, const float
                               int width, float* x, void* act, int ld_act, bool f32, cudaStream_t s) {
     if (f32) embed_rows_kernel<float><<<n, 256, 0, s>>>(embed, ld_embed, pos_tab, tokens, pos0, width, x, (float*)act, ld_act);
     else embed_rows_kernel<__nv_bfloat16><<<n, 256, 0, s>>>(embed, ld_embed, pos_tab, tokens, pos0, width, x, (__nv_bfloat16*)act, ld_act);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_gemm_f32(const GemmF32& g, cudaStream_t s) {
-    gemm_f32_kernel<<<dim3((g.rows + 63) / 64, (g.n + 63) / 64), 256, 0, s>>>(g);
     return cudaGetLastError();
 }
 
