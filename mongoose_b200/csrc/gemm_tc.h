@@ -19,9 +19,9 @@ bool make_head_map(CUtensorMap* map, const void* base, int k, int batch, int row
                    int box_rows);
 
 struct GemmTC {
-    CUtensorMap a, b;       // a: boxes of 128 rows; b: boxes of `bn` rows (64 for GEMM_SILU_BF16)
-    CUtensorMap b2;         // GEMM_SILU_BF16: the second matrix, boxes of 64 rows
-    int bn;                 // 64 or 128; GEMM_SILU_BF16: 128, n in steps of 64
+    CUtensorMap a, b;       // a: boxes of 128 rows; b: boxes of `bn` rows (bn / 2 for GEMM_SILU_BF16)
+    CUtensorMap b2;         // GEMM_SILU_BF16: the second matrix, boxes of bn / 2 rows
+    int bn;                 // columns of a tile, 64, 128 or 256 (gemm_tc_bn); GEMM_SILU_BF16: 128 or 256, half of them of each matrix
     int m, n, k;            // out[m][n], k columns (rounded up to 64 inside)
     int b_steps;            // > 0: b has this many steps of 64 columns, a several times as many: a = [a1 a2 ..] multiplies [b b ..]
     const float* bias;      // [n], GEMM_DECAY_F32
@@ -33,6 +33,8 @@ struct GemmTC {
     int mode;
     int* status;
 };
+// The width of tile for m x n results of each of `batch` products.
+int gemm_tc_bn(int m, int n, int batch);
 cudaError_t launch_gemm_tc(const GemmTC& g, cudaStream_t s);
 
 }  // namespace mg

@@ -262,14 +262,14 @@ cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0
     GemmTC g{};
     g.batch = 1; g.b_group = 1; g.causal_pos0 = -1; g.k = at.ld; g.mode = GEMM_BF16; g.status = status;
     // keys[len][heads * dim_s] = c U_k^T
-    g.m = len; g.n = at.heads * at.dim_s; g.bn = g.n > 64 ? 128 : 64; g.out = keys; g.ldc = g.n;
+    g.m = len; g.n = at.heads * at.dim_s; g.bn = gemm_tc_bn(g.m, g.n, 1); g.out = keys; g.ldc = g.n;
     if (!make_tile_map(&g.a, at.cache, at.rank_s, at.max_seq, 1, at.row(), (long long)at.max_seq * at.row(), 128) ||
         !make_tile_map(&g.b, at.uk, at.ld, g.n, 1, at.ld, (long long)g.n * at.ld, g.bn))
         return cudaErrorInvalidValue;
     cudaError_t c = launch_gemm_tc(g, s);
     if (c != cudaSuccess) return c;
     // vt[heads * vdim][len] = U_v c^T
-    g.m = at.heads * at.vdim; g.n = len; g.bn = len > 64 ? 128 : 64; g.out = vt; g.ldc = ldv;
+    g.m = at.heads * at.vdim; g.n = len; g.bn = gemm_tc_bn(g.m, g.n, 1); g.out = vt; g.ldc = ldv;
     if (!make_tile_map(&g.a, at.uv, at.ld, g.m, 1, at.ld, (long long)g.m * at.ld, 128) ||
         !make_tile_map(&g.b, at.cache, at.rank_s, at.max_seq, 1, at.row(), (long long)at.max_seq * at.row(), g.bn))
         return cudaErrorInvalidValue;

@@ -757,7 +757,7 @@ int layered_matmul(mg_engine* e, const void* act, int act_rows, int ld, const ui
         return MG_OK;
     }
     GemmTC g{};
-    g.bn = rows > 64 ? 128 : 64;
+    g.bn = gemm_tc_bn(n, rows, 1);
     if (!make_tile_map(&g.a, act, ld, act_rows, 1, ld, (long long)act_rows * ld, 128) ||
         !make_tile_map(&g.b, w, ld, rows, 1, ld, (long long)rows * ld, g.bn))
         return fail(e, MG_ERR_CUDA, "tensor map of a %d x %d product failed", rows, ld);
@@ -779,7 +779,7 @@ int layered_matmul_batch(mg_engine* e, const void* act, long long stride, int ac
     }
     e->launches += 1;
     GemmTC g{};
-    g.bn = rows > 64 ? 128 : 64;
+    g.bn = gemm_tc_bn(n, rows, count);
     if (!make_tile_map(&g.a, act, ld, act_rows, count, ld, stride, 128) || !make_tile_map(&g.b, w, ld, rows, count, ld, (long long)rows * ld, g.bn))
         return fail(e, MG_ERR_CUDA, "tensor map of %d %d x %d products failed", count, rows, ld);
     g.m = n; g.n = rows; g.k = ld; g.batch = count; g.b_group = 1; g.causal_pos0 = -1;
@@ -829,13 +829,13 @@ int layered_glu(mg_engine* e, const void* act, int act_rows, int ld, const uint8
         return MG_OK;
     }
     GemmTC g{};
-    g.bn = 128; g.m = n; g.n = ff; g.k = ld; g.batch = 1; g.b_group = 1; g.causal_pos0 = -1; g.group = group;
+    g.bn = std::max(128, gemm_tc_bn(n, 2 * ff, 1)); g.m = n; g.n = ff; g.k = ld; g.batch = 1; g.b_group = 1; g.causal_pos0 = -1; g.group = group;
     g.out = m.xmid; g.ldc = ffs; g.mode = GEMM_SILU_BF16; g.status = m.status;
     if (!make_tile_map(&g.a, act, ld, act_rows, 1, ld, (long long)act_rows * ld, 128) ||
-        !make_tile_map(&g.b, gate, ld, ff, count, ld, (long long)ff * ld, 64) || !make_tile_map(&g.b2, up, ld, ff, count, ld, (long long)ff * ld, 64))
+        !make_tile_map(&g.b, gate, ld, ff, count, ld, (long long)ff * ld, g.bn / 2) || !make_tile_map(&g.b2, up, ld, ff, count, ld, (long long)ff * ld, g.bn / 2))
         return fail(e, MG_ERR_CUDA, "tensor map of a %d x %d feed-forward failed", ff, ld);
     MG_CUDA(e, launch_gemm_tc(g, e->stream));
-    g.bn = W > 64 ? 128 : 64; g.n = W; g.k = ffs; g.out = z; g.ldc = W; g.mode = z_act ? GEMM_BF16 : GEMM_F32;
+    g.bn = gemm_tc_bn(n, W, 1); g.n = W; g.k = ffs; g.out = z; g.ldc = W; g.mode = z_act ? GEMM_BF16 : GEMM_F32;
     if (!make_tile_map(&g.a, m.xmid, ffs, act_rows, 1, ffs, (long long)act_rows * ffs, 128) ||
         !make_tile_map(&g.b, down, ffs, W, count, ffs, (long long)W * ffs, g.bn))
         return fail(e, MG_ERR_CUDA, "tensor map of a %d x %d feed-forward failed", W, ffs);
@@ -916,7 +916,7 @@ int wkv_rows(mg_engine* e, const LayerRun& run, LayerWeights& l, int pos, int n)
         const int ld = 2 * wk.ld2;
         MG_CUDA(e, launch_wkv_inner(m.inner32, ldi, slices, wk.rank, n, m.inner, ld, s));
         GemmTC g{};
-        g.bn = d > 64 ? 128 : 64;
+        g.bn = gemm_tc_bn(n, d, 1);
         if (!make_tile_map(&g.a, m.inner, ld, m.max_rows, 1, ld, (long long)m.max_rows * ld, 128) ||
             !make_tile_map(&g.b, l.w2, wk.ld2, d, 1, wk.ld2, (long long)d * wk.ld2, g.bn))
             return fail(e, MG_ERR_CUDA, "tensor map of a %d x %d product failed", d, ld);
