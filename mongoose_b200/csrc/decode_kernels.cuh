@@ -597,13 +597,48 @@ __device__ __forceinline__ void load_stage(const Tile<EPI, R>& t, int c, bool va
     }
 }
 
+// CTA-level argmax of the threads' keys, one atomic per CTA, last CTA advances the cursor.  `sbest`: a word of
+// shared memory per warp.  All threads call.
+__device__ __forceinline__ void publish_best(const PhaseArgs& a, unsigned long long best, unsigned long long* sbest, int nblocks) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long other = __shfl_xor_sync(MG_FULL_MASK, best, o);
+        best = other > best ? other : best;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sbest[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    unsigned long long b = sbest[0];
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) b = sbest[w] > b ? sbest[w] : b;
+    StepState* s = a.st;
+    if (b) atomicMax(&s->best, b);
+    __threadfence();
+    const unsigned int ticket = atomicAdd(&s->done, 1u);
+    if (ticket != (unsigned)nblocks - 1) return;
+    if (a.defer_finalize) {
+        s->done = 0u;
+        return;
+    }
+    __threadfence();
+    const unsigned long long key = atomicMax(&s->best, 0ull);
+    const int tok = (int)(0xffffffffu - (unsigned int)(key & 0xffffffffull));
+    if (a.out_tokens && s->step < s->out_cap) a.out_tokens[s->step] = tok;
+    s->token = tok;
+    s->step += 1;
+    s->pos += 1;
+    s->best = 0ull;
+    s->done = 0u;
+}
+
 // ---------------------------------------------------------------------
 // The phase kernel.  R rows per tile, D pipeline stages per warp.
 // Dynamic shared memory: K floats (x) + 40 floats (reductions).
 // ---------------------------------------------------------------------
 template <int FMT, int EPI, int R, int D>
-__device__ __forceinline__ void phase_body(const PhaseArgs& a, const int bid, const int nblocks, const bool keep) {
+__global__ void __launch_bounds__(256) phase_kernel(const PhaseArgs a) {
     using C = Chunk<FMT>;
+    const int bid = blockIdx.x, nblocks = gridDim.x;
     extern __shared__ __align__(16) float smem[];
     float* xs = smem;
     float* red = smem + a.K;
@@ -638,10 +673,9 @@ __device__ __forceinline__ void phase_body(const PhaseArgs& a, const int bid, co
     pdl_launch_dependents();
     pdl_wait();
 
-    constexpr bool kInt = (FMT != FMT_F16 && FMT != FMT_BF16);          // int8 / 4-bit weights: integer dot products
+    constexpr bool kInt = FMT != FMT_F16;          // int8 / 4-bit weights: integer dot products
     float rms = 1.0f;
     if (kInt) rms = stage_xq(a, reinterpret_cast<uint8_t*>(smem), red, FMT == FMT_Q4_0);
-    else if (FMT == FMT_BF16) stage_layered(a, xs, red, keep);
     else stage_x(a, xs, red);
     const uint8_t* P0 = reinterpret_cast<const uint8_t*>(smem);
     const uint8_t* P1 = P0 + a.K;
@@ -769,14 +803,6 @@ __device__ __forceinline__ void phase_body(const PhaseArgs& a, const int bid, co
                                 }
                             }
                         }
-                    } else if (EPI == EPI_STORE || EPI == EPI_GELU) {
-                        if (lane == 0) {
-#pragma unroll
-                            for (int r = 0; r < R; r++) {
-                                const int row = it * R + r;
-                                if (row < a.rows[0]) a.out[row] = EPI == EPI_GELU ? gelu_tanh(acc[r]) : acc[r];
-                            }
-                        }
                     } else {  // EPI_LOGITS
                         if (lane == 0) {
 #pragma unroll
@@ -815,67 +841,8 @@ __device__ __forceinline__ void phase_body(const PhaseArgs& a, const int bid, co
     }
 
     if (EPI == EPI_LOGITS) {
-        // CTA-level argmax, one atomic per CTA, last CTA advances the cursor.
-        unsigned long long* sbest = reinterpret_cast<unsigned long long*>(red);   // 8-byte aligned: K is a multiple of 32
-        __syncthreads();
-        if (lane == 0) sbest[threadIdx.x >> 5] = best;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long b = sbest[0];
-            for (int w = 1; w < wpc; w++) b = sbest[w] > b ? sbest[w] : b;
-            StepState* s = a.st;
-            if (b) atomicMax(&s->best, b);
-            __threadfence();
-            const unsigned int ticket = atomicAdd(&s->done, 1u);
-            if (ticket == (unsigned)nblocks - 1 && a.defer_finalize) {
-                s->done = 0u;
-            } else if (ticket == (unsigned)nblocks - 1) {
-                __threadfence();
-                const unsigned long long key = atomicMax(&s->best, 0ull);
-                const int tok = (int)(0xffffffffu - (unsigned int)(key & 0xffffffffull));
-                if (a.out_tokens && s->step < s->out_cap) a.out_tokens[s->step] = tok;
-                s->token = tok;
-                s->step += 1;
-                s->pos += 1;
-                s->best = 0ull;
-                s->done = 0u;
-            }
-        }
+        publish_best(a, best, reinterpret_cast<unsigned long long*>(red), nblocks);      // 8-byte aligned: K is a multiple of 32
     }
-}
-
-template <int FMT, int EPI, int R, int D>
-__global__ void __launch_bounds__(256) phase_kernel(const PhaseArgs a) {
-    phase_body<FMT, EPI, R, D>(a, blockIdx.x, gridDim.x, blockIdx.x == 0);
-}
-
-// Two independent matrices in one launch: the first `split` CTAs multiply a's, the others b's.
-template <int FMT, int EPI, int R, int D>
-__global__ void __launch_bounds__(256) phase_pair_kernel(const PhaseArgs a, const PhaseArgs b, int split) {
-    const bool first = (int)blockIdx.x < split;
-    phase_body<FMT, EPI, R, D>(first ? a : b, first ? blockIdx.x : blockIdx.x - split, first ? split : gridDim.x - split, first ? blockIdx.x == 0 : (int)blockIdx.x == split);
-}
-
-// Several matrices on mixes of one vector: part p's CTAs multiply its matrix by the mix with its own mu.
-constexpr int kMaxParts = 5;
-struct PhaseParts {
-    int n;
-    int first[kMaxParts + 1];   // CTAs [first[p], first[p + 1])
-    WeightView w[kMaxParts];
-    int rows[kMaxParts];
-    const float* mu[kMaxParts];
-    float* out[kMaxParts];
-};
-
-template <int FMT, int EPI, int R, int D>
-__global__ void __launch_bounds__(256) phase_parts_kernel(const PhaseArgs a, const PhaseParts parts) {
-    int p = 0;
-#pragma unroll
-    for (int i = 1; i < kMaxParts; i++)
-        if (i < parts.n && (int)blockIdx.x >= parts.first[i]) p = i;
-    PhaseArgs b = a;
-    b.w[0] = parts.w[p]; b.rows[0] = parts.rows[p]; b.nitems = (parts.rows[p] + R - 1) / R; b.mix_mu = parts.mu[p]; b.out = parts.out[p];
-    phase_body<FMT, EPI, R, D>(b, blockIdx.x - parts.first[p], parts.first[p + 1] - parts.first[p], blockIdx.x == 0);
 }
 
 // Sum of the received rows into a plain vector (the hidden state a layer range hands back to the

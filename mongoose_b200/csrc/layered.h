@@ -92,15 +92,22 @@ struct Moe {
 constexpr int kMaxExperts = 1024, kMaxTop = 64;
 
 // ---- one token (layered_decode.cu) -------------------------------------------------------------
-phase_fn_t layered_phase(int epi, int R);
-typedef void (*phase_pair_fn_t)(const PhaseArgs, const PhaseArgs, int);
-phase_pair_fn_t layered_phase_pair(int R);
-
-typedef void (*phase_parts_fn_t)(const PhaseArgs, const PhaseParts);
-phase_parts_fn_t layered_phase_parts(int R);
-
-// Largest dynamic shared memory the phase kernels may be launched with.
-cudaError_t layered_phase_smem(size_t bytes);
+// Products with bf16 matrices (layered_rows.cuh), K a multiple of 64.
+cudaError_t rows_attrs(int K);          // for rows of up to K columns
+cudaError_t launch_rows(const PhaseArgs& a, int epi, int sms, bool pdl, cudaStream_t s);
+// two independent matrices
+cudaError_t launch_rows_pair(const PhaseArgs& a, const PhaseArgs& b, int sms, bool pdl, cudaStream_t s);
+// Several matrices on mixes of one vector, each by its own mu.
+constexpr int kMaxParts = 5;
+struct PhaseParts {
+    int n;
+    int first[kMaxParts + 1];   // CTAs [first[p], first[p + 1]), filled in by the launch
+    WeightView w[kMaxParts];
+    int rows[kMaxParts];
+    const float* mu[kMaxParts];
+    float* out[kMaxParts];
+};
+cudaError_t launch_rows_parts(const PhaseArgs& a, PhaseParts& p, int sms, bool pdl, cudaStream_t s);
 
 struct MixerStep {
     GateAttn at;

@@ -1,27 +1,12 @@
-// One token of a layer-described model: bf16 instances of the phase kernels, and the mixer step, in
+// One token of a layer-described model: products, and the mixer step, in
 // which the attention branch (split over keys) and the matrix-memory branch run side by side.
-#include "kernel_table.h"
+#include <algorithm>
+#include <type_traits>
+
 #include "layered_ops.cuh"
+#include "layered_rows.cuh"
 
 namespace mg {
-
-phase_fn_t layered_phase(int epi, int R) {
-    switch (epi) {
-        case EPI_GELU:
-            return R == 4 ? phase_kernel<FMT_BF16, EPI_GELU, 4, 2> : R == 2 ? phase_kernel<FMT_BF16, EPI_GELU, 2, 4> : phase_kernel<FMT_BF16, EPI_GELU, 1, 8>;
-        case EPI_LOGITS: return phase_kernel<FMT_BF16, EPI_LOGITS, 4, 2>;
-        default:
-            return R == 4 ? phase_kernel<FMT_BF16, EPI_STORE, 4, 2> : R == 2 ? phase_kernel<FMT_BF16, EPI_STORE, 2, 4> : phase_kernel<FMT_BF16, EPI_STORE, 1, 8>;
-    }
-}
-
-phase_pair_fn_t layered_phase_pair(int R) {
-    return R == 4 ? phase_pair_kernel<FMT_BF16, EPI_STORE, 4, 2> : R == 2 ? phase_pair_kernel<FMT_BF16, EPI_STORE, 2, 4> : phase_pair_kernel<FMT_BF16, EPI_STORE, 1, 8>;
-}
-
-phase_parts_fn_t layered_phase_parts(int R) {
-    return R == 4 ? phase_parts_kernel<FMT_BF16, EPI_STORE, 4, 2> : R == 2 ? phase_parts_kernel<FMT_BF16, EPI_STORE, 2, 4> : phase_parts_kernel<FMT_BF16, EPI_STORE, 1, 8>;
-}
 
 namespace {
 
@@ -202,18 +187,72 @@ cudaError_t step_for(const MixerStep& a, size_t smem, bool pdl, cudaStream_t s) 
 
 }  // namespace
 
-cudaError_t layered_phase_smem(size_t bytes) {
-    for (int R = 1; R <= 4; R *= 2) {
-        for (int epi : {EPI_STORE, EPI_GELU, EPI_LOGITS}) {
-            cudaError_t c = cudaFuncSetAttribute((const void*)layered_phase(epi, R), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+namespace {
+
+template <typename F>
+cudaError_t by_rows(int R, int K, F f) {
+    auto go = [&](auto r, auto ahead) { return f(r, ahead); };
+    using std::integral_constant;
+    if (K <= 2048)
+        return R == 8 ? go(integral_constant<int, 8>{}, integral_constant<int, 1>{}) : R == 4 ? go(integral_constant<int, 4>{}, integral_constant<int, 1>{})
+             : R == 2 ? go(integral_constant<int, 2>{}, integral_constant<int, 1>{}) : go(integral_constant<int, 1>{}, integral_constant<int, 1>{});
+    return R == 4 ? go(integral_constant<int, 4>{}, integral_constant<int, 3>{}) : R == 2 ? go(integral_constant<int, 2>{}, integral_constant<int, 3>{})
+                  : go(integral_constant<int, 1>{}, integral_constant<int, 3>{});
+}
+inline size_t rows_smem(int K) { return ((size_t)K + 72) * sizeof(float); }
+inline int rows_grid(int K, int rows, int R, int most) {
+    const int per = R * (kRowThreads / row_group(K));
+    return std::max(1, std::min((rows + per - 1) / per, most));
+}
+
+}  // namespace
+
+cudaError_t rows_attrs(int K) {
+    const int bytes = (int)rows_smem(K);
+    auto allow = [&](const void* kern) { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+    for (int k : {2048, 4096})
+        for (int R : {1, 2, 4, 8}) {
+            const cudaError_t c = by_rows(R, k, [&](auto r, auto ahead) {
+                constexpr int RR = decltype(r)::value, A = decltype(ahead)::value;
+                for (const void* f : {(const void*)rows_kernel<EPI_STORE, RR, A>, (const void*)rows_kernel<EPI_GELU, RR, A>, (const void*)rows_kernel<EPI_LOGITS, RR, A>,
+                                      (const void*)rows_pair_kernel<RR, A>, (const void*)rows_parts_kernel<RR, A>})
+                    if (cudaError_t e = allow(f)) return e;
+                return cudaSuccess;
+            });
             if (c != cudaSuccess) return c;
         }
-        for (const void* f : {(const void*)layered_phase_pair(R), (const void*)layered_phase_parts(R)}) {
-            cudaError_t c = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (c != cudaSuccess) return c;
-        }
-    }
     return cudaSuccess;
+}
+
+cudaError_t launch_rows(const PhaseArgs& a, int epi, int sms, bool pdl, cudaStream_t s) {
+    const int R = rows_at_a_time(a.K, a.rows[0], sms);
+    return by_rows(R, a.K, [&](auto r, auto ahead) {
+        constexpr int RR = decltype(r)::value, A = decltype(ahead)::value;
+        auto kern = epi == EPI_GELU ? rows_kernel<EPI_GELU, RR, A> : epi == EPI_LOGITS ? rows_kernel<EPI_LOGITS, RR, A> : rows_kernel<EPI_STORE, RR, A>;
+        return launch_pdl(kern, rows_grid(a.K, a.rows[0], R, 2 * sms), kRowThreads, rows_smem(a.K), pdl, s, a);
+    });
+}
+
+cudaError_t launch_rows_pair(const PhaseArgs& a, const PhaseArgs& b, int sms, bool pdl, cudaStream_t s) {
+    const int K = std::max(a.K, b.K);
+    const int R = rows_at_a_time(K, a.rows[0] + b.rows[0], sms);
+    // CTAs in proportion to the bytes
+    const long long wa = (long long)a.rows[0] * a.K, wb = (long long)b.rows[0] * b.K;
+    const int most = (int)std::max(1ll, std::min(2ll * sms - 1, (wa * 2 * sms + (wa + wb) / 2) / (wa + wb)));
+    const int ga = rows_grid(a.K, a.rows[0], R, most), gb = rows_grid(b.K, b.rows[0], R, 2 * sms - most);
+    return by_rows(R, K, [&](auto r, auto ahead) {
+        return launch_pdl(rows_pair_kernel<decltype(r)::value, decltype(ahead)::value>, ga + gb, kRowThreads, rows_smem(K), pdl, s, a, b, ga);
+    });
+}
+
+cudaError_t launch_rows_parts(const PhaseArgs& a, PhaseParts& p, int sms, bool pdl, cudaStream_t s) {
+    long long all = 0;
+    for (int k = 0; k < p.n; k++) all += p.rows[k];
+    const int R = rows_at_a_time(a.K, all, sms);
+    for (int k = 0; k < p.n; k++) p.first[k + 1] = p.first[k] + rows_grid(a.K, p.rows[k], R, std::max(1, (int)(2ll * sms * p.rows[k] / all)));
+    return by_rows(R, a.K, [&](auto r, auto ahead) {
+        return launch_pdl(rows_parts_kernel<decltype(r)::value, decltype(ahead)::value>, p.first[p.n], kRowThreads, rows_smem(a.K), pdl, s, a, p);
+    });
 }
 
 size_t mixer_step_smem(const GateAttn& at, const MatMem& mem, bool f32_cache, int* tile) {

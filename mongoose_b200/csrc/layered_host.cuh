@@ -330,7 +330,7 @@ int layered_shapes(Layered& m, int sms, std::string* why) {
     }
     // the phase kernels stage a whole input vector per CTA
     if (kmax > 48 * 1024) { *why = "a matrix with rows of more than 49152 values"; return MG_ERR_UNSUPPORTED; }
-    if (layered_phase_smem(((size_t)kmax + 72) * sizeof(float)) != cudaSuccess) { *why = "kernel attributes"; return MG_ERR_CUDA; }
+    if (rows_attrs(kmax) != cudaSuccess) { *why = "kernel attributes"; return MG_ERR_CUDA; }
     if (moe_smem && moe_step_attrs(moe_smem) != cudaSuccess) { *why = "kernel attributes"; return MG_ERR_CUDA; }
     return MG_OK;
 }
@@ -533,8 +533,6 @@ void layered_reset(mg_engine* e) {
     for (LayerRun& r : e->lm->runs) r.next_pos = 0;
 }
 
-void layered_phase_shape(const mg_engine* e, int nitems, int* grid) { *grid = std::max(1, std::min((nitems + 7) / 8, 2 * e->num_sms)); }
-
 // One token through the layer runs [ls, le) (+ head).  The residual sum after a sublayer is formed by the kernel
 // that next reads it; its CTA 0 stores it into the other of the two hidden buffers, so that the others can
 // still read the old one.  Where layers loop, the embedding is kept in x0 and every pass's input is a store too.
@@ -594,11 +592,8 @@ int enqueue_layered_step(mg_engine* e, cudaStream_t s, int ls, int le, int mode,
         pending = PRO_X;
     };
     auto phase = [&](PhaseArgs& a, int epi) -> int {
-        const int R = epi == EPI_LOGITS ? 4 : pick_rows_per_tile(e, a.rows[0]);
-        a.nitems = (a.rows[0] + R - 1) / R;
-        int grid;
-        layered_phase_shape(e, a.nitems, &grid);
-        MG_CUDA(e, launch(e, s, layered_phase(epi, R), grid, 256, ((size_t)a.K + 72) * sizeof(float), a));
+        MG_CUDA(e, launch_rows(a, epi, e->num_sms, e->use_pdl, s));
+        e->capture_kernels += 1;
         return MG_OK;
     };
     // a matrix on a plain vector, normed first where a weight is given
@@ -627,16 +622,12 @@ int enqueue_layered_step(mg_engine* e, cudaStream_t s, int ls, int le, int mode,
         e->capture_kernels += 2;
         {   // both output projections
             PhaseArgs a{}, b{};
-            const int R = pick_rows_per_tile(e, 2 * W);
             a.pro = b.pro = PRO_X; a.st = b.st = e->st;
             a.x_src = m.attn; a.k_valid = l.kat(); a.K = pad_to(l.kat(), 64); a.w[0] = WeightView{l.at_o, nullptr}; a.out = m.y[0];
             b.x_src = m.mem_y; b.k_valid = l.kmem(); b.K = pad_to(l.kmem(), 64); b.w[0] = WeightView{l.mem_o, nullptr}; b.out = m.y[1];
             a.rows[0] = b.rows[0] = W;
-            a.nitems = b.nitems = (W + R - 1) / R;
-            int ga;
-            layered_phase_shape(e, a.nitems, &ga);
-            const int gb = ga;
-            MG_CUDA(e, launch(e, s, layered_phase_pair(R), ga + gb, 256, ((size_t)std::max(a.K, b.K) + 72) * sizeof(float), a, b, ga));
+            MG_CUDA(e, launch_rows_pair(a, b, e->num_sms, e->use_pdl, s));
+            e->capture_kernels += 1;
         }
         pending = PRO_POST_PAIR; z0 = m.y[0]; z1 = m.y[1]; w0 = l.at_out; w1 = l.mem_out; pw = l.norm1;
         if (l.c.ffn_dim) {
@@ -673,20 +664,17 @@ int enqueue_layered_step(mg_engine* e, cudaStream_t s, int ls, int le, int mode,
         a.mix_prev = run.prev;
         PhaseParts p{};
         p.n = 5;
-        const int R = pick_rows_per_tile(e, l.proj_rows());
         for (int k = 0; k < 5; k++) {
             p.rows[k] = k < 4 ? n : l.wk.rank;
             p.w[k] = WeightView{l.proj + (size_t)k * n * m.kw * 2, nullptr};
             p.out[k] = m.row + (size_t)k * n;
             p.mu[k] = l.mu[k];
-            const int items = (p.rows[k] + R - 1) / R, most = std::max(1, (int)((long long)2 * e->num_sms * p.rows[k] / l.proj_rows()));
-            p.first[k + 1] = p.first[k] + std::max(1, std::min((items + 7) / 8, most));
         }
-        MG_CUDA(e, launch(e, s, layered_phase_parts(R), p.first[5], 256, ((size_t)a.K + 72) * sizeof(float), a, p));
+        MG_CUDA(e, launch_rows_parts(a, p, e->num_sms, e->use_pdl, s));
         WkvStep t{};
         t.wk = run.wk(l); t.row = m.row; t.st = e->st; t.y = m.attn;
         MG_CUDA(e, launch_wkv_step(t, e->use_pdl, s));
-        e->capture_kernels += 1;
+        e->capture_kernels += 2;
         return product(m.attn, n, l.o, W, m.z, nullptr);
     };
 
