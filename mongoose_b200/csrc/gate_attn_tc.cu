@@ -288,11 +288,14 @@ __global__ void __launch_bounds__(kThreads, Geo<HP>::per_sm) gate_scores_kernel(
 // multiplied by the keys first and the heads are mixed in the outputs.  A head then multiplies the keys of
 // EVERY key head, kv_heads times the products, which the tensor cores do not notice, and mixing falls from
 // every (query, key) pair to every query.  A CTA owns 128 queries of one head and up to 256 output columns
-// and walks the keys in tiles of 64: scores into one of two TMEM buffers, sigmoids in fp32 on eight warps,
+// and walks the keys in tiles of 64: scores into one of two TMEM buffers, sigmoids in fp32 on sixteen warps
+// (a row's 64 keys belong to four threads: a sigmoid is a chain of a dozen instructions; with eight warps, 139 us
+// and 34 % tensor-pipe activity for 2048 queries of 32 heads, with sixteen 122 us),
 // weights as two bf16 parts, high and low, into one of two shared-memory buffers, O += (P_high + P_low) V
 // in TMEM.  The weights carry 16 bits of mantissa into an fp32 sum and are never rounded to 8.
 constexpr int kFlashKeys = 64;
 constexpr int kFlashCols = 256;
+constexpr int kFlashThreads = 576;         // TMA warp, MMA warp, 16 sigmoid warps
 
 struct FlashArgs {
     CUtensorMap q, k, v;            // [rows][heads][dim_s] in boxes of 128 rows; [max_seq][kv][dim_s], 64 rows; [kv * dim][ldv], `cols` rows
@@ -307,7 +310,18 @@ struct FlashArgs {
 
 constexpr int flash_smem(int kb, int cols) { return kb * 128 * 128 + 4 * 128 * 128 + 2 * kb * kFlashKeys * 128 + 2 * ((cols * 128 + 1023) & ~1023) + 1024 + 256 + 8 * 2 * 32 * 4; }
 
-__global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_constant__ FlashArgs a) {
+__device__ __forceinline__ void tmem_load16(uint32_t addr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(addr));
+    tmem_wait_load();
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+
+__global__ void __launch_bounds__(kFlashThreads, 1) gate_flash_kernel(const __grid_constant__ FlashArgs a) {
     extern __shared__ uint8_t raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
     const GateAttn& A = a.at;
@@ -320,7 +334,7 @@ __global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_const
     uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = bars + 3, *v_full = bars + 5, *v_empty = bars + 7, *s_full = bars + 9, *p_empty = bars + 11,
              *s_empty = bars + 13, *p_full = bars + 15;
     uint32_t* tmem_base = reinterpret_cast<uint32_t*>(bars + 17);
-    float* rms = reinterpret_cast<float*>(Vs + 2 * vbytes + 256);               // [warp][2][32]: -log2 e / rms of the warp's keys
+    float* rms = reinterpret_cast<float*>(Vs + 2 * vbytes + 256);               // [warp][2][16]: -log2 e / rms of the warp's keys
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = blockIdx.y, c = h / (A.heads / A.kv_heads), c0 = blockIdx.z * a.per;
@@ -330,7 +344,7 @@ __global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_const
     const int tiles = last / kFlashKeys + 1;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 17; i++) bar_init(bars + i, i >= 13 ? 8 : 1);
+        for (int i = 0; i < 17; i++) bar_init(bars + i, i >= 13 ? 16 : 1);
         bar_init_fence();
         tma_prefetch_map(&a.q); tma_prefetch_map(&a.k); tma_prefetch_map(&a.v);
     }
@@ -399,42 +413,42 @@ __global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_const
         __syncwarp();
     } else {
         constexpr float kLog2e = 1.4426950408889634f;
-        const int quarter = warp & 3, half = (warp - 2) >> 2, r = quarter * 32 + lane;
+        const int quarter = warp & 3, part = (warp - 2) >> 2, r = quarter * 32 + lane;
         const uint32_t mine = (uint32_t)(quarter * 32) << 16;
         const float slope = A.slopes[h] * kLog2e, bias = -A.head_bias[h] * kLog2e;
-        float* kr = rms + (warp - 2) * 64;
+        float* kr = rms + (warp - 2) * 32;
         auto key_rms = [&](int j) {
-            const int key = j * kFlashKeys + half * 32 + lane;
+            const int key = j * kFlashKeys + part * 16 + (lane & 15);
             return key <= last ? -kLog2e * A.cache_r[(size_t)key * A.kv_heads + c] : 0.f;
         };
         const int pos = first + r;
         float next = key_rms(0);
         bool ok = true;
         for (int j = 0; j < tiles; j++) {
-            const int b = j & 1, k0 = j * kFlashKeys + half * 32;
-            kr[b * 32 + lane] = next;
+            const int b = j & 1, k0 = j * kFlashKeys + part * 16;
+            if (lane < 16) kr[b * 16 + lane] = next;
             __syncwarp();
             if (j + 1 < tiles) next = key_rms(j + 1);
             ok = __all_sync(MG_FULL_MASK, bar_wait(s_full + b, (j >> 1) & 1, a.status));
             if (!ok) break;
             tc_fence_after();
-            float s[32];
-            tmem_load32(S0 + mine + b * kFlashKeys + half * 32, s);
+            float s[16];
+            tmem_load16(S0 + mine + b * kFlashKeys + part * 16, s);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) bar_arrive(s_empty + b);
-            const int seen = pos - k0 + 1;                  // keys of this half that the row sees
-            const bool cut = __any_sync(MG_FULL_MASK, seen < 32);
+            const int seen = pos - k0 + 1;                  // keys of this part that the row sees
+            const bool cut = __any_sync(MG_FULL_MASK, seen < 16);
             if (cut) {                                      // rows of the cache behind the query hold anything
 #pragma unroll
-                for (int i = 0; i < 32; i++)
+                for (int i = 0; i < 16; i++)
                     if (i >= seen) s[i] = 0.f;
             }
             // 1 / (1 + 2^t), two at a time: 1 / x = y / (x y).  Exponents are cut off at 60, where a weight is 2^-60.
             const float line = fmaf(slope, (float)(pos - k0), bias);
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-                const float4 k4 = *reinterpret_cast<const float4*>(kr + b * 32 + i);
+            for (int i = 0; i < 16; i += 4) {
+                const float4 k4 = *reinterpret_cast<const float4*>(kr + b * 16 + i);
                 const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
                 float e[4];
 #pragma unroll
@@ -454,7 +468,7 @@ __global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_const
             }
             if (cut) {
 #pragma unroll
-                for (int i = 0; i < 32; i++)
+                for (int i = 0; i < 16; i++)
                     if (i >= seen) s[i] = 0.f;
             }
             if (j >= 2) {
@@ -463,7 +477,7 @@ __global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_const
             }
             uint8_t* high = P + b * 2 * 128 * 128 + r * 128;
 #pragma unroll
-            for (int x = 0; x < 4; x++) {
+            for (int x = 0; x < 2; x++) {
                 uint32_t w[4], u[4];
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
@@ -471,7 +485,7 @@ __global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_const
                     w[i] = bf16_pair(p, q);
                     u[i] = bf16_pair(p - __uint_as_float(w[i] << 16), q - __uint_as_float(w[i] & 0xffff0000u));
                 }
-                const int at = ((half * 4 + x) ^ (r & 7)) << 4;
+                const int at = ((part * 2 + x) ^ (r & 7)) << 4;
                 *reinterpret_cast<uint4*>(high + at) = make_uint4(w[0], w[1], w[2], w[3]);
                 *reinterpret_cast<uint4*>(high + 128 * 128 + at) = make_uint4(u[0], u[1], u[2], u[3]);
             }
@@ -486,7 +500,7 @@ __global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_const
             const int wide = A.kv_heads * A.dim, cols = min(a.per, A.kv_heads - c0) * A.dim, row = tile_row + r;
             float* out = a.o + ((size_t)row * A.heads + h) * wide + c0 * A.dim;
             const bool vec = (A.dim & 3) == 0;
-            for (int x = half * 32; x < cols; x += 64) {
+            for (int x = part * 32; x < cols; x += 128) {
                 float o[32];
                 tmem_load32(O + mine + x, o);
                 if (row < a.rows) {
@@ -511,31 +525,54 @@ __global__ void __launch_bounds__(kThreads) gate_flash_kernel(const __grid_const
     if (warp == 1) tmem_free(S0, a.tmem_cols);
 }
 
-// out[row][h][d] = sum over g of T[h][g] o[row][g][key head of h][d]: a CTA per row, every element of o read once, eight heads
-// of a group at a time.
-__global__ void __launch_bounds__(256) gate_mix_kernel(GateAttn A, const float* o, __nv_bfloat16* out, int ld_out) {
-    __shared__ __align__(16) float talk[32][32];            // [g][h], heads of a group side by side
-    const int H = A.heads, group = H / A.kv_heads, wide = A.kv_heads * A.dim;
-    for (int i = threadIdx.x; i < 32 * 32; i += 256) {
-        const int h = i & 31, g = i >> 5;
+// out[row][h][d] = sum over g of T[h][g] o[row][g][key head of h][d]: every element of o is read once, V at a time (dim a
+// multiple of V), for eight heads of its group at a time; a CTA takes V rows.
+template <int V>
+__global__ void __launch_bounds__(256) gate_mix_kernel(GateAttn A, int rows, const float* o, __nv_bfloat16* out, int ld_out) {
+    __shared__ __align__(16) float talk[32][36];            // [g][h], heads of a group side by side
+    const int H = A.heads, group = H / A.kv_heads, wide = A.kv_heads * A.dim, units = wide / V;
+    for (int i = threadIdx.x; i < 32 * 36; i += 256) {
+        const int h = i % 36, g = i / 36;
         talk[g][h] = h < H && g < H ? A.talk[h * H + g] : 0.f;
     }
     __syncthreads();
-    const size_t row = blockIdx.x;
-    for (int e = threadIdx.x; e < wide; e += 256) {
-        const int c = e / A.dim, d = e - c * A.dim;
+    const bool quads = (group & 3) == 0;
+    for (int u = threadIdx.x; u < V * units; u += 256) {
+        const size_t row = (size_t)blockIdx.x * V + u / units;
+        if (row >= rows) return;
+        const int e = u % units * V, c = e / A.dim, d = e - c * A.dim;
         const float* p = o + row * H * wide + e;
         for (int h0 = 0; h0 < group; h0 += 8) {
-            float acc[8] = {};
+            const int first = c * group + h0, n = min(8, group - h0);
+            float acc[8][V] = {};
 #pragma unroll 8
             for (int g = 0; g < H; g++) {
-                const float v = p[(size_t)g * wide];
+                float v[V], t[8];
+                if constexpr (V == 2) {
+                    const float2 f = *reinterpret_cast<const float2*>(p + (size_t)g * wide);
+                    v[0] = f.x; v[1] = f.y;
+                } else {
+                    v[0] = p[(size_t)g * wide];
+                }
+                if (quads) {                                // heads past the group are in the row, and not stored
+                    const float4 x = *reinterpret_cast<const float4*>(&talk[g][first]), y = *reinterpret_cast<const float4*>(&talk[g][first + 4]);
+                    t[0] = x.x; t[1] = x.y; t[2] = x.z; t[3] = x.w; t[4] = y.x; t[5] = y.y; t[6] = y.z; t[7] = y.w;
+                } else {
 #pragma unroll
-                for (int i = 0; i < 8; i++) acc[i] = fmaf(talk[g][min(c * group + h0 + i, 31)], v, acc[i]);
+                    for (int i = 0; i < 8; i++) t[i] = talk[g][min(first + i, 35)];
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+#pragma unroll
+                    for (int q = 0; q < V; q++) acc[i][q] = fmaf(t[i], v[q], acc[i][q]);
             }
 #pragma unroll
             for (int i = 0; i < 8; i++)
-                if (h0 + i < group) out[row * ld_out + (size_t)(c * group + h0 + i) * A.dim + d] = __float2bfloat16_rn(acc[i]);
+                if (i < n) {
+                    __nv_bfloat16* to = out + row * ld_out + (size_t)(first + i) * A.dim + d;
+                    if constexpr (V == 2) *reinterpret_cast<__nv_bfloat162*>(to) = __floats2bfloat162_rn(acc[i][0], acc[i][1]);
+                    else *to = __float2bfloat16_rn(acc[i][0]);
+                }
         }
     }
 }
@@ -589,8 +626,10 @@ cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, in
     if (attr != cudaSuccess) return attr;
     for (int q0 = 0; q0 < n; q0 += block_rows) {
         a.row0 = q0; a.rows = std::min(block_rows, n - q0);
-        gate_flash_kernel<<<dim3((a.rows + 127) / 128, at.heads, (at.kv_heads + a.per - 1) / a.per), kThreads, flash_smem(a.kb, a.cols), s>>>(a);
-        gate_mix_kernel<<<a.rows, 256, 0, s>>>(at, a.o, (__nv_bfloat16*)out + (size_t)q0 * ld_out, ld_out);
+        gate_flash_kernel<<<dim3((a.rows + 127) / 128, at.heads, (at.kv_heads + a.per - 1) / a.per), kFlashThreads, flash_smem(a.kb, a.cols), s>>>(a);
+        __nv_bfloat16* to = (__nv_bfloat16*)out + (size_t)q0 * ld_out;
+        if (at.dim % 2 == 0) gate_mix_kernel<2><<<(a.rows + 1) / 2, 256, 0, s>>>(at, a.rows, a.o, to, ld_out);
+        else gate_mix_kernel<1><<<a.rows, 256, 0, s>>>(at, a.rows, a.o, to, ld_out);
         *launches += 2;
     }
     return cudaGetLastError();

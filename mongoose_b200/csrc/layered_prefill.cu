@@ -357,18 +357,28 @@ __global__ void __launch_bounds__(256) mem_chunk_kernel(MatMem M, int k_col, int
     const int t0 = ch * kMemChunk, T = min(kMemChunk, n - t0);
     const double bT = w.b[(size_t)h * n + t0 + T - 1];
     const float mT = w.mm[(size_t)h * n + t0 + T - 1];
-    for (int i = threadIdx.x; i < kMemChunk * 64; i += 256) {
-        const int s = i >> 6, c = i & 63;
-        float k = 0.f, v = 0.f;
-        if (s < T) {
-            const float* row = proj + (size_t)(t0 + s) * ldp;
-            if (d0 + c < M.dim)
-                k = row[k_col + h * M.dim + d0 + c] *
-                    expf((float)(bT - w.b[(size_t)h * n + t0 + s]) + w.ig[(size_t)h * n + t0 + s] - mT);
-            if (v0 + c < M.vdim) v = row[v_col + h * M.vdim + v0 + c];
-        }
-        Ks[s][c] = k;
-        Vs[s][c] = v;
+    // every load at once; a token's factor is formed by one thread, not by each that holds one of its values
+    __shared__ float fs[kMemChunk];
+    constexpr int kLoads = kMemChunk * 64 / 256;
+    const int c = threadIdx.x & 63, s0 = threadIdx.x >> 6;
+    float k[kLoads], v[kLoads];
+#pragma unroll
+    for (int r = 0; r < kLoads; r++) {
+        const int s = s0 + 4 * r;
+        const float* row = proj + (size_t)(t0 + s) * ldp;
+        k[r] = s < T && d0 + c < M.dim ? row[k_col + h * M.dim + d0 + c] : 0.f;
+        v[r] = s < T && v0 + c < M.vdim ? row[v_col + h * M.vdim + v0 + c] : 0.f;
+    }
+    if (threadIdx.x < kMemChunk) {
+        const int s = threadIdx.x;
+        fs[s] = s < T ? expf((float)(bT - w.b[(size_t)h * n + t0 + s]) + w.ig[(size_t)h * n + t0 + s] - mT) : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kLoads; r++) {
+        const int s = s0 + 4 * r;
+        Ks[s][c] = s < T && d0 + c < M.dim ? k[r] * fs[s] : 0.f;
+        Vs[s][c] = v[r];
     }
     __syncthreads();
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -390,9 +400,14 @@ __global__ void __launch_bounds__(256) mem_chunk_kernel(MatMem M, int k_col, int
         const int d = d0 + ty * 4 + i;
         if (d >= M.dim) continue;
         if (v0 == 0 && tx == 0) w.nU[((size_t)ch * M.heads + h) * M.dim + d] = nk[i];
+        float* to = U + (size_t)d * M.vdim + v0 + tx * 4;
+        if ((M.vdim & 3) == 0) {
+            if (v0 + tx * 4 < M.vdim) *reinterpret_cast<float4*>(to) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            continue;
+        }
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            if (v0 + tx * 4 + j < M.vdim) U[(size_t)d * M.vdim + v0 + tx * 4 + j] = acc[i][j];
+            if (v0 + tx * 4 + j < M.vdim) to[j] = acc[i][j];
     }
 }
 
@@ -451,24 +466,33 @@ __global__ void __launch_bounds__(256) mem_out_kernel(MatMem M, int q_col, int k
     const float* nU = w.nU + ((size_t)ch * M.heads + h) * M.dim;
     float pa[4][4] = {}, oa[4][4] = {};         // rows t = ty*4.., columns s or v = tx*4..
     float nq = 0.f;                             // thread t < 64: n_prev . q_t
+    // the next 32 columns are under way while these are multiplied
+    float q[8], k[8], u[8], nn = 0.f;
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+            const int i = threadIdx.x + 256 * r, t = i >> 5, d = i & 31, sd = i >> 6, sv = i & 63;
+            const float* row = proj + (size_t)(t0 + t) * ldp + h * M.dim + k0 + d;
+            const bool in = t < T && k0 + d < M.dim;
+            q[r] = in ? row[q_col] : 0.f;
+            k[r] = in ? row[k_col] : 0.f;
+            u[r] = k0 + sd < M.dim && v0 + sv < M.vdim ? U[(size_t)(k0 + sd) * M.vdim + v0 + sv] : 0.f;
+        }
+        if (threadIdx.x < 32) nn = k0 + threadIdx.x < M.dim ? nU[k0 + threadIdx.x] : 0.f;
+    };
+    load(0);
     for (int k0 = 0; k0 < M.dim; k0 += 32) {
         __syncthreads();
 #pragma unroll
-        for (int i = threadIdx.x; i < 32 * 64; i += 256) {
-            const int t = i >> 5, d = i & 31;
-            float q = 0.f, k = 0.f;
-            if (t < T && k0 + d < M.dim) {
-                const float* row = proj + (size_t)(t0 + t) * ldp + h * M.dim + k0 + d;
-                q = row[q_col] * qscale;
-                k = row[k_col];
-            }
-            Qs[d][t] = q;
-            Ks[d][t] = k;
-            const int sd = i >> 6, sv = i & 63;
-            Ss[sd][sv] = k0 + sd < M.dim && v0 + sv < M.vdim ? U[(size_t)(k0 + sd) * M.vdim + v0 + sv] : 0.f;
+        for (int r = 0; r < 8; r++) {
+            const int i = threadIdx.x + 256 * r;
+            Qs[i & 31][i >> 5] = q[r] * qscale;
+            Ks[i & 31][i >> 5] = k[r];
+            Ss[i >> 6][i & 63] = u[r];
         }
-        if (threadIdx.x < 32) ns[threadIdx.x] = k0 + threadIdx.x < M.dim ? nU[k0 + threadIdx.x] : 0.f;
+        if (threadIdx.x < 32) ns[threadIdx.x] = nn;
         __syncthreads();
+        if (k0 + 32 < M.dim) load(k0 + 32);
         if (threadIdx.x < kMemChunk) {
 #pragma unroll 8
             for (int d = 0; d < 32; d++) nq = fmaf(ns[d], Qs[d][threadIdx.x], nq);
@@ -488,6 +512,12 @@ __global__ void __launch_bounds__(256) mem_out_kernel(MatMem M, int q_col, int k
         }
     }
     __syncthreads();
+    float val[kMemChunk * 64 / 256];
+#pragma unroll
+    for (int r = 0; r < kMemChunk * 64 / 256; r++) {
+        const int s = (threadIdx.x >> 6) + 4 * r, c = threadIdx.x & 63;
+        val[r] = s < T && v0 + c < M.vdim ? proj[(size_t)(t0 + s) * ldp + v_col + h * M.vdim + v0 + c] : 0.f;
+    }
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int t = ty * 4 + i;
@@ -499,10 +529,8 @@ __global__ void __launch_bounds__(256) mem_out_kernel(MatMem M, int q_col, int k
             oa[i][j] *= inter;
         }
     }
-    for (int i = threadIdx.x; i < kMemChunk * 64; i += 256) {
-        const int s = i >> 6, c = i & 63;
-        Vs[s][c] = s < T && v0 + c < M.vdim ? proj[(size_t)(t0 + s) * ldp + v_col + h * M.vdim + v0 + c] : 0.f;
-    }
+#pragma unroll
+    for (int r = 0; r < kMemChunk * 64 / 256; r++) Vs[(threadIdx.x >> 6) + 4 * r][threadIdx.x & 63] = val[r];
     __syncthreads();
     if (threadIdx.x < kMemChunk) {
         const int t = threadIdx.x;
