@@ -47,6 +47,13 @@ __device__ __forceinline__ void rows_body(const PhaseArgs& a, int bid, int nbloc
     int r0 = bid * per;
     if (r0 < rows) load(t, r0);
 
+    // the norms' weights on their way to this SM's L1, where they would cost a trip to L2 behind every sum
+    const float* const vecs[] = {a.z_w[0], a.z_w[1], a.post_w, a.last_w, a.mix_mu};
+#pragma unroll
+    for (const float* v : vecs)
+        if (v)
+            for (int i = threadIdx.x * 32; i < a.k_valid; i += kRowThreads * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(v + i));
+
     pdl_launch_dependents();
     pdl_wait();
     if (a.pro == PRO_X && !a.last_w && !a.cat && !(keep && a.h_store)) {
