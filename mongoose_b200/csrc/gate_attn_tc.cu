@@ -71,6 +71,7 @@ __device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
 
 template <int HP>
 __global__ void __launch_bounds__(kThreads, Geo<HP>::per_sm) gate_scores_kernel(const __grid_constant__ ScoreArgs a) {
+    pdl_wait();
     using G = Geo<HP>;
     constexpr int BN = G::bn, kStages = G::stages;
     const GateAttn& A = a.at;
@@ -352,6 +353,9 @@ __global__ void __launch_bounds__(kFlashThreads, 1) gate_flash_kernel(const __gr
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // behind the allocation of TMEM, as in gemm_tc_kernel
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t S0 = *tmem_base, O = S0 + 2 * kFlashKeys;
 
     if (warp == 0) {
@@ -529,6 +533,8 @@ __global__ void __launch_bounds__(kFlashThreads, 1) gate_flash_kernel(const __gr
 // multiple of V), for eight heads of its group at a time; a CTA takes V rows.
 template <int V>
 __global__ void __launch_bounds__(256) gate_mix_kernel(GateAttn A, int rows, const float* o, __nv_bfloat16* out, int ld_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ __align__(16) float talk[32][36];            // [g][h], heads of a group side by side
     const int H = A.heads, group = H / A.kv_heads, wide = A.kv_heads * A.dim, units = wide / V;
     for (int i = threadIdx.x; i < 32 * 36; i += 256) {
@@ -580,6 +586,8 @@ __global__ void __launch_bounds__(256) gate_mix_kernel(GateAttn A, int rows, con
 // cache [len][kv][dim_s] -> vt [kv][dim][ldv], zero from len to ldv
 __global__ void __launch_bounds__(256) key_transpose_kernel(const __nv_bfloat16* cache, int kv_heads, int dim, int dim_s, int len, int ldv,
                                                             __nv_bfloat16* vt) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ __nv_bfloat16 t[32][34];
     const int p0 = blockIdx.x * 32, d0 = blockIdx.y * 32, c = blockIdx.z, x = threadIdx.x & 31, y = threadIdx.x >> 5;
     for (int i = y; i < 32; i += 8)
@@ -594,7 +602,7 @@ cudaError_t scores(const ScoreArgs& a, cudaStream_t s) {
     using G = Geo<HP>;
     static cudaError_t attr = cudaFuncSetAttribute((const void*)gate_scores_kernel<HP>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::bytes);
     if (attr != cudaSuccess) return attr;
-    gate_scores_kernel<HP><<<dim3(pad_to(a.pos0 + a.row0 + a.rows, 64) / G::bn, (a.rows + 127) / 128), kThreads, G::bytes, s>>>(a);
+    launch_pdl(gate_scores_kernel<HP>, dim3(pad_to(a.pos0 + a.row0 + a.rows, 64) / G::bn, (a.rows + 127) / 128), kThreads, G::bytes, true, s, a);
     return cudaGetLastError();
 }
 
@@ -626,10 +634,10 @@ cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, in
     if (attr != cudaSuccess) return attr;
     for (int q0 = 0; q0 < n; q0 += block_rows) {
         a.row0 = q0; a.rows = std::min(block_rows, n - q0);
-        gate_flash_kernel<<<dim3((a.rows + 127) / 128, at.heads, (at.kv_heads + a.per - 1) / a.per), kFlashThreads, flash_smem(a.kb, a.cols), s>>>(a);
+        launch_pdl(gate_flash_kernel, dim3((a.rows + 127) / 128, at.heads, (at.kv_heads + a.per - 1) / a.per), kFlashThreads, flash_smem(a.kb, a.cols), true, s, a);
         __nv_bfloat16* to = (__nv_bfloat16*)out + (size_t)q0 * ld_out;
-        if (at.dim % 2 == 0) gate_mix_kernel<2><<<(a.rows + 1) / 2, 256, 0, s>>>(at, a.rows, a.o, to, ld_out);
-        else gate_mix_kernel<1><<<a.rows, 256, 0, s>>>(at, a.rows, a.o, to, ld_out);
+        if (at.dim % 2 == 0) launch_pdl(gate_mix_kernel<2>, (a.rows + 1) / 2, 256, 0, true, s, at, a.rows, a.o, to, ld_out);
+        else launch_pdl(gate_mix_kernel<1>, a.rows, 256, 0, true, s, at, a.rows, a.o, to, ld_out);
         *launches += 2;
     }
     return cudaGetLastError();
@@ -650,7 +658,7 @@ int gate_attn_tc_rows(const GateAttn& at, int max_seq, int max_rows, size_t budg
 cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* weights, int block_rows, void* vt,
                                 void* out, int ld_out, int* status, int* launches, cudaStream_t s) {
     const int len = pos0 + n, ldv = pad_to(len, 64);
-    key_transpose_kernel<<<dim3(ldv / 32, (at.dim + 31) / 32, at.kv_heads), 256, 0, s>>>((const __nv_bfloat16*)at.cache, at.kv_heads, at.dim,
+    launch_pdl(key_transpose_kernel, dim3(ldv / 32, (at.dim + 31) / 32, at.kv_heads), 256, 0, true, s, (const __nv_bfloat16*)at.cache, at.kv_heads, at.dim,
                                                                                        at.dim_s, len, ldv, (__nv_bfloat16*)vt);
     *launches += 1;
     if (gate_flash_fits(at)) return launch_flash(at, qh, pos0, n, max_rows, weights, block_rows, vt, ldv, out, ld_out, status, launches, s);

@@ -82,6 +82,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // behind the allocation of TMEM: a dependent that took its share first would wait for this kernel, and this one for it
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t acc = *tmem_base;
 
     if (warp == 0) {
@@ -231,8 +234,7 @@ cudaError_t run(const GemmTC& g, cudaStream_t s) {
     static cudaError_t attr = cudaFuncSetAttribute((const void*)gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<BN>::bytes);
     if (attr != cudaSuccess) return attr;
     const int cols = g.mode == GEMM_SILU_BF16 ? BN / 2 : BN, gx = (g.n + cols - 1) / cols, gy = (g.m + 127) / 128, tiles = gx * gy * g.batch;
-    gemm_tc_kernel<BN><<<tiles < sm_count() ? tiles : sm_count(), kThreads, Geo<BN>::bytes, s>>>(g, gx, gy, tiles);
-    return cudaGetLastError();
+    return launch_pdl(gemm_tc_kernel<BN>, tiles < sm_count() ? tiles : sm_count(), kThreads, Geo<BN>::bytes, true, s, g, gx, gy, tiles);
 }
 
 }  // namespace

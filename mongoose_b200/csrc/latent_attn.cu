@@ -362,6 +362,8 @@ __global__ void __launch_bounds__(kThreads) latent_value_kernel(const LatentStep
 // One CTA per row of a portion.
 template <typename AT>
 __global__ void __launch_bounds__(kThreads) latent_rows_kernel(const LatentAttn A, const float* down, int ldd, int pos0, AT* act, int ld_act) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[40];
     const float* q = down + (size_t)blockIdx.x * ldd;
     float ss = 0.f;
@@ -372,6 +374,8 @@ __global__ void __launch_bounds__(kThreads) latent_rows_kernel(const LatentAttn 
 }
 
 __global__ void __launch_bounds__(kThreads) latent_q_rows_kernel(const LatentAttn A, const float* q, int pos0, float scale, __nv_bfloat16* qh) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int row = A.heads * A.qrow(), qr = A.qrow();
     const float* src = q + (size_t)blockIdx.x * row;
     __nv_bfloat16* dst = qh + (size_t)blockIdx.x * row;
@@ -449,13 +453,13 @@ cudaError_t launch_latent_value(const LatentStep& a, bool f32_out, bool pdl, cud
 }
 
 cudaError_t launch_latent_rows(const LatentAttn& at, const float* down, int ldd, int pos0, int n, void* act, int ld_act, bool f32, cudaStream_t s) {
-    if (f32) latent_rows_kernel<float><<<n, kThreads, 0, s>>>(at, down, ldd, pos0, (float*)act, ld_act);
-    else latent_rows_kernel<__nv_bfloat16><<<n, kThreads, 0, s>>>(at, down, ldd, pos0, (__nv_bfloat16*)act, ld_act);
+    if (f32) launch_pdl(latent_rows_kernel<float>, n, kThreads, 0, true, s, at, down, ldd, pos0, (float*)act, ld_act);
+    else launch_pdl(latent_rows_kernel<__nv_bfloat16>, n, kThreads, 0, true, s, at, down, ldd, pos0, (__nv_bfloat16*)act, ld_act);
     return cudaGetLastError();
 }
 
 cudaError_t launch_latent_q_rows(const LatentAttn& at, const float* q, int pos0, int n, void* qh, cudaStream_t s) {
-    latent_q_rows_kernel<<<n, kThreads, 0, s>>>(at, q, pos0, at.scale * 1.4426950408889634f, (__nv_bfloat16*)qh);
+    launch_pdl(latent_q_rows_kernel, n, kThreads, 0, true, s, at, q, pos0, at.scale * 1.4426950408889634f, (__nv_bfloat16*)qh);
     return cudaGetLastError();
 }
 

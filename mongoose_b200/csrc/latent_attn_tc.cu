@@ -77,6 +77,9 @@ __global__ void __launch_bounds__(kThreads, 2) latent_flash_kernel(const __grid_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // behind the allocation of TMEM, as in gemm_tc_kernel
+    pdl_launch_dependents();
+    pdl_wait();
     const uint32_t tmem = *tmem_base, S0 = tmem, O = tmem + 2 * kKeys;
 
     if (warp == 0) {
@@ -290,7 +293,7 @@ cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0
         return cudaErrorInvalidValue;
     static cudaError_t attr = cudaFuncSetAttribute((const void*)latent_flash_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (attr != cudaSuccess) return attr;
-    latent_flash_kernel<<<dim3((n + 127) / 128, at.heads), kThreads, geo.smem, s>>>(f);
+    launch_pdl(latent_flash_kernel, dim3((n + 127) / 128, at.heads), kThreads, geo.smem, true, s, f);
     *launches += 3;
     return cudaGetLastError();
 }

@@ -13,6 +13,8 @@ namespace {
 template <typename AT>
 __global__ void __launch_bounds__(256) embed_rows_kernel(WeightView embed, int ld_embed, const float* pos_tab, const int* tokens,
                                                          int pos0, int width, float* x, AT* act, int ld_act) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int r = blockIdx.x, token = tokens[r];
     for (int i = threadIdx.x; i < width; i += blockDim.x) {
         const float v = embed_value(embed, FMT_BF16, ld_embed, token, i) + (pos_tab ? pos_tab[(size_t)(pos0 + r) * width + i] : 0.f);
@@ -25,6 +27,8 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(WeightView embed, int l
 template <typename AT>
 __global__ void __launch_bounds__(256) qk_rows_kernel(GateAttn A, const float* proj, int ldp, int q_col, int k_col, int pos0, int n,
                                                       AT* qh) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int per = A.heads + A.kv_heads, t = w / per, h = w - t * per;
     if (t >= n) return;
@@ -39,6 +43,8 @@ __global__ void __launch_bounds__(256) qk_rows_kernel(GateAttn A, const float* p
 // to 64 C values.  A prompt of 2048 tokens, 36 heads of 64: 25 us with a warp per head and a value per load.
 template <typename AT, int C>
 __global__ void __launch_bounds__(256) qk_quads_kernel(GateAttn A, const float* proj, int ldp, int q_col, int k_col, int pos0, int n, AT* qh) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int u = (blockIdx.x * 256 + threadIdx.x) >> 4, l = threadIdx.x & 15;
     const unsigned mask = 0xffffu << (threadIdx.x & 16);
     const int per = A.heads + A.kv_heads, t = u / per, h = u - t * per;
@@ -92,6 +98,8 @@ __global__ void __launch_bounds__(256) qk_quads_kernel(GateAttn A, const float* 
 template <typename KT, int NQ, int EP>
 __global__ void __launch_bounds__(kAttnThreads) gate_attn_rows_kernel(GateAttn A, const KT* qh, int pos0, int n, int tile, KT* out,
                                                                       int ld_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float smem[];
     const AttnSmem<KT> sm(A, NQ, tile, smem);
     const int t0 = (gridDim.x - 1 - blockIdx.x) * NQ;      // the longest rows first
@@ -121,6 +129,8 @@ __global__ void __launch_bounds__(kAttnThreads) gate_attn_rows_kernel(GateAttn A
 template <typename AT>
 __global__ void __launch_bounds__(256) post_rows_kernel(float* x, const float* z0, const float* z1, const float* w0, const float* w1,
                                                         const float* post_w, float eps, int width, AT* act, int ld_act) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float y[];
     __shared__ float red[40];
     const size_t r = blockIdx.x;
@@ -151,6 +161,8 @@ __global__ void __launch_bounds__(256) post_rows_kernel(float* x, const float* z
 template <typename AT, int C>
 __global__ void __launch_bounds__(256) post_quads_kernel(float* x, const float* z0, const float* z1, const float* w0, const float* w1,
                                                          const float* post_w, float eps, int width, AT* act, int ld_act) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[72];
     const size_t r = blockIdx.x;
     const float inv = 1.0f / (float)width;
@@ -228,6 +240,8 @@ __device__ __forceinline__ float2 row_norm(const float* y, int kind, float eps, 
 template <typename AT>
 __global__ void __launch_bounds__(256) last_norm_rows_kernel(const float* x, const int* rows, const float* w, int kind, float eps, int width,
                                                              AT* act, int ld_act) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[40];
     const float* a = x + (size_t)rows[blockIdx.x] * width;
     const float2 n = row_norm<1>(a, kind, eps, width, red);
@@ -237,6 +251,8 @@ __global__ void __launch_bounds__(256) last_norm_rows_kernel(const float* x, con
 
 template <typename AT, int V>
 __global__ void __launch_bounds__(256) prenorm_rows_kernel(const PrenormRows a) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float y[];
     __shared__ float red[40];
     const int W = a.width, step = 256 * V;
@@ -286,6 +302,8 @@ constexpr int kGateWarps = 32;
 
 __global__ void __launch_bounds__(kGateWarps * 32) mem_gates_kernel(MatMem M, int i_col, int f_col, const float* proj, int ldp, int pos0,
                                                                     int n, MemRows w) {
+    pdl_launch_dependents();
+    pdl_wait();
     static_assert(kMemChunk == 64, "a warp holds a chunk as two tokens per lane");
     __shared__ double sum_f[kGateWarps];
     __shared__ float top_i[kGateWarps], m_end;
@@ -352,6 +370,8 @@ __device__ __forceinline__ float mem_before(const MemRows& w, int h, int n, int 
 // U[chunk][head] = sum over the chunk of exp(b_T - b_s + i_s - m_T) k_s v_s^T, a 64 x 64 tile per CTA.
 __global__ void __launch_bounds__(256) mem_chunk_kernel(MatMem M, int k_col, int v_col, const float* proj, int ldp, int n, int vtiles,
                                                         MemRows w) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ __align__(16) float Ks[kMemChunk][68], Vs[kMemChunk][68];
     const int ch = blockIdx.x, h = blockIdx.y, d0 = blockIdx.z / vtiles * 64, v0 = blockIdx.z % vtiles * 64;
     const int t0 = ch * kMemChunk, T = min(kMemChunk, n - t0);
@@ -413,6 +433,8 @@ __global__ void __launch_bounds__(256) mem_chunk_kernel(MatMem M, int k_col, int
 
 // Pass over the chunks: U becomes the state BEFORE each chunk, and the state after the last is stored.
 __global__ void __launch_bounds__(256) mem_scan_kernel(MatMem M, int pos0, int n, int chunks, MemRows w) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t per = (size_t)M.dim * M.vdim, all = M.heads * per, nall = (size_t)M.heads * M.dim;
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= all + nall) return;
@@ -444,6 +466,8 @@ __global__ void __launch_bounds__(256) mem_scan_kernel(MatMem M, int pos0, int n
 // Outputs of one chunk and head, 64 value columns per CTA.
 __global__ void __launch_bounds__(256) mem_out_kernel(MatMem M, int q_col, int k_col, int v_col, const float* proj, int ldp,
                                                       int n, MemRows w) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ __align__(16) float Qs[32][68], Ks[32][68], Ss[32][68];
     __shared__ __align__(16) float P[kMemChunk][68];            // [s][t]
     __shared__ float nq_s[kMemChunk], ns[32];
@@ -564,6 +588,8 @@ __global__ void __launch_bounds__(256) mem_out_kernel(MatMem M, int q_col, int k
 template <typename AT>
 __global__ void __launch_bounds__(256) head_norm_rows_kernel(int heads, int vdim, float eps, const float* norm, const float* gate, int ldg,
                                                              int gate_kind, int n, const float* o, AT* act, int ld_act) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int wq = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int t = wq / heads, h = wq - t * heads;
     if (t >= n) return;
@@ -583,6 +609,8 @@ __global__ void __launch_bounds__(256) head_norm_rows_kernel(int heads, int vdim
 template <typename AT>
 __global__ void __launch_bounds__(256) head_norm_quads_kernel(int heads, int vdim, int lanes, float eps, const float* norm, const float* gate,
                                                               int ldg, int gate_kind, int n, const float* o, AT* act, int ld_act) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int unit = (blockIdx.x * 256 + threadIdx.x) / lanes, sub = threadIdx.x & (lanes - 1);
     const int t = unit / heads, h = unit - t * heads, c = h * vdim + sub * 4;
     const bool in = t < n && sub * 4 < vdim;
@@ -609,7 +637,7 @@ cudaError_t attn_rows_for(const GateAttn& at, const void* qh, int pos0, int n, v
     auto run = [&](auto kern) {
         cudaError_t c = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (c != cudaSuccess) return c;
-        kern<<<(n + NQ - 1) / NQ, kAttnThreads, smem, s>>>(at, (const KT*)qh, pos0, n, tile, (KT*)out, ld_out);
+        launch_pdl(kern, (n + NQ - 1) / NQ, kAttnThreads, smem, true, s, at, (const KT*)qh, pos0, n, tile, (KT*)out, ld_out);
         return cudaGetLastError();
     };
     switch (attn_pairs(at)) {
@@ -626,8 +654,8 @@ cudaError_t attn_rows_for(const GateAttn& at, const void* qh, int pos0, int n, v
 
 cudaError_t launch_embed_rows(const WeightView& embed, int ld_embed, const float* pos_tab, const int* tokens, int pos0, int n,
                               int width, float* x, void* act, int ld_act, bool f32, cudaStream_t s) {
-    if (f32) embed_rows_kernel<float><<<n, 256, 0, s>>>(embed, ld_embed, pos_tab, tokens, pos0, width, x, (float*)act, ld_act);
-    else embed_rows_kernel<__nv_bfloat16><<<n, 256, 0, s>>>(embed, ld_embed, pos_tab, tokens, pos0, width, x, (__nv_bfloat16*)act, ld_act);
+    if (f32) launch_pdl(embed_rows_kernel<float>, n, 256, 0, true, s, embed, ld_embed, pos_tab, tokens, pos0, width, x, (float*)act, ld_act);
+    else launch_pdl(embed_rows_kernel<__nv_bfloat16>, n, 256, 0, true, s, embed, ld_embed, pos_tab, tokens, pos0, width, x, (__nv_bfloat16*)act, ld_act);
     return cudaGetLastError();
 }
 
@@ -637,16 +665,16 @@ cudaError_t launch_qk_rows(const GateAttn& at, const float* proj, int ldp, int q
         auto quads = [&](auto* q) {
             using AT = std::remove_pointer_t<decltype(q)>;
             const int grid = (n * (at.heads + at.kv_heads) + 15) / 16;
-            if (at.dim <= 64) qk_quads_kernel<AT, 1><<<grid, 256, 0, s>>>(at, proj, ldp, q_col, k_col, pos0, n, q);
-            else if (at.dim <= 128) qk_quads_kernel<AT, 2><<<grid, 256, 0, s>>>(at, proj, ldp, q_col, k_col, pos0, n, q);
-            else qk_quads_kernel<AT, 4><<<grid, 256, 0, s>>>(at, proj, ldp, q_col, k_col, pos0, n, q);
+            if (at.dim <= 64) launch_pdl(qk_quads_kernel<AT, 1>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, q);
+            else if (at.dim <= 128) launch_pdl(qk_quads_kernel<AT, 2>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, q);
+            else launch_pdl(qk_quads_kernel<AT, 4>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, q);
             return cudaGetLastError();
         };
         return f32 ? quads((float*)qh) : quads((__nv_bfloat16*)qh);
     }
     const int grid = (n * (at.heads + at.kv_heads) + 7) / 8;
-    if (f32) qk_rows_kernel<float><<<grid, 256, 0, s>>>(at, proj, ldp, q_col, k_col, pos0, n, (float*)qh);
-    else qk_rows_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(at, proj, ldp, q_col, k_col, pos0, n, (__nv_bfloat16*)qh);
+    if (f32) launch_pdl(qk_rows_kernel<float>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, (float*)qh);
+    else launch_pdl(qk_rows_kernel<__nv_bfloat16>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, (__nv_bfloat16*)qh);
     return cudaGetLastError();
 }
 
@@ -665,33 +693,33 @@ cudaError_t launch_post_rows(float* x, const float* z0, const float* z1, const f
     if ((width & 3) == 0 && width <= 4096) {
         auto quads = [&](auto* o) {
             using AT = std::remove_pointer_t<decltype(o)>;
-            if (width <= 1024) post_quads_kernel<AT, 1><<<n, 256, 0, s>>>(x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
-            else if (width <= 2048) post_quads_kernel<AT, 2><<<n, 256, 0, s>>>(x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
-            else post_quads_kernel<AT, 4><<<n, 256, 0, s>>>(x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
+            if (width <= 1024) launch_pdl(post_quads_kernel<AT, 1>, n, 256, 0, true, s, x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
+            else if (width <= 2048) launch_pdl(post_quads_kernel<AT, 2>, n, 256, 0, true, s, x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
+            else launch_pdl(post_quads_kernel<AT, 4>, n, 256, 0, true, s, x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
             return cudaGetLastError();
         };
         return f32 ? quads((float*)act) : quads((__nv_bfloat16*)act);
     }
     const size_t smem = (size_t)width * sizeof(float);
-    if (f32) post_rows_kernel<float><<<n, 256, smem, s>>>(x, z0, z1, w0, w1, post_w, eps, width, (float*)act, ld_act);
-    else post_rows_kernel<__nv_bfloat16><<<n, 256, smem, s>>>(x, z0, z1, w0, w1, post_w, eps, width, (__nv_bfloat16*)act, ld_act);
+    if (f32) launch_pdl(post_rows_kernel<float>, n, 256, smem, true, s, x, z0, z1, w0, w1, post_w, eps, width, (float*)act, ld_act);
+    else launch_pdl(post_rows_kernel<__nv_bfloat16>, n, 256, smem, true, s, x, z0, z1, w0, w1, post_w, eps, width, (__nv_bfloat16*)act, ld_act);
     return cudaGetLastError();
 }
 
 cudaError_t launch_last_norm_rows(const float* x, const int* rows, const float* w, int kind, float eps, int n, int width, void* act,
                                   int ld_act, bool f32, cudaStream_t s) {
-    if (f32) last_norm_rows_kernel<float><<<n, 256, 0, s>>>(x, rows, w, kind, eps, width, (float*)act, ld_act);
-    else last_norm_rows_kernel<__nv_bfloat16><<<n, 256, 0, s>>>(x, rows, w, kind, eps, width, (__nv_bfloat16*)act, ld_act);
+    if (f32) launch_pdl(last_norm_rows_kernel<float>, n, 256, 0, true, s, x, rows, w, kind, eps, width, (float*)act, ld_act);
+    else launch_pdl(last_norm_rows_kernel<__nv_bfloat16>, n, 256, 0, true, s, x, rows, w, kind, eps, width, (__nv_bfloat16*)act, ld_act);
     return cudaGetLastError();
 }
 
 cudaError_t launch_prenorm_rows(const PrenormRows& a, bool f32, cudaStream_t s) {
     const size_t smem = (size_t)a.width * sizeof(float);
     const bool quads = a.width % 4 == 0;
-    if (f32 && quads) prenorm_rows_kernel<float, 4><<<a.n, 256, smem, s>>>(a);
-    else if (f32) prenorm_rows_kernel<float, 1><<<a.n, 256, smem, s>>>(a);
-    else if (quads) prenorm_rows_kernel<__nv_bfloat16, 4><<<a.n, 256, smem, s>>>(a);
-    else prenorm_rows_kernel<__nv_bfloat16, 1><<<a.n, 256, smem, s>>>(a);
+    if (f32 && quads) launch_pdl(prenorm_rows_kernel<float, 4>, a.n, 256, smem, true, s, a);
+    else if (f32) launch_pdl(prenorm_rows_kernel<float, 1>, a.n, 256, smem, true, s, a);
+    else if (quads) launch_pdl(prenorm_rows_kernel<__nv_bfloat16, 4>, a.n, 256, smem, true, s, a);
+    else launch_pdl(prenorm_rows_kernel<__nv_bfloat16, 1>, a.n, 256, smem, true, s, a);
     return cudaGetLastError();
 }
 
@@ -702,9 +730,9 @@ static cudaError_t head_norm_for(int heads, int vdim, float eps, const float* no
     int lanes = 1;
     while (lanes * 4 < vdim) lanes *= 2;
     if (quads)
-        head_norm_quads_kernel<AT><<<(int)(((long long)n * heads * lanes + 255) / 256), 256, 0, s>>>(heads, vdim, lanes, eps, norm, gate, ldg, gate_kind, n, o, act, ld_act);
+        launch_pdl(head_norm_quads_kernel<AT>, (int)(((long long)n * heads * lanes + 255) / 256), 256, 0, true, s, heads, vdim, lanes, eps, norm, gate, ldg, gate_kind, n, o, act, ld_act);
     else
-        head_norm_rows_kernel<AT><<<(n * heads + 7) / 8, 256, 0, s>>>(heads, vdim, eps, norm, gate, ldg, gate_kind, n, o, act, ld_act);
+        launch_pdl(head_norm_rows_kernel<AT>, (n * heads + 7) / 8, 256, 0, true, s, heads, vdim, eps, norm, gate, ldg, gate_kind, n, o, act, ld_act);
     return cudaGetLastError();
 }
 
@@ -717,11 +745,11 @@ cudaError_t launch_head_norm_rows(int heads, int vdim, float eps, const float* n
 cudaError_t launch_mem_rows(const MatMem& mem, const ProjCols& c, const float* proj, int ldp, int pos0, int n, const MemRows& w, void* act,
                             int ld_act, bool f32, cudaStream_t s) {
     const int chunks = (n + kMemChunk - 1) / kMemChunk, dt = (mem.dim + 63) / 64, vt = (mem.vdim + 63) / 64;
-    mem_gates_kernel<<<mem.heads, kGateWarps * 32, 0, s>>>(mem, c.mi, c.mf, proj, ldp, pos0, n, w);
-    mem_chunk_kernel<<<dim3(chunks, mem.heads, dt * vt), 256, 0, s>>>(mem, c.mk, c.mv, proj, ldp, n, vt, w);
+    launch_pdl(mem_gates_kernel, mem.heads, kGateWarps * 32, 0, true, s, mem, c.mi, c.mf, proj, ldp, pos0, n, w);
+    launch_pdl(mem_chunk_kernel, dim3(chunks, mem.heads, dt * vt), 256, 0, true, s, mem, c.mk, c.mv, proj, ldp, n, vt, w);
     const size_t elems = (size_t)mem.heads * mem.dim * (mem.vdim + 1);
-    mem_scan_kernel<<<(unsigned)((elems + 255) / 256), 256, 0, s>>>(mem, pos0, n, chunks, w);
-    mem_out_kernel<<<dim3(chunks, mem.heads, vt), 256, 0, s>>>(mem, c.mq, c.mk, c.mv, proj, ldp, n, w);
+    launch_pdl(mem_scan_kernel, (unsigned)((elems + 255) / 256), 256, 0, true, s, mem, pos0, n, chunks, w);
+    launch_pdl(mem_out_kernel, dim3(chunks, mem.heads, vt), 256, 0, true, s, mem, c.mq, c.mk, c.mv, proj, ldp, n, w);
     return launch_head_norm_rows(mem.heads, mem.vdim, mem.eps, mem.norm, proj + c.mg, ldp, GATE_SIGMOID, n, w.o, act, ld_act, f32, s);
 }
 

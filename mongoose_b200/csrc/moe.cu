@@ -182,6 +182,8 @@ __global__ void __launch_bounds__(kThreads) moe_down_kernel(const MoeStep a) {
 
 // A warp per token: choice, and the token's place among those of its expert.
 __global__ void __launch_bounds__(kThreads) moe_choose_kernel(const Moe m, const float* router, int ldr, int slices, int n, MoeRows w) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float smem[];
     __shared__ int sel[kThreads / 32][kMaxTop];
     __shared__ float wt[kThreads / 32][kMaxTop];
@@ -206,6 +208,8 @@ __global__ void __launch_bounds__(kThreads) moe_choose_kernel(const Moe m, const
 
 // One CTA: first row of every expert (whole tiles of 128), the expert of every tile; clears the counts.
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const Moe m, MoeRows w) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ int tiles[kMaxExperts], first[kMaxExperts + 1];
     for (int e = threadIdx.x; e < m.experts; e += blockDim.x) {
         tiles[e] = (w.count[e] + 127) / 128;
@@ -227,6 +231,8 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const Moe m, MoeRows w) 
 
 // A CTA per token: its row to its place in every chosen expert's group; slot becomes the grouped row.
 __global__ void __launch_bounds__(128) moe_gather_kernel(const Moe m, const uint4* act, int units, MoeRows w) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t t = blockIdx.x;
     for (int k = 0; k < m.top; k++) {
         const size_t at = t * m.top + k;
@@ -238,6 +244,8 @@ __global__ void __launch_bounds__(128) moe_gather_kernel(const Moe m, const uint
 
 template <typename AT, int V>
 __global__ void __launch_bounds__(kThreads) moe_combine_kernel(const Moe m, MoeRows w, float* z) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float wt[kMaxTop];
     __shared__ int row[kMaxTop];
     const size_t t = blockIdx.x;
@@ -292,18 +300,18 @@ cudaError_t launch_moe_down(const MoeStep& a, int sms, bool pdl, cudaStream_t s)
 }
 
 cudaError_t launch_moe_route(const Moe& m, const float* router, int ldr, int slices, int n, const void* act, bool f32, const MoeRows& w, cudaStream_t s) {
-    moe_choose_kernel<<<(n + 7) / 8, kThreads, (size_t)8 * m.experts * sizeof(float), s>>>(m, router, ldr, slices, n, w);
-    moe_plan_kernel<<<1, 1024, 0, s>>>(m, w);
-    moe_gather_kernel<<<n, 128, 0, s>>>(m, (const uint4*)act, m.ldw * (f32 ? 4 : 2) / 16, w);
+    launch_pdl(moe_choose_kernel, (n + 7) / 8, kThreads, (size_t)8 * m.experts * sizeof(float), true, s, m, router, ldr, slices, n, w);
+    launch_pdl(moe_plan_kernel, 1, 1024, 0, true, s, m, w);
+    launch_pdl(moe_gather_kernel, n, 128, 0, true, s, m, (const uint4*)act, m.ldw * (f32 ? 4 : 2) / 16, w);
     return cudaGetLastError();
 }
 
 cudaError_t launch_moe_combine(const Moe& m, int n, const MoeRows& w, float* z, bool f32, cudaStream_t s) {
     const bool quads = m.width % 4 == 0;
-    if (f32 && quads) moe_combine_kernel<float, 4><<<n, kThreads, 0, s>>>(m, w, z);
-    else if (f32) moe_combine_kernel<float, 1><<<n, kThreads, 0, s>>>(m, w, z);
-    else if (quads) moe_combine_kernel<__nv_bfloat16, 4><<<n, kThreads, 0, s>>>(m, w, z);
-    else moe_combine_kernel<__nv_bfloat16, 1><<<n, kThreads, 0, s>>>(m, w, z);
+    if (f32 && quads) launch_pdl(moe_combine_kernel<float, 4>, n, kThreads, 0, true, s, m, w, z);
+    else if (f32) launch_pdl(moe_combine_kernel<float, 1>, n, kThreads, 0, true, s, m, w, z);
+    else if (quads) launch_pdl(moe_combine_kernel<__nv_bfloat16, 4>, n, kThreads, 0, true, s, m, w, z);
+    else launch_pdl(moe_combine_kernel<__nv_bfloat16, 1>, n, kThreads, 0, true, s, m, w, z);
     return cudaGetLastError();
 }
 

@@ -114,6 +114,8 @@ template <typename AT, int V>
 __global__ void __launch_bounds__(256) wkv_mix_kernel(const float* h, const float* prev, const float* m0, const float* m1, const float* m2,
                                                       const float* m3, const float* m4, int pos0, int width, AT* act, int ld_act,
                                                       long long stride) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int t = blockIdx.x;
     const float* cur = h + (size_t)t * width;
     const float* before = t > 0 ? cur - width : prev + (size_t)(pos0 & 1) * width;
@@ -142,6 +144,8 @@ __global__ void __launch_bounds__(256) wkv_mix_kernel(const float* h, const floa
 // act[t] = [high, low]: tanh of the decay's inner projection, the sum of `slices` slabs, as two bf16 parts (16 bits of
 // mantissa together), each padded to ld / 2, so that a product of bf16 operands keeps it.
 __global__ void __launch_bounds__(256) wkv_inner_kernel(const float* inner, int ldp, int slices, int rank, int n, __nv_bfloat16* act, int ld) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int i = blockIdx.x * 256 + threadIdx.x, t = i / rank, c = i - t * rank;
     if (t >= n) return;
     float v = 0.f;
@@ -192,6 +196,8 @@ struct Scan {
 template <int KPT>
 __global__ void __launch_bounds__(kScanThreads) wkv_scan_kernel(const Wkv M, const float* proj, int ldp, const float* decay, int pos0, int n,
                                                                 float* out) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float smem[];
     using G = Scan<KPT>;
     constexpr int rows = G::rows, per = G::per, P = G::P, tile = G::tile, NO = kScanGroup * kScanCols;
@@ -339,15 +345,15 @@ cudaError_t scan_for(const Wkv& wk, const float* proj, int ldp, const float* dec
     constexpr size_t smem = G::smem(G::tile);
     static cudaError_t attr = cudaFuncSetAttribute((const void*)wkv_scan_kernel<KPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (attr != cudaSuccess) return attr;
-    wkv_scan_kernel<KPT><<<dim3(wk.heads, (wk.dim + G::cols - 1) / G::cols), kScanThreads, smem, s>>>(wk, proj, ldp, decay, pos0, n, out);
+    launch_pdl(wkv_scan_kernel<KPT>, dim3(wk.heads, (wk.dim + G::cols - 1) / G::cols), kScanThreads, smem, true, s, wk, proj, ldp, decay, pos0, n, out);
     return cudaGetLastError();
 }
 
 template <typename AT>
 cudaError_t mix_for(const float* h, const float* prev, const float* const mu[5], int pos0, int n, int width, AT* act, int ld_act, long long stride,
                     cudaStream_t s) {
-    if (width % 4 == 0) wkv_mix_kernel<AT, 4><<<n, 256, 0, s>>>(h, prev, mu[0], mu[1], mu[2], mu[3], mu[4], pos0, width, act, ld_act, stride);
-    else wkv_mix_kernel<AT, 1><<<n, 256, 0, s>>>(h, prev, mu[0], mu[1], mu[2], mu[3], mu[4], pos0, width, act, ld_act, stride);
+    if (width % 4 == 0) launch_pdl(wkv_mix_kernel<AT, 4>, n, 256, 0, true, s, h, prev, mu[0], mu[1], mu[2], mu[3], mu[4], pos0, width, act, ld_act, stride);
+    else launch_pdl(wkv_mix_kernel<AT, 1>, n, 256, 0, true, s, h, prev, mu[0], mu[1], mu[2], mu[3], mu[4], pos0, width, act, ld_act, stride);
     return cudaGetLastError();
 }
 
@@ -366,7 +372,7 @@ cudaError_t launch_wkv_mix(const float* h, const float* prev, const float* const
 }
 
 cudaError_t launch_wkv_inner(const float* inner, int ldp, int slices, int rank, int n, void* act, int ld, cudaStream_t s) {
-    wkv_inner_kernel<<<(n * rank + 255) / 256, 256, 0, s>>>(inner, ldp, slices, rank, n, (__nv_bfloat16*)act, ld);
+    launch_pdl(wkv_inner_kernel, (n * rank + 255) / 256, 256, 0, true, s, inner, ldp, slices, rank, n, (__nv_bfloat16*)act, ld);
     return cudaGetLastError();
 }
 
