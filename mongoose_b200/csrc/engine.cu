@@ -1353,6 +1353,9 @@ void read_env(mg_engine* e) {
     if (env && env[0] == '1') e->use_mega = false;
     env = getenv("MG_NO_PDL");
     if (env && env[0] == '1') e->use_pdl = false;
+    // Kernels read the position before they wait for their predecessor, which is right behind the edge between two graph
+    // launches: without graphs a step's kernels could start under the last step's lm_head, which moves it.
+    if (!e->use_graph) e->use_pdl = false;
     // L2 prefetch distance of the persistent kernel's weight stream; 64 KiB measured best on
     // 7B-class widths (layer time 85 -> 75 us), neutral on the 0.5 B model, 384 KiB thrashes L2
     env = getenv("MG_PREFETCH_KB");

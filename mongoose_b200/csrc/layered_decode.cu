@@ -28,7 +28,7 @@ __device__ __forceinline__ void mem_step(const MixerStep& a, int cta, float* sme
     const float* row = a.proj;
     const int v = slice * 32 + lane;
     float* S = M.S + (size_t)head * M.dim * M.vdim + v;
-    // the state's rows come first: nothing they wait for is computed here
+    // the state was left by the last token: it is on its way before the predecessor has finished
     float s0[kStateRows];
     auto load_rows = [&](int d0) {
 #pragma unroll
@@ -38,11 +38,14 @@ __device__ __forceinline__ void mem_step(const MixerStep& a, int cta, float* sme
         }
     };
     load_rows(0);
+    const int cur = pos & 1;
+    const float m0 = fresh ? 0.f : M.m[cur * M.heads + head];
+    const int d_own = threadIdx.x;
+    const float n_own = fresh || d_own >= M.dim ? 0.f : M.nrm[((size_t)cur * M.heads + head) * M.dim + d_own];
+    pdl_wait();
     const float vv = v < M.vdim ? row[a.c.mv + head * M.vdim + v] : 0.f;
     const float ig = soft_cap(row[a.c.mi + head] + M.i_bias[head], M.cap);
     const float fg = log_sigmoid(soft_cap(row[a.c.mf + head] + M.f_bias[head], M.cap));
-    const int cur = pos & 1;
-    const float m0 = fresh ? 0.f : M.m[cur * M.heads + head];
     const float m1 = fmaxf(fg + m0, ig);
     const float keep = expf(fg + m0 - m1), add = expf(ig - m1);
     const float qscale = 1.0f / sqrtf((float)M.dim);
@@ -51,7 +54,7 @@ __device__ __forceinline__ void mem_step(const MixerStep& a, int cta, float* sme
         const float k = row[a.c.mk + head * M.dim + d], q = row[a.c.mq + head * M.dim + d] * qscale;
         ks[d] = k * add;
         qs[d] = q;
-        const float n0 = fresh ? 0.f : M.nrm[((size_t)cur * M.heads + head) * M.dim + d];
+        const float n0 = d == d_own ? n_own : fresh ? 0.f : M.nrm[((size_t)cur * M.heads + head) * M.dim + d];
         const float n1 = keep * n0 + add * k;
         if (slice == 0) M.nrm[((size_t)(cur ^ 1) * M.heads + head) * M.dim + d] = n1;
         nq = fmaf(n1, q, nq);
@@ -84,7 +87,6 @@ template <typename KT, int EP>
 __global__ void __launch_bounds__(kAttnThreads) mixer_step_kernel(const MixerStep a) {
     extern __shared__ __align__(16) float smem[];
     pdl_launch_dependents();
-    pdl_wait();
     if ((int)blockIdx.x < a.n_mem) {
         mem_step(a, blockIdx.x, smem);
         return;
@@ -97,16 +99,23 @@ __global__ void __launch_bounds__(kAttnThreads) mixer_step_kernel(const MixerSte
     const int active = key_split(len, a.splits, a.tile, split, &j0, &j1);
     if (split >= active) return;
     const AttnSmem<KT> sm(A, 1, a.tile, smem);
+    // tables, and keys of earlier tokens, do not wait for the predecessor
+    const bool early = j0 + a.tile <= pos;
+    if (early) {
+        load_keys<KT>(A, sm, KeyCopy(A.dim_s / Chunk16<KT>::n), 0, j0, j1, a.tile);
+        cp_async_commit();
+    }
+    sm.load_tables(A);
+    pdl_wait();
     // this token's query, and its key where this CTA's range ends with it
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const float temp = query_temp(A, pos);
     norm_queries(A, a.proj + a.c.q, temp, sm.q, sm.qs);
     if (j1 == len)
         for (int c = wid; c < A.kv_heads; c += nw) store_key<KT>(A, a.proj + a.c.k + c * A.dim, pos, c, lane);
-    sm.load_tables(A);
     __syncthreads();                        // the cache row above is read back by this CTA only
     float acc[1][EP][2] = {};
-    attend<KT, 1, EP>(A, sm, pos, j0, j1, a.tile, acc);
+    attend<KT, 1, EP>(A, sm, pos, j0, j1, a.tile, acc, early);
 #pragma unroll
     for (int p = 0; p < EP; p++) {
         const int e = 2 * (threadIdx.x + p * kAttnThreads);

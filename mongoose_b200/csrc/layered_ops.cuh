@@ -262,10 +262,11 @@ __device__ __forceinline__ void load_keys(const GateAttn& A, const AttnSmem<KT>&
 
 // acc[q][pair] += sum over keys [j0, j1) of the mixed weights times the raw keys, for the NQ queries in
 // sm.q at positions pos0 .. pos0 + NQ - 1.  Thread t owns elements 2 * (t + p * kAttnThreads) and the next of the
-// [heads][dim_s] output.  A score belongs to one thread, lanes over heads.
+// [heads][dim_s] output.  A score belongs to one thread, lanes over heads.  `loaded`: the first tile's copies have been
+// issued and committed.
 template <typename KT, int NQ, int EP>
 __device__ __forceinline__ void attend(const GateAttn& A, const AttnSmem<KT>& sm, int pos0, int j0, int j1, int tile,
-                                       float (&acc)[NQ][EP][2]) {
+                                       float (&acc)[NQ][EP][2], bool loaded = false) {
     constexpr int CN = Chunk16<KT>::n;
     const int H = A.heads, DS = A.dim_s, KV = A.kv_heads, group = H / KV, row = KV * sm.ks;
     const int chunks = DS / CN;
@@ -279,8 +280,10 @@ __device__ __forceinline__ void attend(const GateAttn& A, const AttnSmem<KT>& sm
         head_of[e] = el < H * DS ? h : -1;
         key_of[e] = h / group * sm.ks + el - h * DS;
     }
-    load_keys<KT>(A, sm, cp, 0, j0, j1, tile);
-    cp_async_commit();
+    if (!loaded) {
+        load_keys<KT>(A, sm, cp, 0, j0, j1, tile);
+        cp_async_commit();
+    }
     int buf = 0;
     for (int j = j0; j < j1; j += tile, buf ^= 1) {
         if (j + tile < j1) load_keys<KT>(A, sm, cp, buf ^ 1, j + tile, j1, tile);

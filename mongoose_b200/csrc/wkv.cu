@@ -33,7 +33,6 @@ __global__ void __launch_bounds__(kStepThreads) wkv_step_kernel(const WkvStep a)
     const float w0 = d_of < D ? M.w0[c0 + d_of] : 0.f;
     for (int i = threadIdx.x; i < D; i += kStepThreads) u[i] = M.u[c0 + i];
     pdl_launch_dependents();
-    pdl_wait();
     const bool fresh = a.st->pos == 0;
     float* S = M.S + (size_t)blockIdx.x * D * D;
     float s0[kStepRows][2];
@@ -45,7 +44,8 @@ __global__ void __launch_bounds__(kStepThreads) wkv_step_kernel(const WkvStep a)
             s0[i][1] = !fresh && col + 32 < D && d < D ? S[(size_t)d * D + col + 32] : 0.f;
         }
     };
-    load_rows(0, lane);
+    load_rows(0, lane);                     // the state was left by the last token, the position by the one before the step
+    pdl_wait();
     for (int i = threadIdx.x; i < D; i += kStepThreads) { r[i] = a.row[c0 + i]; k[i] = a.row[n + c0 + i]; v[i] = a.row[2 * n + c0 + i]; }
     for (int i = threadIdx.x; i < rk; i += kStepThreads) inner[i] = i < M.rank ? tanhf(a.row[4 * (size_t)n + i]) : 0.f;
     __syncthreads();
