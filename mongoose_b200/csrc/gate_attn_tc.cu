@@ -338,8 +338,8 @@ __global__ void __launch_bounds__(kFlashThreads, 1) gate_flash_kernel(const __gr
     float* rms = reinterpret_cast<float*>(Vs + 2 * vbytes + 256);               // [warp][2][16]: -log2 e / rms of the warp's keys
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.y, c = h / (A.heads / A.kv_heads), c0 = blockIdx.z * a.per;
-    const int tile_row = (gridDim.x - 1 - blockIdx.x) * 128;                    // the longest rows first
+    const int h = blockIdx.x, c = h / (A.heads / A.kv_heads), c0 = blockIdx.y * a.per;
+    const int tile_row = (gridDim.z - 1 - blockIdx.z) * 128;                    // the longest rows of every head first
     const int first = a.pos0 + a.row0 + tile_row;                               // position of the first query
     const int last = a.pos0 + a.row0 + min(tile_row + 128, a.rows) - 1;
     const int tiles = last / kFlashKeys + 1;
@@ -426,13 +426,14 @@ __global__ void __launch_bounds__(kFlashThreads, 1) gate_flash_kernel(const __gr
             return key <= last ? -kLog2e * A.cache_r[(size_t)key * A.kv_heads + c] : 0.f;
         };
         const int pos = first + r;
-        float next = key_rms(0);
+        float next = key_rms(0), later = tiles > 1 ? key_rms(1) : 0.f;
         bool ok = true;
         for (int j = 0; j < tiles; j++) {
             const int b = j & 1, k0 = j * kFlashKeys + part * 16;
             if (lane < 16) kr[b * 16 + lane] = next;
             __syncwarp();
-            if (j + 1 < tiles) next = key_rms(j + 1);
+            next = later;
+            if (j + 2 < tiles) later = key_rms(j + 2);
             ok = __all_sync(MG_FULL_MASK, bar_wait(s_full + b, (j >> 1) & 1, a.status));
             if (!ok) break;
             tc_fence_after();
@@ -501,24 +502,20 @@ __global__ void __launch_bounds__(kFlashThreads, 1) gate_flash_kernel(const __gr
         if (ok) ok = __all_sync(MG_FULL_MASK, bar_wait(p_empty + ((tiles - 1) & 1), ((tiles - 1) >> 1) & 1, a.status));
         if (ok) {
             tc_fence_after();
-            const int wide = A.kv_heads * A.dim, cols = min(a.per, A.kv_heads - c0) * A.dim, row = tile_row + r;
-            float* out = a.o + ((size_t)row * A.heads + h) * wide + c0 * A.dim;
-            const bool vec = (A.dim & 3) == 0;
+            // 32 columns of 32 rows through shared memory (queries, weights and keys have been consumed), so that a store is 128
+            // bytes of one row
+            const int wide = A.kv_heads * A.dim, cols = min(a.per, A.kv_heads - c0) * A.dim;
+            float* piece = reinterpret_cast<float*>(base) + (warp - 2) * 32 * 33;
             for (int x = part * 32; x < cols; x += 128) {
                 float o[32];
                 tmem_load32(O + mine + x, o);
-                if (row < a.rows) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        if (vec) {
-                            if (x + i < cols) *reinterpret_cast<float4*>(out + x + i) = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-                        } else {
-#pragma unroll
-                            for (int u = 0; u < 4; u++)
-                                if (x + i + u < cols) out[x + i + u] = o[i + u];
-                        }
-                    }
-                }
+                for (int i = 0; i < 32; i++) piece[lane * 33 + i] = o[i];
+                __syncwarp();
+                float* out = a.o + ((size_t)(tile_row + quarter * 32) * A.heads + h) * wide + c0 * A.dim + x + lane;
+#pragma unroll 8
+                for (int i = 0; i < 32; i++)
+                    if (tile_row + quarter * 32 + i < a.rows && x + lane < cols) out[(size_t)i * A.heads * wide] = piece[i * 33 + lane];
                 __syncwarp();
             }
         }
@@ -634,7 +631,7 @@ cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, in
     if (attr != cudaSuccess) return attr;
     for (int q0 = 0; q0 < n; q0 += block_rows) {
         a.row0 = q0; a.rows = std::min(block_rows, n - q0);
-        launch_pdl(gate_flash_kernel, dim3((a.rows + 127) / 128, at.heads, (at.kv_heads + a.per - 1) / a.per), kFlashThreads, flash_smem(a.kb, a.cols), true, s, a);
+        launch_pdl(gate_flash_kernel, dim3(at.heads, (at.kv_heads + a.per - 1) / a.per, (a.rows + 127) / 128), kFlashThreads, flash_smem(a.kb, a.cols), true, s, a);
         __nv_bfloat16* to = (__nv_bfloat16*)out + (size_t)q0 * ld_out;
         if (at.dim % 2 == 0) launch_pdl(gate_mix_kernel<2>, (a.rows + 1) / 2, 256, 0, true, s, at, a.rows, a.o, to, ld_out);
         else launch_pdl(gate_mix_kernel<1>, a.rows, 256, 0, true, s, at, a.rows, a.o, to, ld_out);

@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kThreads, 2) latent_flash_kernel(const __grid_
     uint32_t* tmem_base = reinterpret_cast<uint32_t*>(bars + 14);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.y, row0 = (gridDim.x - 1 - blockIdx.x) * 128;        // the longest rows first
+    const int h = blockIdx.x, row0 = (gridDim.y - 1 - blockIdx.y) * 128;        // the longest rows of every head first
     const int last = min(a.n - 1, row0 + 127);
     const int len = a.pos0 + a.n;
     const int tiles = (a.pos0 + last) / kKeys + 1;
@@ -293,7 +293,7 @@ cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0
         return cudaErrorInvalidValue;
     static cudaError_t attr = cudaFuncSetAttribute((const void*)latent_flash_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (attr != cudaSuccess) return attr;
-    launch_pdl(latent_flash_kernel, dim3((n + 127) / 128, at.heads), kThreads, geo.smem, true, s, f);
+    launch_pdl(latent_flash_kernel, dim3(at.heads, (n + 127) / 128), kThreads, geo.smem, true, s, f);
     *launches += 3;
     return cudaGetLastError();
 }
