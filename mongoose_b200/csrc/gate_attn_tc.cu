@@ -1,4 +1,5 @@
-// Sigmoid attention with mixed heads over a portion of a prompt, on the tensor cores.
+// Sigmoid attention with mixed heads over a portion of a prompt, on the tensor cores: for heads of up to 128 one head at a
+// time, mixed in the outputs (gate_flash_kernel, gate_mix_kernel); for wider ones as follows.
 //
 // Mixing couples every head at every (query, key) pair, so a CTA owns a tile of 128 queries x BN keys for
 // ALL heads: each head's scores land in their own TMEM columns (heads x BN <= 512), then a thread reads
