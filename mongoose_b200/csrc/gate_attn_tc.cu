@@ -598,8 +598,6 @@ __global__ void __launch_bounds__(256) key_transpose_kernel(const __nv_bfloat16*
 template <int HP>
 cudaError_t scores(const ScoreArgs& a, cudaStream_t s) {
     using G = Geo<HP>;
-    static cudaError_t attr = cudaFuncSetAttribute((const void*)gate_scores_kernel<HP>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::bytes);
-    if (attr != cudaSuccess) return attr;
     launch_pdl(gate_scores_kernel<HP>, dim3(pad_to(a.pos0 + a.row0 + a.rows, 64) / G::bn, (a.rows + 127) / 128), kThreads, G::bytes, true, s, a);
     return cudaGetLastError();
 }
@@ -628,8 +626,6 @@ cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, in
         !make_head_map(&a.k, at.cache, at.dim_s, at.kv_heads, at.max_seq, at.dim_s, (long long)at.kv_heads * at.dim_s, kFlashKeys) ||
         !make_tile_map(&a.v, vt, ldv, at.kv_heads * at.dim, 1, ldv, (long long)at.kv_heads * at.dim * ldv, a.cols))
         return cudaErrorInvalidValue;
-    static const cudaError_t attr = cudaFuncSetAttribute((const void*)gate_flash_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, flash_smem(2, kFlashCols));
-    if (attr != cudaSuccess) return attr;
     for (int q0 = 0; q0 < n; q0 += block_rows) {
         a.row0 = q0; a.rows = std::min(block_rows, n - q0);
         launch_pdl(gate_flash_kernel, dim3(at.heads, (at.kv_heads + a.per - 1) / a.per, (a.rows + 127) / 128), kFlashThreads, flash_smem(a.kb, a.cols), true, s, a);
@@ -642,6 +638,14 @@ cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, in
 }
 
 }  // namespace
+
+cudaError_t gate_attn_tc_attrs() {
+    if (cudaError_t c = allow_smem(gate_scores_kernel<4>, Geo<4>::bytes)) return c;
+    if (cudaError_t c = allow_smem(gate_scores_kernel<8>, Geo<8>::bytes)) return c;
+    if (cudaError_t c = allow_smem(gate_scores_kernel<16>, Geo<16>::bytes)) return c;
+    if (cudaError_t c = allow_smem(gate_scores_kernel<32>, Geo<32>::bytes)) return c;
+    return allow_smem(gate_flash_kernel, flash_smem(2, kFlashCols));
+}
 
 bool gate_attn_tc_fits(const GateAttn& at) { return at.heads <= 32; }
 

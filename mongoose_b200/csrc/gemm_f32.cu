@@ -243,8 +243,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_kernel(const __grid_cons
 
 template <int NT>
 cudaError_t run(const Args& a, int parts, cudaStream_t s) {
-    static const cudaError_t attr = cudaFuncSetAttribute((const void*)gemm_f32_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<NT>::bytes);
-    if (attr != cudaSuccess) return attr;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((a.g.rows + 127) / 128, (a.g.n + NT - 1) / NT, parts);
     cfg.blockDim = dim3(kThreads);
@@ -269,6 +267,11 @@ int sm_count() {
 }
 
 }  // namespace
+
+cudaError_t gemm_f32_attrs() {
+    if (cudaError_t c = allow_smem(gemm_f32_kernel<32>, Shape<32>::bytes)) return c;
+    return allow_smem(gemm_f32_kernel<64>, Shape<64>::bytes);
+}
 
 cudaError_t launch_gemm_f32(const GemmF32& g, cudaStream_t s) {
     Args a{};

@@ -231,8 +231,6 @@ int sm_count() {
 
 template <int BN>
 cudaError_t run(const GemmTC& g, cudaStream_t s) {
-    static cudaError_t attr = cudaFuncSetAttribute((const void*)gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<BN>::bytes);
-    if (attr != cudaSuccess) return attr;
     const int cols = g.mode == GEMM_SILU_BF16 ? BN / 2 : BN, gx = (g.n + cols - 1) / cols, gy = (g.m + 127) / 128, tiles = gx * gy * g.batch;
     return launch_pdl(gemm_tc_kernel<BN>, tiles < sm_count() ? tiles : sm_count(), kThreads, Geo<BN>::bytes, true, s, g, gx, gy, tiles);
 }
@@ -265,6 +263,12 @@ int gemm_tc_bn(int m, int n, int batch) {
         if (bn == 64 || t < least) { best = bn; least = t; }
     }
     return best;
+}
+
+cudaError_t gemm_tc_attrs() {
+    if (cudaError_t c = allow_smem(gemm_tc_kernel<64>, Geo<64>::bytes)) return c;
+    if (cudaError_t c = allow_smem(gemm_tc_kernel<128>, Geo<128>::bytes)) return c;
+    return allow_smem(gemm_tc_kernel<256>, Geo<256>::bytes);
 }
 
 cudaError_t launch_gemm_tc(const GemmTC& g, cudaStream_t s) {

@@ -259,6 +259,8 @@ bool latent_attn_tc_fits(const LatentAttn& at) {
     return at.vdim <= 256 && at.dim_s <= 256 && at.rot_s <= 256 && geometry(at).smem <= 226 * 1024;
 }
 
+cudaError_t latent_attn_tc_attrs() { return allow_smem(latent_flash_kernel, 226 * 1024); }
+
 cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0, int n, void* keys, void* vt, int ldv, void* out, int ld_out,
                                   int* status, int* launches, cudaStream_t s) {
     const int len = pos0 + n;
@@ -291,8 +293,6 @@ cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0
         !make_tile_map(&f.kr, (const __nv_bfloat16*)at.cache + at.rank_s, at.rot_s, len, 1, at.row(), (long long)at.max_seq * at.row(), kKeys) ||
         !make_tile_map(&f.v, vt, len, at.vdim, at.heads, ldv, (long long)at.vdim * ldv, geo.vp))
         return cudaErrorInvalidValue;
-    static cudaError_t attr = cudaFuncSetAttribute((const void*)latent_flash_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (attr != cudaSuccess) return attr;
     launch_pdl(latent_flash_kernel, dim3(at.heads, (n + 127) / 128), kThreads, geo.smem, true, s, f);
     *launches += 3;
     return cudaGetLastError();

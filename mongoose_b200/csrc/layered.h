@@ -162,6 +162,7 @@ cudaError_t launch_latent_q_rows(const LatentAttn& at, const float* q, int pos0,
 // bf16 prompts on the tensor cores (latent_attn_tc.cu): keys [max_seq][heads * dim_s] and values, transposed,
 // [heads * vdim][ldv] of positions [0, pos0 + n) are formed from the cache, then attention in tiles of 128 queries.
 bool latent_attn_tc_fits(const LatentAttn& at);
+cudaError_t latent_attn_tc_attrs();
 cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0, int n, void* keys, void* vt, int ldv, void* out, int ld_out,
                                   int* status, int* launches, cudaStream_t s);
 
@@ -180,6 +181,7 @@ cudaError_t launch_wkv_mix(const float* h, const float* prev, const float* const
 // act[n][ld] = tanh of the decay's inner projection (the sum of `slices` slabs [n][ldp]) as two bf16 parts
 cudaError_t launch_wkv_inner(const float* inner, int ldp, int slices, int rank, int n, void* act, int ld, cudaStream_t s);
 bool wkv_rows_fits(const Wkv& wk);
+cudaError_t wkv_attrs();
 // proj rows as WkvStep's, decays [n][heads * dim]; out [n][heads * dim] raw outputs
 cudaError_t launch_wkv_rows(const Wkv& wk, const float* proj, int ldp, const float* decay, int pos0, int n, float* out, cudaStream_t s);
 
@@ -237,6 +239,7 @@ struct GemmF32 {
     long long group_stride;         // elements between them
     int* status;                    // set by a wait that ran out
 };
+cudaError_t gemm_f32_attrs();
 cudaError_t launch_gemm_f32(const GemmF32& g, cudaStream_t s);
 // queries: normed, times temperature, score scale and key-norm weight; keys: raw rows into the cache
 cudaError_t launch_qk_rows(const GateAttn& at, const float* proj, int ldp, int q_col, int k_col, int pos0, int n, void* qh,
@@ -249,6 +252,7 @@ size_t gate_attn_rows_smem(const GateAttn& at, bool f32, int* tile);
 bool gate_attn_tc_fits(const GateAttn& at);
 int gate_attn_tc_rows(const GateAttn& at, int max_seq, int max_rows, size_t budget);
 size_t gate_attn_tc_bytes(const GateAttn& at, int max_seq, int block_rows);
+cudaError_t gate_attn_tc_attrs();
 cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* weights, int block_rows, void* vt,
                                 void* out, int ld_out, int* status, int* launches, cudaStream_t s);
 // x += norm(z) or x += norm(half the sum of two normed branches); act = x

@@ -331,6 +331,8 @@ int layered_shapes(Layered& m, int sms, std::string* why) {
     // the phase kernels stage a whole input vector per CTA
     if (kmax > 48 * 1024) { *why = "a matrix with rows of more than 49152 values"; return MG_ERR_UNSUPPORTED; }
     if (rows_attrs(kmax) != cudaSuccess) { *why = "kernel attributes"; return MG_ERR_CUDA; }
+    for (cudaError_t (*attrs)() : {gemm_tc_attrs, gemm_f32_attrs, gate_attn_tc_attrs, latent_attn_tc_attrs, wkv_attrs})
+        if (attrs() != cudaSuccess) { *why = "kernel attributes"; return MG_ERR_CUDA; }
     if (moe_smem && moe_step_attrs(moe_smem) != cudaSuccess) { *why = "kernel attributes"; return MG_ERR_CUDA; }
     return MG_OK;
 }

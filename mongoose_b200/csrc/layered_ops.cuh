@@ -359,6 +359,13 @@ __device__ __forceinline__ void attend(const GateAttn& A, const AttnSmem<KT>& sm
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
 
+// Dynamic shared memory that a kernel may be launched with on the current device.  The limit belongs to the device, so every engine
+// sets it when it is created.
+template <typename F>
+inline cudaError_t allow_smem(F* kern, size_t bytes) {
+    return cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 // Launch with the programmatic attribute, so that the kernel may start under its predecessor's tail.
 template <typename F, typename... Args>
 inline cudaError_t launch_pdl(F kern, dim3 grid, int threads, size_t smem, bool pdl, cudaStream_t s, Args... args) {

@@ -343,11 +343,12 @@ template <int KPT>
 cudaError_t scan_for(const Wkv& wk, const float* proj, int ldp, const float* decay, int pos0, int n, float* out, cudaStream_t s) {
     using G = Scan<KPT>;
     constexpr size_t smem = G::smem(G::tile);
-    static cudaError_t attr = cudaFuncSetAttribute((const void*)wkv_scan_kernel<KPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (attr != cudaSuccess) return attr;
     launch_pdl(wkv_scan_kernel<KPT>, dim3(wk.heads, (wk.dim + G::cols - 1) / G::cols), kScanThreads, smem, true, s, wk, proj, ldp, decay, pos0, n, out);
     return cudaGetLastError();
 }
+
+template <int KPT>
+cudaError_t allow_scan() { return allow_smem(wkv_scan_kernel<KPT>, Scan<KPT>::smem(Scan<KPT>::tile)); }
 
 template <typename AT>
 cudaError_t mix_for(const float* h, const float* prev, const float* const mu[5], int pos0, int n, int width, AT* act, int ld_act, long long stride,
@@ -377,6 +378,12 @@ cudaError_t launch_wkv_inner(const float* inner, int ldp, int slices, int rank, 
 }
 
 bool wkv_rows_fits(const Wkv& wk) { return wk.dim <= 256; }
+
+cudaError_t wkv_attrs() {
+    if (cudaError_t c = allow_scan<2>()) return c;
+    if (cudaError_t c = allow_scan<4>()) return c;
+    return allow_scan<8>();
+}
 
 cudaError_t launch_wkv_rows(const Wkv& wk, const float* proj, int ldp, const float* decay, int pos0, int n, float* out, cudaStream_t s) {
     if (wk.dim <= 64) return scan_for<2>(wk, proj, ldp, decay, pos0, n, out, s);

@@ -1,0 +1,71 @@
+"""What the engine's host code asks of the CUDA runtime, seen through a stand-in for it (fake_cuda.cpp):
+the library's own objects, host memory for device memory, kernels that do nothing.  Its results mean nothing;
+which launches it makes, and which a device would refuse, does."""
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from mongoose_b200 import _lib, build
+from mongoose_b200.layered import (MATH_BF16, MATH_F32, GateAttention, LatentAttention, LayeredConfig, LayeredInference, MatrixMemory,
+                                   MixtureOfExperts, ParallelLayer, PrenormLayer, Wkv, slot_shapes)
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def fake_path(tmp_path_factory):
+    build.build()
+    out = str(tmp_path_factory.mktemp("fake") / "libmongoose_fake.so")
+    objs = [os.path.join(build.HERE, "build", u.replace(".cu", ".o")) for u in build.UNITS]
+    subprocess.run(["g++", "-O1", "-fPIC", "-shared", "-I", os.path.join(os.path.dirname(os.path.dirname(build._nvcc())), "include"), "-Wl,-Bsymbolic",
+                    *objs, os.path.join(HERE, "fake_cuda.cpp"), "-o", out, "-ldl", "-lpthread"], check=True, capture_output=True, text=True)
+    return out
+
+
+@pytest.fixture
+def fake(fake_path, monkeypatch):
+    lib = _lib._open(fake_path, True)
+    lib.fake_in_use.restype = _lib.sz
+    lib.fake_memory.argtypes = [_lib.sz]
+    monkeypatch.setattr(_lib, "_lib", lib)
+    lib.fake_memory(8 << 30)
+    lib.fake_forget()
+    return lib
+
+
+def layered(fake, layers, math=MATH_BF16, width=96, device=0, **kw):
+    cfg = LayeredConfig("t", width, 50, tuple(layers), 1e-5, max_seq=512, math=math, **kw)
+    e = LayeredInference(cfg, device)
+    for idx, _, _, r, c in slot_shapes(cfg):
+        e.SetWeightBF16(idx, np.zeros(max(r, 1) * c, np.uint16))
+    e.BuildFusedDispatch()
+    return e
+
+
+def parallel(dim=64, heads=4, kv=2, ffn=160):
+    return ParallelLayer(GateAttention(heads, kv, dim, 0.2), MatrixMemory(2, 16, 24, 5.0), ffn)
+
+
+def prenorm():
+    moe = MixtureOfExperts(4, 2, 40, 72)
+    return [PrenormLayer(LatentAttention(4, 32, 16, 40, 72, 64, 0.1, 1e4), moe), PrenormLayer(Wkv(3, 32, 24), moe)]
+
+
+def use(e, n=300):
+    e.Forward([1] * n, 0, [n - 1])
+    e.Forward([1] * 7, n, [6])
+    e.Forward([1], n + 7, [0])
+
+
+@pytest.mark.parametrize("kind", ["dim64", "dim256", "latent"])
+@pytest.mark.parametrize("math", [MATH_BF16, MATH_F32])
+def test_every_device_of_a_process_takes_the_kernels(fake, kind, math):
+    """How much shared memory a kernel may be launched with belongs to the device."""
+    layers = prenorm() if kind == "latent" else [parallel(int(kind[3:]))]
+    for device in (0, 1, 2):
+        e = layered(fake, layers, math, device=device)
+        use(e)
+        e.close()
+    assert fake.fake_refused() == 0
