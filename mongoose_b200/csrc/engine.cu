@@ -900,10 +900,12 @@ int build_mega(mg_engine* e) {
     std::string why;
     bool ok = mega_feasible(e, &why);
     if (ok) {
-        int per_sm = 0;
+        int per_sm = 0, most = 0;
         const void* kern = mega_fn(e);
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->mk_smem) != cudaSuccess ||
-            cudaFuncSetAttribute(mega_fn(e, true), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->mk_smem) != cudaSuccess ||
+        // all that a device has, not what this model needs: the limit is shared by the engines of a process
+        if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->cfg.device) != cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
+            cudaFuncSetAttribute(mega_fn(e, true), cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, MK_THREADS, e->mk_smem) != cudaSuccess ||
             per_sm < 1) {
             cudaGetLastError();

@@ -399,7 +399,7 @@ template <typename KT>
 cudaError_t attend_for(const LatentStep& a, size_t smem, bool pdl, cudaStream_t s) {
     const dim3 grid(a.splits, (a.at.heads + a.group - 1) / a.group, a.tokens);
     auto run = [&](auto kern) {
-        cudaError_t c = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t c = allow_smem(kern, kModelSmem);
         return c != cudaSuccess ? c : launch_pdl(kern, grid, kThreads, smem, pdl, s, a);
     };
     switch (attend_sets(a.at, a.group)) {
@@ -444,8 +444,7 @@ cudaError_t launch_latent_value(const LatentStep& a, bool f32_out, bool pdl, cud
     const dim3 grid(a.at.heads * ((a.at.vdim + kValueRows - 1) / kValueRows), a.tokens);
     const size_t smem = (size_t)(kValueGroups * a.at.ld + a.splits) * sizeof(float);
     if (smem > 48 * 1024) {
-        cudaError_t c = cudaFuncSetAttribute(f32_out ? (const void*)latent_value_kernel<float> : (const void*)latent_value_kernel<__nv_bfloat16>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t c = allow_smem(f32_out ? latent_value_kernel<float> : latent_value_kernel<__nv_bfloat16>, std::max(smem, kModelSmem));
         if (c != cudaSuccess) return c;
     }
     return f32_out ? launch_pdl(latent_value_kernel<float>, grid, kThreads, smem, pdl, s, a)

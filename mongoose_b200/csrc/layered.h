@@ -93,7 +93,8 @@ constexpr int kMaxExperts = 1024, kMaxTop = 64;
 
 // ---- one token (layered_decode.cu) -------------------------------------------------------------
 // Products with bf16 matrices (layered_rows.cuh), K a multiple of 64.
-cudaError_t rows_attrs(int K);          // for rows of up to K columns
+constexpr int kMaxRow = 48 * 1024;      // columns, at most: a CTA holds a whole vector
+cudaError_t rows_attrs();
 cudaError_t launch_rows(const PhaseArgs& a, int epi, int sms, bool pdl, cudaStream_t s);
 // two independent matrices
 cudaError_t launch_rows_pair(const PhaseArgs& a, const PhaseArgs& b, int sms, bool pdl, cudaStream_t s);
@@ -195,7 +196,7 @@ struct MoeStep {
     float* out;                 // [width]
 };
 size_t moe_step_smem(const Moe& m);
-cudaError_t moe_step_attrs(size_t bytes);
+cudaError_t moe_attrs();
 cudaError_t launch_moe_up(const MoeStep& a, int sms, bool pdl, cudaStream_t s);
 cudaError_t launch_moe_down(const MoeStep& a, int sms, bool pdl, cudaStream_t s);
 struct MoeRows {                // workspace of a portion

@@ -181,7 +181,7 @@ cudaError_t step_for(const MixerStep& a, size_t smem, bool pdl, cudaStream_t s) 
     const int ep = attn_pairs(a.at);
     const int grid = a.n_mem + a.splits;
     auto run = [&](auto kern) {
-        cudaError_t c = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t c = allow_smem(kern, std::max(smem, kModelSmem));
         return c != cudaSuccess ? c : launch_pdl(kern, grid, kAttnThreads, smem, pdl, s, a);
     };
     switch (ep) {
@@ -216,17 +216,15 @@ inline int rows_grid(int K, int rows, int R, int most) {
 
 }  // namespace
 
-cudaError_t rows_attrs(int K) {
-    const int bytes = (int)rows_smem(K);
-    auto allow = [&](const void* kern) { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+cudaError_t rows_attrs() {
     for (int k : {2048, 4096})
         for (int R : {1, 2, 4, 8}) {
             const cudaError_t c = by_rows(R, k, [&](auto r, auto ahead) {
                 constexpr int RR = decltype(r)::value, A = decltype(ahead)::value;
-                for (const void* f : {(const void*)rows_kernel<EPI_STORE, RR, A>, (const void*)rows_kernel<EPI_GELU, RR, A>, (const void*)rows_kernel<EPI_LOGITS, RR, A>,
-                                      (const void*)rows_pair_kernel<RR, A>, (const void*)rows_parts_kernel<RR, A>})
-                    if (cudaError_t e = allow(f)) return e;
-                return cudaSuccess;
+                for (auto* f : {rows_kernel<EPI_STORE, RR, A>, rows_kernel<EPI_GELU, RR, A>, rows_kernel<EPI_LOGITS, RR, A>})
+                    if (cudaError_t e = allow_smem(f, rows_smem(kMaxRow))) return e;
+                if (cudaError_t e = allow_smem(rows_pair_kernel<RR, A>, rows_smem(kMaxRow))) return e;
+                return allow_smem(rows_parts_kernel<RR, A>, rows_smem(kMaxRow));
             });
             if (c != cudaSuccess) return c;
         }
@@ -283,7 +281,7 @@ cudaError_t launch_mixer_join(const MixerStep& a, bool pdl, cudaStream_t s) {
 
 cudaError_t launch_resolve(const ResolveArgs& a, bool pdl, cudaStream_t s) {
     const size_t smem = ((size_t)a.p.K + 72) * sizeof(float);
-    cudaError_t c = cudaFuncSetAttribute((const void*)resolve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t c = allow_smem(resolve_kernel, kModelSmem);
     return c != cudaSuccess ? c : launch_pdl(resolve_kernel, 1, 256, smem, pdl, s, a);
 }
 

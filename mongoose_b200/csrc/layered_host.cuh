@@ -308,7 +308,6 @@ int layered_shapes(Layered& m, int sms, std::string* why) {
     m.kw = pad_to(c.width, 64);
     m.kl = pad_to(2 * c.width, 64);
     int kmax = std::max(m.kw, c.loop_times ? m.kl : 0);
-    size_t moe_smem = 0;
     m.max_rows = std::min(c.max_seq, 2048);
     m.logit_rows = std::max(1, std::min(std::min(128, m.max_rows), (int)((64u << 20) / ((size_t)c.vocab * 4))));
     for (LayerWeights& l : m.layers) {
@@ -317,7 +316,6 @@ int layered_shapes(Layered& m, int sms, std::string* why) {
         m.np = std::max(m.np, pad_to(l.proj_rows(), 4));
         for (int k : {l.parallel() ? l.kat() : l.kout(), l.parallel() ? l.kmem() : 0, l.parallel() ? l.c.ffn_dim : 0, l.la.q_rank})
             kmax = std::max(kmax, pad_to(k, 64));
-        if (l.moe.experts) moe_smem = std::max(moe_smem, moe_step_smem(l.moe));
     }
     for (int pass = 0, i = 0; i < c.n_layers;) {
         const bool looped = c.loop_times && i >= c.loop_start && i < c.loop_stop;
@@ -329,11 +327,9 @@ int layered_shapes(Layered& m, int sms, std::string* why) {
         if (looped && i == c.loop_stop && ++pass < c.loop_times) i = c.loop_start;
     }
     // the phase kernels stage a whole input vector per CTA
-    if (kmax > 48 * 1024) { *why = "a matrix with rows of more than 49152 values"; return MG_ERR_UNSUPPORTED; }
-    if (rows_attrs(kmax) != cudaSuccess) { *why = "kernel attributes"; return MG_ERR_CUDA; }
-    for (cudaError_t (*attrs)() : {gemm_tc_attrs, gemm_f32_attrs, gate_attn_tc_attrs, latent_attn_tc_attrs, wkv_attrs})
+    if (kmax > kMaxRow) { *why = "a matrix with rows of more than 49152 values"; return MG_ERR_UNSUPPORTED; }
+    for (cudaError_t (*attrs)() : {rows_attrs, moe_attrs, gemm_tc_attrs, gemm_f32_attrs, gate_attn_tc_attrs, latent_attn_tc_attrs, wkv_attrs})
         if (attrs() != cudaSuccess) { *why = "kernel attributes"; return MG_ERR_CUDA; }
-    if (moe_smem && moe_step_attrs(moe_smem) != cudaSuccess) { *why = "kernel attributes"; return MG_ERR_CUDA; }
     return MG_OK;
 }
 

@@ -360,7 +360,9 @@ __device__ __forceinline__ void attend(const GateAttn& A, const AttnSmem<KT>& sm
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
 
 // Dynamic shared memory that a kernel may be launched with on the current device.  The limit belongs to the device, so every engine
-// sets it when it is created.
+// sets it when it is created.  All engines of a process share it: a kernel whose need depends on the model gets what any of them
+// may need, kModelSmem, so that a small model does not take it from a large one.
+constexpr size_t kModelSmem = 224 * 1024;
 template <typename F>
 inline cudaError_t allow_smem(F* kern, size_t bytes) {
     return cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

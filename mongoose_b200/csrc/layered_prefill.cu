@@ -635,7 +635,7 @@ cudaError_t attn_rows_for(const GateAttn& at, const void* qh, int pos0, int n, v
     const size_t smem = attn_smem(at, NQ, sizeof(KT), 32, &tile);
     if (!smem) return cudaErrorInvalidValue;
     auto run = [&](auto kern) {
-        cudaError_t c = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t c = allow_smem(kern, kModelSmem);
         if (c != cudaSuccess) return c;
         launch_pdl(kern, (n + NQ - 1) / NQ, kAttnThreads, smem, true, s, at, (const KT*)qh, pos0, n, tile, (KT*)out, ld_out);
         return cudaGetLastError();

@@ -281,9 +281,9 @@ constexpr int kDownRows = 4;
 
 size_t moe_step_smem(const Moe& m) { return (size_t)std::max(m.ldw + m.experts, m.top * m.ffs + m.shared_ffs) * sizeof(float); }
 
-cudaError_t moe_step_attrs(size_t bytes) {
-    cudaError_t c = cudaFuncSetAttribute((const void*)moe_up_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return c != cudaSuccess ? c : cudaFuncSetAttribute((const void*)moe_down_kernel<kDownRows>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+cudaError_t moe_attrs() {
+    cudaError_t c = allow_smem(moe_up_kernel, kModelSmem);
+    return c != cudaSuccess ? c : allow_smem(moe_down_kernel<kDownRows>, kModelSmem);
 }
 
 cudaError_t launch_moe_up(const MoeStep& a, int sms, bool pdl, cudaStream_t s) {

@@ -1,6 +1,7 @@
 """What the engine's host code asks of the CUDA runtime, seen through a stand-in for it (fake_cuda.cpp):
 the library's own objects, host memory for device memory, kernels that do nothing.  Its results mean nothing;
 which launches it makes, and which a device would refuse, does."""
+import glob
 import os
 import subprocess
 
@@ -8,6 +9,8 @@ import numpy as np
 import pytest
 
 from mongoose_b200 import _lib, build
+from mongoose_b200 import configs as mc
+from mongoose_b200.fused_infer import CUDAFusedInference
 from mongoose_b200.layered import (MATH_BF16, MATH_F32, GateAttention, LatentAttention, LayeredConfig, LayeredInference, MatrixMemory,
                                    MixtureOfExperts, ParallelLayer, PrenormLayer, Wkv, slot_shapes)
 
@@ -69,3 +72,43 @@ def test_every_device_of_a_process_takes_the_kernels(fake, kind, math):
         use(e)
         e.close()
     assert fake.fake_refused() == 0
+
+
+@pytest.mark.parametrize("math", [MATH_BF16, MATH_F32])
+def test_a_smaller_engine_takes_nothing_from_a_larger_one(fake, math):
+    for layers, small, w in (([parallel(128, 8, 8, 30000)], [parallel(16, 2, 1, 64)], 128),
+                             ([PrenormLayer(l.mixer, MixtureOfExperts(4, 2, 12000, 16000)) for l in prenorm()], prenorm(), 2048)):
+        a = layered(fake, layers, math, width=w)
+        b = layered(fake, small, math, width=32)
+        use(b)
+        use(a)
+        a.close()
+        b.close()
+    assert fake.fake_refused() == 0
+
+
+def dense(fake, cfg):
+    e = CUDAFusedInference(cfg)
+    for idx in range(12 * cfg.n_layers + 2):
+        s = idx % 12 if idx < 12 * cfg.n_layers else -1
+        if s in mc.MATRIX_SLOTS:
+            e.SetWeight(idx, np.zeros(cfg.matrix_shape(s), np.float32))
+        elif s in (mc.SLOT_NORM1, mc.SLOT_NORM2) or idx == 12 * cfg.n_layers:
+            e.SetWeight(idx, np.zeros(cfg.dim, np.float32))
+        elif s == -1:
+            e.SetWeight(idx, np.zeros((cfg.vocab, cfg.dim), np.float32))
+    e.BuildFusedDispatch()
+    return e
+
+
+@pytest.mark.parametrize("mega", [True, False])
+@pytest.mark.parametrize("sizes", [({"ffn_dim": 9600}, {}), ({"max_seq": 16000}, {}), ({"ffn_dim": 9600, "max_seq": 9000}, {"max_seq": 64})])
+def test_dense_engines_take_nothing_from_each_other(fake, monkeypatch, mega, sizes):
+    if not mega:
+        monkeypatch.setenv("MG_NO_MEGA", "1")
+    engines = [dense(fake, mc.TINY.with_(**s)) for s in (*sizes, sizes[0])]
+    for e in engines:
+        e.Generate([1] * 40, 3)
+    assert fake.fake_refused() == 0
+    for e in engines:
+        e.close()
