@@ -12,6 +12,9 @@
 // B200: prompt of 512 tokens, six layers of 1.1B widths, Q8_0: 101 ms one by one, 2.2 ms so (0.25 PFLOP/s counting
 // each of the three parts' products).  Short prompts are bound by the nine launches of a layer, long ones by the products.
 #include "dense_prompt.h"
+
+#include <type_traits>
+
 #include "gemm_tc.h"
 #include "umma.cuh"
 
@@ -390,7 +393,7 @@ __global__ void __launch_bounds__(128) prompt_attn_kernel(const PromptAttn a) {
         if (q0 + r < a.tokens) v = *reinterpret_cast<const float4*>(a.q + (size_t)(q0 + r) * q_dim + head * HD + 4 * c);
         reinterpret_cast<float4*>(Q)[i] = v;
     }
-    const int last = a.pos0 + min(q0 + kAttnQ, a.tokens) - 1;      // position of the last query
+    const int first = a.pos0 + q0, last = a.pos0 + min(q0 + kAttnQ, a.tokens) - 1;      // positions of the first and the last query
     float o[4][E] = {}, mx[4], l[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) { mx[i] = -INFINITY; l[i] = 0.f; }
@@ -431,7 +434,7 @@ __global__ void __launch_bounds__(128) prompt_attn_kernel(const PromptAttn a) {
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const int pos = a.pos0 + q0 + 4 * ty + i;
+            const int pos = first + 4 * ty + i;
             float m = mx[i];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -456,28 +459,34 @@ __global__ void __launch_bounds__(128) prompt_attn_kernel(const PromptAttn a) {
         }
         __syncwarp();                                   // a query's 16 threads are in one warp
         const int n = min(kAttnK, (last - k0 + 4) & ~3);        // rows past `last` are zeros with zero weight
-        for (int k = 0; k < n; k += 4) {
-            float4 p[4];
+        auto add_values = [&](auto masked) {
+            for (int k = 0; k < n; k += 4) {
+                float4 p[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) p[i] = *reinterpret_cast<const float4*>(P + (4 * ty + i) * PS + k);
+                for (int i = 0; i < 4; i++) p[i] = *reinterpret_cast<const float4*>(P + (4 * ty + i) * PS + k);
 #pragma unroll
-            for (int kk = 0; kk < 4; kk++) {
-                const float* v = V + (k + kk) * HD;
-                float x[E];
-                if (HD == 32) {
-                    *reinterpret_cast<float2*>(x) = *reinterpret_cast<const float2*>(v + 2 * tx);
-                } else {
+                for (int kk = 0; kk < 4; kk++) {
+                    const float* v = V + (k + kk) * HD;
+                    float x[E];
+                    if (HD == 32) {
+                        *reinterpret_cast<float2*>(x) = *reinterpret_cast<const float2*>(v + 2 * tx);
+                    } else {
 #pragma unroll
-                    for (int e = 0; e < E / 4; e++) *reinterpret_cast<float4*>(x + 4 * e) = *reinterpret_cast<const float4*>(v + 4 * tx + 64 * e);
-                }
+                        for (int e = 0; e < E / 4; e++) *reinterpret_cast<float4*>(x + 4 * e) = *reinterpret_cast<const float4*>(v + 4 * tx + 64 * e);
+                    }
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float w = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
+                    for (int i = 0; i < 4; i++) {
+                        if (decltype(masked)::value && k0 + k + kk > first + 4 * ty + i) continue;
+                        const float w = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
 #pragma unroll
-                    for (int e = 0; e < E; e++) o[i][e] = fmaf(w, x[e], o[i][e]);
+                        for (int e = 0; e < E; e++) o[i][e] = fmaf(w, x[e], o[i][e]);
+                    }
                 }
             }
-        }
+        };
+        // a row behind a query counts for nothing, not for zero times what it holds: its values may have overflowed fp16
+        if (k0 + n - 1 <= first) add_values(std::false_type{});
+        else add_values(std::true_type{});
         __syncwarp();
     }
 #pragma unroll

@@ -89,3 +89,31 @@ def test_batches_on_the_graph_of_kernels(cuda, mglib, monkeypatch):
         same_cache(cfg, a, b, 50)
     finally:
         a.close(); b.close()
+
+
+@pytest.mark.parametrize("cfg", [ODD, HD64, HD128], ids=lambda c: c.name)
+def test_a_value_that_overflows_leaves_earlier_tokens_alone(cuda, mglib, cfg):
+    """One token's value is beyond fp16 (infinite in the cache): the tokens before it, in the same tile of keys or
+    an earlier one, are as they are without it."""
+    n, at = 90, 77
+    tokens = [int(t) % (cfg.vocab - 1) for t in gen.prompt_ids(11, n, cfg.vocab)]
+    tokens[at] = cfg.vocab - 1
+    embed = gen.tensor_f32(12, 1, cfg.vocab, cfg.dim)
+    embed[:, 0] = 0
+    embed[-1] = 0
+    embed[-1, 0] = 1                        # of the normed input nothing but column 0, which is 0 for every other token
+    wv = gen.tensor_f32(12, 2, cfg.kv_dim, cfg.dim)
+    wv[0, 0] = 2e4
+    a, b = CUDAFusedInference(cfg), CUDAFusedInference(cfg)
+    try:
+        for e in (a, b):
+            fill_models(cfg, seed=12, jitter=0.1, engine=e)
+            e.SetWeight(12 * cfg.n_layers + 1, embed)
+            e.SetWeight(mc.SLOT_WV, wv)
+        a.Forward(tokens, 0)
+        for i, t in enumerate(tokens[:at]):
+            b.StepToken(t, i)
+        assert np.isinf(a.ReadKV(0, at, 1)[1].view(np.float16)[0, 0])
+        same_cache(cfg, a, b, at)
+    finally:
+        a.close(); b.close()
