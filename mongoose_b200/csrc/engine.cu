@@ -217,7 +217,8 @@ struct mg_engine {
     size_t tape_bytes = 0;
     bool built = false;
     bool use_graph = true;
-    bool use_pdl = true;
+    bool use_pdl = true;                // kernels of a step start under their predecessors
+    bool prompt_pdl = true;             // those of a layer-described model's prompt
     long long launches = 0;
     int capture_kernels = 0;            // kernels enqueued by the current enqueue_step
     size_t dev_bytes = 0;
@@ -1354,7 +1355,7 @@ void read_env(mg_engine* e) {
     env = getenv("MG_NO_MEGA");
     if (env && env[0] == '1') e->use_mega = false;
     env = getenv("MG_NO_PDL");
-    if (env && env[0] == '1') e->use_pdl = false;
+    if (env && env[0] == '1') e->use_pdl = e->prompt_pdl = false;
     // Kernels read the position before they wait for their predecessor, which is right behind the edge between two graph
     // launches: without graphs a step's kernels could start under the last step's lm_head, which moves it.
     if (!e->use_graph) e->use_pdl = false;

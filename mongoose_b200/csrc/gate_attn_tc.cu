@@ -596,9 +596,9 @@ __global__ void __launch_bounds__(256) key_transpose_kernel(const __nv_bfloat16*
 }
 
 template <int HP>
-cudaError_t scores(const ScoreArgs& a, cudaStream_t s) {
+cudaError_t scores(const ScoreArgs& a, bool pdl, cudaStream_t s) {
     using G = Geo<HP>;
-    launch_pdl(gate_scores_kernel<HP>, dim3(pad_to(a.pos0 + a.row0 + a.rows, 64) / G::bn, (a.rows + 127) / 128), kThreads, G::bytes, true, s, a);
+    launch_pdl(gate_scores_kernel<HP>, dim3(pad_to(a.pos0 + a.row0 + a.rows, 64) / G::bn, (a.rows + 127) / 128), kThreads, G::bytes, pdl, s, a);
     return cudaGetLastError();
 }
 
@@ -615,7 +615,7 @@ size_t bytes_per_row(const GateAttn& at, int max_seq) {
 }
 
 cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* work, int block_rows, const void* vt, int ldv,
-                         void* out, int ld_out, int* status, int* launches, cudaStream_t s) {
+                         void* out, int ld_out, int* status, int* launches, bool pdl, cudaStream_t s) {
     FlashArgs a{};
     a.at = at; a.pos0 = pos0; a.o = (float*)work; a.status = status;
     a.kb = (at.dim_s + 63) / 64;
@@ -628,10 +628,10 @@ cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, in
         return cudaErrorInvalidValue;
     for (int q0 = 0; q0 < n; q0 += block_rows) {
         a.row0 = q0; a.rows = std::min(block_rows, n - q0);
-        launch_pdl(gate_flash_kernel, dim3(at.heads, (at.kv_heads + a.per - 1) / a.per, (a.rows + 127) / 128), kFlashThreads, flash_smem(a.kb, a.cols), true, s, a);
+        launch_pdl(gate_flash_kernel, dim3(at.heads, (at.kv_heads + a.per - 1) / a.per, (a.rows + 127) / 128), kFlashThreads, flash_smem(a.kb, a.cols), pdl, s, a);
         __nv_bfloat16* to = (__nv_bfloat16*)out + (size_t)q0 * ld_out;
-        if (at.dim % 2 == 0) launch_pdl(gate_mix_kernel<2>, (a.rows + 1) / 2, 256, 0, true, s, at, a.rows, a.o, to, ld_out);
-        else launch_pdl(gate_mix_kernel<1>, a.rows, 256, 0, true, s, at, a.rows, a.o, to, ld_out);
+        if (at.dim % 2 == 0) launch_pdl(gate_mix_kernel<2>, (a.rows + 1) / 2, 256, 0, pdl, s, at, a.rows, a.o, to, ld_out);
+        else launch_pdl(gate_mix_kernel<1>, a.rows, 256, 0, pdl, s, at, a.rows, a.o, to, ld_out);
         *launches += 2;
     }
     return cudaGetLastError();
@@ -658,12 +658,12 @@ int gate_attn_tc_rows(const GateAttn& at, int max_seq, int max_rows, size_t budg
 }
 
 cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* weights, int block_rows, void* vt,
-                                void* out, int ld_out, int* status, int* launches, cudaStream_t s) {
+                                void* out, int ld_out, int* status, int* launches, bool pdl, cudaStream_t s) {
     const int len = pos0 + n, ldv = pad_to(len, 64);
-    launch_pdl(key_transpose_kernel, dim3(ldv / 32, (at.dim + 31) / 32, at.kv_heads), 256, 0, true, s, (const __nv_bfloat16*)at.cache, at.kv_heads, at.dim,
+    launch_pdl(key_transpose_kernel, dim3(ldv / 32, (at.dim + 31) / 32, at.kv_heads), 256, 0, pdl, s, (const __nv_bfloat16*)at.cache, at.kv_heads, at.dim,
                                                                                        at.dim_s, len, ldv, (__nv_bfloat16*)vt);
     *launches += 1;
-    if (gate_flash_fits(at)) return launch_flash(at, qh, pos0, n, max_rows, weights, block_rows, vt, ldv, out, ld_out, status, launches, s);
+    if (gate_flash_fits(at)) return launch_flash(at, qh, pos0, n, max_rows, weights, block_rows, vt, ldv, out, ld_out, status, launches, pdl, s);
     const int hp = at.heads <= 4 ? 4 : at.heads <= 8 ? 8 : at.heads <= 16 ? 16 : 32;
     ScoreArgs a{};
     a.at = at; a.pos0 = pos0; a.w = (__nv_bfloat16*)weights; a.status = status;
@@ -677,12 +677,12 @@ cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, in
     for (int q0 = 0; q0 < n; q0 += block_rows) {
         const int rows = std::min(block_rows, n - q0);
         a.row0 = q0; a.rows = rows; a.ldp = pad_to(pos0 + q0 + rows, 64); a.head_stride = (long long)block_rows * a.ldp;
-        cudaError_t c = hp == 4 ? scores<4>(a, s) : hp == 8 ? scores<8>(a, s) : hp == 16 ? scores<16>(a, s) : scores<32>(a, s);
+        cudaError_t c = hp == 4 ? scores<4>(a, pdl, s) : hp == 8 ? scores<8>(a, pdl, s) : hp == 16 ? scores<16>(a, pdl, s) : scores<32>(a, pdl, s);
         if (c != cudaSuccess) return c;
         if (!make_tile_map(&g.a, weights, a.ldp, block_rows, at.heads, a.ldp, a.head_stride, 128)) return cudaErrorInvalidValue;
         g.m = rows; g.k = a.ldp; g.causal_pos0 = pos0 + q0;
         g.out = (__nv_bfloat16*)out + (size_t)q0 * ld_out;
-        if ((c = launch_gemm_tc(g, s)) != cudaSuccess) return c;
+        if ((c = launch_gemm_tc(g, pdl, s)) != cudaSuccess) return c;
         *launches += 2;
     }
     return cudaSuccess;

@@ -230,9 +230,9 @@ int sm_count() {
 }
 
 template <int BN>
-cudaError_t run(const GemmTC& g, cudaStream_t s) {
+cudaError_t run(const GemmTC& g, bool pdl, cudaStream_t s) {
     const int cols = g.mode == GEMM_SILU_BF16 ? BN / 2 : BN, gx = (g.n + cols - 1) / cols, gy = (g.m + 127) / 128, tiles = gx * gy * g.batch;
-    return launch_pdl(gemm_tc_kernel<BN>, tiles < sm_count() ? tiles : sm_count(), kThreads, Geo<BN>::bytes, true, s, g, gx, gy, tiles);
+    return launch_pdl(gemm_tc_kernel<BN>, tiles < sm_count() ? tiles : sm_count(), kThreads, Geo<BN>::bytes, pdl, s, g, gx, gy, tiles);
 }
 
 }  // namespace
@@ -271,10 +271,10 @@ cudaError_t gemm_tc_attrs() {
     return allow_smem(gemm_tc_kernel<256>, Geo<256>::bytes);
 }
 
-cudaError_t launch_gemm_tc(const GemmTC& g, cudaStream_t s) {
-    if (g.bn == 64 && g.mode != GEMM_SILU_BF16) return run<64>(g, s);
-    if (g.bn == 128) return run<128>(g, s);
-    if (g.bn == 256) return run<256>(g, s);
+cudaError_t launch_gemm_tc(const GemmTC& g, bool pdl, cudaStream_t s) {
+    if (g.bn == 64 && g.mode != GEMM_SILU_BF16) return run<64>(g, pdl, s);
+    if (g.bn == 128) return run<128>(g, pdl, s);
+    if (g.bn == 256) return run<256>(g, pdl, s);
     return cudaErrorInvalidValue;
 }
 

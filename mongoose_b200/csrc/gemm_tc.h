@@ -36,6 +36,6 @@ struct GemmTC {
 // The width of tile for m x n results of each of `batch` products.
 int gemm_tc_bn(int m, int n, int batch);
 cudaError_t gemm_tc_attrs();
-cudaError_t launch_gemm_tc(const GemmTC& g, cudaStream_t s);
+cudaError_t launch_gemm_tc(const GemmTC& g, bool pdl, cudaStream_t s);
 
 }  // namespace mg

@@ -451,14 +451,14 @@ cudaError_t launch_latent_value(const LatentStep& a, bool f32_out, bool pdl, cud
                    : launch_pdl(latent_value_kernel<__nv_bfloat16>, grid, kThreads, smem, pdl, s, a);
 }
 
-cudaError_t launch_latent_rows(const LatentAttn& at, const float* down, int ldd, int pos0, int n, void* act, int ld_act, bool f32, cudaStream_t s) {
-    if (f32) launch_pdl(latent_rows_kernel<float>, n, kThreads, 0, true, s, at, down, ldd, pos0, (float*)act, ld_act);
-    else launch_pdl(latent_rows_kernel<__nv_bfloat16>, n, kThreads, 0, true, s, at, down, ldd, pos0, (__nv_bfloat16*)act, ld_act);
+cudaError_t launch_latent_rows(const LatentAttn& at, const float* down, int ldd, int pos0, int n, void* act, int ld_act, bool f32, bool pdl, cudaStream_t s) {
+    if (f32) launch_pdl(latent_rows_kernel<float>, n, kThreads, 0, pdl, s, at, down, ldd, pos0, (float*)act, ld_act);
+    else launch_pdl(latent_rows_kernel<__nv_bfloat16>, n, kThreads, 0, pdl, s, at, down, ldd, pos0, (__nv_bfloat16*)act, ld_act);
     return cudaGetLastError();
 }
 
-cudaError_t launch_latent_q_rows(const LatentAttn& at, const float* q, int pos0, int n, void* qh, cudaStream_t s) {
-    launch_pdl(latent_q_rows_kernel, n, kThreads, 0, true, s, at, q, pos0, at.scale * 1.4426950408889634f, (__nv_bfloat16*)qh);
+cudaError_t launch_latent_q_rows(const LatentAttn& at, const float* q, int pos0, int n, void* qh, bool pdl, cudaStream_t s) {
+    launch_pdl(latent_q_rows_kernel, n, kThreads, 0, pdl, s, at, q, pos0, at.scale * 1.4426950408889634f, (__nv_bfloat16*)qh);
     return cudaGetLastError();
 }
 

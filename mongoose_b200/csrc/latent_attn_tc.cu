@@ -262,7 +262,7 @@ bool latent_attn_tc_fits(const LatentAttn& at) {
 cudaError_t latent_attn_tc_attrs() { return allow_smem(latent_flash_kernel, 226 * 1024); }
 
 cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0, int n, void* keys, void* vt, int ldv, void* out, int ld_out,
-                                  int* status, int* launches, cudaStream_t s) {
+                                  int* status, int* launches, bool pdl, cudaStream_t s) {
     const int len = pos0 + n;
     GemmTC g{};
     g.batch = 1; g.b_group = 1; g.causal_pos0 = -1; g.k = at.ld; g.mode = GEMM_BF16; g.status = status;
@@ -271,14 +271,14 @@ cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0
     if (!make_tile_map(&g.a, at.cache, at.rank_s, at.max_seq, 1, at.row(), (long long)at.max_seq * at.row(), 128) ||
         !make_tile_map(&g.b, at.uk, at.ld, g.n, 1, at.ld, (long long)g.n * at.ld, g.bn))
         return cudaErrorInvalidValue;
-    cudaError_t c = launch_gemm_tc(g, s);
+    cudaError_t c = launch_gemm_tc(g, pdl, s);
     if (c != cudaSuccess) return c;
     // vt[heads * vdim][len] = U_v c^T
     g.m = at.heads * at.vdim; g.n = len; g.bn = gemm_tc_bn(g.m, g.n, 1); g.out = vt; g.ldc = ldv;
     if (!make_tile_map(&g.a, at.uv, at.ld, g.m, 1, at.ld, (long long)g.m * at.ld, 128) ||
         !make_tile_map(&g.b, at.cache, at.rank_s, at.max_seq, 1, at.row(), (long long)at.max_seq * at.row(), g.bn))
         return cudaErrorInvalidValue;
-    if ((c = launch_gemm_tc(g, s)) != cudaSuccess) return c;
+    if ((c = launch_gemm_tc(g, pdl, s)) != cudaSuccess) return c;
 
     const Geometry geo = geometry(at);
     FlashArgs f{};
@@ -293,7 +293,7 @@ cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0
         !make_tile_map(&f.kr, (const __nv_bfloat16*)at.cache + at.rank_s, at.rot_s, len, 1, at.row(), (long long)at.max_seq * at.row(), kKeys) ||
         !make_tile_map(&f.v, vt, len, at.vdim, at.heads, ldv, (long long)at.vdim * ldv, geo.vp))
         return cudaErrorInvalidValue;
-    launch_pdl(latent_flash_kernel, dim3(at.heads, (n + 127) / 128), kThreads, geo.smem, true, s, f);
+    launch_pdl(latent_flash_kernel, dim3(at.heads, (n + 127) / 128), kThreads, geo.smem, pdl, s, f);
     *launches += 3;
     return cudaGetLastError();
 }

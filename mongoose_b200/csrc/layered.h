@@ -157,15 +157,15 @@ cudaError_t launch_latent_query(const LatentStep& a, bool f32_cache, bool pdl, c
 cudaError_t launch_latent_attend(const LatentStep& a, bool f32_cache, bool pdl, cudaStream_t s);
 cudaError_t launch_latent_value(const LatentStep& a, bool f32_out, bool pdl, cudaStream_t s);
 // rows of a portion: act = normed query latent; normed latent and rotated key part into the cache
-cudaError_t launch_latent_rows(const LatentAttn& at, const float* down, int ldd, int pos0, int n, void* act, int ld_act, bool f32, cudaStream_t s);
+cudaError_t launch_latent_rows(const LatentAttn& at, const float* down, int ldd, int pos0, int n, void* act, int ld_act, bool f32, bool pdl, cudaStream_t s);
 // rows of a portion: qh = queries with their rotated part rotated, times scale * log2 e (bf16)
-cudaError_t launch_latent_q_rows(const LatentAttn& at, const float* q, int pos0, int n, void* qh, cudaStream_t s);
+cudaError_t launch_latent_q_rows(const LatentAttn& at, const float* q, int pos0, int n, void* qh, bool pdl, cudaStream_t s);
 // bf16 prompts on the tensor cores (latent_attn_tc.cu): keys [max_seq][heads * dim_s] and values, transposed,
 // [heads * vdim][ldv] of positions [0, pos0 + n) are formed from the cache, then attention in tiles of 128 queries.
 bool latent_attn_tc_fits(const LatentAttn& at);
 cudaError_t latent_attn_tc_attrs();
 cudaError_t launch_latent_attn_tc(const LatentAttn& at, const void* qh, int pos0, int n, void* keys, void* vt, int ldv, void* out, int ld_out,
-                                  int* status, int* launches, cudaStream_t s);
+                                  int* status, int* launches, bool pdl, cudaStream_t s);
 
 // ---- linear recurrence (wkv.cu) ----
 struct WkvStep {
@@ -178,13 +178,13 @@ cudaError_t launch_wkv_step(const WkvStep& a, bool pdl, cudaStream_t s);
 size_t wkv_step_smem(const Wkv& wk);
 // act[j][r] = the mix of row r and the one before it (prev before the first) with mu[j]
 cudaError_t launch_wkv_mix(const float* h, const float* prev, const float* const mu[5], int pos0, int n, int width, void* act, int ld_act,
-                           long long act_stride, bool f32, cudaStream_t s);
+                           long long act_stride, bool f32, bool pdl, cudaStream_t s);
 // act[n][ld] = tanh of the decay's inner projection (the sum of `slices` slabs [n][ldp]) as two bf16 parts
-cudaError_t launch_wkv_inner(const float* inner, int ldp, int slices, int rank, int n, void* act, int ld, cudaStream_t s);
+cudaError_t launch_wkv_inner(const float* inner, int ldp, int slices, int rank, int n, void* act, int ld, bool pdl, cudaStream_t s);
 bool wkv_rows_fits(const Wkv& wk);
 cudaError_t wkv_attrs();
 // proj rows as WkvStep's, decays [n][heads * dim]; out [n][heads * dim] raw outputs
-cudaError_t launch_wkv_rows(const Wkv& wk, const float* proj, int ldp, const float* decay, int pos0, int n, float* out, cudaStream_t s);
+cudaError_t launch_wkv_rows(const Wkv& wk, const float* proj, int ldp, const float* decay, int pos0, int n, float* out, bool pdl, cudaStream_t s);
 
 // ---- mixture of experts (moe.cu) ----
 struct MoeStep {
@@ -213,14 +213,14 @@ struct MoeRows {                // workspace of a portion
 inline int moe_tiles(const Moe& m, int n) { return (int)(((long long)n * m.top + 127) / 128) + m.experts; }
 // choice, grouping, the grouped inputs and the shared expert's gate; the router rows are the sum of `slices` slabs
 // [n][ldr]
-cudaError_t launch_moe_route(const Moe& m, const float* router, int ldr, int slices, int n, const void* act, bool f32, const MoeRows& w, cudaStream_t s);
+cudaError_t launch_moe_route(const Moe& m, const float* router, int ldr, int slices, int n, const void* act, bool f32, const MoeRows& w, bool pdl, cudaStream_t s);
 // z = weighted sum of the grouped rows (+ z times the shared expert's gate)
-cudaError_t launch_moe_combine(const Moe& m, int n, const MoeRows& w, float* z, bool f32, cudaStream_t s);
+cudaError_t launch_moe_combine(const Moe& m, int n, const MoeRows& w, float* z, bool f32, bool pdl, cudaStream_t s);
 
 // ---- portions of a prompt (layered_prefill.cu) -----------------------------------------------------
 // `act` buffers hold bf16 or fp32 (f32 = true) rows padded to a multiple of 64 with zeros.
 cudaError_t launch_embed_rows(const WeightView& embed, int ld_embed, const float* pos_tab, const int* tokens, int pos0, int n,
-                              int width, float* x, void* act, int ld_act, bool f32, cudaStream_t s);
+                              int width, float* x, void* act, int ld_act, bool f32, bool pdl, cudaStream_t s);
 // out[n][ldc] = A[n][K] W[rows][K]^T with fp32 accuracy (32-bit mode; gemm_f32.cu).  lda a multiple of 4, ldw of 8; W is zero
 // from K to ldw.
 enum : int { F32_STORE = 0, F32_GELU = 1,
@@ -244,9 +244,9 @@ cudaError_t gemm_f32_attrs();
 cudaError_t launch_gemm_f32(const GemmF32& g, cudaStream_t s);
 // queries: normed, times temperature, score scale and key-norm weight; keys: raw rows into the cache
 cudaError_t launch_qk_rows(const GateAttn& at, const float* proj, int ldp, int q_col, int k_col, int pos0, int n, void* qh,
-                           bool f32, cudaStream_t s);
+                           bool f32, bool pdl, cudaStream_t s);
 cudaError_t launch_gate_attn_rows(const GateAttn& at, const void* qh, int pos0, int n, void* out, int ld_out, bool f32,
-                                  cudaStream_t s);
+                                  bool pdl, cudaStream_t s);
 size_t gate_attn_rows_smem(const GateAttn& at, bool f32, int* tile);
 // The same on the tensor cores (bf16 only, gate_attn_tc.cu): `weights` is a workspace for blocks of block_rows queries
 // (gate_attn_tc_rows of them fit `budget`, gate_attn_tc_bytes), `vt` the keys transposed; qh has max_rows rows.
@@ -255,13 +255,13 @@ int gate_attn_tc_rows(const GateAttn& at, int max_seq, int max_rows, size_t budg
 size_t gate_attn_tc_bytes(const GateAttn& at, int max_seq, int block_rows);
 cudaError_t gate_attn_tc_attrs();
 cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* weights, int block_rows, void* vt,
-                                void* out, int ld_out, int* status, int* launches, cudaStream_t s);
+                                void* out, int ld_out, int* status, int* launches, bool pdl, cudaStream_t s);
 // x += norm(z) or x += norm(half the sum of two normed branches); act = x
 cudaError_t launch_post_rows(float* x, const float* z0, const float* z1, const float* w0, const float* w1, const float* post_w,
-                             float eps, int n, int width, void* act, int ld_act, bool f32, cudaStream_t s);
+                             float eps, int n, int width, void* act, int ld_act, bool f32, bool pdl, cudaStream_t s);
 // act[r] = norm(x[rows[r]]) of the kind NORM_*
 cudaError_t launch_last_norm_rows(const float* x, const int* rows, const float* w, int kind, float eps, int n, int width, void* act,
-                                  int ld_act, bool f32, cudaStream_t s);
+                                  int ld_act, bool f32, bool pdl, cudaStream_t s);
 // x += mult * ls * z (where z is given); then act (or h, 32-bit rows without padding) = norm(x), or, where cat is
 // given, act = [x, cat]
 struct PrenormRows {
@@ -277,11 +277,11 @@ struct PrenormRows {
     float* h;
     const float* cat;
 };
-cudaError_t launch_prenorm_rows(const PrenormRows& a, bool f32, cudaStream_t s);
+cudaError_t launch_prenorm_rows(const PrenormRows& a, bool f32, bool pdl, cudaStream_t s);
 // act[t] = unit rms per head of o[t] (a norm weight over all heads) times a gate
 enum : int { GATE_SIGMOID = 0, GATE_SILU = 1 };
 cudaError_t launch_head_norm_rows(int heads, int vdim, float eps, const float* norm, const float* gate, int ldg, int gate_kind, int n,
-                                  const float* o, void* act, int ld_act, bool f32, cudaStream_t s);
+                                  const float* o, void* act, int ld_act, bool f32, bool pdl, cudaStream_t s);
 
 struct MemRows {                // workspace of the chunked memory for up to n tokens
     double* b;                  // [heads][n] log-forget sum inside the chunk
@@ -294,6 +294,6 @@ struct MemRows {                // workspace of the chunked memory for up to n t
     float* o;                   // [n][heads * vdim]
 };
 cudaError_t launch_mem_rows(const MatMem& mem, const ProjCols& c, const float* proj, int ldp, int pos0, int n, const MemRows& w,
-                            void* act, int ld_act, bool f32, cudaStream_t s);
+                            void* act, int ld_act, bool f32, bool pdl, cudaStream_t s);
 
 }  // namespace mg

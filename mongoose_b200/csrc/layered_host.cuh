@@ -749,7 +749,7 @@ int layered_matmul(mg_engine* e, const void* act, int act_rows, int ld, const ui
         return fail(e, MG_ERR_CUDA, "tensor map of a %d x %d product failed", rows, ld);
     g.m = n; g.n = rows; g.k = ld; g.batch = 1; g.b_group = 1; g.causal_pos0 = -1;
     g.out = out; g.ldc = ldc; g.mode = gelu ? GEMM_GELU_BF16 : GEMM_F32; g.status = m.status;
-    MG_CUDA(e, launch_gemm_tc(g, e->stream));
+    MG_CUDA(e, launch_gemm_tc(g, e->prompt_pdl, e->stream));
     return MG_OK;
 }
 
@@ -770,7 +770,7 @@ int layered_matmul_batch(mg_engine* e, const void* act, long long stride, int ac
         return fail(e, MG_ERR_CUDA, "tensor map of %d %d x %d products failed", count, rows, ld);
     g.m = n; g.n = rows; g.k = ld; g.batch = count; g.b_group = 1; g.causal_pos0 = -1;
     g.out = out; g.ldc = ldc; g.batch_c = rows; g.mode = GEMM_F32; g.status = m.status;
-    MG_CUDA(e, launch_gemm_tc(g, e->stream));
+    MG_CUDA(e, launch_gemm_tc(g, e->prompt_pdl, e->stream));
     return MG_OK;
 }
 
@@ -790,7 +790,7 @@ int layered_matmul_thin(mg_engine* e, const void* act, int act_rows, int ld, con
         return fail(e, MG_ERR_CUDA, "tensor map of a %d x %d product in %d slices failed", rows, ld, S);
     g.m = n; g.n = rows; g.k = k; g.batch = S; g.b_group = 1; g.causal_pos0 = -1;
     g.out = out; g.ldc = ldc; g.batch_c = (long long)n * ldc; g.mode = GEMM_F32; g.status = m.status;
-    MG_CUDA(e, launch_gemm_tc(g, e->stream));
+    MG_CUDA(e, launch_gemm_tc(g, e->prompt_pdl, e->stream));
     return MG_OK;
 }
 
@@ -820,12 +820,12 @@ int layered_glu(mg_engine* e, const void* act, int act_rows, int ld, const uint8
     if (!make_tile_map(&g.a, act, ld, act_rows, 1, ld, (long long)act_rows * ld, 128) ||
         !make_tile_map(&g.b, gate, ld, ff, count, ld, (long long)ff * ld, g.bn / 2) || !make_tile_map(&g.b2, up, ld, ff, count, ld, (long long)ff * ld, g.bn / 2))
         return fail(e, MG_ERR_CUDA, "tensor map of a %d x %d feed-forward failed", ff, ld);
-    MG_CUDA(e, launch_gemm_tc(g, e->stream));
+    MG_CUDA(e, launch_gemm_tc(g, e->prompt_pdl, e->stream));
     g.bn = gemm_tc_bn(n, W, 1); g.n = W; g.k = ffs; g.out = z; g.ldc = W; g.mode = z_act ? GEMM_BF16 : GEMM_F32;
     if (!make_tile_map(&g.a, m.xmid, ffs, act_rows, 1, ffs, (long long)act_rows * ffs, 128) ||
         !make_tile_map(&g.b, down, ffs, W, count, ffs, (long long)W * ffs, g.bn))
         return fail(e, MG_ERR_CUDA, "tensor map of a %d x %d feed-forward failed", W, ffs);
-    MG_CUDA(e, launch_gemm_tc(g, e->stream));
+    MG_CUDA(e, launch_gemm_tc(g, e->prompt_pdl, e->stream));
     return MG_OK;
 }
 
@@ -837,15 +837,15 @@ int parallel_rows(mg_engine* e, const LayerRun& run, LayerWeights& l, int pos, i
     const GateAttn at = run.at(l);
     int rc;
     if ((rc = layered_matmul(e, m.act, m.max_rows, m.kw, l.proj, m.P, np, n, l.cols.total, false))) return rc;
-    MG_CUDA(e, launch_qk_rows(at, m.P, np, l.cols.q, l.cols.k, pos, n, m.qh, m.f32, s));
+    MG_CUDA(e, launch_qk_rows(at, m.P, np, l.cols.q, l.cols.k, pos, n, m.qh, m.f32, e->prompt_pdl, s));
     if (l.block_rows) {
         int k = 0;
-        MG_CUDA(e, launch_gate_attn_tc(at, m.qh, pos, n, m.max_rows, m.aw, l.block_rows, m.vt, m.ao, kat, m.status, &k, s));
+        MG_CUDA(e, launch_gate_attn_tc(at, m.qh, pos, n, m.max_rows, m.aw, l.block_rows, m.vt, m.ao, kat, m.status, &k, e->prompt_pdl, s));
         e->launches += k - 1;
     } else {
-        MG_CUDA(e, launch_gate_attn_rows(at, m.qh, pos, n, m.ao, kat, m.f32, s));
+        MG_CUDA(e, launch_gate_attn_rows(at, m.qh, pos, n, m.ao, kat, m.f32, e->prompt_pdl, s));
     }
-    MG_CUDA(e, launch_mem_rows(run.mem(l), l.cols, m.P, np, pos, n, m.mw, m.my, kmem, m.f32, s));
+    MG_CUDA(e, launch_mem_rows(run.mem(l), l.cols, m.P, np, pos, n, m.mw, m.my, kmem, m.f32, e->prompt_pdl, s));
     e->launches += 7;
     if ((rc = layered_matmul(e, m.ao, m.max_rows, kat, l.at_o, m.yr[0], W, n, W, false))) return rc;
     return layered_matmul(e, m.my, m.max_rows, kmem, l.mem_o, m.yr[1], W, n, W, false);
@@ -859,12 +859,12 @@ int latent_rows(mg_engine* e, const LayerRun& run, LayerWeights& l, int pos, int
     cudaStream_t s = e->stream;
     int rc;
     if ((rc = layered_matmul(e, m.act, m.max_rows, m.kw, l.proj, m.P, np, n, l.proj_rows(), false))) return rc;
-    MG_CUDA(e, launch_latent_rows(at, m.P, np, pos, n, m.cq, kq, m.f32, s));
+    MG_CUDA(e, launch_latent_rows(at, m.P, np, pos, n, m.cq, kq, m.f32, e->prompt_pdl, s));
     if ((rc = layered_matmul(e, m.cq, m.max_rows, kq, l.uq, m.q32, qrows, n, qrows, false))) return rc;
     if (l.latent_tc) {
         int k = 0;
-        MG_CUDA(e, launch_latent_q_rows(at, m.q32, pos, n, m.qh, s));
-        MG_CUDA(e, launch_latent_attn_tc(at, m.qh, pos, n, m.keys, m.vt, pad_to(m.c.max_seq, 64), m.ao, ko, m.status, &k, s));
+        MG_CUDA(e, launch_latent_q_rows(at, m.q32, pos, n, m.qh, e->prompt_pdl, s));
+        MG_CUDA(e, launch_latent_attn_tc(at, m.qh, pos, n, m.keys, m.vt, pad_to(m.c.max_seq, 64), m.ao, ko, m.status, &k, e->prompt_pdl, s));
         e->launches += 2 + k;
     } else {
         LatentStep t{};
@@ -886,7 +886,7 @@ int wkv_rows(mg_engine* e, const LayerRun& run, LayerWeights& l, int pos, int n)
     const long long stride = (long long)m.max_rows * kw;
     cudaStream_t s = e->stream;
     int rc;
-    MG_CUDA(e, launch_wkv_mix(m.hr, run.prev, l.mu, pos, n, W, m.mix, kw, stride, m.f32, s));
+    MG_CUDA(e, launch_wkv_mix(m.hr, run.prev, l.mu, pos, n, W, m.mix, kw, stride, m.f32, e->prompt_pdl, s));
     MG_CUDA(e, cudaMemcpyAsync(run.prev + (size_t)((pos + n) & 1) * W, m.hr + (size_t)(n - 1) * W, (size_t)W * 4, cudaMemcpyDeviceToDevice, s));
     if ((rc = layered_matmul_batch(e, m.mix, stride, m.max_rows, kw, l.proj, m.P, np, n, d, 4))) return rc;
     int slices;
@@ -900,7 +900,7 @@ int wkv_rows(mg_engine* e, const LayerRun& run, LayerWeights& l, int pos, int n)
         MG_CUDA(e, launch_gemm_f32(g, s));
     } else {
         const int ld = 2 * wk.ld2;
-        MG_CUDA(e, launch_wkv_inner(m.inner32, ldi, slices, wk.rank, n, m.inner, ld, s));
+        MG_CUDA(e, launch_wkv_inner(m.inner32, ldi, slices, wk.rank, n, m.inner, ld, e->prompt_pdl, s));
         GemmTC g{};
         g.bn = gemm_tc_bn(n, d, 1);
         if (!make_tile_map(&g.a, m.inner, ld, m.max_rows, 1, ld, (long long)m.max_rows * ld, 128) ||
@@ -908,11 +908,11 @@ int wkv_rows(mg_engine* e, const LayerRun& run, LayerWeights& l, int pos, int n)
             return fail(e, MG_ERR_CUDA, "tensor map of a %d x %d product failed", d, ld);
         g.m = n; g.n = d; g.k = ld; g.batch = 1; g.b_group = 1; g.causal_pos0 = -1; g.b_steps = wk.ld2 / 64;
         g.out = m.decay; g.ldc = d; g.mode = GEMM_DECAY_F32; g.bias = l.w0; g.status = m.status;
-        MG_CUDA(e, launch_gemm_tc(g, s));
+        MG_CUDA(e, launch_gemm_tc(g, e->prompt_pdl, s));
         e->launches += 1;
     }
-    MG_CUDA(e, launch_wkv_rows(wk, m.P, np, m.decay, pos, n, m.wo, s));
-    MG_CUDA(e, launch_head_norm_rows(wk.heads, wk.dim, wk.eps, wk.norm, m.P + (size_t)3 * d, np, GATE_SILU, n, m.wo, m.ao, ko, m.f32, s));
+    MG_CUDA(e, launch_wkv_rows(wk, m.P, np, m.decay, pos, n, m.wo, e->prompt_pdl, s));
+    MG_CUDA(e, launch_head_norm_rows(wk.heads, wk.dim, wk.eps, wk.norm, m.P + (size_t)3 * d, np, GATE_SILU, n, m.wo, m.ao, ko, m.f32, e->prompt_pdl, s));
     e->launches += 4;
     return layered_matmul(e, m.ao, m.max_rows, ko, l.o, m.zr, W, n, W, false);
 }
@@ -928,11 +928,11 @@ int moe_rows(mg_engine* e, LayerWeights& l, int n) {
     int rc;
     int slices;
     if ((rc = layered_matmul_thin(e, m.act, m.max_rows, m.kw, l.router, m.rtr, ldr, n, cols, &slices))) return rc;
-    MG_CUDA(e, launch_moe_route(x, m.rtr, ldr, slices, n, m.act, m.f32, w, s));
+    MG_CUDA(e, launch_moe_route(x, m.rtr, ldr, slices, n, m.act, m.f32, w, e->prompt_pdl, s));
     if ((rc = layered_glu(e, w.x, w.tiles * 128, m.kw, l.e_gate, l.e_up, l.e_down, x.ff, x.ffs, x.experts, w.group, w.y, true, w.tiles * 128))) return rc;
     if (x.shared_ff && (rc = layered_glu(e, m.act, m.max_rows, m.kw, l.router_row(x.sg_col() + 1), l.router_row(x.sg_col() + 1 + x.shared_ff),
                                          l.shared_down, x.shared_ff, x.shared_ffs, 1, nullptr, m.zr, false, n))) return rc;
-    MG_CUDA(e, launch_moe_combine(x, n, w, m.zr, m.f32, s));
+    MG_CUDA(e, launch_moe_combine(x, n, w, m.zr, m.f32, e->prompt_pdl, s));
     e->launches += 4;
     return MG_OK;
 }
@@ -943,7 +943,7 @@ int layered_rows(mg_engine* e, int pos, int n) {
     const int W = m.c.width, kw = m.kw;
     cudaStream_t s = e->stream;
     int rc;
-    MG_CUDA(e, launch_embed_rows(WeightView{m.embed, nullptr}, kw, m.pos_tab, m.tokens, pos, n, W, m.x, m.act, kw, m.f32, s));
+    MG_CUDA(e, launch_embed_rows(WeightView{m.embed, nullptr}, kw, m.pos_tab, m.tokens, pos, n, W, m.x, m.act, kw, m.f32, e->prompt_pdl, s));
     e->launches += 1;
     if (m.c.loop_times) MG_CUDA(e, cudaMemcpyAsync(m.x0r, m.x, (size_t)n * W * 4, cudaMemcpyDeviceToDevice, s));
     const float* scale = nullptr;               // m.zr, scaled by this vector, is still to be added
@@ -952,7 +952,7 @@ int layered_rows(mg_engine* e, int pos, int n) {
         if (scale) { a.z = m.zr; a.ls = scale; a.mult = m.c.residual_mult; }
         scale = nullptr;
         e->launches += 1;
-        MG_CUDA(e, launch_prenorm_rows(a, m.f32, s));
+        MG_CUDA(e, launch_prenorm_rows(a, m.f32, e->prompt_pdl, s));
         return MG_OK;
     };
     auto normed = [&](const float* w, float* h) -> int {
@@ -973,14 +973,14 @@ int layered_rows(mg_engine* e, int pos, int n) {
         if (l.parallel()) {
             if (!raw && (rc = normed(nullptr, nullptr))) return rc;
             if ((rc = parallel_rows(e, run, l, pos, n))) return rc;
-            MG_CUDA(e, launch_post_rows(m.x, m.yr[0], m.yr[1], l.at_out, l.mem_out, l.norm1, m.c.norm_eps, n, W, m.act, kw, m.f32, s));
+            MG_CUDA(e, launch_post_rows(m.x, m.yr[0], m.yr[1], l.at_out, l.mem_out, l.norm1, m.c.norm_eps, n, W, m.act, kw, m.f32, e->prompt_pdl, s));
             e->launches += 1;
             raw = true;
             if (!l.c.ffn_dim) continue;
             const int kff = pad_to(l.c.ffn_dim, 64);
             if ((rc = layered_matmul(e, m.act, m.max_rows, kw, l.up, m.midr, kff, n, l.c.ffn_dim, true))) return rc;
             if ((rc = layered_matmul(e, m.midr, m.max_rows, kff, l.down, m.zr, W, n, W, false))) return rc;
-            MG_CUDA(e, launch_post_rows(m.x, m.zr, nullptr, nullptr, nullptr, l.norm2, m.c.norm_eps, n, W, m.act, kw, m.f32, s));
+            MG_CUDA(e, launch_post_rows(m.x, m.zr, nullptr, nullptr, nullptr, l.norm2, m.c.norm_eps, n, W, m.act, kw, m.f32, e->prompt_pdl, s));
             e->launches += 1;
             continue;
         }
@@ -1018,7 +1018,7 @@ int layered_forward(mg_engine* e, const int* tokens, int n, int pos, const int* 
             MG_CUDA(e, cudaStreamSynchronize(e->stream));
             while (w + k < n_want && want[w + k] < b + nb && k < m.logit_rows) { e->pin_i[8 + k] = want[w + k] - b; k++; }
             MG_CUDA(e, cudaMemcpyAsync(m.want, e->pin_i + 8, (size_t)k * 4, cudaMemcpyHostToDevice, e->stream));
-            MG_CUDA(e, launch_last_norm_rows(m.x, m.want, m.final_norm, m.c.norm, m.c.norm_eps, k, m.c.width, m.fin, m.kw, m.f32, e->stream));
+            MG_CUDA(e, launch_last_norm_rows(m.x, m.want, m.final_norm, m.c.norm, m.c.norm_eps, k, m.c.width, m.fin, m.kw, m.f32, e->prompt_pdl, e->stream));
             e->launches += 1;
             if ((rc = layered_matmul(e, m.fin, m.logit_rows, m.kw, m.head, m.logits, m.c.vocab, k, m.c.vocab, false))) return rc;
             MG_CUDA(e, cudaMemcpyAsync(logits_out + (size_t)w * m.c.vocab, m.logits, (size_t)k * m.c.vocab * 4, cudaMemcpyDeviceToHost, e->stream));

@@ -630,14 +630,14 @@ __global__ void __launch_bounds__(256) head_norm_quads_kernel(int heads, int vdi
 }
 
 template <typename KT, int NQ>
-cudaError_t attn_rows_for(const GateAttn& at, const void* qh, int pos0, int n, void* out, int ld_out, cudaStream_t s) {
+cudaError_t attn_rows_for(const GateAttn& at, const void* qh, int pos0, int n, void* out, int ld_out, bool pdl, cudaStream_t s) {
     int tile;
     const size_t smem = attn_smem(at, NQ, sizeof(KT), 32, &tile);
     if (!smem) return cudaErrorInvalidValue;
     auto run = [&](auto kern) {
         cudaError_t c = allow_smem(kern, kModelSmem);
         if (c != cudaSuccess) return c;
-        launch_pdl(kern, (n + NQ - 1) / NQ, kAttnThreads, smem, true, s, at, (const KT*)qh, pos0, n, tile, (KT*)out, ld_out);
+        launch_pdl(kern, (n + NQ - 1) / NQ, kAttnThreads, smem, pdl, s, at, (const KT*)qh, pos0, n, tile, (KT*)out, ld_out);
         return cudaGetLastError();
     };
     switch (attn_pairs(at)) {
@@ -653,104 +653,104 @@ cudaError_t attn_rows_for(const GateAttn& at, const void* qh, int pos0, int n, v
 }  // namespace
 
 cudaError_t launch_embed_rows(const WeightView& embed, int ld_embed, const float* pos_tab, const int* tokens, int pos0, int n,
-                              int width, float* x, void* act, int ld_act, bool f32, cudaStream_t s) {
-    if (f32) launch_pdl(embed_rows_kernel<float>, n, 256, 0, true, s, embed, ld_embed, pos_tab, tokens, pos0, width, x, (float*)act, ld_act);
-    else launch_pdl(embed_rows_kernel<__nv_bfloat16>, n, 256, 0, true, s, embed, ld_embed, pos_tab, tokens, pos0, width, x, (__nv_bfloat16*)act, ld_act);
+                              int width, float* x, void* act, int ld_act, bool f32, bool pdl, cudaStream_t s) {
+    if (f32) launch_pdl(embed_rows_kernel<float>, n, 256, 0, pdl, s, embed, ld_embed, pos_tab, tokens, pos0, width, x, (float*)act, ld_act);
+    else launch_pdl(embed_rows_kernel<__nv_bfloat16>, n, 256, 0, pdl, s, embed, ld_embed, pos_tab, tokens, pos0, width, x, (__nv_bfloat16*)act, ld_act);
     return cudaGetLastError();
 }
 
 cudaError_t launch_qk_rows(const GateAttn& at, const float* proj, int ldp, int q_col, int k_col, int pos0, int n, void* qh, bool f32,
-                           cudaStream_t s) {
+                           bool pdl, cudaStream_t s) {
     if (((at.dim | ldp | q_col | k_col) & 3) == 0 && at.dim <= 256) {
         auto quads = [&](auto* q) {
             using AT = std::remove_pointer_t<decltype(q)>;
             const int grid = (n * (at.heads + at.kv_heads) + 15) / 16;
-            if (at.dim <= 64) launch_pdl(qk_quads_kernel<AT, 1>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, q);
-            else if (at.dim <= 128) launch_pdl(qk_quads_kernel<AT, 2>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, q);
-            else launch_pdl(qk_quads_kernel<AT, 4>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, q);
+            if (at.dim <= 64) launch_pdl(qk_quads_kernel<AT, 1>, grid, 256, 0, pdl, s, at, proj, ldp, q_col, k_col, pos0, n, q);
+            else if (at.dim <= 128) launch_pdl(qk_quads_kernel<AT, 2>, grid, 256, 0, pdl, s, at, proj, ldp, q_col, k_col, pos0, n, q);
+            else launch_pdl(qk_quads_kernel<AT, 4>, grid, 256, 0, pdl, s, at, proj, ldp, q_col, k_col, pos0, n, q);
             return cudaGetLastError();
         };
         return f32 ? quads((float*)qh) : quads((__nv_bfloat16*)qh);
     }
     const int grid = (n * (at.heads + at.kv_heads) + 7) / 8;
-    if (f32) launch_pdl(qk_rows_kernel<float>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, (float*)qh);
-    else launch_pdl(qk_rows_kernel<__nv_bfloat16>, grid, 256, 0, true, s, at, proj, ldp, q_col, k_col, pos0, n, (__nv_bfloat16*)qh);
+    if (f32) launch_pdl(qk_rows_kernel<float>, grid, 256, 0, pdl, s, at, proj, ldp, q_col, k_col, pos0, n, (float*)qh);
+    else launch_pdl(qk_rows_kernel<__nv_bfloat16>, grid, 256, 0, pdl, s, at, proj, ldp, q_col, k_col, pos0, n, (__nv_bfloat16*)qh);
     return cudaGetLastError();
 }
 
 size_t gate_attn_rows_smem(const GateAttn& at, bool f32, int* tile) { return attn_smem(at, 1, f32 ? 4 : 2, 32, tile); }
 
-cudaError_t launch_gate_attn_rows(const GateAttn& at, const void* qh, int pos0, int n, void* out, int ld_out, bool f32, cudaStream_t s) {
+cudaError_t launch_gate_attn_rows(const GateAttn& at, const void* qh, int pos0, int n, void* out, int ld_out, bool f32, bool pdl, cudaStream_t s) {
     int tile;
     const bool four = attn_pairs(at) <= 8 && attn_smem(at, 4, f32 ? 4 : 2, 32, &tile) > 0;
-    if (f32) return four ? attn_rows_for<float, 4>(at, qh, pos0, n, out, ld_out, s) : attn_rows_for<float, 1>(at, qh, pos0, n, out, ld_out, s);
-    return four ? attn_rows_for<__nv_bfloat16, 4>(at, qh, pos0, n, out, ld_out, s)
-                : attn_rows_for<__nv_bfloat16, 1>(at, qh, pos0, n, out, ld_out, s);
+    if (f32) return four ? attn_rows_for<float, 4>(at, qh, pos0, n, out, ld_out, pdl, s) : attn_rows_for<float, 1>(at, qh, pos0, n, out, ld_out, pdl, s);
+    return four ? attn_rows_for<__nv_bfloat16, 4>(at, qh, pos0, n, out, ld_out, pdl, s)
+                : attn_rows_for<__nv_bfloat16, 1>(at, qh, pos0, n, out, ld_out, pdl, s);
 }
 
 cudaError_t launch_post_rows(float* x, const float* z0, const float* z1, const float* w0, const float* w1, const float* post_w, float eps,
-                             int n, int width, void* act, int ld_act, bool f32, cudaStream_t s) {
+                             int n, int width, void* act, int ld_act, bool f32, bool pdl, cudaStream_t s) {
     if ((width & 3) == 0 && width <= 4096) {
         auto quads = [&](auto* o) {
             using AT = std::remove_pointer_t<decltype(o)>;
-            if (width <= 1024) launch_pdl(post_quads_kernel<AT, 1>, n, 256, 0, true, s, x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
-            else if (width <= 2048) launch_pdl(post_quads_kernel<AT, 2>, n, 256, 0, true, s, x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
-            else launch_pdl(post_quads_kernel<AT, 4>, n, 256, 0, true, s, x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
+            if (width <= 1024) launch_pdl(post_quads_kernel<AT, 1>, n, 256, 0, pdl, s, x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
+            else if (width <= 2048) launch_pdl(post_quads_kernel<AT, 2>, n, 256, 0, pdl, s, x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
+            else launch_pdl(post_quads_kernel<AT, 4>, n, 256, 0, pdl, s, x, z0, z1, w0, w1, post_w, eps, width, o, ld_act);
             return cudaGetLastError();
         };
         return f32 ? quads((float*)act) : quads((__nv_bfloat16*)act);
     }
     const size_t smem = (size_t)width * sizeof(float);
-    if (f32) launch_pdl(post_rows_kernel<float>, n, 256, smem, true, s, x, z0, z1, w0, w1, post_w, eps, width, (float*)act, ld_act);
-    else launch_pdl(post_rows_kernel<__nv_bfloat16>, n, 256, smem, true, s, x, z0, z1, w0, w1, post_w, eps, width, (__nv_bfloat16*)act, ld_act);
+    if (f32) launch_pdl(post_rows_kernel<float>, n, 256, smem, pdl, s, x, z0, z1, w0, w1, post_w, eps, width, (float*)act, ld_act);
+    else launch_pdl(post_rows_kernel<__nv_bfloat16>, n, 256, smem, pdl, s, x, z0, z1, w0, w1, post_w, eps, width, (__nv_bfloat16*)act, ld_act);
     return cudaGetLastError();
 }
 
 cudaError_t launch_last_norm_rows(const float* x, const int* rows, const float* w, int kind, float eps, int n, int width, void* act,
-                                  int ld_act, bool f32, cudaStream_t s) {
-    if (f32) launch_pdl(last_norm_rows_kernel<float>, n, 256, 0, true, s, x, rows, w, kind, eps, width, (float*)act, ld_act);
-    else launch_pdl(last_norm_rows_kernel<__nv_bfloat16>, n, 256, 0, true, s, x, rows, w, kind, eps, width, (__nv_bfloat16*)act, ld_act);
+                                  int ld_act, bool f32, bool pdl, cudaStream_t s) {
+    if (f32) launch_pdl(last_norm_rows_kernel<float>, n, 256, 0, pdl, s, x, rows, w, kind, eps, width, (float*)act, ld_act);
+    else launch_pdl(last_norm_rows_kernel<__nv_bfloat16>, n, 256, 0, pdl, s, x, rows, w, kind, eps, width, (__nv_bfloat16*)act, ld_act);
     return cudaGetLastError();
 }
 
-cudaError_t launch_prenorm_rows(const PrenormRows& a, bool f32, cudaStream_t s) {
+cudaError_t launch_prenorm_rows(const PrenormRows& a, bool f32, bool pdl, cudaStream_t s) {
     const size_t smem = (size_t)a.width * sizeof(float);
     const bool quads = a.width % 4 == 0;
-    if (f32 && quads) launch_pdl(prenorm_rows_kernel<float, 4>, a.n, 256, smem, true, s, a);
-    else if (f32) launch_pdl(prenorm_rows_kernel<float, 1>, a.n, 256, smem, true, s, a);
-    else if (quads) launch_pdl(prenorm_rows_kernel<__nv_bfloat16, 4>, a.n, 256, smem, true, s, a);
-    else launch_pdl(prenorm_rows_kernel<__nv_bfloat16, 1>, a.n, 256, smem, true, s, a);
+    if (f32 && quads) launch_pdl(prenorm_rows_kernel<float, 4>, a.n, 256, smem, pdl, s, a);
+    else if (f32) launch_pdl(prenorm_rows_kernel<float, 1>, a.n, 256, smem, pdl, s, a);
+    else if (quads) launch_pdl(prenorm_rows_kernel<__nv_bfloat16, 4>, a.n, 256, smem, pdl, s, a);
+    else launch_pdl(prenorm_rows_kernel<__nv_bfloat16, 1>, a.n, 256, smem, pdl, s, a);
     return cudaGetLastError();
 }
 
 template <typename AT>
 static cudaError_t head_norm_for(int heads, int vdim, float eps, const float* norm, const float* gate, int ldg, int gate_kind, int n, const float* o,
-                                 AT* act, int ld_act, cudaStream_t s) {
+                                 AT* act, int ld_act, bool pdl, cudaStream_t s) {
     const bool quads = vdim % 4 == 0 && vdim <= 128 && ldg % 4 == 0 && (reinterpret_cast<uintptr_t>(gate) & 15) == 0;
     int lanes = 1;
     while (lanes * 4 < vdim) lanes *= 2;
     if (quads)
-        launch_pdl(head_norm_quads_kernel<AT>, (int)(((long long)n * heads * lanes + 255) / 256), 256, 0, true, s, heads, vdim, lanes, eps, norm, gate, ldg, gate_kind, n, o, act, ld_act);
+        launch_pdl(head_norm_quads_kernel<AT>, (int)(((long long)n * heads * lanes + 255) / 256), 256, 0, pdl, s, heads, vdim, lanes, eps, norm, gate, ldg, gate_kind, n, o, act, ld_act);
     else
-        launch_pdl(head_norm_rows_kernel<AT>, (n * heads + 7) / 8, 256, 0, true, s, heads, vdim, eps, norm, gate, ldg, gate_kind, n, o, act, ld_act);
+        launch_pdl(head_norm_rows_kernel<AT>, (n * heads + 7) / 8, 256, 0, pdl, s, heads, vdim, eps, norm, gate, ldg, gate_kind, n, o, act, ld_act);
     return cudaGetLastError();
 }
 
 cudaError_t launch_head_norm_rows(int heads, int vdim, float eps, const float* norm, const float* gate, int ldg, int gate_kind, int n,
-                                  const float* o, void* act, int ld_act, bool f32, cudaStream_t s) {
-    return f32 ? head_norm_for(heads, vdim, eps, norm, gate, ldg, gate_kind, n, o, (float*)act, ld_act, s)
-               : head_norm_for(heads, vdim, eps, norm, gate, ldg, gate_kind, n, o, (__nv_bfloat16*)act, ld_act, s);
+                                  const float* o, void* act, int ld_act, bool f32, bool pdl, cudaStream_t s) {
+    return f32 ? head_norm_for(heads, vdim, eps, norm, gate, ldg, gate_kind, n, o, (float*)act, ld_act, pdl, s)
+               : head_norm_for(heads, vdim, eps, norm, gate, ldg, gate_kind, n, o, (__nv_bfloat16*)act, ld_act, pdl, s);
 }
 
 cudaError_t launch_mem_rows(const MatMem& mem, const ProjCols& c, const float* proj, int ldp, int pos0, int n, const MemRows& w, void* act,
-                            int ld_act, bool f32, cudaStream_t s) {
+                            int ld_act, bool f32, bool pdl, cudaStream_t s) {
     const int chunks = (n + kMemChunk - 1) / kMemChunk, dt = (mem.dim + 63) / 64, vt = (mem.vdim + 63) / 64;
-    launch_pdl(mem_gates_kernel, mem.heads, kGateWarps * 32, 0, true, s, mem, c.mi, c.mf, proj, ldp, pos0, n, w);
-    launch_pdl(mem_chunk_kernel, dim3(chunks, mem.heads, dt * vt), 256, 0, true, s, mem, c.mk, c.mv, proj, ldp, n, vt, w);
+    launch_pdl(mem_gates_kernel, mem.heads, kGateWarps * 32, 0, pdl, s, mem, c.mi, c.mf, proj, ldp, pos0, n, w);
+    launch_pdl(mem_chunk_kernel, dim3(chunks, mem.heads, dt * vt), 256, 0, pdl, s, mem, c.mk, c.mv, proj, ldp, n, vt, w);
     const size_t elems = (size_t)mem.heads * mem.dim * (mem.vdim + 1);
-    launch_pdl(mem_scan_kernel, (unsigned)((elems + 255) / 256), 256, 0, true, s, mem, pos0, n, chunks, w);
-    launch_pdl(mem_out_kernel, dim3(chunks, mem.heads, vt), 256, 0, true, s, mem, c.mq, c.mk, c.mv, proj, ldp, n, w);
-    return launch_head_norm_rows(mem.heads, mem.vdim, mem.eps, mem.norm, proj + c.mg, ldp, GATE_SIGMOID, n, w.o, act, ld_act, f32, s);
+    launch_pdl(mem_scan_kernel, (unsigned)((elems + 255) / 256), 256, 0, pdl, s, mem, pos0, n, chunks, w);
+    launch_pdl(mem_out_kernel, dim3(chunks, mem.heads, vt), 256, 0, pdl, s, mem, c.mq, c.mk, c.mv, proj, ldp, n, w);
+    return launch_head_norm_rows(mem.heads, mem.vdim, mem.eps, mem.norm, proj + c.mg, ldp, GATE_SIGMOID, n, w.o, act, ld_act, f32, pdl, s);
 }
 
 }  // namespace mg

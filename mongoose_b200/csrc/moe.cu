@@ -299,19 +299,19 @@ cudaError_t launch_moe_down(const MoeStep& a, int sms, bool pdl, cudaStream_t s)
     return launch_pdl(moe_down_kernel<kDownRows>, grid, kThreads, smem, pdl, s, a);
 }
 
-cudaError_t launch_moe_route(const Moe& m, const float* router, int ldr, int slices, int n, const void* act, bool f32, const MoeRows& w, cudaStream_t s) {
-    launch_pdl(moe_choose_kernel, (n + 7) / 8, kThreads, (size_t)8 * m.experts * sizeof(float), true, s, m, router, ldr, slices, n, w);
-    launch_pdl(moe_plan_kernel, 1, 1024, 0, true, s, m, w);
-    launch_pdl(moe_gather_kernel, n, 128, 0, true, s, m, (const uint4*)act, m.ldw * (f32 ? 4 : 2) / 16, w);
+cudaError_t launch_moe_route(const Moe& m, const float* router, int ldr, int slices, int n, const void* act, bool f32, const MoeRows& w, bool pdl, cudaStream_t s) {
+    launch_pdl(moe_choose_kernel, (n + 7) / 8, kThreads, (size_t)8 * m.experts * sizeof(float), pdl, s, m, router, ldr, slices, n, w);
+    launch_pdl(moe_plan_kernel, 1, 1024, 0, pdl, s, m, w);
+    launch_pdl(moe_gather_kernel, n, 128, 0, pdl, s, m, (const uint4*)act, m.ldw * (f32 ? 4 : 2) / 16, w);
     return cudaGetLastError();
 }
 
-cudaError_t launch_moe_combine(const Moe& m, int n, const MoeRows& w, float* z, bool f32, cudaStream_t s) {
+cudaError_t launch_moe_combine(const Moe& m, int n, const MoeRows& w, float* z, bool f32, bool pdl, cudaStream_t s) {
     const bool quads = m.width % 4 == 0;
-    if (f32 && quads) launch_pdl(moe_combine_kernel<float, 4>, n, kThreads, 0, true, s, m, w, z);
-    else if (f32) launch_pdl(moe_combine_kernel<float, 1>, n, kThreads, 0, true, s, m, w, z);
-    else if (quads) launch_pdl(moe_combine_kernel<__nv_bfloat16, 4>, n, kThreads, 0, true, s, m, w, z);
-    else launch_pdl(moe_combine_kernel<__nv_bfloat16, 1>, n, kThreads, 0, true, s, m, w, z);
+    if (f32 && quads) launch_pdl(moe_combine_kernel<float, 4>, n, kThreads, 0, pdl, s, m, w, z);
+    else if (f32) launch_pdl(moe_combine_kernel<float, 1>, n, kThreads, 0, pdl, s, m, w, z);
+    else if (quads) launch_pdl(moe_combine_kernel<__nv_bfloat16, 4>, n, kThreads, 0, pdl, s, m, w, z);
+    else launch_pdl(moe_combine_kernel<__nv_bfloat16, 1>, n, kThreads, 0, pdl, s, m, w, z);
     return cudaGetLastError();
 }
 

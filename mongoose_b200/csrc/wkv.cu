@@ -340,10 +340,10 @@ __global__ void __launch_bounds__(kScanThreads) wkv_scan_kernel(const Wkv M, con
 }
 
 template <int KPT>
-cudaError_t scan_for(const Wkv& wk, const float* proj, int ldp, const float* decay, int pos0, int n, float* out, cudaStream_t s) {
+cudaError_t scan_for(const Wkv& wk, const float* proj, int ldp, const float* decay, int pos0, int n, float* out, bool pdl, cudaStream_t s) {
     using G = Scan<KPT>;
     constexpr size_t smem = G::smem(G::tile);
-    launch_pdl(wkv_scan_kernel<KPT>, dim3(wk.heads, (wk.dim + G::cols - 1) / G::cols), kScanThreads, smem, true, s, wk, proj, ldp, decay, pos0, n, out);
+    launch_pdl(wkv_scan_kernel<KPT>, dim3(wk.heads, (wk.dim + G::cols - 1) / G::cols), kScanThreads, smem, pdl, s, wk, proj, ldp, decay, pos0, n, out);
     return cudaGetLastError();
 }
 
@@ -352,9 +352,9 @@ cudaError_t allow_scan() { return allow_smem(wkv_scan_kernel<KPT>, Scan<KPT>::sm
 
 template <typename AT>
 cudaError_t mix_for(const float* h, const float* prev, const float* const mu[5], int pos0, int n, int width, AT* act, int ld_act, long long stride,
-                    cudaStream_t s) {
-    if (width % 4 == 0) launch_pdl(wkv_mix_kernel<AT, 4>, n, 256, 0, true, s, h, prev, mu[0], mu[1], mu[2], mu[3], mu[4], pos0, width, act, ld_act, stride);
-    else launch_pdl(wkv_mix_kernel<AT, 1>, n, 256, 0, true, s, h, prev, mu[0], mu[1], mu[2], mu[3], mu[4], pos0, width, act, ld_act, stride);
+                    bool pdl, cudaStream_t s) {
+    if (width % 4 == 0) launch_pdl(wkv_mix_kernel<AT, 4>, n, 256, 0, pdl, s, h, prev, mu[0], mu[1], mu[2], mu[3], mu[4], pos0, width, act, ld_act, stride);
+    else launch_pdl(wkv_mix_kernel<AT, 1>, n, 256, 0, pdl, s, h, prev, mu[0], mu[1], mu[2], mu[3], mu[4], pos0, width, act, ld_act, stride);
     return cudaGetLastError();
 }
 
@@ -367,13 +367,13 @@ cudaError_t launch_wkv_step(const WkvStep& a, bool pdl, cudaStream_t s) {
 }
 
 cudaError_t launch_wkv_mix(const float* h, const float* prev, const float* const mu[5], int pos0, int n, int width, void* act, int ld_act,
-                           long long act_stride, bool f32, cudaStream_t s) {
-    return f32 ? mix_for(h, prev, mu, pos0, n, width, (float*)act, ld_act, act_stride, s)
-               : mix_for(h, prev, mu, pos0, n, width, (__nv_bfloat16*)act, ld_act, act_stride, s);
+                           long long act_stride, bool f32, bool pdl, cudaStream_t s) {
+    return f32 ? mix_for(h, prev, mu, pos0, n, width, (float*)act, ld_act, act_stride, pdl, s)
+               : mix_for(h, prev, mu, pos0, n, width, (__nv_bfloat16*)act, ld_act, act_stride, pdl, s);
 }
 
-cudaError_t launch_wkv_inner(const float* inner, int ldp, int slices, int rank, int n, void* act, int ld, cudaStream_t s) {
-    launch_pdl(wkv_inner_kernel, (n * rank + 255) / 256, 256, 0, true, s, inner, ldp, slices, rank, n, (__nv_bfloat16*)act, ld);
+cudaError_t launch_wkv_inner(const float* inner, int ldp, int slices, int rank, int n, void* act, int ld, bool pdl, cudaStream_t s) {
+    launch_pdl(wkv_inner_kernel, (n * rank + 255) / 256, 256, 0, pdl, s, inner, ldp, slices, rank, n, (__nv_bfloat16*)act, ld);
     return cudaGetLastError();
 }
 
@@ -385,10 +385,10 @@ cudaError_t wkv_attrs() {
     return allow_scan<8>();
 }
 
-cudaError_t launch_wkv_rows(const Wkv& wk, const float* proj, int ldp, const float* decay, int pos0, int n, float* out, cudaStream_t s) {
-    if (wk.dim <= 64) return scan_for<2>(wk, proj, ldp, decay, pos0, n, out, s);
-    if (wk.dim <= 128) return scan_for<4>(wk, proj, ldp, decay, pos0, n, out, s);
-    if (wk.dim <= 256) return scan_for<8>(wk, proj, ldp, decay, pos0, n, out, s);
+cudaError_t launch_wkv_rows(const Wkv& wk, const float* proj, int ldp, const float* decay, int pos0, int n, float* out, bool pdl, cudaStream_t s) {
+    if (wk.dim <= 64) return scan_for<2>(wk, proj, ldp, decay, pos0, n, out, pdl, s);
+    if (wk.dim <= 128) return scan_for<4>(wk, proj, ldp, decay, pos0, n, out, pdl, s);
+    if (wk.dim <= 256) return scan_for<8>(wk, proj, ldp, decay, pos0, n, out, pdl, s);
     return cudaErrorInvalidValue;
 }
 

@@ -112,3 +112,17 @@ def test_dense_engines_take_nothing_from_each_other(fake, monkeypatch, mega, siz
     assert fake.fake_refused() == 0
     for e in engines:
         e.close()
+
+
+@pytest.mark.parametrize("math", [MATH_BF16, MATH_F32])
+@pytest.mark.parametrize("layers", [[parallel()], prenorm()], ids=["mitotar", "kuzipel"])
+def test_no_pdl_covers_prompts(fake, monkeypatch, layers, math):
+    for off in ("0", "1"):
+        monkeypatch.setenv("MG_NO_PDL", off)
+        e = layered(fake, layers, math)
+        fake.fake_forget()
+        e.Forward([1] * 300, 0, [299])
+        e.Forward([1], 300, [0])
+        assert fake.fake_launches(b"", -1) > 20
+        assert (fake.fake_launches(b"", 1) > 0) == (off == "0")
+        e.close()
