@@ -40,11 +40,14 @@ static_assert(sizeof(ActBlock) == 40, "activation block is 40 bytes");
 // rows at a time, which share the activation reads; where rows are fewer than warps, `ks` warps share
 // a row and their sums meet in shared memory, in order.
 //
-// The bound is the instruction rate and, for wide inputs, HBM.  The activation slices of a warp's lanes
+// Two chunks per row are under way while a third is multiplied.  The activation slices of a warp's lanes
 // are 36 floats apart: 32 floats apart, all lanes of an access fell on the same four banks and the reads
 // alone took 60 of 104 us of a 3584 x 18944 Q4_0 product.
 constexpr int kRawStages = 3;
 constexpr int kXStride = 36;                                // floats between the activation slices of two blocks
+// Where the kernel reads activations: slices kXStride apart; slices without gaps, the eight 16-byte pieces of block b in the
+// order of piece ^ (b mod 8), which takes a ninth less room and an instruction per read; global memory.
+enum RawInput : int { RAW_PADDED, RAW_SWIZZLED, RAW_GLOBAL };
 __host__ __device__ constexpr int block_bytes(int fmt) { return fmt == FMT_Q8_0 ? 34 : 18; }
 __host__ __device__ constexpr int chunk_ring(int fmt) { return 32 * block_bytes(fmt) + 16; }        // bytes: whole pieces cover a chunk, whatever its alignment
 
@@ -63,15 +66,15 @@ __device__ __forceinline__ void copy_chunk(uint8_t* dst, const uint8_t* src, int
 }
 
 // V: bytes per copy; 16 where the matrix starts on a 16-byte boundary (so no piece starts before it), else 4.
-// XS: the activations fit shared memory.  ks: warps per row.
-template <int FMT, int R, int V, bool XS>
+// X: where the activations are (RawInput).  ks: warps per row.
+template <int FMT, int R, int V, int X>
 __global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __restrict__ act, const uint8_t* __restrict__ w, float* out, int N,
                                                                int K, int ks) {
     constexpr int BB = block_bytes(FMT), QW = FMT == FMT_Q8_0 ? 8 : 4;       // bytes, 4-byte words of quants per block
     constexpr int ring = chunk_ring(FMT);
-    extern __shared__ __align__(16) float raw_xs[];         // kXStride floats per block, 512 R partial sums, then the rings
+    extern __shared__ __align__(16) float raw_xs[];         // activation slices, 16 R partial sums, then the rings
     const int nb = K / 32, chunks = (nb + 31) / 32;
-    float* sums = raw_xs + (XS ? (size_t)nb * kXStride : 0);
+    float* sums = raw_xs + (size_t)nb * (X == RAW_PADDED ? kXStride : X == RAW_SWIZZLED ? 32 : 0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     uint8_t* stage = reinterpret_cast<uint8_t*>(sums + 16 * R) + (size_t)warp * kRawStages * R * ring;
     const int slots = warps / ks, slot = warp / ks, part = warp - slot * ks;
@@ -97,13 +100,15 @@ __global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __re
 #pragma unroll
     for (int s = 0; s < kRawStages - 1; s++) issue(s);
 
-    if (XS) {
+    if (X != RAW_GLOBAL) {
+        auto place = [&](int b, int piece) {                // four floats of block b
+            return raw_xs + (X == RAW_PADDED ? b * kXStride + piece * 4 : b * 32 + (piece ^ (b & 7)) * 4);
+        };
         if ((reinterpret_cast<uintptr_t>(act) & 15) == 0) {
 #pragma unroll 4
-            for (int i = threadIdx.x; i < nb * 8; i += blockDim.x)
-                *reinterpret_cast<float4*>(raw_xs + (i >> 3) * kXStride + (i & 7) * 4) = reinterpret_cast<const float4*>(act)[i];
+            for (int i = threadIdx.x; i < nb * 8; i += blockDim.x) *reinterpret_cast<float4*>(place(i >> 3, i & 7)) = reinterpret_cast<const float4*>(act)[i];
         } else {
-            for (int i = threadIdx.x; i < K; i += blockDim.x) raw_xs[(i >> 5) * kXStride + (i & 31)] = act[i];
+            for (int i = threadIdx.x; i < K; i += blockDim.x) place(i >> 5, (i & 31) >> 2)[i & 3] = act[i];
         }
         __syncthreads();
     }
@@ -140,9 +145,10 @@ __global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __re
                     }
                     sum[r] = 0.f;
                 }
-                const float* xb = XS ? raw_xs + (size_t)b * kXStride : act + (size_t)b * 32;
+                const float* xb = X == RAW_PADDED ? raw_xs + b * kXStride : X == RAW_SWIZZLED ? raw_xs + b * 32 : act + (size_t)b * 32;
                 auto x4 = [&](int i) {
-                    return XS ? *reinterpret_cast<const float4*>(xb + 4 * i) : make_float4(xb[4 * i], xb[4 * i + 1], xb[4 * i + 2], xb[4 * i + 3]);
+                    if (X == RAW_GLOBAL) return make_float4(xb[4 * i], xb[4 * i + 1], xb[4 * i + 2], xb[4 * i + 3]);
+                    return *reinterpret_cast<const float4*>(xb + 4 * (X == RAW_PADDED ? i : i ^ (lane & 7)));
                 };
                 if (FMT == FMT_Q8_0) {
 #pragma unroll
@@ -264,15 +270,20 @@ int static_fail(int code, const char* fmt, int a, int b) {
     return code;
 }
 
-// Two rows per warp where that still leaves every warp a pair; fewer rows than warps are shared by several
-// warps each.  CTAs of 8 warps, up to three per SM, while the activations are small; wide inputs, whose copy a
-// CTA's warps share, take one CTA of 16.  Measured on B200, back to back: 4864 x 896 Q8_0 10.3 -> 4.3 us
-// (the launch), 3584 x 18944 Q4_0 104 -> 26.8 us, 18944 x 3584 Q8_0 26.4 us = 2.7 TB/s.
+// Two rows per warp where every warp has a row; where tiles are fewer than warps, several warps share a row (pair) each.  CTAs
+// of 8 warps, up to three per SM, while the activations are small; wide inputs, whose copy a CTA's warps share, take one
+// CTA of 16, and those that do not fit beside its rings take, in this order, slices without gaps, single rows and 8 warps: Q8_0
+// from 27872 columns on (39648 where rows are single anyway), Q4_0 from 38784 (45120); beyond 51200 (54272) the
+// activations stay in global memory.
+// Measured on B200, weights in no cache, activations read from global memory / from such slices: Q8_0 8192 x 28672 573 / 74 us, 8192 x
+// 40960 817 / 112 us, 256 x 32768 99 / 7 us.  Elsewhere: 4864 x 896 Q8_0 4.7 us (the launch), 18944 x 3584 Q8_0 27 us = 2.7 TB/s;
+// at 18944 columns of Q8_0, 2368 rows 17 us (two warps a pair), 2400 to 4736 rows 27 to 29 us (the walk of one warp over its pair).
 struct RawShape {
-    int grid, threads, ks;
-    bool pairs, xs;
+    int grid, threads, ks, input;
+    bool pairs;
     size_t smem;
 };
+constexpr size_t kRawSmem = 226 * 1024;
 
 template <int FMT>
 RawShape raw_shape(int N, int K, int sms) {
@@ -280,11 +291,16 @@ RawShape raw_shape(int N, int K, int sms) {
     const int nb = K / 32, chunks = cdiv(nb, 32);
     size_t x = (size_t)nb * kXStride * 4;
     auto rest = [&](int warps, int R) { return (size_t)16 * R * 4 + (size_t)warps * kRawStages * R * chunk_ring(FMT); };
-    p.xs = x + rest(16, 2) <= 226 * 1024;
-    if (!p.xs) x = 0;
     const bool wide = x > 24 * 1024;
-    const int warps = wide ? 16 : 8, most = sms * (wide ? 1 : 3);
+    int warps = wide ? 16 : 8, most = sms * (wide ? 1 : 3);
     p.pairs = N >= most * warps;
+    if (x + rest(warps, p.pairs ? 2 : 1) > kRawSmem) {
+        p.input = RAW_SWIZZLED;
+        x = (size_t)K * 4;
+        if (x + rest(warps, p.pairs ? 2 : 1) > kRawSmem) p.pairs = false;
+        if (x + rest(warps, 1) > kRawSmem) warps = 8;
+        if (x + rest(warps, 1) > kRawSmem) { p.input = RAW_GLOBAL; x = 0; most = sms * 3; p.pairs = N >= most * warps; }
+    }
     const int R = p.pairs ? 2 : 1, tiles = cdiv(N, R);
     p.ks = 1;
     while (2 * p.ks <= warps && 2 * p.ks <= chunks && (long long)tiles * 2 * p.ks <= (long long)most * warps) p.ks *= 2;
@@ -294,9 +310,9 @@ RawShape raw_shape(int N, int K, int sms) {
     return p;
 }
 
-template <int FMT, int R, int V, bool XS>
+template <int FMT, int R, int V, int X>
 void run_raw_matvec(const RawShape& p, int dev, const float* act, const uint8_t* w, float* out, int N, int K, cudaStream_t stream) {
-    auto kern = raw_block_matvec_kernel<FMT, R, V, XS>;
+    auto kern = raw_block_matvec_kernel<FMT, R, V, X>;
     static std::atomic<bool> raised[kMaxDevices];
     if (p.smem > 48 * 1024 && !(dev < kMaxDevices && raised[dev].load(std::memory_order_relaxed))) {
         cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -330,8 +346,10 @@ void launch_raw_matvec(const float* act, const void* w_blocks, float* out, int N
     const RawShape p = raw_shape<FMT>(N, K, sms);
     const uint8_t* w = static_cast<const uint8_t*>(w_blocks);
     auto go = [&](auto r, auto v) {
-        if (p.xs) run_raw_matvec<FMT, decltype(r)::value, decltype(v)::value, true>(p, dev, act, w, out, N, K, stream);
-        else run_raw_matvec<FMT, decltype(r)::value, decltype(v)::value, false>(p, dev, act, w, out, N, K, stream);
+        constexpr int R = decltype(r)::value, V = decltype(v)::value;
+        if (p.input == RAW_PADDED) run_raw_matvec<FMT, R, V, RAW_PADDED>(p, dev, act, w, out, N, K, stream);
+        else if (p.input == RAW_SWIZZLED) run_raw_matvec<FMT, R, V, RAW_SWIZZLED>(p, dev, act, w, out, N, K, stream);
+        else run_raw_matvec<FMT, R, V, RAW_GLOBAL>(p, dev, act, w, out, N, K, stream);
     };
     using std::integral_constant;
     const bool v16 = (reinterpret_cast<uintptr_t>(w) & 15) == 0;

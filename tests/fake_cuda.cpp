@@ -18,6 +18,7 @@ constexpr int kDevices = 4, kSms = 148, kSmemOptin = 227 * 1024, kSmemDefault = 
 struct Launch {
     std::string kernel;
     int device;
+    size_t smem;
     bool programmatic;
 };
 
@@ -43,7 +44,7 @@ cudaError_t launched(const void* f, size_t smem, bool programmatic) {
         S().refused++;
         return cudaErrorInvalidValue;
     }
-    S().launches.push_back({S().names[f], S().device, programmatic});
+    S().launches.push_back({S().names[f], S().device, smem, programmatic});
     return cudaSuccess;
 }
 
@@ -64,6 +65,8 @@ int fake_launches(const char* part, int programmatic) {
         n += l.kernel.find(part) != std::string::npos && (programmatic < 0 || l.programmatic == (programmatic == 1));
     return n;
 }
+// Dynamic shared memory of the last launch.
+size_t fake_smem() { return S().launches.empty() ? 0 : S().launches.back().smem; }
 int fake_refused() { return S().refused; }
 void fake_forget() { S().launches.clear(); S().refused = 0; }
 size_t fake_in_use() { return S().in_use; }

@@ -6,9 +6,11 @@ import pytest
 from mongoose_b200 import kernels as K
 
 pytestmark = pytest.mark.gpu
+# activations without gaps: pairs, single rows on 16 and on 8 warps; the narrowest that stay in global memory
+WIDE = [(2369, 28672), (2369, 32800), (40, 39648), (70, 44640), (33, 50752), (9, 51232), (9, 54304)]
 
 
-@pytest.mark.parametrize("N,K_", [(1, 32), (3, 1056), (100, 8192), (65, 19200), (2369, 2080), (3553, 64), (7105, 1024), (20, 51200)])
+@pytest.mark.parametrize("N,K_", [(1, 32), (3, 1056), (100, 8192), (65, 19200), (2369, 2080), (3553, 64), (7105, 1024), (20, 51200), *WIDE])
 @pytest.mark.parametrize("shift", [0, 2, 4, 8])
 @pytest.mark.parametrize("fmt", [0, 1])
 def test_raw_matvec_shapes(cuda, oracle, mglib, N, K_, shift, fmt):

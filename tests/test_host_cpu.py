@@ -30,7 +30,7 @@ def fake_path(tmp_path_factory):
 @pytest.fixture
 def fake(fake_path, monkeypatch):
     lib = _lib._open(fake_path, True)
-    lib.fake_in_use.restype = _lib.sz
+    lib.fake_in_use.restype = lib.fake_smem.restype = _lib.sz
     lib.fake_memory.argtypes = [_lib.sz]
     monkeypatch.setattr(_lib, "_lib", lib)
     lib.fake_memory(8 << 30)
@@ -126,3 +126,12 @@ def test_no_pdl_covers_prompts(fake, monkeypatch, layers, math):
         assert fake.fake_launches(b"", -1) > 20
         assert (fake.fake_launches(b"", 1) > 0) == (off == "0")
         e.close()
+
+
+@pytest.mark.parametrize("fmt", ["q8_0", "q4_0"])
+@pytest.mark.parametrize("rows", [20, 2400, 8192])
+@pytest.mark.parametrize("cols", [896, 18944, 27872, 28672, 32768, 38784, 40960, 49152, 51200])
+def test_matvecs_stage_wide_inputs_in_shared_memory(fake, fmt, rows, cols):
+    getattr(fake, f"mongoose_{fmt}_matvec")(256, 4096, 8192, rows, cols, None)
+    assert fake.fake_launches(b"raw_block_matvec", -1) == 1 and fake.fake_refused() == 0
+    assert fake.fake_smem() >= 4 * cols
