@@ -1,5 +1,5 @@
-// Sigmoid attention with mixed heads over a portion of a prompt, on the tensor cores: for heads of up to 128 one head at a
-// time, mixed in the outputs (gate_flash_kernel, gate_mix_kernel); for wider ones as follows.
+// Sigmoid attention with mixed heads over a portion of a prompt, on the tensor cores, in one of two ways (gate_flash_pays): one
+// head at a time, mixed in the outputs (gate_flash_kernel, gate_mix_kernel), or all heads of a pair at once, as follows.
 //
 // Mixing couples every head at every (query, key) pair, so a CTA owns a tile of 128 queries x BN keys for
 // ALL heads: each head's scores land in their own TMEM columns (heads x BN <= 512), then a thread reads
@@ -288,9 +288,9 @@ __global__ void __launch_bounds__(kThreads, Geo<HP>::per_sm) gate_scores_kernel(
 // ---- heads one at a time, mixed behind the product with the keys ---------------------------------------
 // sum over keys of (sum over g of T[h][g] w_g) v = sum over g of T[h][g] (sum over keys of w_g v): the weights are
 // multiplied by the keys first and the heads are mixed in the outputs.  A head then multiplies the keys of
-// EVERY key head, kv_heads times the products, which the tensor cores do not notice, and mixing falls from
+// EVERY key head, kv_heads times the products, and mixing falls from
 // every (query, key) pair to every query.  A CTA owns 128 queries of one head and up to 256 output columns
-// and walks the keys in tiles of 64: scores into one of two TMEM buffers, sigmoids in fp32 on sixteen warps
+// (more columns are more CTAs, each of which forms the scores again) and walks the keys in tiles of 64: scores into one of two TMEM buffers, sigmoids in fp32 on sixteen warps
 // (a row's 64 keys belong to four threads: a sigmoid is a chain of a dozen instructions; with eight warps, 139 us
 // and 34 % tensor-pipe activity for 2048 queries of 32 heads, with sixteen 122 us),
 // weights as two bf16 parts, high and low, into one of two shared-memory buffers, O += (P_high + P_low) V
@@ -302,7 +302,7 @@ constexpr int kFlashThreads = 576;         // TMA warp, MMA warp, 16 sigmoid war
 struct FlashArgs {
     CUtensorMap q, k, v;            // [rows][heads][dim_s] in boxes of 128 rows; [max_seq][kv][dim_s], 64 rows; [kv * dim][ldv], `cols` rows
     GateAttn at;
-    int row0, rows, pos0;           // queries [row0, row0 + rows) of the portion, at positions pos0 + row
+    int rows, pos0;                 // queries of the portion, at positions pos0 + row
     int kb;                         // 64-column steps of a query
     int per, cols;                  // key heads per CTA; their columns, padded to 16
     int tmem_cols;
@@ -341,8 +341,8 @@ __global__ void __launch_bounds__(kFlashThreads, 1) gate_flash_kernel(const __gr
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = blockIdx.x, c = h / (A.heads / A.kv_heads), c0 = blockIdx.y * a.per;
     const int tile_row = (gridDim.z - 1 - blockIdx.z) * 128;                    // the longest rows of every head first
-    const int first = a.pos0 + a.row0 + tile_row;                               // position of the first query
-    const int last = a.pos0 + a.row0 + min(tile_row + 128, a.rows) - 1;
+    const int first = a.pos0 + tile_row;                                        // position of the first query
+    const int last = a.pos0 + min(tile_row + 128, a.rows) - 1;
     const int tiles = last / kFlashKeys + 1;
 
     if (threadIdx.x == 0) {
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(kFlashThreads, 1) gate_flash_kernel(const __gr
     if (warp == 0) {
         if (lane == 0) {
             bar_expect(q_full, a.kb * 128 * 128);
-            for (int x = 0; x < a.kb; x++) tma_load_3d(Q + x * 128 * 128, &a.q, x * 64, h, a.row0 + tile_row, q_full);
+            for (int x = 0; x < a.kb; x++) tma_load_3d(Q + x * 128 * 128, &a.q, x * 64, h, tile_row, q_full);
             int ki = 0, vi = 0;
             for (int j = 0; j < tiles; j++) {
                 const int s = j & 1, use = j >> 1;
@@ -602,38 +602,51 @@ cudaError_t scores(const ScoreArgs& a, bool pdl, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-}  // namespace
+int flash_key_heads(const GateAttn& at) { return std::min(at.kv_heads, kFlashCols / at.dim); }     // per CTA
 
-namespace {
-
-// Heads one at a time where a query, two buffers of weights and two stages of keys fit shared memory; wider heads take the
-// kernel that mixes pairs.
-bool gate_flash_fits(const GateAttn& at) { return at.dim_s <= 128; }
-
-size_t bytes_per_row(const GateAttn& at, int max_seq) {
-    return gate_flash_fits(at) ? (size_t)at.heads * at.kv_heads * at.dim * 4 : (size_t)at.heads * pad_to(max_seq, 64) * 2;
+// One head at a time where that is the faster way.  Against it: more columns of key heads than a CTA takes are more CTAs (groups) that
+// form the same scores; and a CTA walks every key of its rows, while the pairs of the other kernel are dealt over keys
+// too, so that few heads behind a long context leave most SMs idle.  B200, Forward of one layer of 256 columns, one head at a time / pairs, us:
+// 2048 tokens, 32 heads of 64 with 4, 8, 16 and 32 key heads 243 / 480, 363 / 477, 610 / 481 and 1139 / 485; 512 tokens behind 3584,
+// 16, 8 and 4 heads of 64 with 4 key heads 175 / 237, 168 / 153 and 168 / 127; 128 tokens, 32 heads of 96 with 8 (four groups)
+// 116 / 142.  The lines were laid through 138 shapes of heads at 13 portions each.
+constexpr int kFlashGroups = 4;
+int flash_groups(const GateAttn& at) { return (at.kv_heads + flash_key_heads(at) - 1) / flash_key_heads(at); }
+bool gate_flash_pays(const GateAttn& at, int pos0, int n) {
+    if (at.dim_s > 128) return false;                       // a query, two buffers of weights and two stages of keys fill shared memory
+    const long long longest = (pos0 + n + kFlashKeys - 1) / kFlashKeys;
+    if (flash_groups(at) > 2) return flash_groups(at) <= kFlashGroups && longest <= 2;
+    long long tiles = 0;
+    for (int r = 0; r < n; r += 128) tiles += (pos0 + std::min(r + 128, n) + kFlashKeys - 1) / kFlashKeys;
+    return (longest - 4) * sm_count() <= 4 * at.heads * tiles;
 }
 
-cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* work, int block_rows, const void* vt, int ldv,
+size_t flash_bytes(const GateAttn& at, int max_rows) {
+    if (at.dim_s > 128 || flash_groups(at) > kFlashGroups) return 0;
+    return (size_t)(flash_groups(at) > 2 ? std::min(max_rows, 2 * kFlashKeys) : max_rows) * at.heads * at.kv_heads * at.dim * 4;
+}
+size_t pair_bytes(const GateAttn& at, int rows) { return (size_t)rows * at.heads * pad_to(at.max_seq, 64) * 2; }
+// Queries of a block whose pairs' weights fit `bytes`.
+int pair_rows(const GateAttn& at, int max_rows, size_t bytes) {
+    return std::max(128, (int)std::min<size_t>(bytes / pair_bytes(at, 1), (size_t)pad_to(max_rows, 128)) / 128 * 128);
+}
+
+cudaError_t launch_flash(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* work, const void* vt, int ldv,
                          void* out, int ld_out, int* status, int* launches, bool pdl, cudaStream_t s) {
     FlashArgs a{};
-    a.at = at; a.pos0 = pos0; a.o = (float*)work; a.status = status;
+    a.at = at; a.pos0 = pos0; a.rows = n; a.o = (float*)work; a.status = status;
     a.kb = (at.dim_s + 63) / 64;
-    a.per = std::min(at.kv_heads, kFlashCols / at.dim);
+    a.per = flash_key_heads(at);
     a.cols = pad_to(a.per * at.dim, 16);
     a.tmem_cols = 2 * kFlashKeys + pad_to(a.cols, 32) <= 256 ? 256 : 512;
     if (!make_head_map(&a.q, qh, at.dim_s, at.heads, max_rows, at.dim_s, (long long)at.heads * at.dim_s, 128) ||
         !make_head_map(&a.k, at.cache, at.dim_s, at.kv_heads, at.max_seq, at.dim_s, (long long)at.kv_heads * at.dim_s, kFlashKeys) ||
         !make_tile_map(&a.v, vt, ldv, at.kv_heads * at.dim, 1, ldv, (long long)at.kv_heads * at.dim * ldv, a.cols))
         return cudaErrorInvalidValue;
-    for (int q0 = 0; q0 < n; q0 += block_rows) {
-        a.row0 = q0; a.rows = std::min(block_rows, n - q0);
-        launch_pdl(gate_flash_kernel, dim3(at.heads, (at.kv_heads + a.per - 1) / a.per, (a.rows + 127) / 128), kFlashThreads, flash_smem(a.kb, a.cols), pdl, s, a);
-        __nv_bfloat16* to = (__nv_bfloat16*)out + (size_t)q0 * ld_out;
-        if (at.dim % 2 == 0) launch_pdl(gate_mix_kernel<2>, (a.rows + 1) / 2, 256, 0, pdl, s, at, a.rows, a.o, to, ld_out);
-        else launch_pdl(gate_mix_kernel<1>, a.rows, 256, 0, pdl, s, at, a.rows, a.o, to, ld_out);
-        *launches += 2;
-    }
+    launch_pdl(gate_flash_kernel, dim3(at.heads, (at.kv_heads + a.per - 1) / a.per, (n + 127) / 128), kFlashThreads, flash_smem(a.kb, a.cols), pdl, s, a);
+    if (at.dim % 2 == 0) launch_pdl(gate_mix_kernel<2>, (n + 1) / 2, 256, 0, pdl, s, at, n, a.o, (__nv_bfloat16*)out, ld_out);
+    else launch_pdl(gate_mix_kernel<1>, n, 256, 0, pdl, s, at, n, a.o, (__nv_bfloat16*)out, ld_out);
+    *launches += 2;
     return cudaGetLastError();
 }
 
@@ -649,21 +662,18 @@ cudaError_t gate_attn_tc_attrs() {
 
 bool gate_attn_tc_fits(const GateAttn& at) { return at.heads <= 32; }
 
-size_t gate_attn_tc_bytes(const GateAttn& at, int max_seq, int block_rows) { return bytes_per_row(at, max_seq) * block_rows; }
-
-int gate_attn_tc_rows(const GateAttn& at, int max_seq, int max_rows, size_t budget) {
-    const size_t per = bytes_per_row(at, max_seq);
-    int rows = (int)std::min<size_t>(budget / per, (size_t)pad_to(max_rows, 128)) / 128 * 128;
-    return rows < 128 ? 128 : rows;
+size_t gate_attn_tc_bytes(const GateAttn& at, int max_rows, size_t budget) {
+    return std::max(pair_bytes(at, pair_rows(at, max_rows, budget)), flash_bytes(at, max_rows));
 }
 
-cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* weights, int block_rows, void* vt,
+cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* weights, size_t bytes, void* vt,
                                 void* out, int ld_out, int* status, int* launches, bool pdl, cudaStream_t s) {
     const int len = pos0 + n, ldv = pad_to(len, 64);
     launch_pdl(key_transpose_kernel, dim3(ldv / 32, (at.dim + 31) / 32, at.kv_heads), 256, 0, pdl, s, (const __nv_bfloat16*)at.cache, at.kv_heads, at.dim,
                                                                                        at.dim_s, len, ldv, (__nv_bfloat16*)vt);
     *launches += 1;
-    if (gate_flash_fits(at)) return launch_flash(at, qh, pos0, n, max_rows, weights, block_rows, vt, ldv, out, ld_out, status, launches, pdl, s);
+    if (gate_flash_pays(at, pos0, n)) return launch_flash(at, qh, pos0, n, max_rows, weights, vt, ldv, out, ld_out, status, launches, pdl, s);
+    const int block_rows = pair_rows(at, max_rows, bytes);
     const int hp = at.heads <= 4 ? 4 : at.heads <= 8 ? 8 : at.heads <= 16 ? 16 : 32;
     ScoreArgs a{};
     a.at = at; a.pos0 = pos0; a.w = (__nv_bfloat16*)weights; a.status = status;

@@ -258,14 +258,6 @@ cudaError_t run(const Args& a, int parts, cudaStream_t s) {
     return cudaLaunchKernelEx(&cfg, gemm_f32_kernel<NT>, a);
 }
 
-int sm_count() {
-    static const int n = [] {
-        int dev = 0, v = 0;
-        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? v : 148;
-    }();
-    return n;
-}
-
 }  // namespace
 
 cudaError_t gemm_f32_attrs() {

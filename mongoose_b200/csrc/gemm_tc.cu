@@ -221,14 +221,6 @@ bool encode(CUtensorMap* map, const void* base, const cuuint64_t dims[3], const 
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-int sm_count() {
-    static const int n = [] {
-        int dev = 0, v = 0;
-        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 148;
-    }();
-    return n;
-}
-
 template <int BN>
 cudaError_t run(const GemmTC& g, bool pdl, cudaStream_t s) {
     const int cols = g.mode == GEMM_SILU_BF16 ? BN / 2 : BN, gx = (g.n + cols - 1) / cols, gy = (g.m + 127) / 128, tiles = gx * gy * g.batch;

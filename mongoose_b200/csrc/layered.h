@@ -248,13 +248,12 @@ cudaError_t launch_qk_rows(const GateAttn& at, const float* proj, int ldp, int q
 cudaError_t launch_gate_attn_rows(const GateAttn& at, const void* qh, int pos0, int n, void* out, int ld_out, bool f32,
                                   bool pdl, cudaStream_t s);
 size_t gate_attn_rows_smem(const GateAttn& at, bool f32, int* tile);
-// The same on the tensor cores (bf16 only, gate_attn_tc.cu): `weights` is a workspace for blocks of block_rows queries
-// (gate_attn_tc_rows of them fit `budget`, gate_attn_tc_bytes), `vt` the keys transposed; qh has max_rows rows.
+// The same on the tensor cores (bf16 only, gate_attn_tc.cu): `weights` is a workspace of `bytes`, gate_attn_tc_bytes of them for
+// portions of max_rows rows (`budget` where the context is long), `vt` the keys transposed; qh has max_rows rows.
 bool gate_attn_tc_fits(const GateAttn& at);
-int gate_attn_tc_rows(const GateAttn& at, int max_seq, int max_rows, size_t budget);
-size_t gate_attn_tc_bytes(const GateAttn& at, int max_seq, int block_rows);
+size_t gate_attn_tc_bytes(const GateAttn& at, int max_rows, size_t budget);
 cudaError_t gate_attn_tc_attrs();
-cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* weights, int block_rows, void* vt,
+cudaError_t launch_gate_attn_tc(const GateAttn& at, const void* qh, int pos0, int n, int max_rows, void* weights, size_t bytes, void* vt,
                                 void* out, int ld_out, int* status, int* launches, bool pdl, cudaStream_t s);
 // x += norm(z) or x += norm(half the sum of two normed branches); act = x
 cudaError_t launch_post_rows(float* x, const float* z0, const float* z1, const float* w0, const float* w1, const float* post_w,

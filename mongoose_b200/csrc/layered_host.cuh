@@ -10,7 +10,7 @@ struct LayerWeights {
     // MG_MIXER_PARALLEL
     ProjCols cols{};
     int splits = 1, tile = 16;
-    int block_rows = 0;                 // queries per block of the tensor-core attention; 0: CUDA-core kernel
+    size_t attn_bytes = 0;              // workspace of the tensor-core attention; 0: CUDA-core kernel
     uint8_t *at_o = nullptr, *mem_o = nullptr, *up = nullptr, *down = nullptr;
     float *at_out = nullptr, *mem_out = nullptr;
     float *q_norm = nullptr, *k_norm = nullptr, *talk = nullptr, *bias = nullptr, *slopes = nullptr;
@@ -139,8 +139,8 @@ int layered_buffers(Layered& m, F take) {
             ff = std::max(ff, (size_t)pad_to(l.c.ffn_dim, 64)); mh = std::max(mh, (size_t)r.heads);
             const size_t chunks = (T + kMemChunk - 1) / kMemChunk;
             u = std::max(u, chunks * r.heads * r.dim * r.vdim); nu = std::max(nu, chunks * r.heads * r.dim);
-            if (l.block_rows) {
-                aw = std::max(aw, gate_attn_tc_bytes(l.at, c.max_seq, l.block_rows));
+            if (l.attn_bytes) {
+                aw = std::max(aw, l.attn_bytes);
                 vt = std::max(vt, (size_t)a.kv_heads * a.dim * ldv);
             }
             part = std::max(part, (size_t)l.splits * a.heads * l.at.dim_s);
@@ -254,7 +254,7 @@ int parallel_shapes(Layered& m, LayerWeights& l, int sms, std::string* why) {
     const int n_mem = r.heads * ((r.vdim + 31) / 32);
     l.splits = std::max(32, sms - n_mem);
     if (!mixer_step_smem(g, q, m.f32, &l.tile)) { *why = "attention heads do not fit one CTA's registers or shared memory"; return MG_ERR_UNSUPPORTED; }
-    if (!m.f32 && gate_attn_tc_fits(g)) l.block_rows = gate_attn_tc_rows(g, c.max_seq, m.max_rows, (size_t)256 << 20);
+    if (!m.f32 && gate_attn_tc_fits(g)) l.attn_bytes = gate_attn_tc_bytes(g, m.max_rows, (size_t)256 << 20);
     ProjCols& p = l.cols;
     int o = 0;
     auto col = [&](int n) { const int at = o; o += n; return at; };
@@ -838,9 +838,9 @@ int parallel_rows(mg_engine* e, const LayerRun& run, LayerWeights& l, int pos, i
     int rc;
     if ((rc = layered_matmul(e, m.act, m.max_rows, m.kw, l.proj, m.P, np, n, l.cols.total, false))) return rc;
     MG_CUDA(e, launch_qk_rows(at, m.P, np, l.cols.q, l.cols.k, pos, n, m.qh, m.f32, e->prompt_pdl, s));
-    if (l.block_rows) {
+    if (l.attn_bytes) {
         int k = 0;
-        MG_CUDA(e, launch_gate_attn_tc(at, m.qh, pos, n, m.max_rows, m.aw, l.block_rows, m.vt, m.ao, kat, m.status, &k, e->prompt_pdl, s));
+        MG_CUDA(e, launch_gate_attn_tc(at, m.qh, pos, n, m.max_rows, m.aw, l.attn_bytes, m.vt, m.ao, kat, m.status, &k, e->prompt_pdl, s));
         e->launches += k - 1;
     } else {
         MG_CUDA(e, launch_gate_attn_rows(at, m.qh, pos, n, m.ao, kat, m.f32, e->prompt_pdl, s));

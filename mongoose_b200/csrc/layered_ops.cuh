@@ -359,6 +359,14 @@ __device__ __forceinline__ void attend(const GateAttn& A, const AttnSmem<KT>& sm
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + expf(-z)); }
 
+inline int sm_count() {
+    static const int n = [] {
+        int dev = 0, v = 0;
+        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 148;
+    }();
+    return n;
+}
+
 // Dynamic shared memory that a kernel may be launched with on the current device.  The limit belongs to the device, so every engine
 // sets it when it is created.  All engines of a process share it: a kernel whose need depends on the model gets what any of them
 // may need, kModelSmem, so that a small model does not take it from a large one.

@@ -135,3 +135,22 @@ def test_matvecs_stage_wide_inputs_in_shared_memory(fake, fmt, rows, cols):
     getattr(fake, f"mongoose_{fmt}_matvec")(256, 4096, 8192, rows, cols, None)
     assert fake.fake_launches(b"raw_block_matvec", -1) == 1 and fake.fake_refused() == 0
     assert fake.fake_smem() >= 4 * cols
+
+
+# heads, key heads, dim, tokens behind position -> the kernel of the bf16 attention
+ROUTES = [(32, 4, 64, 0, 500, "flash"), (32, 8, 64, 0, 500, "flash"), (32, 16, 64, 0, 500, "scores"), (32, 32, 64, 0, 500, "scores"), (32, 32, 64, 0, 2, "scores"),
+          (28, 4, 128, 0, 500, "flash"), (32, 8, 128, 0, 128, "flash"), (32, 8, 128, 0, 129, "scores"), (16, 8, 128, 0, 500, "scores"), (20, 20, 12, 0, 500, "flash"), (6, 6, 136, 0, 300, "scores"),
+          (4, 4, 64, 0, 200, "flash"), (4, 4, 64, 0, 500, "scores"), (32, 4, 64, 400, 100, "flash"), (16, 4, 64, 400, 100, "scores"), (2, 2, 64, 400, 100, "scores")]
+
+
+@pytest.mark.parametrize("heads,kv,dim,pos,n,kernel", ROUTES)
+def test_route_of_the_gate_attention(fake, heads, kv, dim, pos, n, kernel):
+    e = layered(fake, [parallel(dim, heads, kv)])
+    if pos:
+        e.Forward([1] * pos, 0)
+    fake.fake_forget()
+    e.Forward([1] * n, pos)
+    other = {"flash": "scores", "scores": "flash"}[kernel]
+    assert fake.fake_launches(b"gate_%s_kernel" % kernel.encode(), -1) == 1 and fake.fake_launches(b"gate_%s_kernel" % other.encode(), -1) == 0
+    assert fake.fake_refused() == 0
+    e.close()
