@@ -271,7 +271,7 @@ int static_fail(int code, const char* fmt, int a, int b) {
 }
 
 // Two rows per warp where every warp has a row; where tiles are fewer than warps, several warps share a row (pair) each.  CTAs
-// of 8 warps, up to three per SM, while the activations are small; wide inputs, whose copy a CTA's warps share, take one
+// of 8 warps, three per SM (two where no more fit: Q8_0 8192 x 5376 19 us, 29 with a third left for a second round), while the activations are small; wide inputs, whose copy a CTA's warps share, take one
 // CTA of 16, and those that do not fit beside its rings take, in this order, slices without gaps, single rows and 8 warps: Q8_0
 // from 27872 columns on (39648 where rows are single anyway), Q4_0 from 38784 (45120); beyond 51200 (54272) the
 // activations stay in global memory.
@@ -283,7 +283,7 @@ struct RawShape {
     bool pairs;
     size_t smem;
 };
-constexpr size_t kRawSmem = 226 * 1024;
+constexpr size_t kRawSmem = 226 * 1024, kSmSmem = 228 * 1024;      // of a CTA; of an SM, 1 KB of it for each CTA
 
 template <int FMT>
 RawShape raw_shape(int N, int K, int sms) {
@@ -302,11 +302,12 @@ RawShape raw_shape(int N, int K, int sms) {
         if (x + rest(warps, 1) > kRawSmem) { p.input = RAW_GLOBAL; x = 0; most = sms * 3; p.pairs = N >= most * warps; }
     }
     const int R = p.pairs ? 2 : 1, tiles = cdiv(N, R);
+    p.smem = x + rest(warps, R);
+    most = std::min(most, sms * (int)(kSmSmem / (p.smem + 1024)));         // no second round of CTAs
     p.ks = 1;
     while (2 * p.ks <= warps && 2 * p.ks <= chunks && (long long)tiles * 2 * p.ks <= (long long)most * warps) p.ks *= 2;
     p.grid = std::min(cdiv(tiles, warps / p.ks), most);
     p.threads = warps * 32;
-    p.smem = x + rest(warps, R);
     return p;
 }
 

@@ -19,6 +19,7 @@ struct Launch {
     std::string kernel;
     int device;
     size_t smem;
+    int ctas;
     bool programmatic;
 };
 
@@ -30,7 +31,8 @@ struct State {
     std::vector<Launch> launches;
     std::map<void*, size_t> blocks;
     size_t in_use = 0, memory = (size_t)8 << 30;
-    size_t pushed = 0;                  // dynamic shared memory of the launch in the making
+    size_t pushed = 0;                  // dynamic shared memory and grid of the launch in the making
+    dim3 pushed_grid{1, 1, 1};
     int refused = 0;
 };
 State& S() {
@@ -38,13 +40,13 @@ State& S() {
     return *s;
 }
 
-cudaError_t launched(const void* f, size_t smem, bool programmatic) {
+cudaError_t launched(const void* f, dim3 grid, size_t smem, bool programmatic) {
     const auto a = S().allowed.find({f, S().device});
     if (smem > (a == S().allowed.end() ? (size_t)kSmemDefault : a->second)) {
         S().refused++;
         return cudaErrorInvalidValue;
     }
-    S().launches.push_back({S().names[f], S().device, smem, programmatic});
+    S().launches.push_back({S().names[f], S().device, smem, (int)(grid.x * grid.y * grid.z), programmatic});
     return cudaSuccess;
 }
 
@@ -65,8 +67,9 @@ int fake_launches(const char* part, int programmatic) {
         n += l.kernel.find(part) != std::string::npos && (programmatic < 0 || l.programmatic == (programmatic == 1));
     return n;
 }
-// Dynamic shared memory of the last launch.
+// Dynamic shared memory and CTAs of the last launch.
 size_t fake_smem() { return S().launches.empty() ? 0 : S().launches.back().smem; }
+int fake_ctas() { return S().launches.empty() ? 0 : S().launches.back().ctas; }
 int fake_refused() { return S().refused; }
 void fake_forget() { S().launches.clear(); S().refused = 0; }
 size_t fake_in_use() { return S().in_use; }
@@ -78,9 +81,10 @@ void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
 void __cudaRegisterFunction(void**, const char* f, char*, const char* name, int, void*, void*, void*, void*, int*) { S().names[f] = name; }
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
-unsigned __cudaPushCallConfiguration(dim3, dim3, size_t smem, struct CUstream_st*) { S().pushed = smem; return 0; }
+unsigned __cudaPushCallConfiguration(dim3 grid, dim3, size_t smem, struct CUstream_st*) { S().pushed_grid = grid; S().pushed = smem; return 0; }
 cudaError_t __cudaPopCallConfiguration(dim3* grid, dim3* block, size_t* smem, void* stream) {
-    *grid = *block = dim3{1, 1, 1};
+    *grid = S().pushed_grid;
+    *block = dim3{1, 1, 1};
     *smem = S().pushed;
     *(void**)stream = nullptr;
     return cudaSuccess;
@@ -169,13 +173,13 @@ cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
     return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t) { *n = 1; return cudaSuccess; }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) { return launched(f, smem, false); }
-cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3, dim3, void**, size_t smem, cudaStream_t) { return launched(f, smem, false); }
+cudaError_t cudaLaunchKernel(const void* f, dim3 grid, dim3, void**, size_t smem, cudaStream_t) { return launched(f, grid, smem, false); }
+cudaError_t cudaLaunchCooperativeKernel(const void* f, dim3 grid, dim3, void**, size_t smem, cudaStream_t) { return launched(f, grid, smem, false); }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
     bool programmatic = false;
     for (unsigned i = 0; i < c->numAttrs; i++)
         programmatic |= c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization && c->attrs[i].val.programmaticStreamSerializationAllowed;
-    return launched(f, c->dynamicSmemBytes, programmatic);
+    return launched(f, c->gridDim, c->dynamicSmemBytes, programmatic);
 }
 
 }  // extern "C"

@@ -137,6 +137,13 @@ def test_matvecs_stage_wide_inputs_in_shared_memory(fake, fmt, rows, cols):
     assert fake.fake_smem() >= 4 * cols
 
 
+@pytest.mark.parametrize("fmt", ["q8_0", "q4_0"])
+@pytest.mark.parametrize("cols", [896, 5120, 5280, 5376, 5440, 5472, 18944])
+def test_matvecs_launch_no_more_ctas_than_fit(fake, fmt, cols):
+    getattr(fake, f"mongoose_{fmt}_matvec")(256, 4096, 8192, 20000, cols, None)
+    assert fake.fake_ctas() <= 148 * (228 * 1024 // (fake.fake_smem() + 1024))
+
+
 # heads, key heads, dim, tokens behind position -> the kernel of the bf16 attention
 ROUTES = [(32, 4, 64, 0, 500, "flash"), (32, 8, 64, 0, 500, "flash"), (32, 16, 64, 0, 500, "scores"), (32, 32, 64, 0, 500, "scores"), (32, 32, 64, 0, 2, "scores"),
           (28, 4, 128, 0, 500, "flash"), (32, 8, 128, 0, 128, "flash"), (32, 8, 128, 0, 129, "scores"), (16, 8, 128, 0, 500, "scores"), (20, 20, 12, 0, 500, "flash"), (6, 6, 136, 0, 300, "scores"),
