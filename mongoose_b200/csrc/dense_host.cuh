@@ -10,35 +10,44 @@ constexpr int kPromptMin = 4;
 // 512 tokens: 2.2 ms for six layers of 1.1B widths (101 ms one by one), 1.8 ms for two of 7B (134 ms).
 constexpr int kPromptBatch = 512;
 
-template <typename Alloc>
-int dense_prompt_buffers(mg_engine* e, Alloc alloc) {
-    DensePrompt& p = e->prompt;
-    const mg_config& c = e->cfg;
-    const size_t cap = std::min(kPromptBatch, (c.max_seq + 63) & ~63), widest = std::max(2 * c.ffn_dim, c.dim + 2 * c.kv_dim);
-    // a product is cut along K only while its tiles of 128 x 64 leave SMs idle
-    const size_t sums = std::max(cap * widest, (size_t)e->num_sms * 128 * 64);
-    int rc;
-    if ((rc = alloc((void**)&p.tokens, (size_t)e->out_cap * 4)) || (rc = alloc((void**)&p.x, cap * c.dim * 4)) ||
-        (rc = alloc((void**)&p.q, cap * c.dim * 4)) || (rc = alloc((void**)&p.sums, sums * 4)) ||
-        (rc = alloc((void**)&p.act, 3 * cap * c.dim * 2)) || (rc = alloc((void**)&p.mid, 3 * cap * c.ffn_dim * 2)) ||
-        (rc = alloc((void**)&p.status, 4)))
-        return rc;
-    return MG_OK;
+void dense_prompt_free(mg_engine* e) {
+    if (e->prompt.block) cudaFree(e->prompt.block);
+    e->dev_bytes -= e->prompt.bytes;
+    e->prompt = DensePrompt{};
 }
 
-int dense_prompt_create(mg_engine* e) {
+// The workspace, for engines that batch prompts: one GPU and every layer.  It is an allocation of its own, since the arena is made
+// before an engine is told its share of a model; where there is no memory for it, prompts are fed token by token.
+int dense_prompt_build(mg_engine* e) {
     DensePrompt& p = e->prompt;
     const mg_config& c = e->cfg;
-    if (c.dim > kPromptMaxWidth) return MG_OK;
-    int rc = dense_prompt_buffers(e, [&](void** b, size_t bytes) {
-        uint8_t* d = nullptr;
-        const int r = dev_alloc(e, &d, bytes);
-        *b = d;
-        return r;
-    });
-    if (rc) return rc;
-    if (cudaMemset(p.status, 0, 4) != cudaSuccess) return MG_ERR_CUDA;
-    const int cap = std::min(kPromptBatch, (c.max_seq + 63) & ~63);
+    const bool wanted = c.dim <= kPromptMaxWidth && e->sh.size == 1 && e->own_ls == 0 && e->own_le == c.n_layers;
+    if (wanted == (p.cap > 0)) return MG_OK;
+    dense_prompt_free(e);
+    if (!wanted) return MG_OK;
+    const int cap = std::min(kPromptBatch, (c.max_seq + 63) & ~63), widest = std::max(2 * c.ffn_dim, c.dim + 2 * c.kv_dim);
+    // a product is cut along K only while its tiles of 128 x 64 leave SMs idle
+    const size_t sums = std::max((size_t)cap * widest, (size_t)e->num_sms * 128 * 64);
+    size_t at = 0;
+    auto carve = [&](auto** b, size_t count) {              // first the sizes, then the places
+        if (p.block) *b = reinterpret_cast<std::remove_reference_t<decltype(*b)>>(p.block + at);
+        at += (count * sizeof(**b) + 255) & ~(size_t)255;
+    };
+    auto all = [&] {
+        at = 0;
+        carve(&p.tokens, e->out_cap); carve(&p.x, (size_t)cap * c.dim); carve(&p.q, (size_t)cap * c.dim); carve(&p.sums, sums);
+        carve(&p.act, (size_t)3 * cap * c.dim); carve(&p.mid, (size_t)3 * cap * c.ffn_dim); carve(&p.status, 1);
+    };
+    all();
+    if (cudaMalloc((void**)&p.block, at) != cudaSuccess) {
+        cudaGetLastError();
+        p.block = nullptr;
+        return MG_OK;
+    }
+    all();
+    p.bytes = at;
+    e->dev_bytes += at;
+    MG_CUDA(e, cudaMemset(p.status, 0, 4));
     for (int i = 0; i < 2; i++)
         if (!make_tile_map(&p.act_map[i], p.act, c.dim, cap, 3, c.dim, (long long)cap * c.dim, i ? 32 : 64) ||
             !make_tile_map(&p.mid_map[i], p.mid, c.ffn_dim, cap, 3, c.ffn_dim, (long long)cap * c.ffn_dim, i ? 32 : 64))
@@ -47,7 +56,7 @@ int dense_prompt_create(mg_engine* e) {
     return MG_OK;
 }
 
-bool dense_prompt_takes(const mg_engine* e, int n) { return !e->lm && e->prompt.cap && e->sh.size == 1 && n >= kPromptMin; }
+bool dense_prompt_takes(const mg_engine* e, int n) { return e->prompt.cap && n >= kPromptMin; }
 
 // x W^T for up to three matrices on one input, into p.sums.
 int dense_prompt_gemm(mg_engine* e, const CUtensorMap maps[2], int K, int n, const int* slots, int n_mats, PieceSums* out) {

@@ -158,6 +158,8 @@ struct Arena {
 // stream's worth, like its other activations.
 struct DensePrompt {
     int cap = 0;                        // tokens per batch; 0: prompts are fed token by token
+    uint8_t* block = nullptr;           // the allocation that holds what follows
+    size_t bytes = 0;
     int* tokens = nullptr;              // [out_cap]
     float *x = nullptr, *q = nullptr, *sums = nullptr;      // [cap][dim], [cap][dim], pieces of products
     __nv_bfloat16 *act = nullptr, *mid = nullptr;           // [3][cap][dim], [3][cap][ffn]
@@ -1421,7 +1423,6 @@ int mg_create(const mg_config* cfg, mg_engine** out) {
         }
         size_t want = 2 * planes + planes / 16 + kv_elems * 4 + (size_t)c.max_seq * half * 8 + (size_t)c.vocab * 8 +
                       (size_t)(c.dim * 64 + c.ffn_dim * 16) + (size_t)e->out_cap * 4 + (64u << 20);
-        dense_prompt_buffers(e, [&](void**, size_t bytes) { want += (bytes + 511) & ~(size_t)255; return MG_OK; });
         if (const char* mb = getenv("MG_ARENA_MB")) want = (size_t)atoll(mb) << 20;
         if (!e->arena.init(want)) fprintf(stderr, "[mongoose-b200] arena of %zu MB not available: falling back to one allocation per buffer\n", want >> 20);
     }
@@ -1436,7 +1437,6 @@ int mg_create(const mg_config* cfg, mg_engine** out) {
     if ((rc = dev_alloc(e, &e->mid, (size_t)c.ffn_dim))) return bail(rc);
     if ((rc = dev_alloc(e, &e->logits, (size_t)c.vocab))) return bail(rc);
     if ((rc = create_cursor(e))) return bail(rc);
-    if ((rc = dense_prompt_create(e))) return bail(rc);
 
     // RoPE tables in float64 on the host, narrowed to fp32 (cuda_fused_infer.go:181-190).
     {
@@ -1520,6 +1520,7 @@ void mg_destroy(mg_engine* e) {
     if (e->stream) cudaStreamSynchronize(e->stream);
     drop_graphs(e);
     free_mega(e);
+    dense_prompt_free(e);
     for (auto& m : e->mats) {
         if (m.qs) ARENA_FREE(e, m.qs);
         if (m.ds) ARENA_FREE(e, m.ds);
@@ -1627,7 +1628,7 @@ int mg_build(mg_engine* e) {
             return fail(e, MG_ERR_STATE, "mg_build: weight slot %d has not been set", idx);
     }
     drop_graphs(e);
-    if ((rc = build_mega(e))) return rc;
+    if ((rc = build_mega(e)) || (rc = dense_prompt_build(e))) return rc;
     e->built = true;
     return MG_OK;
 }

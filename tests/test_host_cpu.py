@@ -87,7 +87,7 @@ def test_a_smaller_engine_takes_nothing_from_a_larger_one(fake, math):
     assert fake.fake_refused() == 0
 
 
-def dense(fake, cfg):
+def dense(fake, cfg, build=True):
     e = CUDAFusedInference(cfg)
     for idx in range(12 * cfg.n_layers + 2):
         s = idx % 12 if idx < 12 * cfg.n_layers else -1
@@ -97,7 +97,8 @@ def dense(fake, cfg):
             e.SetWeight(idx, np.zeros(cfg.dim, np.float32))
         elif s == -1:
             e.SetWeight(idx, np.zeros((cfg.vocab, cfg.dim), np.float32))
-    e.BuildFusedDispatch()
+    if build:
+        e.BuildFusedDispatch()
     return e
 
 
@@ -160,4 +161,34 @@ def test_route_of_the_gate_attention(fake, heads, kv, dim, pos, n, kernel):
     other = {"flash": "scores", "scores": "flash"}[kernel]
     assert fake.fake_launches(b"gate_%s_kernel" % kernel.encode(), -1) == 1 and fake.fake_launches(b"gate_%s_kernel" % other.encode(), -1) == 0
     assert fake.fake_refused() == 0
+    e.close()
+
+
+def test_prompt_workspace_is_for_engines_that_batch_prompts(fake, monkeypatch):
+    """Not for the stages of a pipeline, and never at the price of an engine that would otherwise be made."""
+    monkeypatch.setenv("MG_NO_MEGA", "1")
+    cfg = mc.TINY.with_(ffn_dim=9600, max_seq=512)
+    least = 3 * 512 * cfg.ffn_dim * 2                       # of one of its buffers
+    e = dense(fake, cfg, build=False)
+    made = fake.fake_in_use()
+    e.BuildFusedDispatch()
+    whole = fake.fake_in_use()
+    assert whole > made + least and e.ArenaStats()["outside"] == 0
+    e.Generate([1] * 40, 3)
+    assert fake.fake_launches(b"prompt_gemm", -1) > 0
+    e.SetLayerRange(0, 1)
+    e.BuildFusedDispatch()
+    assert fake.fake_in_use() == made
+    e.SetLayerRange(0, cfg.n_layers)
+    e.BuildFusedDispatch()
+    assert fake.fake_in_use() == whole
+    # no room: token by token
+    e.close()
+    assert fake.fake_in_use() == 0
+    e = dense(fake, cfg, build=False)
+    fake.fake_memory(fake.fake_in_use() + least)
+    e.BuildFusedDispatch()
+    fake.fake_forget()
+    e.Generate([1] * 40, 3)
+    assert fake.fake_launches(b"prompt_gemm", -1) == 0 and fake.fake_launches(b"", -1) > 0
     e.close()
