@@ -822,7 +822,7 @@ def measure_layered(args, torch, cfg, local_rank, sampler, with_e2e):
 def run_layered_workload(args, cfg, local_rank):
     """Prefill of one portion and greedy decode at several contexts, random-init weights.  A step is one
     decode token at the first context; `closest` is the dense model of the same widths (Q8_0 on its
-    default path, prompts fed token by token as it does), for Kuzipel the Mitotar model of the same widths."""
+    default path, prompts in batches as it takes them), for Kuzipel the Mitotar model of the same widths."""
     import torch
     from mongoose_b200 import layered
     from mongoose_b200.fused_infer import CUDAFusedInference

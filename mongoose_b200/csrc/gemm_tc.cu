@@ -245,7 +245,10 @@ bool make_head_map(CUtensorMap* map, const void* base, int k, int batch, int row
 
 int gemm_tc_bn(int m, int n, int batch) {
     if (n <= 64) return 64;
-    // rounds of tiles over the SMs, times what a tile of each width takes
+    // Rounds of tiles over the SMs, times what a tile of each width takes.  Measured on B200, 2048 columns of K: 11.5, 13.5 and 18.9 us where
+    // a CTA walks several tiles, 12, 15.5 and 24.4 where it has one, whose copies and results nothing hides.  Over the 504 products
+    // of prompts of 128 to 2048 tokens of six models the choices take 17.5 ms and the best ones 17.1; the furthest off are
+    // gated products of experts (75 us for 51), whose row tiles are counted as if every expert's last one were used.
     const int rows = (m + 127) / 128 * batch;
     int best = 64;
     float least = 0.f;

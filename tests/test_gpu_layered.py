@@ -200,8 +200,8 @@ def test_sequences_that_reuse_the_cache(load, dtype):
 
 
 def test_prompts_longer_than_a_block_of_rows(load):
-    """One call that the engine cuts into blocks of rows, and attention into blocks of queries, equals
-    portions that need no cutting, in 32-bit and (within its rounding) in bf16."""
+    """One call that the engine cuts into blocks of rows equals portions that need no cutting, in 32-bit and
+    (within its rounding) in bf16.  (Blocks of queries within a portion: test_gpu_gate_routes.py.)"""
     cfg = U.config(64, 90, 1e-5, [U.layer(32, 8, 8, 0.35, 0.3, 300, 2, 16, 24, 8.0, 48)])
     w = U.weights(cfg, seed=41)
     n = 2175
