@@ -158,7 +158,7 @@ struct Arena {
 // stream's worth, like its other activations.
 struct DensePrompt {
     int cap = 0;                        // tokens per batch; 0: prompts are fed token by token
-    uint8_t* block = nullptr;           // the allocation that holds what follows
+    uint8_t* block = nullptr;           // holds what follows
     size_t bytes = 0;
     int* tokens = nullptr;              // [out_cap]
     float *x = nullptr, *q = nullptr, *sums = nullptr;      // [cap][dim], [cap][dim], pieces of products
@@ -1423,6 +1423,7 @@ int mg_create(const mg_config* cfg, mg_engine** out) {
         }
         size_t want = 2 * planes + planes / 16 + kv_elems * 4 + (size_t)c.max_seq * half * 8 + (size_t)c.vocab * 8 +
                       (size_t)(c.dim * 64 + c.ffn_dim * 16) + (size_t)e->out_cap * 4 + (64u << 20);
+        want += dense_prompt_carve(e, e->prompt, nullptr);
         if (const char* mb = getenv("MG_ARENA_MB")) want = (size_t)atoll(mb) << 20;
         if (!e->arena.init(want)) fprintf(stderr, "[mongoose-b200] arena of %zu MB not available: falling back to one allocation per buffer\n", want >> 20);
     }
@@ -1437,6 +1438,7 @@ int mg_create(const mg_config* cfg, mg_engine** out) {
     if ((rc = dev_alloc(e, &e->mid, (size_t)c.ffn_dim))) return bail(rc);
     if ((rc = dev_alloc(e, &e->logits, (size_t)c.vocab))) return bail(rc);
     if ((rc = create_cursor(e))) return bail(rc);
+    if ((rc = dense_prompt_build(e))) return bail(rc);
 
     // RoPE tables in float64 on the host, narrowed to fp32 (cuda_fused_infer.go:181-190).
     {

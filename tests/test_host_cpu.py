@@ -87,7 +87,7 @@ def test_a_smaller_engine_takes_nothing_from_a_larger_one(fake, math):
     assert fake.fake_refused() == 0
 
 
-def dense(fake, cfg, build=True):
+def dense(fake, cfg):
     e = CUDAFusedInference(cfg)
     for idx in range(12 * cfg.n_layers + 2):
         s = idx % 12 if idx < 12 * cfg.n_layers else -1
@@ -97,8 +97,7 @@ def dense(fake, cfg, build=True):
             e.SetWeight(idx, np.zeros(cfg.dim, np.float32))
         elif s == -1:
             e.SetWeight(idx, np.zeros((cfg.vocab, cfg.dim), np.float32))
-    if build:
-        e.BuildFusedDispatch()
+    e.BuildFusedDispatch()
     return e
 
 
@@ -165,30 +164,29 @@ def test_route_of_the_gate_attention(fake, heads, kv, dim, pos, n, kernel):
 
 
 def test_prompt_workspace_is_for_engines_that_batch_prompts(fake, monkeypatch):
-    """Not for the stages of a pipeline, and never at the price of an engine that would otherwise be made."""
+    """Stages of a pipeline give it back, and it is never the price of an engine that would otherwise be made."""
     monkeypatch.setenv("MG_NO_MEGA", "1")
     cfg = mc.TINY.with_(ffn_dim=9600, max_seq=512)
     least = 3 * 512 * cfg.ffn_dim * 2                       # of one of its buffers
-    e = dense(fake, cfg, build=False)
-    made = fake.fake_in_use()
-    e.BuildFusedDispatch()
-    whole = fake.fake_in_use()
-    assert whole > made + least and e.ArenaStats()["outside"] == 0
+    e = dense(fake, cfg)
+    whole = e.ArenaStats()
+    assert whole["in_use"] > least and whole["outside"] == 0
     e.Generate([1] * 40, 3)
     assert fake.fake_launches(b"prompt_gemm", -1) > 0
     e.SetLayerRange(0, 1)
     e.BuildFusedDispatch()
-    assert fake.fake_in_use() == made
+    assert e.ArenaStats()["in_use"] < whole["in_use"] - least
     e.SetLayerRange(0, cfg.n_layers)
     e.BuildFusedDispatch()
-    assert fake.fake_in_use() == whole
-    # no room: token by token
+    assert e.ArenaStats() == {**whole, "peak": e.ArenaStats()["peak"]}
     e.close()
     assert fake.fake_in_use() == 0
-    e = dense(fake, cfg, build=False)
-    fake.fake_memory(fake.fake_in_use() + least)
-    e.BuildFusedDispatch()
+    # no room: token by token
+    monkeypatch.setenv("MG_ARENA_MB", "1")
+    fake.fake_memory(2 * least)
+    e = dense(fake, cfg)
     fake.fake_forget()
     e.Generate([1] * 40, 3)
     assert fake.fake_launches(b"prompt_gemm", -1) == 0 and fake.fake_launches(b"", -1) > 0
     e.close()
+    assert fake.fake_in_use() == 0
