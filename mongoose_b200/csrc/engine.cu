@@ -212,6 +212,7 @@ struct mg_engine {
     int mk_buf = 0;
     int mk_acc_n = 0;                   // additions that complete an accumulator word
     int mk_qkv_cta0 = 0;                // first CTA that owns QKV rows
+    CUtensorMap mk_kmap, mk_vmap;       // the KV cache as boxes of a head's rows
     int mk_splits = 1;                  // most CTAs that share a query head in the persistent kernel
     DensePrompt prompt;
     PhaseGeom mk_geom[5] = {};
@@ -886,7 +887,7 @@ bool mega_feasible(mg_engine* e, std::string* why) {
         }
     }
     const int xs = ((xs_bytes + 15) / 16) * 4;
-    const int sc = (c.max_seq + 3) & ~3;
+    const int sc = (c.max_seq + 7) & ~7;
     int dev_max = 0;
     cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device);
     int nslot = MK_MAX_SLOTS;
@@ -914,6 +915,15 @@ int build_mega(mg_engine* e) {
             cudaGetLastError();
             ok = false;
             why = "one CTA does not fit an SM";
+        }
+    }
+    if (ok) {
+        int q_rows, v0;
+        const mg_config c = mega_cfg(e, &q_rows, &v0);
+        if (!make_rows_map(&e->mk_kmap, e->kc, c.kv_dim, c.max_seq, c.n_layers, c.head_dim, MK_KV_BOX) ||
+            !make_rows_map(&e->mk_vmap, e->vc, c.kv_dim, c.max_seq, c.n_layers, c.head_dim, MK_KV_BOX)) {
+            ok = false;
+            why = "no tensor map of the KV cache";
         }
     }
     if (e->sh.size > 1 && e->comm) {
@@ -1151,6 +1161,7 @@ int launch_mega_steps(mg_engine* e, int ls, int le, int mode, int head, int n_st
     a.final_norm = e->vecs[L * 12];
     a.embed_w = e->mats[L * 12 + 1].view();
     a.cos_tab = e->cos_tab; a.sin_tab = e->sin_tab; a.kc = e->kc; a.vc = e->vc;
+    a.k_map = e->mk_kmap; a.v_map = e->mk_vmap;
     Tagged* x = e->xbuf;
     a.xh = x; x += c.dim; a.xhm = x; x += c.dim; a.xq = x; x += q_dim; a.xkv = x; x += 2 * c.kv_dim;
     a.xattn = x; x += q_dim; a.xmid = x; x += c.ffn_dim; a.xtok = x; x += 2;
@@ -1188,10 +1199,10 @@ int launch_mega_steps(mg_engine* e, int ls, int le, int mode, int head, int n_st
     return MG_OK;
 }
 
-// Positions from MK_SPLIT_FROM on go to the instance whose CTAs share query heads.  The host's mirror of the position only
+// Positions from mk_split_from() on go to the instance whose CTAs share query heads.  The host's mirror of the position only
 // chooses: both instances are right at any position.
 int launch_mega(mg_engine* e, int ls, int le, int mode, int head, int n_steps) {
-    const int plain = e->mk_splits > 1 ? std::max(0, std::min(MK_SPLIT_FROM - e->cursor, n_steps)) : n_steps;
+    const int plain = e->mk_splits > 1 ? std::max(0, std::min(mk_split_from(e->cfg.head_dim) - e->cursor, n_steps)) : n_steps;
     if (plain > 0)
         if (int rc = launch_mega_steps(e, ls, le, mode, head, plain, false)) return rc;
     if (plain < n_steps)

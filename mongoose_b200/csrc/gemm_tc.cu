@@ -213,11 +213,12 @@ encode_fn_t encode_fn() {
     return fn;
 }
 
-bool encode(CUtensorMap* map, const void* base, const cuuint64_t dims[3], const cuuint64_t strides[2], const cuuint32_t box[3]) {
+bool encode(CUtensorMap* map, const void* base, const cuuint64_t dims[3], const cuuint64_t strides[2], const cuuint32_t box[3],
+            CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
     const cuuint32_t ones[3] = {1, 1, 1};
     encode_fn_t fn = encode_fn();
     return fn && fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, ones,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -241,6 +242,13 @@ bool make_head_map(CUtensorMap* map, const void* base, int k, int batch, int row
     const cuuint64_t strides[2] = {(cuuint64_t)batch_stride * 2, (cuuint64_t)row_stride * 2};
     const cuuint32_t box[3] = {64, 1, (cuuint32_t)box_rows};
     return encode(map, base, dims, strides, box);
+}
+
+bool make_rows_map(CUtensorMap* map, const void* base, int row_len, int rows, int batch, int box_cols, int box_rows) {
+    const cuuint64_t dims[3] = {(cuuint64_t)row_len, (cuuint64_t)rows, (cuuint64_t)batch};
+    const cuuint64_t strides[2] = {(cuuint64_t)row_len * 2, (cuuint64_t)rows * row_len * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+    return encode(map, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 int gemm_tc_bn(int m, int n, int batch) {

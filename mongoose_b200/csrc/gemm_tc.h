@@ -18,6 +18,9 @@ bool make_tile_map(CUtensorMap* map, const void* base, int k, int rows, int batc
 bool make_head_map(CUtensorMap* map, const void* base, int k, int batch, int rows, long long batch_stride, long long row_stride,
                    int box_rows);
 
+// 16-bit rows [batch][rows][row_len] in boxes of box_rows x box_cols, as they lie in memory (no swizzle).
+bool make_rows_map(CUtensorMap* map, const void* base, int row_len, int rows, int batch, int box_cols, int box_rows);
+
 struct GemmTC {
     CUtensorMap a, b;       // a: boxes of 128 rows; b: boxes of `bn` rows (bn / 2 for GEMM_SILU_BF16)
     CUtensorMap b2;         // GEMM_SILU_BF16: the second matrix, boxes of bn / 2 rows

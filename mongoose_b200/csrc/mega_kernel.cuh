@@ -17,6 +17,7 @@
 //    completion) into a ring of shared-memory slots, running up to a ring ahead
 //    of the consumers - weights never depend on activations, so HBM streaming
 //    is off the dependency chain.
+//    Attention's cached K and V rows travel through the same ring, as entries between the weights of QKV and of wo.
 //  * Tagged exchange.  A phase's output vector is written to global memory as
 //    8-byte {fp32 value, 32-bit epoch} words.  Consumers poll the words they
 //    need until the epoch is the one they expect: data and flag arrive in one
@@ -54,6 +55,7 @@
 #pragma once
 
 #include "decode_kernels.cuh"
+#include "umma.cuh"
 
 namespace mg {
 
@@ -61,6 +63,8 @@ constexpr int MK_NW = 15;                       // consumer warps
 constexpr int MK_CONSUMERS = MK_NW * 32;        // 480
 constexpr int MK_THREADS = MK_CONSUMERS + 32;   // + producer warp = 512 threads, 128 registers each
 constexpr int MK_SLOT = 32768;                  // ring slot bytes
+constexpr int MK_KV_BYTES = 30720;               // cached rows in a ring entry: one, two or four blocks of eight rows per warp (mk_attention)
+constexpr int MK_KV_BOX = 40;                   // rows of a copy of cached rows
 constexpr int MK_MAX_SLOTS = 14;
 constexpr int MK_PART_FLOATS = 2048;
 constexpr int MK_EPOCHS_PER_LAYER = 8;
@@ -135,6 +139,7 @@ struct MegaArgs {
     const float* sin_tab;
     __half* kc;             // [layers][max_seq][kv_dim]
     __half* vc;
+    CUtensorMap k_map, v_map;   // the same, as boxes of MK_KV_BOX rows of a head
     // exchange buffers
     Tagged *xh, *xhm, *xq, *xkv, *xattn, *xmid, *xtok;
     Tagged* xpart;          // [head][att_splits - 1][head_dim + 2] partial attention outputs (see mk_attention)
@@ -384,6 +389,7 @@ struct MkCtx {
     __device__ __forceinline__ volatile int* abort_flag() const {
         return reinterpret_cast<volatile int*>(empty() + MK_MAX_SLOTS);
     }
+    __device__ __forceinline__ int* appended() const { return const_cast<int*>(abort_flag()) + 1; }
     // per phase p: [p] first row-group of this CTA, [8+p] its number of row-groups;
     // then per phase and consumer warp (MK_WARP_TAB): row-group slot | K-split index << 8
     __device__ __forceinline__ int* phase_tab() const { return const_cast<int*>(reinterpret_cast<volatile int*>(abort_flag())) + 4; }
@@ -553,6 +559,41 @@ __device__ __forceinline__ float mk_block_sum(MkCtx& c, float v) {
 }
 
 // ---------------------------------------------------------------------
+// CTAs that share a query head at `pos`: CTA s * n_heads + h takes the s-th run of the positions of head h.  A split costs one
+// more exchange, the partial outputs, and on the CTAs that join ring entries that weights would have had.  B200, us per token with
+// one CTA a head / with 480 positions per CTA: six layers of 1.1B widths at 600 positions 164.3 / 164.0, 750 167.5 / 165.4, 1050
+// 176.3 / 170.7, 1300 182.0 / 172.6; six of 0.5B widths 600 127.4 / 129.8, 800 134.9 / 131.9, 1300 144.8 / 134.9; two of 7B widths
+// (head_dim 128) 900 219.6 / 226.7, 1300 225.5 / 228.2, on a slope of 1.5 per 100.  Runs of 120, 160, 240 and 360 positions
+// cost more at every length.
+constexpr int MK_SPLIT_POSITIONS = 480;
+constexpr int MK_MAX_SPLITS = 5;
+__host__ __device__ inline int mk_split_from(int head_dim) { return head_dim > 64 ? 1440 : 720; }
+__device__ __forceinline__ int mk_attn_splits(const MegaArgs& a, int pos) {
+    return pos < mk_split_from(a.head_dim) ? 1 : min((pos + MK_SPLIT_POSITIONS) / MK_SPLIT_POSITIONS, a.att_splits);
+}
+
+// The positions of one of the CTAs that share a head: `first` .. ; rows 0 .. now - 1 of the run are cached, row `now` is the new
+// one where the run ends with it.
+struct AttnRun { int first, now; bool ends; };
+__device__ __forceinline__ AttnRun attn_run(int pos, int split, int splits) {
+    const int run = splits > 1 ? (pos + splits) / splits : pos + 1, first = split * run;
+    const bool ends = first + run > pos;
+    return {first, ends ? pos - first : run, ends};
+}
+// Rows of the cache that this CTA has appended in this launch, counted for its producer, whose copies read them: the warp that
+// stored a row makes the stores known to the async proxy before it counts.
+__device__ __forceinline__ void mk_appended(MkCtx& c, int n) {
+    asm volatile("fence.proxy.async;" ::: "memory");
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(c.appended())), "r"(n) : "memory");
+}
+__device__ __forceinline__ int mk_appended_so_far(MkCtx& c) {
+    int n;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(n) : "r"(smem_u32(c.appended())) : "memory");
+    return n;
+}
+
+// ---------------------------------------------------------------------
 // Producer warp: stream this CTA's tape through the ring.
 // ---------------------------------------------------------------------
 // Whole rounds of `step` tiles that fit a ring entry of tpe tiles (at least one).  Used by the
@@ -619,12 +660,45 @@ __device__ __forceinline__ void mk_produce_down_fused(MkCtx& c, const MegaArgs& 
     }
 }
 
+// The cached rows of this CTA's run of positions in one layer, MK_KV_BYTES at a time (see mk_attention).  `appended`: how many
+// rows this CTA must have appended in this launch before they may be read.
+__device__ __forceinline__ void mk_produce_kv(MkCtx& c, const MegaArgs& a, int layer, int split, const AttnRun& rn, int appended) {
+    if (rn.now == 0) return;
+    if (appended > 0) {
+        const long long t0 = global_ns();
+        while (mk_appended_so_far(c) < appended) {
+            if (*c.abort_flag()) return;
+            if (global_ns() - t0 > a.wait_cycles) { mk_fail(c, MK_ERR_EMPTY, 400000); return; }
+        }
+    }
+    const int rb = 2 * a.head_dim, E = MK_KV_BYTES / rb;
+    const int kvh = ((int)blockIdx.x - split * a.n_heads) / (a.n_heads / a.n_kv_heads);
+    for (int kv = 0; kv < 2; kv++)
+        for (int r0 = 0; r0 < rn.now; r0 += E) {
+            mk_wait_bar(c, &c.empty()[c.slot], c.par ^ 1u, MK_ERR_EMPTY);
+            if (*c.abort_flag()) return;
+            const int boxes = (min(E, rn.now - r0) + MK_KV_BOX - 1) / MK_KV_BOX;      // a box's rows behind the cache read as zero
+            mbar_expect_tx(&c.full()[c.slot], (uint32_t)(boxes * MK_KV_BOX * rb));
+            for (int b = 0; b < boxes; b++)
+                tma_load_3d(c.ring() + (size_t)c.slot * a.slot_bytes + b * MK_KV_BOX * rb, kv ? &a.v_map : &a.k_map, kvh * a.head_dim,
+                            rn.first + r0 + b * MK_KV_BOX, layer, reinterpret_cast<uint64_t*>(&c.full()[c.slot]));
+            c.advance();
+        }
+}
+
+template <bool SHARED>
 __device__ __forceinline__ void mk_producer(MkCtx& c, const MegaArgs& a) {
     if ((threadIdx.x & 31) != 0) return;
     const unsigned long long* off = a.tape_off + (size_t)blockIdx.x * (a.n_layers * 4 + 2);
+    const int pos0 = a.st->pos;
+    const int my_split = (int)blockIdx.x / a.n_heads;
     for (int step = 0; step < a.n_steps; step++) {
+        const int pos = min(pos0 + step, a.max_seq - 1);
+        const int splits = SHARED ? mk_attn_splits(a, pos) : 1;
         for (int l = a.ls; l < a.le; l++)
             for (int p = 0; p < 4; p++) {
+                if (p == PH_WO && my_split < splits)
+                    mk_produce_kv(c, a, l, my_split, attn_run(pos, my_split, splits), step > 0 ? (step - 1) * (a.le - a.ls) + l - a.ls + 1 : 0);
                 if (p == PH_DOWN && a.ffn_fused) mk_produce_down_fused(c, a, a.tape + off[l * 4 + p], c.phase_tab()[8 + p]);
                 else mk_produce_phase(c, a, a.tape + off[l * 4 + p], p, c.phase_tab()[8 + p]);
             }
@@ -1503,37 +1577,25 @@ __device__ __forceinline__ void mk_clear_next(const MegaArgs& a, long long* acc_
 }
 
 // ---------------------------------------------------------------------
-// CTAs that share a query head at `pos`: CTA s * n_heads + h takes the s-th run of the positions of head h.  One CTA
-// keeps up with the other phases as long as its rows sit in registers when q arrives (240 positions); beyond
-// that it fetches them behind q, 256 bytes of K and V per position through one SM.  A split costs one more
-// exchange, the partial outputs.  B200, six layers of 1.1B widths, us per token with one CTA a head / with 240 positions
-// per CTA: at 300 positions 176.8 / 177.3, 360: 182.4 / 178.3, 600: 209.3 / 185.8, 960: 246.7 / 195.4; two layers of
-// 7B widths, at 300: 251.0 / 248.2, 900: 282.7 / 250.5.  Runs of 120, 160 and 300 positions were no better.
-constexpr int MK_SPLIT_FROM = 320;
-constexpr int MK_SPLIT_POSITIONS = 240;
-constexpr int MK_MAX_SPLITS = 5;
-__device__ __forceinline__ int mk_attn_splits(const MegaArgs& a, int pos) {
-    return pos < MK_SPLIT_FROM ? 1 : min((pos + MK_SPLIT_POSITIONS) / MK_SPLIT_POSITIONS, a.att_splits);
-}
-
-// ---------------------------------------------------------------------
-// Attention for one query head on this CTA (fp16 KV cache), three barriers.
-// Cached K/V rows do not depend on this token, so they are loaded into registers BEFORE q is
-// waited for.
-//   scores : four adjacent lanes share a position (a quarter of the head's dims each); unit
-//            u = tid / 4 takes positions u, u + 120, ...; the first NPRE of them come from registers;
-//   softmax: one maximum over the CTA; exp(s - max) is formed where it is used;
-//   P . V  : warp w takes positions w, w + 15, ... (the first NV from registers), a lane HD / 32
-//            adjacent dims; the warps' partial outputs and partial sums of exp meet in shared memory.
+// Attention for one query head on this CTA (fp16 KV cache), two barriers.
+// Cached K and V rows do not depend on this token, so the producer warp copies them into ring entries of their own, between
+// the weights of QKV and those of wo: K rows of the CTA's run of positions, MK_KV_BYTES at a time, then its V rows.
+// Eight consecutive rows are a BLOCK; block b belongs to warp b mod 15, for scores and for P . V, so that a warp's
+// scores never leave it.
+//   scores : four adjacent lanes share a position; lane qp takes the 16-byte chunks qp, qp + 4, ... of the row, rows of odd
+//            number in the other order of each two (all 32 banks are then busy), its part of q in registers;
+//   softmax: a maximum per warp; a lane forms exp(s - max) of one position and leaves it in sc[];
+//   P . V  : a lane HD / 32 adjacent dims, eight positions at a time; the warps' partial outputs and partial sums of exp
+//            meet in shared memory.
+// The new row is one more position, read from shared memory; a warp that does not merge appends it to the cache.
+// Rows fetched by the threads themselves, into registers before q arrives, cost the issue of every load (1.0 to 4.2 thousand
+// cycles a layer), a trip to DRAM that q did not hide (a token's weights push the cache out of L2) and a second for rows beyond
+// the registers; here q finds them in shared memory.  From q's arrival to the output, cycles before / now: 0.5B widths at 130
+// positions 7200 / 4500, 1.1B at 300 13400 / 8500, 7B at 190 21300 / 7700.  B200, tokens after a prompt: 0.5B Q8_0 32 + 200
+// 82.0 -> 76.0 ms, 1.1B widths 512 + 512 99.0 -> 89.3, 7B widths 128 + 128 30.1 -> 27.6.
 // Where several CTAs share the head, each does this for its run of positions and the first of them
 // collects the others' outputs, maxima and sums.  Positions below are relative to the run.
 // ---------------------------------------------------------------------
-template <int VPL>
-__device__ __forceinline__ uint2 ldcg_v(const __half* p) {
-    if (VPL == 1) return make_uint2(__ldcg(reinterpret_cast<const unsigned short*>(p)), 0u);
-    if (VPL == 2) return make_uint2(__ldcg(reinterpret_cast<const unsigned int*>(p)), 0u);
-    return __ldcg(reinterpret_cast<const uint2*>(p));
-}
 template <int VPL>
 __device__ __forceinline__ void fma_v(float (&acc)[VPL], float p, uint2 v) {
     if (VPL == 1) {
@@ -1547,17 +1609,31 @@ __device__ __forceinline__ void fma_v(float (&acc)[VPL], float p, uint2 v) {
         }
     }
 }
-// dot of 8 fp16 K values with 8 floats of q in shared memory
-__device__ __forceinline__ float dot8_kq(uint4 kk, uint32_t q_s) {
+// dot of 8 fp16 K values with 8 floats of q
+__device__ __forceinline__ float dot8_kq(uint4 kk, const float* q, float d) {
     const __half2* h = reinterpret_cast<const __half2*>(&kk);
-    const float4 qa = lds128f(q_s), qb = lds128f(q_s + 16);
     const float2 k0 = __half22float2(h[0]), k1 = __half22float2(h[1]);
     const float2 k2 = __half22float2(h[2]), k3 = __half22float2(h[3]);
-    float d0 = qa.x * k0.x, d1 = qa.y * k0.y;
-    d0 = fmaf(qa.z, k1.x, d0); d1 = fmaf(qa.w, k1.y, d1);
-    d0 = fmaf(qb.x, k2.x, d0); d1 = fmaf(qb.y, k2.y, d1);
-    d0 = fmaf(qb.z, k3.x, d0); d1 = fmaf(qb.w, k3.y, d1);
-    return d0 + d1;
+    float d1 = q[1] * k0.y;
+    d = fmaf(q[0], k0.x, d);
+    d = fmaf(q[2], k1.x, d); d1 = fmaf(q[3], k1.y, d1);
+    d = fmaf(q[4], k2.x, d); d1 = fmaf(q[5], k2.y, d1);
+    d = fmaf(q[6], k3.x, d); d1 = fmaf(q[7], k3.y, d1);
+    return d + d1;
+}
+template <int VPL>
+__device__ __forceinline__ uint2 lds_v(uint32_t addr) {
+    uint2 v = make_uint2(0u, 0u);
+    if (VPL == 1) {
+        unsigned short h;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(addr));
+        v.x = h;
+    } else if (VPL == 2) {
+        v.x = lds32(addr);
+    } else {
+        v = lds64(addr);
+    }
+    return v;
 }
 
 // Element tid of a head's output and the sum of its weights over all the head's splits, from those of the first split
@@ -1598,78 +1674,37 @@ static __device__ __noinline__ float2 mk_merge_splits(volatile int* abort_flag, 
 }
 
 // The new K and V rows of this token on a CTA that will share the head later in this launch: a CTA reads
-// back only cache rows that it has written itself, or that an earlier launch has written.
+// back only cache rows that it has written itself, or that an earlier launch has written.  One warp calls.
 static __device__ __noinline__ void mk_append_row(volatile int* abort_flag, MegaStatus* status, long long limit, const Tagged* k_new, int kv_dim,
                                                   int hd, __half* k_row, __half* v_row, unsigned int tag) {
-    const int i = 2 * (int)threadIdx.x;
-    if (i >= 2 * hd) return;
-    const bool is_k = i < hd;
-    const int at = is_k ? i : i - hd;
-    const Tagged* p = k_new + (is_k ? 0 : kv_dim) + at;
-    uint4 r = ld_poll16(p);
-    if (r.y != tag || r.w != tag) r = mk_poll16_slow(abort_flag, status, limit, p, tag, 0);
-    *reinterpret_cast<__half2*>((is_k ? k_row : v_row) + at) = __floats2half2_rn(__uint_as_float(r.x), __uint_as_float(r.z));
+    for (int i = 2 * (int)(threadIdx.x & 31); i < 2 * hd; i += 64) {
+        const bool is_k = i < hd;
+        const int at = is_k ? i : i - hd;
+        const Tagged* p = k_new + (is_k ? 0 : kv_dim) + at;
+        uint4 r = ld_poll16(p);
+        if (r.y != tag || r.w != tag) r = mk_poll16_slow(abort_flag, status, limit, p, tag, 0);
+        *reinterpret_cast<__half2*>((is_k ? k_row : v_row) + at) = __floats2half2_rn(__uint_as_float(r.x), __uint_as_float(r.z));
+    }
 }
 
 template <int HD, bool SHARED>
-__device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int layer, int pos, int split, int splits,
+__device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int layer, int pos, int split, int splits, int appended,
                                              unsigned int tag_in, unsigned int tag_out) {
-    constexpr int DPL = HD / 4;                // dims per lane in the score phase
-    constexpr int KV4 = DPL / 8;               // 16-byte pieces of K per lane and position
-    constexpr int NPRE = HD == 128 ? 2 : 4;    // score passes whose K rows are held in registers
-    constexpr int PPP = 8;                     // positions per warp and pass (four lanes each)
-    constexpr int VPL = HD / 32;               // dims per lane in P . V
-    constexpr int NV = 16;                     // positions per warp whose V rows are held in registers
+    constexpr int RB = 2 * HD, E = MK_KV_BYTES / RB;           // bytes of a row, rows of a ring entry
+    constexpr int BPW = E / (8 * MK_NW);                       // blocks of a warp in an entry
+    constexpr int NC = HD / 32, VPL = HD / 32;                 // chunks per lane (scores), dims per lane (P . V)
+    static_assert(E % (8 * MK_NW) == 0, "every warp has as many blocks of an entry");
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const uint32_t sm0 = smem_u32(mk_smem);
     const int head = (int)blockIdx.x - (SHARED ? split * a.n_heads : 0);
     const int kvh = head / (a.n_heads / a.n_kv_heads);
-    // this CTA's run of positions: rows 0 .. now - 1 of kc / vc are cached, row `now` is the new one where the run ends with it
-    const int run = SHARED && splits > 1 ? (pos + splits) / splits : pos + 1, first = SHARED ? split * run : 0;
-    const bool ends = !SHARED || first + run > pos;
-    const int now = ends ? pos - first : run, end = ends ? now : now - 1;
-    const size_t lbase = (size_t)layer * a.max_seq * a.kv_dim + kvh * HD;
-    const __half* kc = a.kc + lbase + (size_t)first * a.kv_dim;
-    const __half* vc = a.vc + lbase + (size_t)first * a.kv_dim;
-    const uint32_t xs_s = smem_u32(mk_smem) + c.xs_off;        // q | new k | new v, HD floats each
-    const int uq = lane >> 2, qp = lane & 3;
-    // Warp w owns positions w, w + 15, w + 30, ...: it computes their scores AND their share of
-    // P . V, so the scores never leave the warp; pass i covers its positions number 8 i .. 8 i + 7.
-    const int t_first = w + MK_NW * uq;
+    const AttnRun rn = attn_run(pos, SHARED ? split : 0, SHARED ? splits : 1);
+    const int now = rn.now;
+    const uint32_t xs_s = sm0 + c.xs_off, new_s = xs_s + 4u * HD;      // q, HD floats; new k | new v, HD halves each
+    const uint32_t sc_s = smem_u32(c.sc());
+    const int u = lane >> 2, qp = lane & 3;
 
-    // ---- cached rows (positions < now) into registers ----
-    // Everything below is guarded per warp (a warp's positions of a pass / of a group of four are
-    // known from w and the run alone), so a short context skips the passes it does not have instead of
-    // walking through their predicated-off loads.
-    const int npass = (end - w + MK_NW * PPP) / (MK_NW * PPP);      // score passes in which this warp has a position <= end (w <= end)
-    const int nv = w < now ? (now - w + MK_NW - 1) / MK_NW : 0;     // cached positions of this warp for P . V
-    uint4 kreg[NPRE][KV4];
-#pragma unroll
-    for (int i = 0; i < NPRE; i++) {
-        const int t = t_first + i * (MK_NW * PPP);
-#pragma unroll
-        for (int j = 0; j < KV4; j++) kreg[i][j] = make_uint4(0u, 0u, 0u, 0u);
-        if (w <= end && i < npass && t < now) {
-            const uint4* kp = reinterpret_cast<const uint4*>(kc + (size_t)t * a.kv_dim + qp * DPL);
-#pragma unroll
-            for (int j = 0; j < KV4; j++) kreg[i][j] = __ldcg(kp + j);
-        }
-    }
-    uint2 vreg[NV];
-#pragma unroll
-    for (int j0 = 0; j0 < NV; j0 += 4) {
-#pragma unroll
-        for (int j = j0; j < j0 + 4; j++) vreg[j] = make_uint2(0u, 0u);
-        if (j0 < nv) {
-#pragma unroll
-            for (int j = j0; j < j0 + 4; j++) {
-                const int t = w + j * MK_NW;
-                if (t < now) vreg[j] = ldcg_v<VPL>(vc + (size_t)t * a.kv_dim + lane * VPL);
-            }
-        }
-    }
-    MK_ESTAMP(40);
-
-    // ---- gather q, new k, new v (HD values each); append the new row to the cache ----
+    // ---- gather q, new k, new v (HD values each) ----
     for (int i = 2 * tid; i < 3 * HD; i += 2 * MK_CONSUMERS) {
         const int which = i / HD, d = i - which * HD;
         const Tagged* src = which == 0 ? a.xq + head * HD + d
@@ -1677,123 +1712,104 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
                                        : a.xkv + a.kv_dim + kvh * HD + d;
         float v0, v1;
         mk_poll2(c, src, tag_in, v0, v1);
-        *reinterpret_cast<float2*>(c.xs() + i) = make_float2(v0, v1);
-        // every CTA of the KV group appends the (identical) new row; each CTA later reads back
-        // only addresses it has written itself
-        if (which == 1) *reinterpret_cast<__half2*>(a.kc + lbase + (size_t)pos * a.kv_dim + d) = __floats2half2_rn(v0, v1);
-        if (which == 2) *reinterpret_cast<__half2*>(a.vc + lbase + (size_t)pos * a.kv_dim + d) = __floats2half2_rn(v0, v1);
+        if (which == 0) *reinterpret_cast<float2*>(c.xs() + d) = make_float2(v0, v1);
+        else *reinterpret_cast<__half2*>(c.xs() + HD + ((which - 1) * HD + d) / 2) = __floats2half2_rn(v0, v1);    // rounded already
     }
     consumer_sync();
     MK_ESTAMP(41);
 
     // ---- scores of this warp's positions ----
     const float scale = rsqrtf((float)HD);
-    const uint32_t q_s = xs_s + (uint32_t)(qp * DPL) * 4u;
-    float mx = -INFINITY;
+    const int swap = NC > 1 ? u & 1 : 0;
+    const uint32_t k_off = (uint32_t)(qp * 16);
+    float q[NC * 8];
 #pragma unroll
-    for (int i = 0; i < NPRE; i++) {
-        if (i == 0 || (w <= end && i < npass)) {                   // uniform over the warp
-            const int t = t_first + i * (MK_NW * PPP);
-            if (t == now) {
-                // the new position's K row sits in shared memory (fp16-rounded values: the conversion is exact)
-                const float* kn = c.xs() + HD + qp * DPL;
-#pragma unroll
-                for (int j = 0; j < KV4; j++) {
-                    __half2 h[4];
-#pragma unroll
-                    for (int e = 0; e < 4; e++) h[e] = __floats2half2_rn(kn[8 * j + 2 * e], kn[8 * j + 2 * e + 1]);
-                    kreg[i][j] = *reinterpret_cast<const uint4*>(h);
-                }
-            }
-            float dot = 0.f;
-#pragma unroll
-            for (int j = 0; j < KV4; j++) dot += dot8_kq(kreg[i][j], q_s + j * 32);
-            dot += __shfl_xor_sync(MG_FULL_MASK, dot, 1);
-            dot += __shfl_xor_sync(MG_FULL_MASK, dot, 2);
-            dot *= scale;
-            if (t <= end) { if (qp == 0) c.sc()[t] = dot; mx = fmaxf(mx, dot); }
-        }
+    for (int j = 0; j < NC; j++) {
+        const uint32_t qa = xs_s + (uint32_t)((qp + 4 * (j ^ swap)) * 32);
+        *reinterpret_cast<float4*>(q + 8 * j) = lds128f(qa);
+        *reinterpret_cast<float4*>(q + 8 * j + 4) = lds128f(qa + 16);
     }
-    for (int i = NPRE; w <= end && i < npass; i++) {              // contexts beyond the registers: rows from L2
-        const int t = t_first + i * (MK_NW * PPP);
-        uint4 kk[KV4];
+    auto score = [&](uint32_t row) {
+        uint4 kk[NC];
 #pragma unroll
-        for (int j = 0; j < KV4; j++) kk[j] = make_uint4(0u, 0u, 0u, 0u);
-        if (t < now) {
-            const uint4* kp = reinterpret_cast<const uint4*>(kc + (size_t)t * a.kv_dim + qp * DPL);
+        for (int j = 0; j < NC; j++) kk[j] = lds128(row + k_off + (uint32_t)((j ^ swap) * 64));
+        float d = 0.f;
 #pragma unroll
-            for (int j = 0; j < KV4; j++) kk[j] = __ldcg(kp + j);
-        } else if (t == now) {
-            const float* kn = c.xs() + HD + qp * DPL;
+        for (int j = 0; j < NC; j++) d = dot8_kq(kk[j], q + 8 * j, d);
+        d += __shfl_xor_sync(MG_FULL_MASK, d, 1);
+        d += __shfl_xor_sync(MG_FULL_MASK, d, 2);
+        return d * scale;
+    };
+    const int nblk = (now + 7) >> 3;
+    const bool has_new = rn.ends && w == nblk % MK_NW;         // the new position belongs to the next warp in turn
+    float mx = -INFINITY, s_new = 0.f;
+    for (int r0 = 0; r0 < now; r0 += E) {
+        mk_wait_bar(c, &c.full()[c.slot], c.par, MK_ERR_FULL);
+        const uint32_t rows = sm0 + (uint32_t)c.slot * (uint32_t)a.slot_bytes;
 #pragma unroll
-            for (int j = 0; j < KV4; j++) {
-                __half2 h[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) h[e] = __floats2half2_rn(kn[8 * j + 2 * e], kn[8 * j + 2 * e + 1]);
-                kk[j] = *reinterpret_cast<const uint4*>(h);
+        for (int i = 0; i < BPW; i++) {
+            const int b = 8 * (w + MK_NW * i), t = r0 + b + u;
+            if (r0 + b < now) {                                // uniform over the warp; rows from `now` on are left out below
+                const float s = score(rows + (uint32_t)((b + u) * RB));
+                if (t < now) { if (qp == 0) c.sc()[t] = s; mx = fmaxf(mx, s); }
             }
         }
-        float dot = 0.f;
-#pragma unroll
-        for (int j = 0; j < KV4; j++) dot += dot8_kq(kk[j], q_s + j * 32);
-        dot += __shfl_xor_sync(MG_FULL_MASK, dot, 1);
-        dot += __shfl_xor_sync(MG_FULL_MASK, dot, 2);
-        dot *= scale;
-        if (t <= end) { if (qp == 0) c.sc()[t] = dot; mx = fmaxf(mx, dot); }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&c.empty()[c.slot]);
+        c.advance();
     }
+    if (has_new) { s_new = score(new_s); mx = fmaxf(mx, s_new); }
     mx = warp_max(mx);                       // -inf: the warp has no position
     __syncwarp();                            // the scores in sc[] were written by lanes of this warp
     MK_ESTAMP(42);
-    MK_ESTAMP(43);
 
-    // ---- this warp's share of P . V, relative to its own maximum ----
+    // ---- weights exp(s - mx), and this warp's share of P . V ----
+    float lsum = 0.f;
+    for (int k = lane, n = w < nblk ? (nblk - w + MK_NW - 1) / MK_NW * 8 : 0; k < n; k += 32) {
+        const int t = ((k >> 3) * MK_NW + w) * 8 + (k & 7);
+        const float p = t < now ? __expf(c.sc()[t] - mx) : 0.f;
+        c.sc()[t] = p;
+        lsum += p;
+    }
+    lsum = warp_sum(lsum);
+    __syncwarp();
     float acc[VPL];
 #pragma unroll
     for (int e = 0; e < VPL; e++) acc[e] = 0.f;
-    float lsum = 0.f;
-    const int last = max(now - 1, 0);
+    for (int r0 = 0; r0 < now; r0 += E) {
+        mk_wait_bar(c, &c.full()[c.slot], c.par, MK_ERR_FULL);
+        const uint32_t rows = sm0 + (uint32_t)c.slot * (uint32_t)a.slot_bytes + (uint32_t)(lane * VPL * 2);
 #pragma unroll
-    for (int j0 = 0; j0 < NV; j0 += 4) {
-        if (j0 < nv) {
-            // a group of four, straight-line: positions beyond the context contribute p = 0 (their V registers hold zeros)
+        for (int i = 0; i < BPW; i++) {
+            const int b = 8 * (w + MK_NW * i);
+            if (r0 + b < now) {
+                const float4 p0 = lds128f(sc_s + 4u * (uint32_t)(r0 + b)), p1 = lds128f(sc_s + 4u * (uint32_t)(r0 + b) + 16);
+                const float p[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+                uint2 v[8];
 #pragma unroll
-            for (int j = j0; j < j0 + 4; j++) {
-                const int t = w + j * MK_NW;
-                float p = __expf(c.sc()[min(t, last)] - mx);
-                p = t < now ? p : 0.f;
-                lsum += p;
-                fma_v<VPL>(acc, p, vreg[j]);
+                for (int j = 0; j < 8; j++) {
+                    v[j] = make_uint2(0u, 0u);                 // a row from `now` on may hold anything, an infinity too
+                    if (r0 + b + j < now) v[j] = lds_v<VPL>(rows + (uint32_t)((b + j) * RB));
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++) fma_v<VPL>(acc, p[j], v[j]);
             }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&c.empty()[c.slot]);
+        c.advance();
     }
-    for (int t0 = w + NV * MK_NW; t0 < now; t0 += 4 * MK_NW) {   // remainder, four loads in flight
-        uint2 vv[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int t = t0 + j * MK_NW;
-            vv[j] = make_uint2(0u, 0u);
-            if (t < now) vv[j] = ldcg_v<VPL>(vc + (size_t)t * a.kv_dim + lane * VPL);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int t = t0 + j * MK_NW;
-            float p = __expf(c.sc()[min(t, last)] - mx);
-            p = t < now ? p : 0.f;
-            lsum += p;
-            fma_v<VPL>(acc, p, vv[j]);
-        }
-    }
-    if (ends && w == now % MK_NW) {                                       // the new position belongs to one warp
-        const float p = __expf(c.sc()[now] - mx);
+    if (has_new) {
+        const float p = __expf(s_new - mx);
         lsum += p;
-        const float* vn = c.xs() + 2 * HD + lane * VPL;
-#pragma unroll
-        for (int e = 0; e < VPL; e++) acc[e] = fmaf(p, vn[e], acc[e]);
+        fma_v<VPL>(acc, p, lds_v<VPL>(new_s + (uint32_t)(RB + lane * VPL * 2)));
     }
     MK_ESTAMP(44);
 #pragma unroll
     for (int e = 0; e < VPL; e++) c.part()[w * HD + lane * VPL + e] = acc[e];
     if (lane == 0) { c.red()[32 + w] = mx; c.red()[48 + w] = lsum; }
+    // (read here: behind the barrier xs belongs to the next phase)
+    const uint4 fresh = w == MK_NW - 1 && lane < HD / 4 ? lds128(new_s + (uint32_t)(lane * 16)) : make_uint4(0u, 0u, 0u, 0u);
     consumer_sync();
     MK_ESTAMP(45);
     // ---- merge the warps' partial results: weights exp(m_w - M) ----
@@ -1816,19 +1832,30 @@ __device__ __forceinline__ void mk_attention(const MegaArgs& a, MkCtx& c, int la
             s = fmaf(f, c.part()[g * HD + tid], s);
             lt = fmaf(f, l[g], lt);
         }
+        bool collect = true;
         if (SHARED && splits > 1) {
             Tagged* part = a.xpart + (size_t)head * (a.att_splits - 1) * (HD + 2);
             if (split > 0) {
                 part += (split - 1) * (HD + 2);
                 st_tagged(part + tid, s, tag_out);
                 if (tid == 0) { st_tagged(part + HD, M, tag_out); st_tagged(part + HD + 1, lt, tag_out); }
-                return;
+                collect = false;
+            } else {
+                const float2 all = mk_merge_splits(c.abort_flag(), c.status(), a.wait_cycles, part, splits - 1, HD + 2, tid, tag_out, s, lt, M);
+                s = all.x;
+                lt = all.y;
             }
-            const float2 all = mk_merge_splits(c.abort_flag(), c.status(), a.wait_cycles, part, splits - 1, HD + 2, tid, tag_out, s, lt, M);
-            s = all.x;
-            lt = all.y;
         }
-        st_tagged(a.xattn + head * HD + tid, __fdividef(s, lt), tag_out);
+        if (collect) st_tagged(a.xattn + head * HD + tid, __fdividef(s, lt), tag_out);
+    } else if (w == MK_NW - 1) {
+        // every CTA of the KV group appends the (identical) new row; each CTA later reads back
+        // only addresses it has written itself
+        if (lane < HD / 4) {
+            const bool is_k = lane < HD / 8;
+            const int at = (is_k ? lane : lane - HD / 8) * 8;
+            *reinterpret_cast<uint4*>((is_k ? a.kc : a.vc) + ((size_t)layer * a.max_seq + pos) * a.kv_dim + kvh * HD + at) = fresh;
+        }
+        mk_appended(c, appended);
     }
 }
 
@@ -1880,14 +1907,15 @@ __device__ __forceinline__ void mk_consumer(MkCtx& c, const MegaArgs& a) {
             mk_run_phase<PH_QKV, FMT, TP>(a, c, s0, l, base + 1, l * MK_EV, best);                                 \
             if (my_split < splits) {                                                                               \
                 MK_SET_PROBE(l * MK_EV);                                                                           \
-                if (a.head_dim == 64) mk_attention<64, SHARED>(a, c, l, pos, my_split, splits, base + 1, base + 2); \
-                else if (a.head_dim == 128) mk_attention<128, SHARED>(a, c, l, pos, my_split, splits, base + 1, base + 2); \
-                else mk_attention<32, SHARED>(a, c, l, pos, my_split, splits, base + 1, base + 2);                 \
+                if (a.head_dim == 64) mk_attention<64, SHARED>(a, c, l, pos, my_split, splits, qn + 1, base + 1, base + 2); \
+                else if (a.head_dim == 128) mk_attention<128, SHARED>(a, c, l, pos, my_split, splits, qn + 1, base + 1, base + 2); \
+                else mk_attention<32, SHARED>(a, c, l, pos, my_split, splits, qn + 1, base + 1, base + 2);         \
                 mk_trace(a, step, l * MK_EV + 9);                                                                  \
-            } else if (SHARED && my_split < late_splits) {                                                         \
+            } else if (SHARED && my_split < late_splits && tid < 32) {                                             \
                 const int at = ((int)blockIdx.x - my_split * a.n_heads) / (a.n_heads / a.n_kv_heads) * a.head_dim;  \
                 const size_t row = ((size_t)l * a.max_seq + pos) * a.kv_dim + at;                                  \
                 mk_append_row(c.abort_flag(), c.status(), a.wait_cycles, a.xkv + at, a.kv_dim, a.head_dim, a.kc + row, a.vc + row, base + 1); \
+                mk_appended(c, qn + 1);                                                                            \
             }                                                                                                      \
             if (fused) mk_clear_next(a, a.acc + (size_t)((a.acc_buf0 + qn + 1) % 3) * a.dim);                      \
             const StageSrc s1{SRC_POLL, a.xattn, base + 2, a.q_dim, nullptr, token};                               \
@@ -2021,6 +2049,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) mega_decode_kernel(const __grid
             mbar_init(&c.empty()[i], MK_NW);
         }
         *c.abort_flag() = 0;
+        *c.appended() = 0;
         c.red()[15] = 0.f; c.red()[31] = 0.f;      // 16th entry of the two halves of the RMS partial sums
         for (int p = 0; p <= PH_HEAD; p++) {
             const PhaseShape sh = phase_shape_of(p, a.dim, a.q_dim, a.kv_dim, a.ffn_dim, a.vocab, a.layer_fmt, a.head_fmt);
@@ -2049,7 +2078,7 @@ __global__ void __launch_bounds__(MK_THREADS, 1) mega_decode_kernel(const __grid
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
-    if (threadIdx.x >= MK_CONSUMERS) mk_producer(c, a);
+    if (threadIdx.x >= MK_CONSUMERS) mk_producer<SHARED>(c, a);
     else mk_consumer<TP, SHARED>(c, a);
 }
 
