@@ -18,6 +18,7 @@
 
 #include "../../include/mongoose_kernels.h"
 #include "mg_common.cuh"
+#include "umma.cuh"
 
 using namespace mg;
 
@@ -200,6 +201,272 @@ __global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __re
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// ---------------- the same on the integer tensor path: matrices that keep every SM busy ----------------
+// Above, a lane converts every weight to fp32: about eight instructions per weight of a lane, and the issue slots are what
+// bounds a large product.  Here a warp multiplies 16 rows x one block of 32 columns by ONE mma.sync (m16n8k32, int8): A = the
+// quants as they lie in the block (4-bit ones as 16 (q - 8)), B = the activations as fixed point, four signed byte digits
+// in four of the eight columns.  A block's activations share a power of two, which puts the largest at 2^29 .. 2^30: an
+// element of 2^-6 of the largest or more is exact, a smaller one off by at most 2^-31 of the largest; the sums of a block
+// are exact integers, and fp32 only adds (block scale x power of two x sum) over the blocks, digit by digit.
+//   A CTA owns a contiguous run of rows, taken up to 32 at a time (one or two MMA tiles, which share the activations), and a row's
+// blocks in SEGMENTS of up to 128 (Q8_0: 64), 2 KB of every row.  A producer warp copies a segment (cp.async.bulk, a lane a row: the
+// 16-byte pieces that cover it) into a ring of slots; the 16 other warps share its blocks, and their sums over all
+// segments meet in shared memory.  Rows lie an odd multiple of 16 bytes apart in a slot, so that the eight rows of an access
+// fall on different banks.  (Copies by the warps themselves, ten pieces of 16 bytes per row and turn with cp.async, took half the time.)
+//   What bounds it is the number of loads from shared memory, one per two cycles and SM.  Blocks are taken in PAIRS, 9 (17) aligned
+// words of a row: the scale of the first and two of its quants share word 0, its last two and the scale of the second word 4 (8).
+// Lane t = 0 of a row completes its half word from there, so that no lane re-aligns what it loads: 2 (3) loads per
+// block and row where re-aligned words took 3 (5).  The activations of even blocks are staged in that order of elements.
+// B200, passes among others, the kernel above -> this one: Q4_0 3584 x 18944 26.9 -> 13.0 us (2.9 TB/s), 3584 x 3584 10.8 -> 4.4, 18944 x 3584
+// 24.2 -> 10.7; Q8_0 3584 x 18944 27.5 -> 17.0, 20000 x 19200 114 -> 75 (5.4 TB/s).  Error against 64 bits at 3584 x 18944 Q4_0 1.4e-7 -> 0.7e-7.
+//   A row whose sum is not finite is computed again in plain fp32 (activations or scales that are not, or sums beyond the range).
+constexpr int kMmaWarps = 16, kMmaRows = 32, kMmaSlots = 4;
+constexpr int kMmaThreads = (kMmaWarps + 1) * 32;
+__host__ __device__ constexpr int mma_seg(int fmt) { return fmt == FMT_Q8_0 ? 32 : 64; }       // pairs
+__host__ __device__ constexpr int mma_stride(int fmt) { return 2 * mma_seg(fmt) * block_bytes(fmt) + 16; }
+static_assert(mma_stride(FMT_Q8_0) / 16 % 2 == 1 && mma_stride(FMT_Q4_0) / 16 % 2 == 1, "rows on different banks");
+__host__ __device__ constexpr int mma_digit_bytes(int nb) { return (nb * 32 + 127) / 128 * 128 + 32; }     // from digit to digit: the four on different banks
+__host__ __device__ constexpr size_t mma_input_bytes(int nb) { return (size_t)4 * mma_digit_bytes(nb) + ((size_t)nb * 4 + 15) / 16 * 16; }
+constexpr size_t kMmaSums = (size_t)2 * kMmaWarps * kMmaRows * 4, kMmaBars = 2 * kMmaSlots * 8 + 16;
+
+// Re-computes one row; every lane returns it.
+template <int FMT>
+__device__ __noinline__ float raw_row_plain(const float* __restrict__ act, const uint8_t* __restrict__ row, int nb) {
+    constexpr int BB = block_bytes(FMT);
+    float acc = 0.f;
+    for (int b = threadIdx.x & 31; b < nb; b += 32) {
+        const uint8_t* p = row + (size_t)b * BB;
+        const float* x = act + (size_t)b * 32;
+        const float d = half_bits_to_float(*reinterpret_cast<const unsigned short*>(p));
+        float sum = 0.f;
+        for (int i = 0; i < 32; i++) {
+            const int q = FMT == FMT_Q8_0 ? (int)(int8_t)p[2 + i] : (i < 16 ? p[2 + i] & 15 : p[2 + i - 16] >> 4) - 8;
+            sum = fmaf((float)q, x[i], sum);
+        }
+        acc = fmaf(d, sum, acc);
+    }
+    return warp_sum(acc);
+}
+
+// `n` pairs of blocks for NT tiles of 16 rows.  at: this lane's rows g + 8 r, offset of the first pair in shared memory; digits,
+// scales: of its first block.  Column 2 p of a product is digit p, which lane t = p receives.  acc: even and odd blocks, so that fewer
+// roundings follow one another.
+template <int FMT, int NT>
+__device__ __forceinline__ void mma_pairs(const uint8_t* smem, const uint32_t (&at)[2 * NT], int n, uint32_t digits, uint32_t scales, bool bvalid, int t,
+                                          float (&acc)[2][4]) {
+    constexpr int PB = 2 * block_bytes(FMT), QW = block_bytes(FMT) / 4 * 4;        // bytes of a pair; where the word that both blocks share lies
+    const unsigned join = t == 0 ? 0x3254u : 0x3210u;
+    auto word = [&](uint32_t p) { return *reinterpret_cast<const uint32_t*>(smem + p); };
+#pragma unroll 2
+    for (int k = 0; k < n; k++) {
+        uint2 B[2];
+        float s[2], d[2][2 * NT];
+        uint32_t a[2][NT][4];
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            B[j] = bvalid ? *reinterpret_cast<const uint2*>(smem + digits + (2 * k + j) * 32) : make_uint2(0u, 0u);
+            s[j] = *reinterpret_cast<const float*>(smem + scales + (2 * k + j) * 4);
+        }
+#pragma unroll
+        for (int r = 0; r < 2 * NT; r++) {
+            const uint32_t p = at[r] + k * PB;
+            const uint32_t both = word(p + QW);
+            uint32_t(&e)[4] = a[0][r >> 1], (&o)[4] = a[1][r >> 1];
+            d[0][r] = half_bits_to_float(*reinterpret_cast<const unsigned short*>(smem + p));
+            d[1][r] = half_bits_to_float((unsigned short)(both >> 16));
+            const uint32_t v0 = __byte_perm(word(p + 4 * t), both, join), v1 = word(p + QW + 4 + 4 * t);
+            if (FMT == FMT_Q8_0) {
+                e[r & 1] = v0; e[2 + (r & 1)] = word(p + 16 + 4 * t);
+                o[r & 1] = v1; o[2 + (r & 1)] = word(p + QW + 20 + 4 * t);
+            } else {
+                e[r & 1] = ((v0 << 4) & 0xf0f0f0f0u) ^ 0x80808080u; e[2 + (r & 1)] = (v0 & 0xf0f0f0f0u) ^ 0x80808080u;
+                o[r & 1] = ((v1 << 4) & 0xf0f0f0f0u) ^ 0x80808080u; o[2 + (r & 1)] = (v1 & 0xf0f0f0f0u) ^ 0x80808080u;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int i = 0; i < NT; i++) {
+                const uint32_t(&o)[4] = a[j][i];
+                int c[4];
+                asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                    : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+                    : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(B[j].x), "r"(B[j].y), "r"(0));
+                acc[j][2 * i] = fmaf(d[j][2 * i] * s[j], __int2float_rn(c[0]), acc[j][2 * i]);         // |sum| <= 32 * 128 * 128: exact
+                acc[j][2 * i + 1] = fmaf(d[j][2 * i + 1] * s[j], __int2float_rn(c[2]), acc[j][2 * i + 1]);
+            }
+    }
+}
+
+// An even number of blocks, and a matrix on a 16-byte boundary.  slot_rows: rows taken at a time; slots: of the ring.
+template <int FMT>
+__global__ void __launch_bounds__(kMmaThreads, 1) raw_block_mma_kernel(const float* __restrict__ act, const uint8_t* __restrict__ w, float* out, int N, int K,
+                                                                       int slot_rows, int slots) {
+    constexpr int BB = block_bytes(FMT), SEG = mma_seg(FMT), STRIDE = mma_stride(FMT);
+    extern __shared__ __align__(16) uint8_t mma_smem[];     // digits [digit][block][32], scales; sums [2][warp][row]; barriers; slots
+    const int nb = K / 32, np = nb / 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int digit_bytes = mma_digit_bytes(nb);
+    const size_t rb = (size_t)nb * BB;
+    float* part = reinterpret_cast<float*>(mma_smem + mma_input_bytes(nb));
+    uint64_t* full = reinterpret_cast<uint64_t*>(mma_smem + mma_input_bytes(nb) + kMmaSums);
+    uint64_t* empty = full + kMmaSlots;
+    int* status = reinterpret_cast<int*>(empty + kMmaSlots);
+    const uint32_t ring = (uint32_t)(mma_input_bytes(nb) + kMmaSums + kMmaBars), slot_bytes = (uint32_t)slot_rows * STRIDE;
+    const int row_lo = (int)((long long)N * blockIdx.x / gridDim.x), row_hi = (int)((long long)N * (blockIdx.x + 1) / gridDim.x);
+    const int segs = (np + SEG - 1) / SEG;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < slots; i++) { bar_init(full + i, 1); bar_init(empty + i, kMmaWarps); }
+        *status = 0;
+        bar_init_fence();
+    }
+    __syncthreads();
+    pdl_launch_dependents();
+    pdl_wait();
+
+    if (warp == kMmaWarps) {
+        int s = 0, par = 1, n = 0;
+        bool ok = true;
+        for (int row0 = row_lo; ok && row0 < row_hi; row0 += slot_rows)
+            for (int k = 0; k < segs; k++, n++) {
+                if (n >= slots && !(ok = __all_sync(MG_FULL_MASK, bar_wait(empty + s, par, status)))) break;
+                const int p0 = np * k / segs, p1 = np * (k + 1) / segs;
+                const uint8_t* src = w;
+                uint8_t* to = mma_smem + ring + s * slot_bytes + lane * STRIDE;
+                unsigned bytes = 0;
+                if (lane < min(slot_rows, row_hi - row0)) {
+                    src += (size_t)(row0 + lane) * rb + (size_t)p0 * 2 * BB;
+                    const unsigned lead = (unsigned)(reinterpret_cast<uintptr_t>(src) & 15u), need = lead + (unsigned)(p1 - p0) * 2 * BB;
+                    src -= lead;
+                    const size_t left = (size_t)(w + (size_t)N * rb - src);         // nothing behind the matrix is read
+                    bytes = (unsigned)min((size_t)((need + 15u) & ~15u), left & ~(size_t)15);
+                    for (unsigned i = bytes; i < need; i += 2) *reinterpret_cast<unsigned short*>(to + i) = *reinterpret_cast<const unsigned short*>(src + i);
+                }
+                const unsigned all = __reduce_add_sync(MG_FULL_MASK, bytes);
+                if (lane == 0) bar_expect(full + s, all);
+                __syncwarp();
+                if (bytes)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(to)), "l"(src), "r"(bytes),
+                                 "r"(smem_addr(full + s)) : "memory");
+                if (++s == slots) { s = 0; par ^= 1; }
+            }
+        // no copy may be in flight when the CTA leaves
+        for (int i = max(0, n - slots); i < n; i++) bar_wait(full + i % slots, (i / slots) & 1, status);
+        return;
+    }
+
+    // Activations.  A warp stages the blocks that it multiplies, with the rows it takes first: eight lanes share a block, lane e
+    // the elements that the MMA wants in word e, in even blocks 4 e - 2 .. 4 e + 1 (the first two from the end of the block, or of
+    // its half, where e begins it).  A segment's are on the way while the one before is multiplied.
+    constexpr int PART = FMT == FMT_Q8_0 ? 32 : 16, TURNS = SEG / kMmaWarps / 2;
+    static_assert(TURNS * 4 * kMmaWarps == 2 * SEG, "four blocks a turn");
+    const bool x8 = (reinterpret_cast<uintptr_t>(act) & 7) == 0;
+    float4 xs[TURNS];
+    auto load_x = [&](int k) {
+        const int p0 = np * k / segs, here = np * (k + 1) / segs - p0, lo = here * warp / kMmaWarps, n = here * (warp + 1) / kMmaWarps - lo;
+#pragma unroll
+        for (int j = 0; j < TURNS; j++) {
+            const int i = j * 32 + lane, own = (p0 + lo) * 64 + 4 * i;
+            const int other = i & 8 ? own + 2 : own % PART ? own - 2 : own + PART - 2, x0 = i & 8 ? own : other, x1 = i & 8 ? other : own;
+            xs[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < n * 16) {
+                if (x8) {
+                    const float2 u = *reinterpret_cast<const float2*>(act + x0), v = *reinterpret_cast<const float2*>(act + x1);
+                    xs[j] = make_float4(u.x, u.y, v.x, v.y);
+                } else {
+                    xs[j] = make_float4(act[x0], act[x0 + 1], act[x1], act[x1 + 1]);
+                }
+            }
+        }
+    };
+    auto store_x = [&](int first, int n) {                  // of the warp's n pairs from pair `first` on
+#pragma unroll
+        for (int j = 0; j < TURNS; j++) {
+            const int i = j * 32 + lane, b = first * 2 + (i >> 3), e = lane & 7;
+            const float x[4] = {xs[j].x, xs[j].y, xs[j].z, xs[j].w};
+            unsigned m = max(max(__float_as_uint(fabsf(x[0])), __float_as_uint(fabsf(x[1]))), max(__float_as_uint(fabsf(x[2])), __float_as_uint(fabsf(x[3]))));
+#pragma unroll
+            for (int o = 1; o < 8; o *= 2) m = max(m, __shfl_xor_sync(MG_FULL_MASK, m, o));
+            m >>= 23;                                       // exponent of the largest
+            // times 2^(156 - m): the largest lies in 2^29 .. 2^30 (below 2^-96 the factor stays at 2^125)
+            const unsigned f = m < 31 ? 252u : m == 255 ? 0u : 283u - m;
+            const float up = __uint_as_float(f << 23);
+            // signed digits: byte p of v + 128 (1 + 256 + 65536), less 128 below the top one
+            uint32_t v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[k] = (uint32_t)(__float2int_rn(x[k] * up) + 0x808080);
+            if (i < n * 16) {
+                const uint32_t u0 = __byte_perm(v[0], v[1], 0x5140), u1 = __byte_perm(v[2], v[3], 0x5140);     // bytes 0 and 1 of two
+                const uint32_t u2 = __byte_perm(v[0], v[1], 0x7362), u3 = __byte_perm(v[2], v[3], 0x7362);     // bytes 2 and 3
+                uint8_t* to = mma_smem + b * 32 + 8 * (e & 3) + 4 * (e >> 2);
+                *reinterpret_cast<uint32_t*>(to) = __byte_perm(u0, u1, 0x5410) ^ 0x80808080u;
+                *reinterpret_cast<uint32_t*>(to + digit_bytes) = __byte_perm(u0, u1, 0x7632) ^ 0x80808080u;
+                *reinterpret_cast<uint32_t*>(to + 2 * digit_bytes) = __byte_perm(u2, u3, 0x5410) ^ 0x80808080u;
+                *reinterpret_cast<uint32_t*>(to + 3 * digit_bytes) = __byte_perm(u2, u3, 0x7632);
+                if (e == 0) reinterpret_cast<float*>(mma_smem + 4 * digit_bytes)[b] = m == 255 ? __uint_as_float(0x7fc00000u) : __uint_as_float((254u - f) << 23);
+            }
+        }
+        __syncwarp();
+    };
+    load_x(0);
+
+    auto all_consumers = [] { asm volatile("bar.sync 1, %0;" ::"n"(kMmaWarps * 32) : "memory"); };
+    const int g = lane >> 2, t = lane & 3;
+    const bool bvalid = (g & 1) == 0;
+    const float weight = (t == 0 ? 1.0f : t == 1 ? 256.0f : t == 2 ? 65536.0f : 16777216.0f) * (FMT == FMT_Q8_0 ? 1.0f : 0.0625f);
+    int s = 0, par = 0, buf = 0;
+    for (int row0 = row_lo; row0 < row_hi; row0 += slot_rows, buf ^= 1) {
+        const int rows = min(slot_rows, row_hi - row0);
+        float acc[2][4] = {};
+        for (int k = 0; k < segs; k++) {
+            const int p0 = np * k / segs, here = np * (k + 1) / segs - p0, lo = here * warp / kMmaWarps, n = here * (warp + 1) / kMmaWarps - lo;
+            const uint32_t first = (uint32_t)reinterpret_cast<uintptr_t>(w) + (uint32_t)((size_t)row0 * rb + (size_t)p0 * 2 * BB);  // its low bits
+            const uint32_t from = ring + s * slot_bytes + lo * 2 * BB, digits = (p0 + lo) * 64 + (g >> 1) * digit_bytes + t * 8, sc = 4 * digit_bytes + (p0 + lo) * 8;
+            auto row_at = [&](int r) { return from + r * STRIDE + ((first + (uint32_t)r * (uint32_t)rb) & 15u); };
+            if (row0 == row_lo) {
+                store_x(p0 + lo, n);
+                if (k + 1 < segs) load_x(k + 1);
+            }
+            bar_wait(full + s, par, status);
+            if (rows > 16) {
+                const uint32_t at[4] = {row_at(g), row_at(g + 8), row_at(g + 16), row_at(g + 24)};
+                mma_pairs<FMT, 2>(mma_smem, at, n, digits, sc, bvalid, t, acc);
+            } else {
+                const uint32_t at[2] = {row_at(g), row_at(g + 8)};
+                mma_pairs<FMT, 1>(mma_smem, at, n, digits, sc, bvalid, t, acc);
+            }
+            __syncwarp();
+            if (lane == 0) bar_arrive(empty + s);
+            if (++s == slots) { s = 0; par ^= 1; }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float v = (acc[0][i] + acc[1][i]) * weight;
+            v += __shfl_xor_sync(MG_FULL_MASK, v, 1);
+            v += __shfl_xor_sync(MG_FULL_MASK, v, 2);
+            if (t == 0) part[(buf * kMmaWarps + warp) * kMmaRows + g + 8 * i] = v;
+        }
+        all_consumers();                                    // (two buffers: a sum is read while the next rows are multiplied)
+        if (warp == 0) {
+            float u[kMmaWarps];
+#pragma unroll
+            for (int p = 0; p < kMmaWarps; p++) u[p] = part[(buf * kMmaWarps + p) * kMmaRows + lane];
+#pragma unroll
+            for (int h = kMmaWarps / 2; h > 0; h /= 2)
+#pragma unroll
+                for (int p = 0; p < h; p++) u[p] += u[p + h];
+            float v = u[0];
+            const bool plain = lane < rows && !(fabsf(v) <= 3.402823466e38f);
+            for (unsigned left = __ballot_sync(MG_FULL_MASK, plain); left; left &= left - 1) {
+                const int r = __ffs(left) - 1;
+                const float again = raw_row_plain<FMT>(act, w + (size_t)(row0 + r) * rb, nb);
+                if (lane == r) v = again;
+            }
+            if (*reinterpret_cast<volatile int*>(status)) v = __uint_as_float(0x7fc00000u);     // a copy never came
+            if (lane < rows) out[row0 + lane] = v;
+        }
+    }
+}
+
 // ---------------- activation quantizer: one warp per block of 32 ----------------
 __global__ void __launch_bounds__(256) quantize_act_kernel(const float* __restrict__ act, ActBlock* out,
                                                           int nblocks_total) {
@@ -311,25 +578,48 @@ RawShape raw_shape(int N, int K, int sms) {
     return p;
 }
 
-template <int FMT, int R, int V, int X>
-void run_raw_matvec(const RawShape& p, int dev, const float* act, const uint8_t* w, float* out, int N, int K, cudaStream_t stream) {
-    auto kern = raw_block_matvec_kernel<FMT, R, V, X>;
-    static std::atomic<bool> raised[kMaxDevices];
-    if (p.smem > 48 * 1024 && !(dev < kMaxDevices && raised[dev].load(std::memory_order_relaxed))) {
+// A launch that may begin while the one before it ends (the kernels wait before they read).  raised: is the kernel's limit
+// of shared memory up on a device?
+template <typename... P, typename... A>
+void launch_raw(void (*kern)(P...), std::atomic<bool>* raised, int dev, int grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+    if (smem > 48 * 1024 && !(dev < kMaxDevices && raised[dev].load(std::memory_order_relaxed))) {
         cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (dev < kMaxDevices) raised[dev].store(true, std::memory_order_relaxed);
     }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)p.grid);
-    cfg.blockDim = dim3((unsigned)p.threads);
-    cfg.dynamicSmemBytes = p.smem;
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];        // a launch may begin while the one before it ends; the kernel waits before it reads
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, act, w, out, N, K, p.ks);
+    cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <int FMT, int R, int V, int X>
+void run_raw_matvec(const RawShape& p, int dev, const float* act, const uint8_t* w, float* out, int N, int K, cudaStream_t stream) {
+    static std::atomic<bool> raised[kMaxDevices];
+    launch_raw(raw_block_matvec_kernel<FMT, R, V, X>, raised, dev, p.grid, p.threads, p.smem, stream, act, w, out, N, K, p.ks);
+}
+
+// Rows a CTA of the integer kernel takes at a time, 32, 16 or all it has, and slots of its ring; no rows: shared memory holds no two slots.
+struct MmaShape {
+    int rows, slots;
+    size_t smem;
+};
+template <int FMT>
+MmaShape mma_shape(int N, int K, int sms) {
+    const size_t fixed = mma_input_bytes(K / 32) + kMmaSums + kMmaBars;
+    for (int rows = std::min(kMmaRows, cdiv(N, sms)); rows > 0; rows = rows > 16 ? 16 : 0) {
+        // (behind the last slot: rows that a tile of 16 has and the slot has not are read, and dropped)
+        const size_t slot = (size_t)rows * mma_stride(FMT), spare = (size_t)kMmaRows * mma_stride(FMT) - slot;
+        for (int slots = kMmaSlots; slots >= 2; slots--)
+            if (fixed + slots * slot + spare <= kRawSmem) return {rows, slots, fixed + slots * slot + spare};
+    }
+    return {};
 }
 
 template <int FMT>
@@ -344,8 +634,18 @@ void launch_raw_matvec(const float* act, const void* w_blocks, float* out, int N
         if (sms <= 0) sms = 148;
         if (dev < kMaxDevices) sm_count[dev].store(sms, std::memory_order_relaxed);
     }
-    const RawShape p = raw_shape<FMT>(N, K, sms);
     const uint8_t* w = static_cast<const uint8_t*>(w_blocks);
+    // The integer kernel, us of Q8_0 / Q4_0, the other -> this: 1024 columns 20000 rows 8.6 -> 9.2 / 8.5 -> 9.4, 7200 rows 4.5 -> 4.8 / 5.0 -> 4.9;
+    // 1536 columns 20000 rows 14.4 -> 9.5 / 13.5 -> 9.8; 8192 columns 300 rows 4.4 -> 5.9 / 4.0 -> 5.0, 600 rows 6.0 -> 5.9 / 5.6 -> 5.1; 24576
+    // columns 900 rows 12.7 -> 13.7 / 12.0 -> 11.3, 1200 rows 21.7 -> 13.7 / 20.3 -> 11.3 (every CTA stages the whole input).
+    const bool ints = K > 1024 && K % 64 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && N >= (K > 20480 ? 8 : 4) * sms;
+    const MmaShape q = ints ? mma_shape<FMT>(N, K, sms) : MmaShape{};
+    if (q.rows > 0) {
+        static std::atomic<bool> raised[kMaxDevices];
+        launch_raw(raw_block_mma_kernel<FMT>, raised, dev, std::min(sms, N), kMmaThreads, q.smem, stream, act, w, out, N, K, q.rows, q.slots);
+        return;
+    }
+    const RawShape p = raw_shape<FMT>(N, K, sms);
     auto go = [&](auto r, auto v) {
         constexpr int R = decltype(r)::value, V = decltype(v)::value;
         if (p.input == RAW_PADDED) run_raw_matvec<FMT, R, V, RAW_PADDED>(p, dev, act, w, out, N, K, stream);
