@@ -219,7 +219,8 @@ __global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __re
 // block and row where re-aligned words took 3 (5).  The activations of even blocks are staged in that order of elements.
 // B200, passes among others, the kernel above -> this one: Q4_0 3584 x 18944 26.9 -> 13.0 us (2.9 TB/s), 3584 x 3584 10.8 -> 4.4, 18944 x 3584
 // 24.2 -> 10.7; Q8_0 3584 x 18944 27.5 -> 17.0, 20000 x 19200 114 -> 75 (5.4 TB/s).  Error against 64 bits at 3584 x 18944 Q4_0 1.4e-7 -> 0.7e-7.
-//   A row whose sum is not finite is computed again in plain fp32 (activations or scales that are not, or sums beyond the range).
+//   A row whose sum is not finite is computed again in plain fp32 (activations or scales that are not, or sums beyond the range); so is one
+// below 2^-80 where a block of activations lies below 2^-96, whose digits would not hold fp32's.
 constexpr int kMmaWarps = 16, kMmaRows = 32, kMmaSlots = 4;
 constexpr int kMmaThreads = (kMmaWarps + 1) * 32;
 __host__ __device__ constexpr int mma_seg(int fmt) { return fmt == FMT_Q8_0 ? 32 : 64; }       // pairs
@@ -310,13 +311,13 @@ __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_mma_kernel(const flo
     float* part = reinterpret_cast<float*>(mma_smem + mma_input_bytes(nb));
     uint64_t* full = reinterpret_cast<uint64_t*>(mma_smem + mma_input_bytes(nb) + kMmaSums);
     uint64_t* empty = full + kMmaSlots;
-    int* status = reinterpret_cast<int*>(empty + kMmaSlots);
+    int* status = reinterpret_cast<int*>(empty + kMmaSlots), *small = status + 1;      // small: a block below the digits' range
     const uint32_t ring = (uint32_t)(mma_input_bytes(nb) + kMmaSums + kMmaBars), slot_bytes = (uint32_t)slot_rows * STRIDE;
     const int row_lo = (int)((long long)N * blockIdx.x / gridDim.x), row_hi = (int)((long long)N * (blockIdx.x + 1) / gridDim.x);
     const int segs = (np + SEG - 1) / SEG;
     if (threadIdx.x == 0) {
         for (int i = 0; i < slots; i++) { bar_init(full + i, 1); bar_init(empty + i, kMmaWarps); }
-        *status = 0;
+        *status = *small = 0;
         bar_init_fence();
     }
     __syncthreads();
@@ -386,6 +387,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_mma_kernel(const flo
             unsigned m = max(max(__float_as_uint(fabsf(x[0])), __float_as_uint(fabsf(x[1]))), max(__float_as_uint(fabsf(x[2])), __float_as_uint(fabsf(x[3]))));
 #pragma unroll
             for (int o = 1; o < 8; o *= 2) m = max(m, __shfl_xor_sync(MG_FULL_MASK, m, o));
+            if (m > 0 && m < 31u << 23) *small = 1;
             m >>= 23;                                       // exponent of the largest
             // times 2^(156 - m): the largest lies in 2^29 .. 2^30 (below 2^-96 the factor stays at 2^125)
             const unsigned f = m < 31 ? 252u : m == 255 ? 0u : 283u - m;
@@ -455,7 +457,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_mma_kernel(const flo
 #pragma unroll
                 for (int p = 0; p < h; p++) u[p] += u[p + h];
             float v = u[0];
-            const bool plain = lane < rows && !(fabsf(v) <= 3.402823466e38f);
+            const bool plain = lane < rows && (!(fabsf(v) <= 3.402823466e38f) || (*small && fabsf(v) < 0x1p-80f));
             for (unsigned left = __ballot_sync(MG_FULL_MASK, plain); left; left &= left - 1) {
                 const int r = __ffs(left) - 1;
                 const float again = raw_row_plain<FMT>(act, w + (size_t)(row0 + r) * rb, nb);
