@@ -119,7 +119,8 @@ struct MixerStep {
     int n_mem;              // CTAs of the memory part (0: no such branch)
     int vslices;            // value slices of 32 columns per head
     int splits;             // CTAs of the attention part
-    int tile;               // keys per shared-memory tile
+    int tile, grain;        // keys per shared-memory tile; keys are dealt to the CTAs in runs of a multiple of `grain`
+    bool key_copy;          // launch_mixer_step: shared memory has room for the new key
     float* part;            // [splits][heads * dim_s]
     float* mem_o;           // [heads * vdim] raw outputs
     float* attn_out;        // [heads * dim]

@@ -10,6 +10,7 @@ namespace mg {
 
 namespace {
 
+constexpr int kStepThreads = 512;
 constexpr int kStateRows = 16;      // rows of the state a warp holds at a time
 
 // One token of the matrix memory: CTA (head, slice of 32 value columns); lanes over columns, warps over
@@ -83,53 +84,190 @@ __device__ __forceinline__ void mem_step(const MixerStep& a, int cta, float* sme
     }
 }
 
+// Shared memory of the attention part: AttnSmem, and behind it
+//   rnew [kv_heads], knew [kv_heads][dim_s] the new key as it is stored (read back
+//   from the cache where shared memory has no room for it).
+inline size_t step_extra(const GateAttn& A) { return ((size_t)pad_to(A.kv_heads, 4) + 3) * 4; }
+inline size_t step_key(const GateAttn& A, size_t kt_bytes) { return (size_t)A.kv_heads * A.dim_s * kt_bytes; }
+
+// What bounds the step is the latency of one tile of keys: loads that follow one another, each phase behind a barrier, on the CTAs of
+// a few keys each.  So four lanes share a score and a mixed weight, sixteen a query's norm, keys are dealt four by four, and
+// everything that no predecessor leaves (cached keys, tables, the norms' weights, addresses) is there before the wait; the new key
+// reaches the CTA that ends with it through shared memory, not through the cache.  B200, 1.1B widths, 320 positions, us from the
+// wait to the end of this kernel: 9.2 with 256 threads, a thread per score, eight lanes per norm and tiles of eight keys, 4.3 now;
+// 300 + 64 tokens of six layers 18.20 -> 16.92 ms.  Runs of eight keys per CTA: 17.17 ms.
 template <typename KT, int EP>
-__global__ void __launch_bounds__(kAttnThreads) mixer_step_kernel(const MixerStep a) {
+__global__ void __launch_bounds__(kStepThreads) mixer_step_kernel(const MixerStep a) {
     extern __shared__ __align__(16) float smem[];
     pdl_launch_dependents();
     if ((int)blockIdx.x < a.n_mem) {
         mem_step(a, blockIdx.x, smem);
         return;
     }
+    constexpr int CN = Chunk16<KT>::n;
     const GateAttn& A = a.at;
+    const int H = A.heads, DS = A.dim_s, KV = A.kv_heads, group = H / KV, chunks = DS / CN;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = kStepThreads / 32;
+    const AttnSmem<KT> sm(A, 1, a.tile, smem);
+    const int row = KV * sm.ks;
+    // tables and the norms' weights are on the way before the position is known
     const int pos = a.st->pos, len = pos + 1;
-    if (pos >= A.max_seq) return;
+    for (int h = wid; h < H; h += nw)
+        for (int g = lane; g < H; g += 32) cp_async4(sm.talk + h * sm.ts + g, A.talk + h * H + g);
+    for (int i = tid; i < H; i += kStepThreads) { cp_async4(sm.bias + i, A.head_bias + i); cp_async4(sm.slope + i, A.slopes + i); }
+    const int part16 = lane & 15;
+    float qk[8];                                    // of the first 128 elements
+#pragma unroll
+    for (int i = 0; i < 8; i++) qk[i] = part16 + 16 * i < A.dim ? A.q_norm[part16 + 16 * i] * A.k_norm[part16 + 16 * i] : 0.f;
+    int head_of[EP], key_of[EP];                    // this thread's output elements
+#pragma unroll
+    for (int e = 0; e < EP; e++) {
+        const int el = 2 * (tid + e * kStepThreads), h = el / DS;
+        head_of[e] = el < H * DS ? h : -1;
+        key_of[e] = h / group * sm.ks + el - h * DS;
+    }
     const int split = blockIdx.x - a.n_mem;
     int j0, j1;
-    const int active = key_split(len, a.splits, a.tile, split, &j0, &j1);
-    if (split >= active) return;
-    const AttnSmem<KT> sm(A, 1, a.tile, smem);
-    // tables, and keys of earlier tokens, do not wait for the predecessor
-    const bool early = j0 + a.tile <= pos;
-    if (early) {
-        load_keys<KT>(A, sm, KeyCopy(A.dim_s / Chunk16<KT>::n), 0, j0, j1, a.tile);
+    const int active = key_split(len, a.splits, a.grain, split, &j0, &j1);
+    if (split >= active || pos >= A.max_seq) {
         cp_async_commit();
+        cp_async_wait<0>();
+        return;
     }
-    sm.load_tables(A);
+    const int tile = j1 - j0 <= a.grain ? a.grain : a.tile, tsh = 31 - __clz(tile);      // powers of two
+    float* rnew = sm.slope + A.heads;
+    KT* knew = a.key_copy ? reinterpret_cast<KT*>((reinterpret_cast<uintptr_t>(rnew + A.kv_heads) + 15) & ~(uintptr_t)15)
+                          : static_cast<KT*>(A.cache) + (size_t)pos * A.kv_heads * A.dim_s;
+
+    // cached keys of a tile, rows behind them zero
+    const int pieces = chunks, step = kStepThreads / pieces, first = tid / pieces, piece = tid - first * pieces;
+    auto load_tile = [&](int buf, int j) {
+        const int rows = tile * KV, valid = max(0, min(rows, (min(j1, pos) - j) * KV));
+        KT* dst = sm.k + (size_t)buf * a.tile * row + piece * CN;
+        const KT* src = static_cast<const KT*>(A.cache) + (size_t)j * KV * DS + piece * CN;
+        if (first < step)
+            for (int r = first; r < rows; r += step) {
+                if (r < valid) cp_async16(dst + r * sm.ks, src + (size_t)r * DS);
+                else *reinterpret_cast<uint4*>(dst + r * sm.ks) = make_uint4(0u, 0u, 0u, 0u);
+            }
+        for (int i = tid; i < valid; i += kStepThreads) cp_async4(sm.r + buf * a.tile * KV + i, A.cache_r + (size_t)j * KV + i);
+        cp_async_commit();
+    };
+    load_tile(0, j0);
+    const float temp = query_temp(A, pos) * A.scale;
     pdl_wait();
-    // this token's query, and its key where this CTA's range ends with it
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const float temp = query_temp(A, pos);
-    norm_queries(A, a.proj + a.c.q, temp, sm.q, sm.qs);
-    if (j1 == len)
-        for (int c = wid; c < A.kv_heads; c += nw) store_key<KT>(A, a.proj + a.c.k + c * A.dim, pos, c, lane);
-    __syncthreads();                        // the cache row above is read back by this CTA only
-    float acc[1][EP][2] = {};
-    attend<KT, 1, EP>(A, sm, pos, j0, j1, a.tile, acc, early);
+
+    // this token's query, sixteen lanes per head, and its key where this CTA's range ends with it
+    {
+        const int sub = part16;
+        const unsigned mask = 0xffffu << (lane & 16);
+        for (int h = tid >> 4; h < H; h += kStepThreads / 16) {
+            const float* p = a.proj + a.c.q + h * A.dim;
+            float v[8], ss = 0.f;                   // the first 128 values are loaded at once
 #pragma unroll
-    for (int p = 0; p < EP; p++) {
-        const int e = 2 * (threadIdx.x + p * kAttnThreads);
-        if (e < A.heads * A.dim_s)
-            *reinterpret_cast<float2*>(a.part + (size_t)split * A.heads * A.dim_s + e) = make_float2(acc[0][p][0], acc[0][p][1]);
+            for (int i = 0; i < 8; i++) {
+                v[i] = sub + 16 * i < A.dim ? p[sub + 16 * i] : 0.f;
+                ss = fmaf(v[i], v[i], ss);
+            }
+            for (int d = sub + 128; d < A.dim; d += 16) ss = fmaf(p[d], p[d], ss);
+#pragma unroll
+            for (int o = 1; o < 16; o *= 2) ss += __shfl_xor_sync(mask, ss, o);
+            const float r = temp / sqrtf(ss / (float)A.dim + A.eps);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int d = sub + 16 * i;
+                if (d < DS) sm.q[h * sm.qs + d] = v[i] * r * qk[i];
+            }
+            for (int d = sub + 128; d < DS; d += 16) sm.q[h * sm.qs + d] = d < A.dim ? p[d] * r * A.q_norm[d] * A.k_norm[d] : 0.f;
+        }
     }
+    if (j1 == len)
+        for (int c = nw - 1 - wid; c < KV; c += nw) store_key<KT>(A, a.proj + a.c.k + c * A.dim, pos, c, lane, a.key_copy ? knew + c * DS : nullptr, rnew + c);
+
+    float2 acc[EP];
+#pragma unroll
+    for (int e = 0; e < EP; e++) acc[e] = make_float2(0.f, 0.f);
+    const int sub = lane & 3;
+    const unsigned quad = 0xfu << (lane & 28);
+    int buf = 0;
+    for (int j = j0; j < j1; j += tile, buf ^= 1) {
+        if (j + tile < j1) load_tile(buf ^ 1, j + tile);
+        else cp_async_commit();
+        cp_async_wait<1>();
+        KT* K = sm.k + (size_t)buf * a.tile * row;
+        float* R = sm.r + buf * a.tile * KV;
+        if (pos >= j && pos < j + tile) {           // (the rows of the copies end before it)
+            __syncthreads();
+            KT* to = K + (size_t)(pos - j) * row;
+            for (int i = tid; i < KV * DS; i += kStepThreads) to[i / DS * sm.ks + i % DS] = knew[i];
+            for (int i = tid; i < KV; i += kStepThreads) R[(pos - j) * KV + i] = rnew[i];
+        }
+        __syncthreads();
+        const int keys = min(tile, j1 - j), units = H << tsh;
+        for (int u = tid >> 2; u < units; u += kStepThreads / 4) {
+            const int h = u >> tsh, p = u & (tile - 1), c = h / group;
+            const KT* kp = K + p * row + c * sm.ks;
+            const float* qp = sm.q + h * sm.qs;
+            float d0 = 0.f, d1 = 0.f;
+#pragma unroll 2
+            for (int ch = sub; ch < chunks; ch += 4) {
+                float kk[CN];
+                Chunk16<KT>::load(kp + ch * CN, kk);
+#pragma unroll
+                for (int i = 0; i < CN; i += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(qp + ch * CN + i);
+                    d0 = fmaf(kk[i], v.x, d0);
+                    d1 = fmaf(kk[i + 1], v.y, d1);
+                    d0 = fmaf(kk[i + 2], v.z, d0);
+                    d1 = fmaf(kk[i + 3], v.w, d1);
+                }
+            }
+            d0 += d1;
+            d0 += __shfl_xor_sync(quad, d0, 1);
+            d0 += __shfl_xor_sync(quad, d0, 2);
+            if (sub == 0) {
+                const float s = d0 * (p < keys ? R[p * KV + c] : 0.f) - sm.slope[h] * (float)(pos - (j + p)) + sm.bias[h];
+                sm.w[h * sm.ws + p] = p < keys ? sigmoid(s) : 0.f;
+            }
+        }
+        __syncthreads();
+        for (int u = tid >> 2; u < units; u += kStepThreads / 4) {
+            const int h = u >> tsh, p = u & (tile - 1);
+            const float* t = sm.talk + h * sm.ts;
+            float v = 0.f;
+#pragma unroll 8
+            for (int g = sub; g < H; g += 4) v = fmaf(t[g], sm.w[g * sm.ws + p], v);
+            v += __shfl_xor_sync(quad, v, 1);
+            v += __shfl_xor_sync(quad, v, 2);
+            if (sub == 0) sm.mix[h * sm.ws + p] = v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < EP; e++)
+            if (head_of[e] >= 0) {
+#pragma unroll 4
+                for (int p = 0; p < keys; p++) {
+                    const float2 kv = pair_f32(K + p * row + key_of[e]);
+                    const float m = sm.mix[head_of[e] * sm.ws + p];
+                    acc[e].x = fmaf(m, kv.x, acc[e].x);
+                    acc[e].y = fmaf(m, kv.y, acc[e].y);
+                }
+            }
+        if (j + tile < j1) __syncthreads();         // w, mix and this buffer are used again
+    }
+#pragma unroll
+    for (int e = 0; e < EP; e++)
+        if (head_of[e] >= 0) *reinterpret_cast<float2*>(a.part + (size_t)split * H * DS + 2 * (tid + e * kStepThreads)) = acc[e];
 }
 
-constexpr int kJoinCols = 32, kJoinParts = 8;      // outputs per CTA, threads that share one output's splits
+constexpr int kJoinCols = 16, kJoinParts = 16;      // outputs per CTA, threads that share one output's splits
 
 // Joins the key splits, and norms and gates the memory's outputs (one CTA per memory head).
 __global__ void __launch_bounds__(kJoinCols * kJoinParts) mixer_join_kernel(const MixerStep a) {
     __shared__ float red[40];
     pdl_launch_dependents();
+    int j0, j1;
+    const int active = key_split(a.st->pos + 1, a.splits, a.grain, 0, &j0, &j1);
     pdl_wait();
     const MatMem& M = a.mem;
     const int nm = a.n_mem ? M.heads : 0;
@@ -149,8 +287,6 @@ __global__ void __launch_bounds__(kJoinCols * kJoinParts) mixer_join_kernel(cons
     const int col = threadIdx.x % kJoinCols, grp = threadIdx.x / kJoinCols;
     const int e = (blockIdx.x - nm) * kJoinCols + col;
     const bool ok = e < A.heads * A.dim;
-    int j0, j1;
-    const int active = key_split(a.st->pos + 1, a.splits, a.tile, 0, &j0, &j1);
     const int src = ok ? e / A.dim * A.dim_s + e % A.dim : 0;
     const size_t stride = (size_t)A.heads * A.dim_s;
     float v = 0.f;
@@ -178,19 +314,16 @@ __global__ void __launch_bounds__(256) resolve_kernel(const ResolveArgs a) {
 
 template <typename KT>
 cudaError_t step_for(const MixerStep& a, size_t smem, bool pdl, cudaStream_t s) {
-    const int ep = attn_pairs(a.at);
+    const int pairs = (a.at.heads * a.at.dim_s / 2 + kStepThreads - 1) / kStepThreads;
     const int grid = a.n_mem + a.splits;
     auto run = [&](auto kern) {
         cudaError_t c = allow_smem(kern, std::max(smem, kModelSmem));
-        return c != cudaSuccess ? c : launch_pdl(kern, grid, kAttnThreads, smem, pdl, s, a);
+        return c != cudaSuccess ? c : launch_pdl(kern, grid, kStepThreads, smem, pdl, s, a);
     };
-    switch (ep) {
-        case 1: return run(mixer_step_kernel<KT, 1>);
-        case 2: return run(mixer_step_kernel<KT, 2>);
-        case 4: return run(mixer_step_kernel<KT, 4>);
-        case 8: return run(mixer_step_kernel<KT, 8>);
-        case 16: return run(mixer_step_kernel<KT, 16>);
-    }
+    if (pairs <= 1) return run(mixer_step_kernel<KT, 1>);
+    if (pairs <= 2) return run(mixer_step_kernel<KT, 2>);
+    if (pairs <= 4) return run(mixer_step_kernel<KT, 4>);
+    if (pairs <= 8) return run(mixer_step_kernel<KT, 8>);
     return cudaErrorInvalidValue;
 }
 
@@ -263,15 +396,20 @@ cudaError_t launch_rows_parts(const PhaseArgs& a, PhaseParts& p, int sms, bool p
 }
 
 size_t mixer_step_smem(const GateAttn& at, const MatMem& mem, bool f32_cache, int* tile) {
-    const size_t need_mem = (40 + kAttnThreads + 2 * (size_t)mem.dim) * sizeof(float);
-    const size_t need = attn_smem(at, 1, f32_cache ? 4 : 2, 8, tile);
-    return need == 0 ? 0 : need > need_mem ? need : need_mem;
+    const size_t need_mem = (40 + kStepThreads + 2 * (size_t)mem.dim) * sizeof(float);
+    size_t need = attn_smem(at, 1, f32_cache ? 4 : 2, 8, tile);
+    if (need == 0) return 0;
+    need += step_extra(at);
+    if (const size_t key = step_key(at, f32_cache ? 4 : 2); need + key <= kModelSmem) need += key;
+    return need > need_mem ? need : need_mem;
 }
 
 cudaError_t launch_mixer_step(const MixerStep& a, bool f32_cache, bool pdl, cudaStream_t s) {
+    MixerStep b = a;
     int tile;
-    const size_t smem = mixer_step_smem(a.at, a.mem, f32_cache, &tile);
-    return f32_cache ? step_for<float>(a, smem, pdl, s) : step_for<__nv_bfloat16>(a, smem, pdl, s);
+    const size_t smem = mixer_step_smem(a.at, a.mem, f32_cache, &tile), kt = f32_cache ? 4 : 2;
+    b.key_copy = smem >= attn_smem(a.at, 1, (int)kt, 8, &tile) + step_extra(a.at) + step_key(a.at, kt);
+    return f32_cache ? step_for<float>(b, smem, pdl, s) : step_for<__nv_bfloat16>(b, smem, pdl, s);
 }
 
 cudaError_t launch_mixer_join(const MixerStep& a, bool pdl, cudaStream_t s) {

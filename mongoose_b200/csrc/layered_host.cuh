@@ -613,7 +613,7 @@ int enqueue_layered_step(mg_engine* e, cudaStream_t s, int ls, int le, int mode,
         }
         MixerStep ms{};
         ms.at = run.at(l); ms.mem = run.mem(l); ms.c = l.cols; ms.proj = m.row; ms.st = e->st;
-        ms.vslices = (l.mem.vdim + 31) / 32; ms.n_mem = l.mem.heads * ms.vslices; ms.splits = l.splits; ms.tile = l.tile;
+        ms.vslices = (l.mem.vdim + 31) / 32; ms.n_mem = l.mem.heads * ms.vslices; ms.splits = l.splits; ms.tile = l.tile; ms.grain = std::min(l.tile, 4);
         ms.part = m.part; ms.mem_o = m.mem_raw; ms.attn_out = m.attn; ms.mem_y = m.mem_y;
         MG_CUDA(e, launch_mixer_step(ms, m.f32, e->use_pdl, s));
         MG_CUDA(e, launch_mixer_join(ms, e->use_pdl, s));

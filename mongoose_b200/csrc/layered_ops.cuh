@@ -93,47 +93,25 @@ __device__ __forceinline__ void norm_query(const GateAttn& A, const float* q, fl
     for (int d = lane; d < A.dim_s; d += 32) from_f32(d < A.dim ? q[d] * r * A.q_norm[d] * A.k_norm[d] : 0.f, out + d);
 }
 
-// The same for every head of one token by the whole CTA, eight lanes per head.
-__device__ __forceinline__ void norm_queries(const GateAttn& A, const float* q, float temp, float* out, int qs) {
-    const int sub = threadIdx.x & 7;
-    const unsigned mask = 0xffu << (threadIdx.x & 24);
-    for (int h = threadIdx.x >> 3; h < A.heads; h += kAttnThreads / 8) {
-        const float* p = q + h * A.dim;
-        float v[16], ss = 0.f;              // the first 128 values are loaded at once
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const int d = sub + 8 * i;
-            v[i] = d < A.dim ? p[d] : 0.f;
-            ss = fmaf(v[i], v[i], ss);
-        }
-        for (int d = sub + 128; d < A.dim; d += 8) ss = fmaf(p[d], p[d], ss);
-        ss += __shfl_xor_sync(mask, ss, 1);
-        ss += __shfl_xor_sync(mask, ss, 2);
-        ss += __shfl_xor_sync(mask, ss, 4);
-        const float r = temp * A.scale / sqrtf(ss / (float)A.dim + A.eps);
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const int d = sub + 8 * i;
-            if (d < A.dim_s) out[h * qs + d] = d < A.dim ? v[i] * r * A.q_norm[d] * A.k_norm[d] : 0.f;
-        }
-        for (int d = sub + 128; d < A.dim_s; d += 8) out[h * qs + d] = d < A.dim ? p[d] * r * A.q_norm[d] * A.k_norm[d] : 0.f;
-    }
-}
-
-// One warp: key head c of position pos into the cache, with the 1 / rms of the row as stored.
+// One warp: key head c of position pos into the cache, with the 1 / rms of the row as stored; a copy of both where it is wanted.
 template <typename KT>
-__device__ __forceinline__ void store_key(const GateAttn& A, const float* k, int pos, int c, int lane) {
+__device__ __forceinline__ void store_key(const GateAttn& A, const float* k, int pos, int c, int lane, KT* copy = nullptr, float* copy_r = nullptr) {
     KT* dst = static_cast<KT*>(A.cache) + ((size_t)pos * A.kv_heads + c) * A.dim_s;
     float ss = 0.f;
     for (int d = lane; d < A.dim_s; d += 32) {
         KT t;
         from_f32(d < A.dim ? k[d] : 0.f, &t);
         dst[d] = t;
+        if (copy) copy[d] = t;
         const float v = to_f32(t);
         ss = fmaf(v, v, ss);
     }
     ss = warp_sum(ss);
-    if (lane == 0) A.cache_r[(size_t)pos * A.kv_heads + c] = 1.0f / sqrtf(ss / (float)A.dim + A.eps);
+    if (lane == 0) {
+        const float r = 1.0f / sqrtf(ss / (float)A.dim + A.eps);
+        A.cache_r[(size_t)pos * A.kv_heads + c] = r;
+        if (copy_r) *copy_r = r;
+    }
 }
 
 // Keys [j0, j1) of part `split` when `len` keys are cut into at most `splits` parts of whole tiles;
@@ -262,11 +240,10 @@ __device__ __forceinline__ void load_keys(const GateAttn& A, const AttnSmem<KT>&
 
 // acc[q][pair] += sum over keys [j0, j1) of the mixed weights times the raw keys, for the NQ queries in
 // sm.q at positions pos0 .. pos0 + NQ - 1.  Thread t owns elements 2 * (t + p * kAttnThreads) and the next of the
-// [heads][dim_s] output.  A score belongs to one thread, lanes over heads.  `loaded`: the first tile's copies have been
-// issued and committed.
+// [heads][dim_s] output.  A score belongs to one thread, lanes over heads. 
 template <typename KT, int NQ, int EP>
 __device__ __forceinline__ void attend(const GateAttn& A, const AttnSmem<KT>& sm, int pos0, int j0, int j1, int tile,
-                                       float (&acc)[NQ][EP][2], bool loaded = false) {
+                                       float (&acc)[NQ][EP][2]) {
     constexpr int CN = Chunk16<KT>::n;
     const int H = A.heads, DS = A.dim_s, KV = A.kv_heads, group = H / KV, row = KV * sm.ks;
     const int chunks = DS / CN;
@@ -280,10 +257,8 @@ __device__ __forceinline__ void attend(const GateAttn& A, const AttnSmem<KT>& sm
         head_of[e] = el < H * DS ? h : -1;
         key_of[e] = h / group * sm.ks + el - h * DS;
     }
-    if (!loaded) {
-        load_keys<KT>(A, sm, cp, 0, j0, j1, tile);
-        cp_async_commit();
-    }
+    load_keys<KT>(A, sm, cp, 0, j0, j1, tile);
+    cp_async_commit();
     int buf = 0;
     for (int j = j0; j < j1; j += tile, buf ^= 1) {
         if (j + tile < j1) load_keys<KT>(A, sm, cp, buf ^ 1, j + tile, j1, tile);
