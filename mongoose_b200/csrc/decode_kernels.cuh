@@ -260,7 +260,27 @@ __device__ __forceinline__ float2 block_sum2(float u, float v, float* red) {
     return make_float2(warp_sum(u), warp_sum(v));
 }
 
-// Prologue of layer-described models.  xs gets K floats, zero behind the vector; with `keep` the residual sum
+// Sums over a CTA of eight warps behind ONE barrier; every thread gets them, in the same order.  `red` is 8 N floats of shared
+// memory, 16-byte aligned, that nothing else uses between two barriers of the caller: a prologue's sums each have their own.
+template <int N>
+__device__ __forceinline__ void sums8(float (&v)[N], float* red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < N; i++) v[i] += __shfl_xor_sync(MG_FULL_MASK, v[i], o);
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i++) red[8 * i + (threadIdx.x >> 5)] = v[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const float4 a = *reinterpret_cast<const float4*>(red + 8 * i), b = *reinterpret_cast<const float4*>(red + 8 * i + 4);
+        v[i] = ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
+    }
+}
+
+// Prologue of layer-described models, 256 threads.  xs gets K floats, zero behind the vector; with `keep` the residual sum
 // goes to h_store (never the buffer x_src names: other CTAs still read that one), the normed vector to
 // n_store and, for a mixed one, to the other slot of mix_prev.  `red` is 72 floats.  A vector of up to 8
 // values per thread stays in registers from the first load to the last norm; a longer one goes through xs
@@ -285,9 +305,10 @@ __device__ __forceinline__ void stage_layered(const PhaseArgs& a, float* xs, flo
                 s0 += y.squares();
                 s1 += z.squares();
             }
-            const float2 t = block_sum2(s0, s1, red);
-            r0 = 0.5f / sqrtf(t.x * inv_n + a.eps);
-            r1 = 0.5f / sqrtf(t.y * inv_n + a.eps);
+            float t[2] = {s0, s1};
+            sums8(t, red);
+            r0 = 0.5f / sqrtf(t[0] * inv_n + a.eps);
+            r1 = 0.5f / sqrtf(t[1] * inv_n + a.eps);
         }
         for (int b = 0; b < n; b += step) {
             if (!(one && pair)) {
@@ -305,7 +326,9 @@ __device__ __forceinline__ void stage_layered(const PhaseArgs& a, float* xs, flo
             ss += y.squares();
             if (!one) y.store(xs, b, n);
         }
-        r = 1.0f / sqrtf(block_sum2(ss, 0.f, red).x * inv_n + a.eps);
+        float t[1] = {ss};
+        sums8(t, red + 16);
+        r = 1.0f / sqrtf(t[0] * inv_n + a.eps);
     }
     const int token = a.pro == PRO_EMBED_POS ? a.st->token : 0;
     const int pos = a.pro == PRO_EMBED_POS || a.mix_mu ? a.st->pos : 0;
@@ -344,10 +367,11 @@ __device__ __forceinline__ void stage_layered(const PhaseArgs& a, float* xs, flo
         if (!(one && a.last_w)) x.store(xs, b, n);
     }
     if (a.last_w) {
-        const float2 t = block_sum2(ss, sum, red);
-        float mean = 0.f, var = t.x * inv_n;
+        float t[2] = {ss, sum};
+        sums8(t, red + 24);
+        float mean = 0.f, var = t[0] * inv_n;
         if (a.last_kind == NORM_LAYER) {            // the mean square of the deviations themselves
-            mean = t.y * inv_n;
+            mean = t[1] * inv_n;
             float dd = 0.f;
             for (int b = 0; b < n; b += step) {
                 if (!one) x.load(xs, b, n);
@@ -357,7 +381,9 @@ __device__ __forceinline__ void stage_layered(const PhaseArgs& a, float* xs, flo
                     dd = fmaf(d, d, dd);
                 }
             }
-            var = block_sum2(dd, 0.f, red).x * inv_n;
+            float u[1] = {dd};
+            sums8(u, red + 40);
+            var = u[0] * inv_n;
         }
         const float rl = 1.0f / sqrtf(var + a.eps);
         const float one_more = a.last_kind == NORM_RMS_AROUND_ZERO ? 1.0f : 0.0f;

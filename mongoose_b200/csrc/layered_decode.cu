@@ -264,7 +264,7 @@ constexpr int kJoinCols = 16, kJoinParts = 16;      // outputs per CTA, threads 
 
 // Joins the key splits, and norms and gates the memory's outputs (one CTA per memory head).
 __global__ void __launch_bounds__(kJoinCols * kJoinParts) mixer_join_kernel(const MixerStep a) {
-    __shared__ float red[40];
+    __shared__ __align__(16) float red[8];
     pdl_launch_dependents();
     int j0, j1;
     const int active = key_split(a.st->pos + 1, a.splits, a.grain, 0, &j0, &j1);
@@ -276,7 +276,9 @@ __global__ void __launch_bounds__(kJoinCols * kJoinParts) mixer_join_kernel(cons
         const float* o = a.mem_o + head * M.vdim;
         float ss = 0.f;
         for (int v = threadIdx.x; v < M.vdim; v += blockDim.x) ss = fmaf(o[v], o[v], ss);
-        const float r = 1.0f / sqrtf(block_sum(ss, red) / (float)M.vdim + M.eps);
+        float total[1] = {ss};
+        sums8(total, red);
+        const float r = 1.0f / sqrtf(total[0] / (float)M.vdim + M.eps);
         for (int v = threadIdx.x; v < M.vdim; v += blockDim.x) {
             const int c = head * M.vdim + v;
             a.mem_y[c] = o[v] * r * M.norm[c] * sigmoid(a.proj[a.c.mg + c]);

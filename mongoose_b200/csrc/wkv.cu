@@ -14,7 +14,7 @@ constexpr int kStepRows = 8;        // rows of the state a warp holds at a time,
 // One token: a CTA per head, lanes over value channels, warps over key channels.
 __global__ void __launch_bounds__(kStepThreads) wkv_step_kernel(const WkvStep a) {
     extern __shared__ __align__(16) float smem[];
-    __shared__ float red[40];
+    __shared__ __align__(16) float red[8];
     const Wkv& M = a.wk;
     const int D = M.dim, n = M.heads * D, c0 = blockIdx.x * D, rk = pad_to(M.rank, 8);
     float *r = smem, *k = r + D, *w = k + D, *v = w + D, *u = v + D, *inner = smem + pad_to(5 * D, 4);
@@ -104,7 +104,9 @@ __global__ void __launch_bounds__(kStepThreads) wkv_step_kernel(const WkvStep a)
         part[i] = o;                        // row 0 of this column is read by this thread only
         ss = fmaf(o, o, ss);
     }
-    const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)D + M.eps);
+    float total[1] = {ss};
+    sums8(total, red);
+    const float inv = 1.0f / sqrtf(total[0] / (float)D + M.eps);
     for (int i = threadIdx.x; i < D; i += kStepThreads)
         a.y[c0 + i] = part[i] * inv * M.norm[c0 + i] * silu(a.row[3 * (size_t)n + c0 + i]);
 }
