@@ -301,7 +301,7 @@ __device__ __forceinline__ void mma_pairs(const uint8_t* smem, const uint32_t (&
 
 // An even number of blocks, and a matrix on a 16-byte boundary.  slot_rows: rows taken at a time; slots: of the ring.
 template <int FMT>
-__global__ void __launch_bounds__(kMmaThreads, 1) raw_block_mma_kernel(const float* __restrict__ act, const uint8_t* __restrict__ w, float* out, int N, int K,
+__global__ void __launch_bounds__(kMmaThreads, 1) raw_block_matvec_mma_kernel(const float* __restrict__ act, const uint8_t* __restrict__ w, float* out, int N, int K,
                                                                        int slot_rows, int slots) {
     constexpr int BB = block_bytes(FMT), SEG = mma_seg(FMT), STRIDE = mma_stride(FMT);
     extern __shared__ __align__(16) uint8_t mma_smem[];     // digits [digit][block][32], scales; sums [2][warp][row]; barriers; slots
@@ -644,7 +644,7 @@ void launch_raw_matvec(const float* act, const void* w_blocks, float* out, int N
     const MmaShape q = ints ? mma_shape<FMT>(N, K, sms) : MmaShape{};
     if (q.rows > 0) {
         static std::atomic<bool> raised[kMaxDevices];
-        launch_raw(raw_block_mma_kernel<FMT>, raised, dev, std::min(sms, N), kMmaThreads, q.smem, stream, act, w, out, N, K, q.rows, q.slots);
+        launch_raw(raw_block_matvec_mma_kernel<FMT>, raised, dev, std::min(sms, N), kMmaThreads, q.smem, stream, act, w, out, N, K, q.rows, q.slots);
         return;
     }
     const RawShape p = raw_shape<FMT>(N, K, sms);

@@ -240,7 +240,7 @@ __device__ __forceinline__ void load_keys(const GateAttn& A, const AttnSmem<KT>&
 
 // acc[q][pair] += sum over keys [j0, j1) of the mixed weights times the raw keys, for the NQ queries in
 // sm.q at positions pos0 .. pos0 + NQ - 1.  Thread t owns elements 2 * (t + p * kAttnThreads) and the next of the
-// [heads][dim_s] output.  A score belongs to one thread, lanes over heads. 
+// [heads][dim_s] output.  A score belongs to one thread, lanes over heads.
 template <typename KT, int NQ, int EP>
 __device__ __forceinline__ void attend(const GateAttn& A, const AttnSmem<KT>& sm, int pos0, int j0, int j1, int tile,
                                        float (&acc)[NQ][EP][2]) {

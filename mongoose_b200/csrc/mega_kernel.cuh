@@ -1590,7 +1590,7 @@ __device__ __forceinline__ void mk_clear_next(const MegaArgs& a, long long* acc_
 // The new row is one more position, read from shared memory; a warp that does not merge appends it to the cache.
 // Rows fetched by the threads themselves, into registers before q arrives, cost the issue of every load (1.0 to 4.2 thousand
 // cycles a layer), a trip to DRAM that q did not hide (a token's weights push the cache out of L2) and a second for rows beyond
-// the registers; here q finds them in shared memory.  From q's arrival to the output, cycles before / now: 0.5B widths at 130
+// the registers; here q finds them in shared memory.  From the end of QKV to the output, cycles before / now: 0.5B widths at 130
 // positions 7200 / 4500, 1.1B at 300 13400 / 8500, 7B at 190 21300 / 7700.  B200, tokens after a prompt: 0.5B Q8_0 32 + 200
 // 82.0 -> 76.0 ms, 1.1B widths 512 + 512 99.0 -> 89.3, 7B widths 128 + 128 30.1 -> 27.6.
 // Where several CTAs share the head, each does this for its run of positions and the first of them
