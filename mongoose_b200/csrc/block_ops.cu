@@ -343,6 +343,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_matvec_mma_kernel(co
                     for (unsigned i = bytes; i < need; i += 2) *reinterpret_cast<unsigned short*>(to + i) = *reinterpret_cast<const unsigned short*>(src + i);
                 }
                 const unsigned all = __reduce_add_sync(MG_FULL_MASK, bytes);
+                __syncwarp();                               // the bytes that a lane stored itself are there before lane 0 arrives
                 if (lane == 0) bar_expect(full + s, all);
                 __syncwarp();
                 if (bytes)

@@ -43,6 +43,20 @@ def test_rows_and_segments(cuda, oracle, mglib, N, K_, off, fmt):
     assert np.all(np.abs(got - values @ x64) <= (9 + K_ / 1024) * 2.0 ** -24 * 2 * size + 2.0 ** -31 * (np.abs(values) @ top))
 
 
+# matrices that end 4, 12 and 8 bytes behind a multiple of 16: those bytes of the last row do not come with its copy
+@pytest.mark.parametrize("N,K_", [(593, 1088), (595, 1088), (593, 1152)])
+@pytest.mark.parametrize("fmt", [0, 1])
+def test_bytes_behind_the_last_whole_piece(cuda, oracle, mglib, N, K_, fmt):
+    blocks, x = quantized(oracle, fmt, N, K_, N)
+    other = quantized(oracle, fmt, N, K_, N + 1)[0]
+    x[:-32] = 0                                             # the last row's sum hangs on them
+    for b in (other, blocks, other, blocks):                # (shared memory holds the other matrix's)
+        got = product(cuda, fmt, b, x, N, K_)
+        values = oracle.dequant(fmt, b, N, K_).astype(np.float64)
+        size = np.abs(values) @ np.abs(x.astype(np.float64))
+        assert np.all(np.abs(got - values @ x.astype(np.float64)) <= 50 * 2.0 ** -24 * size + 2.0 ** -30 * np.abs(x).max() * np.abs(values[:, -32:]).sum(1))
+
+
 @pytest.mark.parametrize("fmt", [0, 1])
 @pytest.mark.parametrize("kind", ["inf", "two infs", "nan", "scale inf", "huge", "tiny", "zeros"])
 def test_numbers_off_the_range(cuda, oracle, mglib, fmt, kind):
