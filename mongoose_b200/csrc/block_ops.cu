@@ -204,10 +204,12 @@ __global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __re
 // ---------------- the same on the integer tensor path: matrices that keep every SM busy ----------------
 // Above, a lane converts every weight to fp32: about eight instructions per weight of a lane, and the issue slots are what
 // bounds a large product.  Here a warp multiplies 16 rows x one block of 32 columns by ONE mma.sync (m16n8k32, int8): A = the
-// quants as they lie in the block (4-bit ones as 16 (q - 8)), B = the activations as fixed point, four signed byte digits
-// in four of the eight columns.  A block's activations share a power of two, which puts the largest at 2^29 .. 2^30: an
-// element of 2^-6 of the largest or more is exact, a smaller one off by at most 2^-31 of the largest; the sums of a block
-// are exact integers, and fp32 only adds (block scale x power of two x sum) over the blocks, digit by digit.
+// quants as they lie in the block (4-bit ones as 16 (q - 8)), B = the activations as fixed point, two whole numbers of three signed byte
+// digits each in six of the eight columns.  A block's activations share a power of two, which puts the largest at 2^20 .. 2^21: the first number is what is
+// whole of that, the second what is left, in steps of 2^-22.  So the digits hold EVERY bit of an element that has 2^-19 of its block's largest or more.
+// A block with an element of which they do not is PLAIN (scale 0): multiplied in fp32 as the kernel above does; so is one that is not finite, lies
+// below 2^-82, where the product of its scales would not hold fp32's bits, or spans more than fp32's exponents.  A block's sums are integers of up
+// to 27 bits, which fp32 rounds once and adds (block scale x power of two x sum) over the blocks, one or two digits at a time.
 //   A CTA owns a contiguous run of rows, taken up to 32 at a time (one or two MMA tiles, which share the activations), and a row's
 // blocks in SEGMENTS of up to 128 (Q8_0: 64), 2 KB of every row.  A producer warp copies a segment (cp.async.bulk, a lane a row: the
 // 16-byte pieces that cover it) into a ring of slots; the 16 other warps share its blocks, and their sums over all
@@ -217,18 +219,21 @@ __global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __re
 // words of a row: the scale of the first and two of its quants share word 0, its last two and the scale of the second word 4 (8).
 // Lane t = 0 of a row completes its half word from there, so that no lane re-aligns what it loads: 2 (3) loads per
 // block and row where re-aligned words took 3 (5).  The activations of even blocks are staged in that order of elements.
-// B200, passes among others, the kernel above -> this one: Q4_0 3584 x 18944 26.9 -> 13.0 us (2.9 TB/s), 3584 x 3584 10.8 -> 4.4, 18944 x 3584
-// 24.2 -> 10.7; Q8_0 3584 x 18944 27.5 -> 17.0, 20000 x 19200 114 -> 75 (5.4 TB/s).  Error against 64 bits at 3584 x 18944 Q4_0 1.4e-7 -> 0.7e-7.
-//   A row whose sum is not finite is computed again in plain fp32 (activations or scales that are not, or sums beyond the range); so is one
-// below 2^-80 where a block of activations lies below 2^-96, whose digits would not hold fp32's.
+// B200, the kernel above -> this one, weights in no cache (the same matrix again and again): Q4_0 3584 x 18944 26.1 -> 15.0 us (25.8 -> 14.0), 3584 x 3584 11.0 -> 5.4,
+// 18944 x 3584 23.9 -> 12.9; Q8_0 3584 x 18944 27.2 -> 18.5, 18944 x 3584 26.1 -> 15.3, 9000 x 18944 51.2 -> 40.8.  Four digits, which keep 30 bits below the largest, took
+// 13.1, 4.8, 11.3, 17.6, 14.9 and 34.7, and lost what lies below: one large activation under a small weight took its block's other terms with it.  Where
+// every block is plain (activations e^(8 N(0, 1))): Q4_0 3584 x 18944 34 us, Q8_0 38, slower than above; N(0, 1) and gated inputs have a plain block in none to one of
+// twenty products.  Error against 64 bits at 3584 x 18944 Q4_0 1.4e-7 -> 0.7e-7.
+//   A row whose sum over digits is not finite (a scale that is not, sums beyond the range) is computed again in plain fp32.
 constexpr int kMmaWarps = 16, kMmaRows = 32, kMmaSlots = 4;
 constexpr int kMmaThreads = (kMmaWarps + 1) * 32;
 __host__ __device__ constexpr int mma_seg(int fmt) { return fmt == FMT_Q8_0 ? 32 : 64; }       // pairs
-__host__ __device__ constexpr int mma_stride(int fmt) { return 2 * mma_seg(fmt) * block_bytes(fmt) + 16; }
-static_assert(mma_stride(FMT_Q8_0) / 16 % 2 == 1 && mma_stride(FMT_Q4_0) / 16 % 2 == 1, "rows on different banks");
-__host__ __device__ constexpr int mma_digit_bytes(int nb) { return (nb * 32 + 127) / 128 * 128 + 32; }     // from digit to digit: the four on different banks
-__host__ __device__ constexpr size_t mma_input_bytes(int nb) { return (size_t)4 * mma_digit_bytes(nb) + ((size_t)nb * 4 + 15) / 16 * 16; }
-constexpr size_t kMmaSums = (size_t)2 * kMmaWarps * kMmaRows * 4, kMmaBars = 2 * kMmaSlots * 8 + 16;
+// From row to row of a slot: whole pieces that cover a row's part of a segment of `per` pairs, an odd number of them.
+__host__ __device__ constexpr int mma_stride(int fmt, int per) { return ((per * 2 * block_bytes(fmt) + 30) / 16 | 1) * 16; }
+constexpr int kMmaDigits = 6;
+__host__ __device__ constexpr int mma_digit_bytes(int nb) { return (nb * 32 + 127) / 128 * 128 + 32; }     // from digit to digit: four in turn on different banks
+__host__ __device__ constexpr size_t mma_input_bytes(int nb) { return (size_t)kMmaDigits * mma_digit_bytes(nb) + ((size_t)nb * 4 + 15) / 16 * 16; }
+constexpr size_t kMmaSums = (size_t)2 * kMmaWarps * kMmaRows * 4, kMmaBars = 2 * kMmaSlots * 8 + 16, kMmaFixed = kMmaSums + kMmaBars;
 
 // Re-computes one row; every lane returns it.
 template <int FMT>
@@ -249,9 +254,34 @@ __device__ __noinline__ float raw_row_plain(const float* __restrict__ act, const
     return warp_sum(acc);
 }
 
+// A row's block at `p` in shared memory, an even address, times its activations, of which lane i holds the i-th; in fp32.  Lanes are rows.
+template <int FMT>
+__device__ __noinline__ float mma_plain_block(uint32_t p, float x, float acc) {
+    constexpr int QW = FMT == FMT_Q8_0 ? 8 : 4;
+    auto word = [&](int i) {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"((p & ~3u) + 4 * i));
+        return v;
+    };
+    auto xi = [&](int i) { return __shfl_sync(MG_FULL_MASK, x, i); };
+    auto x4 = [&](int i) { return make_float4(xi(4 * i), xi(4 * i + 1), xi(4 * i + 2), xi(4 * i + 3)); };
+    const int sh = p & 2 ? 32 : 16;                         // quants start 2 bytes after the scale
+    uint32_t lo = word(0);
+    const float d = half_bits_to_float((unsigned short)(p & 2 ? lo >> 16 : lo & 0xffffu));
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < QW; i++) {
+        const uint32_t hi = word(i + 1), q = __funnelshift_rc(lo, hi, sh);
+        if (FMT == FMT_Q8_0) sum = dot4_s8(q, x4(i), sum);
+        else sum = dot4_u4(q >> 4 & 0x0f0f0f0fu, x4(4 + i), dot4_u4(q & 0x0f0f0f0fu, x4(i), sum));
+        lo = hi;
+    }
+    return fmaf(d, sum, acc);
+}
+
 // `n` pairs of blocks for NT tiles of 16 rows.  at: this lane's rows g + 8 r, offset of the first pair in shared memory; digits,
-// scales: of its first block.  Column 2 p of a product is digit p, which lane t = p receives.  acc: even and odd blocks, so that fewer
-// roundings follow one another.
+// scales: of its first block.  A lane t gets columns 2 t and 2 t + 1 of a product, two digits that follow one another, high and low.  acc: even and odd
+// blocks, so that fewer roundings follow one another.
 template <int FMT, int NT>
 __device__ __forceinline__ void mma_pairs(const uint8_t* smem, const uint32_t (&at)[2 * NT], int n, uint32_t digits, uint32_t scales, bool bvalid, int t,
                                           float (&acc)[2][4]) {
@@ -293,8 +323,8 @@ __device__ __forceinline__ void mma_pairs(const uint8_t* smem, const uint32_t (&
                 asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                     : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
                     : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(B[j].x), "r"(B[j].y), "r"(0));
-                acc[j][2 * i] = fmaf(d[j][2 * i] * s[j], __int2float_rn(c[0]), acc[j][2 * i]);         // |sum| <= 32 * 128 * 128: exact
-                acc[j][2 * i + 1] = fmaf(d[j][2 * i + 1] * s[j], __int2float_rn(c[2]), acc[j][2 * i + 1]);
+                acc[j][2 * i] = fmaf(d[j][2 * i] * s[j], __int2float_rn(c[0] * 256 + c[1]), acc[j][2 * i]);        // |c| <= 32 * 128 * 128
+                acc[j][2 * i + 1] = fmaf(d[j][2 * i + 1] * s[j], __int2float_rn(c[2] * 256 + c[3]), acc[j][2 * i + 1]);
             }
     }
 }
@@ -302,22 +332,23 @@ __device__ __forceinline__ void mma_pairs(const uint8_t* smem, const uint32_t (&
 // An even number of blocks, and a matrix on a 16-byte boundary.  slot_rows: rows taken at a time; slots: of the ring.
 template <int FMT>
 __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_matvec_mma_kernel(const float* __restrict__ act, const uint8_t* __restrict__ w, float* out, int N, int K,
-                                                                       int slot_rows, int slots) {
-    constexpr int BB = block_bytes(FMT), SEG = mma_seg(FMT), STRIDE = mma_stride(FMT);
+                                                                       int slot_rows, int slots, int per) {
+    constexpr int BB = block_bytes(FMT), SEG = mma_seg(FMT);
     extern __shared__ __align__(16) uint8_t mma_smem[];     // digits [digit][block][32], scales; sums [2][warp][row]; barriers; slots
-    const int nb = K / 32, np = nb / 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nb = K / 32, np = nb / 2, segs = (np + per - 1) / per, stride = mma_stride(FMT, per), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int digit_bytes = mma_digit_bytes(nb);
     const size_t rb = (size_t)nb * BB;
     float* part = reinterpret_cast<float*>(mma_smem + mma_input_bytes(nb));
     uint64_t* full = reinterpret_cast<uint64_t*>(mma_smem + mma_input_bytes(nb) + kMmaSums);
     uint64_t* empty = full + kMmaSlots;
-    int* status = reinterpret_cast<int*>(empty + kMmaSlots), *small = status + 1;      // small: a block below the digits' range
-    const uint32_t ring = (uint32_t)(mma_input_bytes(nb) + kMmaSums + kMmaBars), slot_bytes = (uint32_t)slot_rows * STRIDE;
+    int* status = reinterpret_cast<int*>(empty + kMmaSlots), *inputs_off = status + 1;    // inputs_off: an activation is not finite
+    unsigned* again = reinterpret_cast<unsigned*>(status + 2);     // [2] rows whose sum over digits is not finite
+    const uint32_t ring = (uint32_t)(mma_input_bytes(nb) + kMmaFixed), slot_bytes = (uint32_t)slot_rows * stride;
     const int row_lo = (int)((long long)N * blockIdx.x / gridDim.x), row_hi = (int)((long long)N * (blockIdx.x + 1) / gridDim.x);
-    const int segs = (np + SEG - 1) / SEG;
     if (threadIdx.x == 0) {
         for (int i = 0; i < slots; i++) { bar_init(full + i, 1); bar_init(empty + i, kMmaWarps); }
-        *status = *small = 0;
+        *status = *inputs_off = 0;
+        again[0] = again[1] = 0;
         bar_init_fence();
     }
     __syncthreads();
@@ -330,9 +361,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_matvec_mma_kernel(co
         for (int row0 = row_lo; ok && row0 < row_hi; row0 += slot_rows)
             for (int k = 0; k < segs; k++, n++) {
                 if (n >= slots && !(ok = __all_sync(MG_FULL_MASK, bar_wait(empty + s, par, status)))) break;
-                const int p0 = np * k / segs, p1 = np * (k + 1) / segs;
+                const int p0 = k * per, p1 = min(p0 + per, np);
                 const uint8_t* src = w;
-                uint8_t* to = mma_smem + ring + s * slot_bytes + lane * STRIDE;
+                uint8_t* to = mma_smem + ring + s * slot_bytes + lane * stride;
                 unsigned bytes = 0;
                 if (lane < min(slot_rows, row_hi - row0)) {
                     src += (size_t)(row0 + lane) * rb + (size_t)p0 * 2 * BB;
@@ -356,78 +387,119 @@ __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_matvec_mma_kernel(co
         return;
     }
 
-    // Activations.  A warp stages the blocks that it multiplies, with the rows it takes first: eight lanes share a block, lane e
-    // the elements that the MMA wants in word e, in even blocks 4 e - 2 .. 4 e + 1 (the first two from the end of the block, or of
-    // its half, where e begins it).  A segment's are on the way while the one before is multiplied.
-    constexpr int PART = FMT == FMT_Q8_0 ? 32 : 16, TURNS = SEG / kMmaWarps / 2;
-    static_assert(TURNS * 4 * kMmaWarps == 2 * SEG, "four blocks a turn");
-    const bool x8 = (reinterpret_cast<uintptr_t>(act) & 7) == 0;
-    float4 xs[TURNS];
-    auto load_x = [&](int k) {
-        const int p0 = np * k / segs, here = np * (k + 1) / segs - p0, lo = here * warp / kMmaWarps, n = here * (warp + 1) / kMmaWarps - lo;
-#pragma unroll
-        for (int j = 0; j < TURNS; j++) {
-            const int i = j * 32 + lane, own = (p0 + lo) * 64 + 4 * i;
-            const int other = i & 8 ? own + 2 : own % PART ? own - 2 : own + PART - 2, x0 = i & 8 ? own : other, x1 = i & 8 ? other : own;
-            xs[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < n * 16) {
-                if (x8) {
-                    const float2 u = *reinterpret_cast<const float2*>(act + x0), v = *reinterpret_cast<const float2*>(act + x1);
-                    xs[j] = make_float4(u.x, u.y, v.x, v.y);
-                } else {
-                    xs[j] = make_float4(act[x0], act[x0 + 1], act[x1], act[x1 + 1]);
-                }
-            }
-        }
+    // Activations.  A warp stages the blocks that it multiplies, with the rows it takes first, eight blocks at a time (Q8_0: of two segments): four
+    // lanes share a block, lane q the elements that the MMA wants in words q and q + 4, in even blocks 4 q - 2 .. 4 q + 1 and so on (the first two
+    // from the end of the block, or of its half, where q is 0).  The next ones are on the way meanwhile.
+    constexpr int PART = FMT == FMT_Q8_0 ? 32 : 16, OWN = 2 * SEG / kMmaWarps, AHEAD = 8 / OWN;     // OWN: blocks of a segment; AHEAD: segments
+    static_assert(OWN * AHEAD == 8 && AHEAD <= 2, "eight blocks");
+    const int q = lane & 3, sub = lane / (4 * OWN);
+    const bool odd = lane & 4, x8 = (reinterpret_cast<uintptr_t>(act) & 7) == 0;
+    const int col[4] = {odd ? 4 * q : q ? 4 * q - 2 : PART - 2, odd ? 4 * q + 2 : 4 * q, odd ? 4 * q + 16 : q || PART == 32 ? 4 * q + 14 : 30, odd ? 4 * q + 18 : 4 * q + 16};
+    float2 xs[4];                                           // elements col[i], col[i] + 1 of block xb (-1: none)
+    int xb;
+    auto share = [&](int k, int& lo) {                      // this warp's pairs of segment k: their number, the first
+        const int p0 = k * per, here = min(per, np - p0);
+        lo = here * warp / kMmaWarps;
+        return here * (warp + 1) / kMmaWarps - lo;
     };
-    auto store_x = [&](int first, int n) {                  // of the warp's n pairs from pair `first` on
+    auto load_x = [&](int k) {
+        int lo;
+        k += sub;
+        const int blk = lane / 4 % OWN, n = k < segs ? share(k, lo) : 0;
+        xb = blk < 2 * n ? (k * per + lo) * 2 + blk : -1;
+        const float* x = act + (size_t)max(xb, 0) * 32;
 #pragma unroll
-        for (int j = 0; j < TURNS; j++) {
-            const int i = j * 32 + lane, b = first * 2 + (i >> 3), e = lane & 7;
-            const float x[4] = {xs[j].x, xs[j].y, xs[j].z, xs[j].w};
-            unsigned m = max(max(__float_as_uint(fabsf(x[0])), __float_as_uint(fabsf(x[1]))), max(__float_as_uint(fabsf(x[2])), __float_as_uint(fabsf(x[3]))));
+        for (int i = 0; i < 4; i++)
+            xs[i] = xb < 0 ? make_float2(0.f, 0.f) : x8 ? *reinterpret_cast<const float2*>(x + col[i]) : make_float2(x[col[i]], x[col[i] + 1]);
+    };
+    bool plains = false;                                    // does one of this warp's blocks go without digits?
+    auto store_x = [&] {
+        auto bits = [](float v) { return __float_as_uint(fabsf(v)); };
+        uint32_t m = 0;
 #pragma unroll
-            for (int o = 1; o < 8; o *= 2) m = max(m, __shfl_xor_sync(MG_FULL_MASK, m, o));
-            if (m > 0 && m < 31u << 23) *small = 1;
-            m >>= 23;                                       // exponent of the largest
-            // times 2^(156 - m): the largest lies in 2^29 .. 2^30 (below 2^-96 the factor stays at 2^125)
-            const unsigned f = m < 31 ? 252u : m == 255 ? 0u : 283u - m;
-            const float up = __uint_as_float(f << 23);
-            // signed digits: byte p of v + 128 (1 + 256 + 65536), less 128 below the top one
-            uint32_t v[4];
+        for (int i = 0; i < 4; i++) m = max(m, max(bits(xs[i].x), bits(xs[i].y)));
 #pragma unroll
-            for (int k = 0; k < 4; k++) v[k] = (uint32_t)(__float2int_rn(x[k] * up) + 0x808080);
-            if (i < n * 16) {
-                const uint32_t u0 = __byte_perm(v[0], v[1], 0x5140), u1 = __byte_perm(v[2], v[3], 0x5140);     // bytes 0 and 1 of two
-                const uint32_t u2 = __byte_perm(v[0], v[1], 0x7362), u3 = __byte_perm(v[2], v[3], 0x7362);     // bytes 2 and 3
-                uint8_t* to = mma_smem + b * 32 + 8 * (e & 3) + 4 * (e >> 2);
-                *reinterpret_cast<uint32_t*>(to) = __byte_perm(u0, u1, 0x5410) ^ 0x80808080u;
-                *reinterpret_cast<uint32_t*>(to + digit_bytes) = __byte_perm(u0, u1, 0x7632) ^ 0x80808080u;
-                *reinterpret_cast<uint32_t*>(to + 2 * digit_bytes) = __byte_perm(u2, u3, 0x5410) ^ 0x80808080u;
-                *reinterpret_cast<uint32_t*>(to + 3 * digit_bytes) = __byte_perm(u2, u3, 0x7632);
-                if (e == 0) reinterpret_cast<float*>(mma_smem + 4 * digit_bytes)[b] = m == 255 ? __uint_as_float(0x7fc00000u) : __uint_as_float((254u - f) << 23);
+        for (int o = 1; o < 4; o *= 2) m = max(m, __shfl_xor_sync(MG_FULL_MASK, m, o));
+        bool plain = m - 1u < (45u << 23) - 1u || m >= 255u << 23;
+        const bool far = m >= 148u << 23;
+        m = max(m >> 23, 45u);                              // exponent of the largest
+        const float up = __uint_as_float((274u - m) << 23);
+        // whole numbers by additions that leave no place behind the point; the constant's low bytes make those of signed digits, xor 128
+        constexpr float kWhole = 12582912.0f + 32896.0f;
+        const unsigned long long up2 = pack2(up, up), whole = pack2(kWhole, kWhole), minus = pack2(-1.0f, -1.0f), more = pack2(4194304.0f, 4194304.0f);
+        uint32_t u[2][8], any = 0;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const unsigned long long x = pack2(xs[i].x, xs[i].y), a = fma2(x, up2, whole), left = fma2(x, up2, fma2(a, minus, whole));      // exact, as what follows
+            const unsigned long long b = fma2(left, more, whole), rest = fma2(left, more, fma2(b, minus, whole));
+            u[0][2 * i] = (uint32_t)b; u[0][2 * i + 1] = (uint32_t)(b >> 32);
+            u[1][2 * i] = (uint32_t)a; u[1][2 * i + 1] = (uint32_t)(a >> 32);
+            any |= (uint32_t)rest | (uint32_t)(rest >> 32);
+        }
+        if (xb >= 0) {
+            uint8_t* to = mma_smem + xb * 32 + 8 * q;
+#pragma unroll
+            for (int h = 0; h < 2; h++, to += 3 * digit_bytes) {
+                uint32_t lo[2], mid[2], hi[2];
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const uint32_t* a = u[h] + 4 * i;
+                    const uint32_t u0 = __byte_perm(a[0], a[1], 0x5140), u1 = __byte_perm(a[2], a[3], 0x5140);     // bytes 0 and 1 of two
+                    lo[i] = __byte_perm(u0, u1, 0x5410) ^ 0x80808080u;
+                    mid[i] = __byte_perm(u0, u1, 0x7632) ^ 0x80808080u;
+                    hi[i] = __byte_perm(__byte_perm(a[0], a[1], 0x0062), __byte_perm(a[2], a[3], 0x0062), 0x5410);     // each 64 more than the digit
+                    hi[i] = ((hi[i] | 0x80808080u) - 0x40404040u) ^ 0x80808080u;
+                }
+                *reinterpret_cast<uint2*>(to) = make_uint2(mid[0], mid[1]);
+                *reinterpret_cast<uint2*>(to + digit_bytes) = make_uint2(lo[0], lo[1]);
+                *reinterpret_cast<uint2*>(to + 2 * digit_bytes) = make_uint2(hi[0], hi[1]);
             }
         }
+        any &= 0x7fffffffu;
+        if (__any_sync(MG_FULL_MASK, any || far || plain)) {
+            // rests, and blocks beyond 2^21, where a product with `up` may leave fp32's exponents
+            bool off = any != 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) off |= far && ((xs[i].x != 0.f && fabsf(xs[i].x * up) < 0x1p-126f) || (xs[i].y != 0.f && fabsf(xs[i].y * up) < 0x1p-126f));
+            plain |= (__ballot_sync(MG_FULL_MASK, off) & 15u << (lane & 28)) != 0;          // the block's lanes
+            plains |= __any_sync(MG_FULL_MASK, plain);
+            if (m == 255) *inputs_off = 1;
+        }
+        if (xb >= 0 && q == 0) reinterpret_cast<float*>(mma_smem + kMmaDigits * digit_bytes)[xb] = plain ? 0.f : __uint_as_float((m - 20u) << 23);
         __syncwarp();
     };
     load_x(0);
 
     auto all_consumers = [] { asm volatile("bar.sync 1, %0;" ::"n"(kMmaWarps * 32) : "memory"); };
     const int g = lane >> 2, t = lane & 3;
-    const bool bvalid = (g & 1) == 0;
-    const float weight = (t == 0 ? 1.0f : t == 1 ? 256.0f : t == 2 ? 65536.0f : 16777216.0f) * (FMT == FMT_Q8_0 ? 1.0f : 0.0625f);
+    const int digit = g - (g > 2) - (g > 6);                // columns 2 and 6 are empty: a number's first digit has no lower one beside it
+    const bool bvalid = (g & 3) != 2;
+    const float weight = (t == 0 ? 0x1p-22f : t == 1 ? 0x1p-6f : t == 2 ? 1.0f : 65536.0f) * (FMT == FMT_Q8_0 ? 1.0f : 0.0625f);
     int s = 0, par = 0, buf = 0;
     for (int row0 = row_lo; row0 < row_hi; row0 += slot_rows, buf ^= 1) {
         const int rows = min(slot_rows, row_hi - row0);
-        float acc[2][4] = {};
+        float acc[2][4] = {}, plain = 0.f;                  // plain: what row `lane` has in fp32
         for (int k = 0; k < segs; k++) {
-            const int p0 = np * k / segs, here = np * (k + 1) / segs - p0, lo = here * warp / kMmaWarps, n = here * (warp + 1) / kMmaWarps - lo;
+            int lo;
+            const int n = share(k, lo), p0 = k * per;
             const uint32_t first = (uint32_t)reinterpret_cast<uintptr_t>(w) + (uint32_t)((size_t)row0 * rb + (size_t)p0 * 2 * BB);  // its low bits
-            const uint32_t from = ring + s * slot_bytes + lo * 2 * BB, digits = (p0 + lo) * 64 + (g >> 1) * digit_bytes + t * 8, sc = 4 * digit_bytes + (p0 + lo) * 8;
-            auto row_at = [&](int r) { return from + r * STRIDE + ((first + (uint32_t)r * (uint32_t)rb) & 15u); };
-            if (row0 == row_lo) {
-                store_x(p0 + lo, n);
-                if (k + 1 < segs) load_x(k + 1);
+            const uint32_t from = ring + s * slot_bytes + lo * 2 * BB, digits = (p0 + lo) * 64 + digit * digit_bytes + t * 8,
+                           sc = kMmaDigits * digit_bytes + (p0 + lo) * 8;
+            // (rows that a tile has and the slot has not: its last one again, dropped)
+            auto row_at = [&](int row) {
+                const uint32_t r = min(row, slot_rows - 1);
+                return from + r * stride + ((first + r * (uint32_t)rb) & 15u);
+            };
+            if (row0 == row_lo && k % AHEAD == 0) {
+                store_x();
+                if (k + AHEAD < segs) load_x(k + AHEAD);
+            }
+            unsigned off = 0;                               // blocks without digits, and their activations, a lane an element
+            float x_off[OWN];
+            if (plains) {
+                off = __ballot_sync(MG_FULL_MASK, lane < 2 * n && *reinterpret_cast<const float*>(mma_smem + sc + 4 * lane) == 0.f);
+#pragma unroll
+                for (int b = 0; b < OWN; b++) x_off[b] = off >> b & 1 ? act[(size_t)((p0 + lo) * 2 + b) * 32 + lane] : 0.f;
             }
             bar_wait(full + s, par, status);
             if (rows > 16) {
@@ -436,6 +508,11 @@ __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_matvec_mma_kernel(co
             } else {
                 const uint32_t at[2] = {row_at(g), row_at(g + 8)};
                 mma_pairs<FMT, 1>(mma_smem, at, n, digits, sc, bvalid, t, acc);
+            }
+            if (off) {
+#pragma unroll
+                for (int b = 0; b < OWN; b++)
+                    if (off >> b & 1) plain = mma_plain_block<FMT>(smem_addr(mma_smem) + row_at(lane) + b * BB, x_off[b], plain);
             }
             __syncwarp();
             if (lane == 0) bar_arrive(empty + s);
@@ -446,7 +523,14 @@ __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_matvec_mma_kernel(co
             float v = (acc[0][i] + acc[1][i]) * weight;
             v += __shfl_xor_sync(MG_FULL_MASK, v, 1);
             v += __shfl_xor_sync(MG_FULL_MASK, v, 2);
-            if (t == 0) part[(buf * kMmaWarps + warp) * kMmaRows + g + 8 * i] = v;
+            if (t == 0) {
+                part[(buf * kMmaWarps + warp) * kMmaRows + g + 8 * i] = v;
+                if (!(fabsf(v) <= 3.402823466e38f)) atomicOr(again + buf, 1u << (g + 8 * i));
+            }
+        }
+        if (plains) {
+            __syncwarp();
+            part[(buf * kMmaWarps + warp) * kMmaRows + lane] += plain;
         }
         all_consumers();                                    // (two buffers: a sum is read while the next rows are multiplied)
         if (warp == 0) {
@@ -458,11 +542,13 @@ __global__ void __launch_bounds__(kMmaThreads, 1) raw_block_matvec_mma_kernel(co
 #pragma unroll
                 for (int p = 0; p < h; p++) u[p] += u[p + h];
             float v = u[0];
-            const bool plain = lane < rows && (!(fabsf(v) <= 3.402823466e38f) || (*small && fabsf(v) < 0x1p-80f));
-            for (unsigned left = __ballot_sync(MG_FULL_MASK, plain); left; left &= left - 1) {
+            const bool off = lane < rows && ((again[buf] >> lane & 1) || (!(fabsf(v) <= 3.402823466e38f) && !*inputs_off));
+            __syncwarp();
+            if (lane == 0) again[buf] = 0;
+            for (unsigned left = __ballot_sync(MG_FULL_MASK, off); left; left &= left - 1) {
                 const int r = __ffs(left) - 1;
-                const float again = raw_row_plain<FMT>(act, w + (size_t)(row0 + r) * rb, nb);
-                if (lane == r) v = again;
+                const float sum = raw_row_plain<FMT>(act, w + (size_t)(row0 + r) * rb, nb);
+                if (lane == r) v = sum;
             }
             if (*reinterpret_cast<volatile int*>(status)) v = __uint_as_float(0x7fc00000u);     // a copy never came
             if (lane < rows) out[row0 + lane] = v;
@@ -608,19 +694,26 @@ void run_raw_matvec(const RawShape& p, int dev, const float* act, const uint8_t*
     launch_raw(raw_block_matvec_kernel<FMT, R, V, X>, raised, dev, p.grid, p.threads, p.smem, stream, act, w, out, N, K, p.ks);
 }
 
-// Rows a CTA of the integer kernel takes at a time, 32, 16 or all it has, and slots of its ring; no rows: shared memory holds no two slots.
+// Rows a CTA of the integer kernel takes at a time, slots of its ring, and pairs of a segment; no rows: shared memory holds no two slots.  Two tiles of
+// rows at a time (as even as may be) where that takes no more than a third more segments than there may be fewest, else one.  B200, us of Q8_0 / Q4_0, two
+// tiles in so many segments, one tile: 9000 x 18944 40.8 in 12, 40.9 in 10 / 30.9 in 7, 29.0 in 5; 3584 x 24576 28.3 in 18, 28.7 in 12 / 21.8 in 10, 21.4 in 6;
+// 2400 x 26624 24.4 in 17, 25.5 in 13 / 20.4 in 9, 21.8 in 7.
 struct MmaShape {
-    int rows, slots;
+    int rows, slots, per;
     size_t smem;
 };
 template <int FMT>
 MmaShape mma_shape(int N, int K, int sms) {
-    const size_t fixed = mma_input_bytes(K / 32) + kMmaSums + kMmaBars;
-    for (int rows = std::min(kMmaRows, cdiv(N, sms)); rows > 0; rows = rows > 16 ? 16 : 0) {
-        // (behind the last slot: rows that a tile of 16 has and the slot has not are read, and dropped)
-        const size_t slot = (size_t)rows * mma_stride(FMT), spare = (size_t)kMmaRows * mma_stride(FMT) - slot;
-        for (int slots = kMmaSlots; slots >= 2; slots--)
-            if (fixed + slots * slot + spare <= kRawSmem) return {rows, slots, fixed + slots * slot + spare};
+    const int pairs = K / 64, most = cdiv(N, sms), least = cdiv(pairs, mma_seg(FMT));
+    const size_t fixed = mma_input_bytes(K / 32) + kMmaFixed;
+    for (int tiles = 2; tiles > 0; tiles--) {
+        const int rows = cdiv(most, cdiv(most, 16 * tiles));
+        for (int segs = least; 3 * segs <= 4 * least; segs++) {
+            const int per = cdiv(pairs, segs);
+            const size_t slot = (size_t)rows * mma_stride(FMT, per);
+            for (int slots = kMmaSlots; slots >= 2; slots--)
+                if (fixed + slots * slot <= kRawSmem) return {rows, slots, per, fixed + slots * slot};
+        }
     }
     return {};
 }
@@ -638,14 +731,19 @@ void launch_raw_matvec(const float* act, const void* w_blocks, float* out, int N
         if (dev < kMaxDevices) sm_count[dev].store(sms, std::memory_order_relaxed);
     }
     const uint8_t* w = static_cast<const uint8_t*>(w_blocks);
-    // The integer kernel, us of Q8_0 / Q4_0, the other -> this: 1024 columns 20000 rows 8.6 -> 9.2 / 8.5 -> 9.4, 7200 rows 4.5 -> 4.8 / 5.0 -> 4.9;
-    // 1536 columns 20000 rows 14.4 -> 9.5 / 13.5 -> 9.8; 8192 columns 300 rows 4.4 -> 5.9 / 4.0 -> 5.0, 600 rows 6.0 -> 5.9 / 5.6 -> 5.1; 24576
-    // columns 900 rows 12.7 -> 13.7 / 12.0 -> 11.3, 1200 rows 21.7 -> 13.7 / 20.3 -> 11.3 (every CTA stages the whole input).
-    const bool ints = K > 1024 && K % 64 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && N >= (K > 20480 ? 8 : 4) * sms;
+    // The integer kernel, us of Q8_0 / Q4_0 on weights in no cache, the other -> this: 1088 columns 600 rows 3.43 -> 3.20 / 3.16 -> 3.22, 18944 rows 13.4 -> 9.2 / 12.6 ->
+    // 9.4; 4864 columns 800 rows 4.4 -> 5.2 / 5.2 -> 4.9, 1200 rows 6.1 -> 5.4 / 8.0 -> 5.1; 8192
+    // columns 600 rows 6.3 -> 6.0 / 7.8 -> 5.4; 18944 columns 800 rows 11.0 -> 11.6 / 14.7 -> 10.6, 1200 rows 17.6 -> 11.8 / 23.3 -> 10.6; 24576 columns 1200 rows 21.3
+    // -> 14.3 / 20.0 -> 12.5.  Every CTA stages the whole input, so few rows do not pay for it.  Q8_0 of four to eight rows per SM: 3072 columns 4.4 to 5.1 -> 4.0 to 4.2,
+    // 5120 columns 600 rows 4.3 -> 5.0, 1000 rows 6.1 -> 5.3, 6144 columns (the other kernel has one CTA per SM from 5472 on) 6.2 to 6.6 -> 5.3 to 5.6, 12288 columns
+    // 8.5 to 11.1 -> 8.0 to 8.4 (at 1180 rows 7.9), 14336 columns 8.6 to 8.9 -> 9.4 to 9.7.
+    const int r = N / sms;
+    const bool enough = r >= 8 || (r >= 4 && (FMT == FMT_Q4_0 ? K <= 20480 : K <= 3072 || (K <= 12288 && (r >= 6 || K > 5440))));
+    const bool ints = K > 1024 && K % 64 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 && enough;
     const MmaShape q = ints ? mma_shape<FMT>(N, K, sms) : MmaShape{};
     if (q.rows > 0) {
         static std::atomic<bool> raised[kMaxDevices];
-        launch_raw(raw_block_matvec_mma_kernel<FMT>, raised, dev, std::min(sms, N), kMmaThreads, q.smem, stream, act, w, out, N, K, q.rows, q.slots);
+        launch_raw(raw_block_matvec_mma_kernel<FMT>, raised, dev, std::min(sms, N), kMmaThreads, q.smem, stream, act, w, out, N, K, q.rows, q.slots, q.per);
         return;
     }
     const RawShape p = raw_shape<FMT>(N, K, sms);

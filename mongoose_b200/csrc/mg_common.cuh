@@ -67,6 +67,23 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return red[32];
 }
 
+// Two fp32 operations at once.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ float lo(unsigned long long v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
+
 // ---------------------------------------------------------------------
 // int8 -> fp32 without the conversion pipe: a byte placed in the low
 // mantissa of 2^23 reads as 8388608 + u; with u = q xor 0x80 (= q + 128)
