@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kStepThreads) mixer_step_kernel(const MixerSte
         cp_async_wait<1>();
         KT* K = sm.k + (size_t)buf * a.tile * row;
         float* R = sm.r + buf * a.tile * KV;
-        if (pos >= j && pos < j + tile) {           // (the rows of the copies end before it)
+        if (j1 == len && pos < j + tile) {          // the new key is this CTA's, and in this tile (the rows of the copies end before it)
             __syncthreads();
             KT* to = K + (size_t)(pos - j) * row;
             for (int i = tid; i < KV * DS; i += kStepThreads) to[i / DS * sm.ks + i % DS] = knew[i];
