@@ -96,6 +96,13 @@ inline size_t step_key(const GateAttn& A, size_t kt_bytes) { return (size_t)A.kv
 // reaches the CTA that ends with it through shared memory, not through the cache.  B200, 1.1B widths, 320 positions, us from the
 // wait to the end of this kernel: 9.2 with 256 threads, a thread per score, eight lanes per norm and tiles of eight keys, 4.3 now;
 // 300 + 64 tokens of six layers 18.20 -> 16.92 ms.  Runs of eight keys per CTA: 17.17 ms.
+//   Many keys per CTA (the memory leaves 84 CTAs at 1.1B widths) are bound by instructions instead: a tile holds the range, up to 16 keys, and from
+// 192 scores on a lane has one for itself.  us per token, tiles of eight and four lanes per score -> now: six layers of 1.1B widths at 300, 700, 1200, 2000 and 4500
+// positions 238.5, 249.8, 278.9, 308.2, 370.5 -> 239.3, 240.7, 243.1, 255.2, 276.0; two of 7B widths at 300, 2000 and 4500 221.3, 242.2, 266.9 -> 221.1, 231.4, 248.8;
+// four of 0.5B at 330, 2000 and 7000 144.3, 154.8, 209.2 -> 143.8, 145.5, 182.7.  (A thread per score on 256 threads, tiles of eight: four layers of 1.1B 182.3 at
+// 300, 211.1 at 2000, where four lanes per score took 214.7.)  Tiles of 32 take 251.2 at 2000 and 171.2 at 7000, and 240.4 at 300, where nothing but the shared memory differs.
+// From 256 or 128 scores on: 243.7 or 240.4 at 700, else the same.
+constexpr int kStepTile = 16, kStepShared = 192;        // keys of a tile; scores of one that four lanes each share
 template <typename KT, int EP>
 __global__ void __launch_bounds__(kStepThreads) mixer_step_kernel(const MixerStep a) {
     extern __shared__ __align__(16) float smem[];
@@ -134,7 +141,9 @@ __global__ void __launch_bounds__(kStepThreads) mixer_step_kernel(const MixerSte
         cp_async_wait<0>();
         return;
     }
-    const int tile = j1 - j0 <= a.grain ? a.grain : a.tile, tsh = 31 - __clz(tile);      // powers of two
+    int tile = a.grain;                             // a power of two
+    while (tile < j1 - j0 && tile < a.tile) tile *= 2;
+    const int tsh = 31 - __clz(tile);
     float* rnew = sm.slope + A.heads;
     KT* knew = a.key_copy ? reinterpret_cast<KT*>((reinterpret_cast<uintptr_t>(rnew + A.kv_heads) + 15) & ~(uintptr_t)15)
                           : static_cast<KT*>(A.cache) + (size_t)pos * A.kv_heads * A.dim_s;
@@ -187,7 +196,6 @@ __global__ void __launch_bounds__(kStepThreads) mixer_step_kernel(const MixerSte
     float2 acc[EP];
 #pragma unroll
     for (int e = 0; e < EP; e++) acc[e] = make_float2(0.f, 0.f);
-    const int sub = lane & 3;
     const unsigned quad = 0xfu << (lane & 28);
     int buf = 0;
     for (int j = j0; j < j1; j += tile, buf ^= 1) {
@@ -203,44 +211,67 @@ __global__ void __launch_bounds__(kStepThreads) mixer_step_kernel(const MixerSte
             for (int i = tid; i < KV; i += kStepThreads) R[(pos - j) * KV + i] = rnew[i];
         }
         __syncthreads();
-        const int keys = min(tile, j1 - j), units = H << tsh;
-        for (int u = tid >> 2; u < units; u += kStepThreads / 4) {
-            const int h = u >> tsh, p = u & (tile - 1), c = h / group;
-            const KT* kp = K + p * row + c * sm.ks;
-            const float* qp = sm.q + h * sm.qs;
-            float d0 = 0.f, d1 = 0.f;
-#pragma unroll 2
-            for (int ch = sub; ch < chunks; ch += 4) {
-                float kk[CN];
-                Chunk16<KT>::load(kp + ch * CN, kk);
-#pragma unroll
-                for (int i = 0; i < CN; i += 4) {
-                    const float4 v = *reinterpret_cast<const float4*>(qp + ch * CN + i);
-                    d0 = fmaf(kk[i], v.x, d0);
-                    d1 = fmaf(kk[i + 1], v.y, d1);
-                    d0 = fmaf(kk[i + 2], v.z, d0);
-                    d1 = fmaf(kk[i + 3], v.w, d1);
+        const int keys = min(tile, j1 - j);
+        // every head and key: four lanes for each, lanes over the tile's rows, or one, lanes over heads
+        auto each = [&](auto lanes, auto unit) {
+            if constexpr (lanes == 4) {
+                for (int u = tid >> 2; u < H << tsh; u += kStepThreads / 4) unit(u >> tsh, u & (tile - 1));
+            } else {
+                const int p_step = kStepThreads / H, h_step = kStepThreads - p_step * H;
+                for (int p = tid / H, h = tid % H; p < keys;) {
+                    unit(h, p);
+                    p += p_step;
+                    h += h_step;
+                    if (h >= H) { h -= H; p++; }
                 }
             }
-            d0 += d1;
-            d0 += __shfl_xor_sync(quad, d0, 1);
-            d0 += __shfl_xor_sync(quad, d0, 2);
-            if (sub == 0) {
-                const float s = d0 * (p < keys ? R[p * KV + c] : 0.f) - sm.slope[h] * (float)(pos - (j + p)) + sm.bias[h];
-                sm.w[h * sm.ws + p] = p < keys ? sigmoid(s) : 0.f;
-            }
-        }
-        __syncthreads();
-        for (int u = tid >> 2; u < units; u += kStepThreads / 4) {
-            const int h = u >> tsh, p = u & (tile - 1);
-            const float* t = sm.talk + h * sm.ts;
-            float v = 0.f;
+        };
+        auto weights = [&](auto lanes) {
+            constexpr int LANES = lanes;
+            const int sub = LANES == 4 ? lane & 3 : 0;
+            auto total = [&](float v) {
+                if (LANES == 4) {
+                    v += __shfl_xor_sync(quad, v, 1);
+                    v += __shfl_xor_sync(quad, v, 2);
+                }
+                return v;
+            };
+            each(lanes, [&](int h, int p) {
+                const int c = h / group;
+                const KT* kp = K + p * row + c * sm.ks;
+                const float* qp = sm.q + h * sm.qs;
+                float d0 = 0.f, d1 = 0.f;
+#pragma unroll 2
+                for (int ch = sub; ch < chunks; ch += LANES) {
+                    float kk[CN];
+                    Chunk16<KT>::load(kp + ch * CN, kk);
+#pragma unroll
+                    for (int i = 0; i < CN; i += 4) {
+                        const float4 v = *reinterpret_cast<const float4*>(qp + ch * CN + i);
+                        d0 = fmaf(kk[i], v.x, d0);
+                        d1 = fmaf(kk[i + 1], v.y, d1);
+                        d0 = fmaf(kk[i + 2], v.z, d0);
+                        d1 = fmaf(kk[i + 3], v.w, d1);
+                    }
+                }
+                d0 = total(d0 + d1);
+                if (sub == 0) {
+                    const float z = d0 * (p < keys ? R[p * KV + c] : 0.f) - sm.slope[h] * (float)(pos - (j + p)) + sm.bias[h];
+                    sm.w[h * sm.ws + p] = p < keys ? sigmoid(z) : 0.f;
+                }
+            });
+            __syncthreads();
+            each(lanes, [&](int h, int p) {
+                const float* t = sm.talk + h * sm.ts;
+                float v = 0.f;
 #pragma unroll 8
-            for (int g = sub; g < H; g += 4) v = fmaf(t[g], sm.w[g * sm.ws + p], v);
-            v += __shfl_xor_sync(quad, v, 1);
-            v += __shfl_xor_sync(quad, v, 2);
-            if (sub == 0) sm.mix[h * sm.ws + p] = v;
-        }
+                for (int g = sub; g < H; g += LANES) v = fmaf(t[g], sm.w[g * sm.ws + p], v);
+                v = total(v);
+                if (sub == 0) sm.mix[h * sm.ws + p] = v;
+            });
+        };
+        if (H << tsh <= kStepShared) weights(std::integral_constant<int, 4>{});
+        else weights(std::integral_constant<int, 1>{});
         __syncthreads();
 #pragma unroll
         for (int e = 0; e < EP; e++)
@@ -399,7 +430,7 @@ cudaError_t launch_rows_parts(const PhaseArgs& a, PhaseParts& p, int sms, bool p
 
 size_t mixer_step_smem(const GateAttn& at, const MatMem& mem, bool f32_cache, int* tile) {
     const size_t need_mem = (40 + kStepThreads + 2 * (size_t)mem.dim) * sizeof(float);
-    size_t need = attn_smem(at, 1, f32_cache ? 4 : 2, 8, tile);
+    size_t need = attn_smem(at, 1, f32_cache ? 4 : 2, kStepTile, tile);
     if (need == 0) return 0;
     need += step_extra(at);
     if (const size_t key = step_key(at, f32_cache ? 4 : 2); need + key <= kModelSmem) need += key;
@@ -410,7 +441,7 @@ cudaError_t launch_mixer_step(const MixerStep& a, bool f32_cache, bool pdl, cuda
     MixerStep b = a;
     int tile;
     const size_t smem = mixer_step_smem(a.at, a.mem, f32_cache, &tile), kt = f32_cache ? 4 : 2;
-    b.key_copy = smem >= attn_smem(a.at, 1, (int)kt, 8, &tile) + step_extra(a.at) + step_key(a.at, kt);
+    b.key_copy = smem >= attn_smem(a.at, 1, (int)kt, kStepTile, &tile) + step_extra(a.at) + step_key(a.at, kt);
     return f32_cache ? step_for<float>(b, smem, pdl, s) : step_for<__nv_bfloat16>(b, smem, pdl, s);
 }
 
