@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __re
 // 16-byte pieces that cover it) into a ring of slots; the 16 other warps share its blocks, and their sums over all
 // segments meet in shared memory.  Rows lie an odd multiple of 16 bytes apart in a slot, so that the eight rows of an access
 // fall on different banks.  (Copies by the warps themselves, ten pieces of 16 bytes per row and turn with cp.async, took half the time.)
-//   What bounds it is the number of loads from shared memory, one per two cycles and SM.  Blocks are taken in PAIRS, 9 (17) aligned
+//   What bounds it is instruction issue (66 % of the slots of a launch by itself, Q4_0 3584 x 18944, 53 % of the ALU's; shared memory 26 %), and in front
+// of the first rows the staging of the whole input by every CTA.  Blocks are taken in PAIRS, 9 (17) aligned
 // words of a row: the scale of the first and two of its quants share word 0, its last two and the scale of the second word 4 (8).
 // Lane t = 0 of a row completes its half word from there, so that no lane re-aligns what it loads: 2 (3) loads per
 // block and row where re-aligned words took 3 (5).  The activations of even blocks are staged in that order of elements.
@@ -632,8 +633,7 @@ int static_fail(int code, const char* fmt, int a, int b) {
 // from 27872 columns on (39648 where rows are single anyway), Q4_0 from 38784 (45120); beyond 51200 (54272) the
 // activations stay in global memory.
 // Measured on B200, weights in no cache, activations read from global memory / from such slices: Q8_0 8192 x 28672 573 / 74 us, 8192 x
-// 40960 817 / 112 us, 256 x 32768 99 / 7 us.  Elsewhere: 4864 x 896 Q8_0 4.7 us (the launch), 18944 x 3584 Q8_0 27 us = 2.7 TB/s;
-// at 18944 columns of Q8_0, 2368 rows 17 us (two warps a pair), 2400 to 4736 rows 27 to 29 us (the walk of one warp over its pair).
+// 40960 817 / 112 us, 256 x 32768 99 / 7 us.  Elsewhere: 4864 x 896 Q8_0 4.4 us, 3584 x 36864 51.5, 600 x 18944 10.8 (what the integer kernel takes: there).
 struct RawShape {
     int grid, threads, ks, input;
     bool pairs;

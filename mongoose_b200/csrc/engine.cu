@@ -832,8 +832,9 @@ bool mega_feasible(mg_engine* e, std::string* why) {
         e->mk_geom[p] = choose_geom(s.fmt, s.K, s.items, s.rpi, G, MK_NW, slot, p == PH_HEAD, fw, fs);
         if (e->mk_geom[p].nkt == 0) { *why = "no tile layout for a phase"; return false; }
         if (p == PH_QKV) {
-            // Leave the CTAs that run attention without QKV rows where the busiest CTA gets no more rows
-            // for it: they then fetch their cached K/V rows while the others multiply.  MG_QKV_ALL=1 keeps them in.
+            // Leave the CTAs that run attention without QKV rows where the busiest CTA gets no more rows for it: their rings then
+            // hold cached rows instead of QKV's weights.  us per token without / with QKV rows: four layers of 1.1B widths 111.0 / 114.1 at 64
+            // positions, 125.3 / 127.5 at 1000; 0.5B widths the same.  MG_QKV_ALL=1 keeps them in.
             const int sh = e->mk_geom[p].ipg_shift, units = (s.items + (1 << sh) - 1) >> sh, rest = G - c.n_heads;
             const char* all = getenv("MG_QKV_ALL");
             e->mk_qkv_cta0 = (rest > 0 && !(all && all[0] == '1') && (units + rest - 1) / rest == (units + G - 1) / G) ? c.n_heads : 0;

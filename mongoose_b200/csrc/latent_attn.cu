@@ -94,8 +94,9 @@ __global__ void __launch_bounds__(kThreads) latent_query_kernel(const LatentStep
 
 // ---- attention over a range of cached rows ----
 // Rows are dealt to the CTAs in runs of a multiple of kGrain, or of a tile where that is less: at a few hundred positions a tile of
-// sixteen rows kept 21 of 148 CTAs busy for 17 us.  300 + 64 tokens of Kuzipel 1.1B, six layers: 22.63 -> 22.21 ms with runs of four rows, 22.23
-// with eight.
+// sixteen rows kept 21 of 148 CTAs busy for 17 us.  us per token with runs of 4 / 8 / 16 rows: Kuzipel 1.1B, three layers, at 20 positions 216.2 / 218.3 / 222.2, 300
+// 219.4 / 219.7 / 222.7, 1200 226.4 / 225.3 / 225.4, 4000 239.7 / 239.0 / 239.0; 0.5B at 20 178.1 / 179.6 / 181.6, 4000 194.2 / 193.5 / 193.6; 7B widths at 300 444.1 / 441.1 / 442.1,
+// 4000 479.4 / 479.4 / 478.8.
 constexpr int kGrain = 4;
 // Shared memory: rows [2][tile][row + 16 bytes], queries [group][row + 4], weights [tile][group4], then per head
 // the running maximum, sum and this tile's correction.

@@ -95,7 +95,9 @@ inline size_t step_key(const GateAttn& A, size_t kt_bytes) { return (size_t)A.kv
 // everything that no predecessor leaves (cached keys, tables, the norms' weights, addresses) is there before the wait; the new key
 // reaches the CTA that ends with it through shared memory, not through the cache.  B200, 1.1B widths, 320 positions, us from the
 // wait to the end of this kernel: 9.2 with 256 threads, a thread per score, eight lanes per norm and tiles of eight keys, 4.3 now;
-// 300 + 64 tokens of six layers 18.20 -> 16.92 ms.  Runs of eight keys per CTA: 17.17 ms.
+// 300 + 64 tokens of six layers 18.20 -> 16.92 ms.  Runs of 4 / 8 keys per CTA, us per token of the kernel as it is: four layers of 1.1B widths at 20
+// positions 162.4 / 161.6, 300 169.6 / 165.6 (a lane per score), 1200 171.9 / 171.4, 4000 192.8 / 194.1; 0.5B 143.0 / 141.8, 143.3 / 147.4, 147.9 / 145.8, 160.9 / 161.0;
+// two of 7B widths at 300 220.9 / 220.6, 4000 245.9 / 246.7.
 //   Many keys per CTA (the memory leaves 84 CTAs at 1.1B widths) are bound by instructions instead: a tile holds the range, up to 16 keys, and from
 // 192 scores on a lane has one for itself.  us per token, tiles of eight and four lanes per score -> now: six layers of 1.1B widths at 300, 700, 1200, 2000 and 4500
 // positions 238.5, 249.8, 278.9, 308.2, 370.5 -> 239.3, 240.7, 243.1, 255.2, 276.0; two of 7B widths at 300, 2000 and 4500 221.3, 242.2, 266.9 -> 221.1, 231.4, 248.8;

@@ -124,7 +124,7 @@ struct MegaArgs {
     int xs_floats;          // size of the staged-activation buffer (multiple of 4)
     long long wait_cycles;  // limit of every wait inside the kernel, in SM clocks
     PhaseGeom geom[5];
-    int sc_floats;          // attention score buffer: max_seq rounded up to a multiple of 4
+    int sc_floats;          // attention score buffer: max_seq rounded up to a multiple of 8 (attention reads and writes whole blocks of eight)
     // weight tape
     const uint8_t* tape;
     const unsigned long long* tape_off;   // [grid][n_layers*4 + 2]
@@ -169,7 +169,7 @@ struct MegaArgs {
     int ffn_fused;
     int acc_buf0;           // accumulator (0..2) of this launch's first layer
     int qkv_cta0;           // the QKV rows are dealt to CTAs qkv_cta0 .. grid-1 (n_heads where that keeps the balance: the
-                            // CTAs that run attention then load their cached K/V rows while the others multiply)
+                            // rings of the CTAs that run attention then hold cached rows instead of QKV's weights)
     int acc_n;              // additions that complete a word: the CTAs that own gate/up rows + 1 (the residual)
     long long* acc;         // [3][dim]
 };
@@ -564,7 +564,8 @@ __device__ __forceinline__ float mk_block_sum(MkCtx& c, float v) {
 // one CTA a head / with 480 positions per CTA: six layers of 1.1B widths at 600 positions 164.3 / 164.0, 750 167.5 / 165.4, 1050
 // 176.3 / 170.7, 1300 182.0 / 172.6; six of 0.5B widths 600 127.4 / 129.8, 800 134.9 / 131.9, 1300 144.8 / 134.9; two of 7B widths
 // (head_dim 128) 900 219.6 / 226.7, 1300 225.5 / 228.2, on a slope of 1.5 per 100.  Runs of 120, 160, 240 and 360 positions
-// cost more at every length.
+// cost more at every length.  With these limits: two of 7B widths 1350 225.2, 1500 (shared) 227.6, 2000 232.9; heads of 32, which take the line of 64, six
+// of 0.5B widths with 28 heads 500 119.1, 700 125.9, 900 (shared) 128.4.
 constexpr int MK_SPLIT_POSITIONS = 480;
 constexpr int MK_MAX_SPLITS = 5;
 __host__ __device__ inline int mk_split_from(int head_dim) { return head_dim > 64 ? 1440 : 720; }
@@ -1590,9 +1591,9 @@ __device__ __forceinline__ void mk_clear_next(const MegaArgs& a, long long* acc_
 // The new row is one more position, read from shared memory; a warp that does not merge appends it to the cache.
 // Rows fetched by the threads themselves, into registers before q arrives, cost the issue of every load (1.0 to 4.2 thousand
 // cycles a layer), a trip to DRAM that q did not hide (a token's weights push the cache out of L2) and a second for rows beyond
-// the registers; here q finds them in shared memory.  From the end of QKV to the output, cycles before / now: 0.5B widths at 130
-// positions 7200 / 4500, 1.1B at 300 13400 / 8500, 7B at 190 21300 / 7700.  B200, tokens after a prompt: 0.5B Q8_0 32 + 200
-// 82.0 -> 76.0 ms, 1.1B widths 512 + 512 99.0 -> 89.3, 7B widths 128 + 128 30.1 -> 27.6.
+// the registers; here q finds them in shared memory.  From the CTA's last QKV row to the output (mg_trace_step), cycles before / now: 0.5B
+// widths at 130 positions 7000 / 5000, 1.1B at 300 14700 / 9100, 7B at 190 19400 / 8300; a layer 29500 / 26500, 46800 / 40000 and 117400 / 105100.
+// B200, tokens after a prompt: 0.5B Q8_0 32 + 200 81.5 -> 74.7 ms, 1.1B widths 512 + 512 99.0 -> 89.3, 7B widths 128 + 128 30.8 -> 28.7.
 // Where several CTAs share the head, each does this for its run of positions and the first of them
 // collects the others' outputs, maxima and sums.  Positions below are relative to the run.
 // ---------------------------------------------------------------------

@@ -1,10 +1,8 @@
-"""Decode attention beyond the positions the kernels keep in registers.
+"""Decode attention over more than one entry of the weight ring.
 
-The persistent kernel's attention holds the first cached K rows (480 positions for head_dim 32 / 64,
-240 for head_dim 128) and V rows (240 positions) in registers and takes longer contexts from L2 in
-separate loops; the benchmark configurations run to 1024 (TinyLlama) and 384 (7B-class) positions.
-Here small models with those head sizes are decoded past 500 positions and the logits are compared
-with the CPU oracle, which replays the engine's own tokens.
+The persistent kernel's attention gets its cached K and V rows through the ring, 480, 240 or 120 rows an entry (head_dim 32, 64, 128);
+the benchmark configurations run to 1024 (TinyLlama) and 384 (7B-class) positions.  Here small models with those head sizes
+are decoded past 500 positions and the logits are compared with the CPU oracle, which replays the engine's own tokens.
 """
 import numpy as np
 import pytest
@@ -35,8 +33,7 @@ def test_logits_beyond_500_positions(cuda, oracle, mglib, monkeypatch, cfg, kern
         n_prompt, n_new = 8, 540
         prompt = gen.prompt_ids(4, n_prompt, cfg.vocab)
         toks = eng.Generate(prompt, n_new)
-        # teacher-forced replay on the oracle; logits are checked at positions around and past every
-        # boundary of the register-held part (240, 480) and at the end
+        # teacher-forced replay on the oracle; logits are checked at positions around ends of entries (240, 480) and at the end
         check = {100, 239, 240, 241, 300, 479, 480, 481, 500, n_prompt + n_new - 2}
         logits = np.empty(cfg.vocab, np.float32)
         seq = list(prompt) + [int(x) for x in toks]
