@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(512) raw_block_matvec_kernel(const float* __re
 // B200, the kernel above -> this one, weights in no cache (the same matrix again and again): Q4_0 3584 x 18944 26.1 -> 15.0 us (25.8 -> 14.0), 3584 x 3584 11.0 -> 5.4,
 // 18944 x 3584 23.9 -> 12.9; Q8_0 3584 x 18944 27.2 -> 18.5, 18944 x 3584 26.1 -> 15.3, 9000 x 18944 51.2 -> 40.8.  Four digits, which keep 30 bits below the largest, took
 // 13.1, 4.8, 11.3, 17.6, 14.9 and 34.7, and lost what lies below: one large activation under a small weight took its block's other terms with it.  Where
-// every block is plain (activations e^(8 N(0, 1))): Q4_0 3584 x 18944 34 us, Q8_0 38, slower than above; N(0, 1) and gated inputs have a plain block in none to one of
-// twenty products.  Error against 64 bits at 3584 x 18944 Q4_0 1.4e-7 -> 0.7e-7.
+// every block is plain (activations e^(8 N(0, 1))): Q4_0 3584 x 18944 34 us, Q8_0 38, slower than above; of 18944 columns N(0, 1) inputs have a plain
+// block in one of 27 products, gated ones (silu(u) v) in every second, which takes no longer.  Error against 64 bits at 3584 x 18944 Q4_0 1.4e-7 -> 0.7e-7.
 //   A row whose sum over digits is not finite (a scale that is not, sums beyond the range) is computed again in plain fp32.
 constexpr int kMmaWarps = 16, kMmaRows = 32, kMmaSlots = 4;
 constexpr int kMmaThreads = (kMmaWarps + 1) * 32;
